@@ -584,6 +584,15 @@ __global__ void k_collect_overflow(const pb_pair_out *out, int n, int *list, int
     }
 }
 
+__global__ void k_count_overflow(const pb_pair_out *__restrict__ out, size_t n, int *__restrict__ count)
+{
+    int c = 0;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+        c += (out[i].status & PB_ST_OVERFLOW16) != 0;
+    for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, c);
+}
+
 __global__ void k_scatter(const pb_pair_out *src, const int *list, int n, pb_pair_out *dst)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -593,9 +602,9 @@ __global__ void k_scatter(const pb_pair_out *src, const int *list, int n, pb_pai
 }  // namespace
 
 /* Everything the score kernel needs for a batch that depends only on the
- * profiles and the target lengths: the length order of the targets, the
- * task list (most cells first, team tasks at the front), the concatenated
- * int8 profiles and the per-warp pass buffers. Buffers come from st's pool
+ * profiles and the target lengths: the task list (most cells first, team
+ * tasks at the front), the concatenated int8 profiles and the sizes of the
+ * per-warp pass buffers. Buffers come from st's pool
  * and are released by sw16_release. */
 struct Sw16Prep {
     pb::Sw16Params p;
@@ -604,7 +613,8 @@ struct Sw16Prep {
     int wave_rl;                  /* its rows per lane */
     size_t prof_bytes;
     int *counter;                 /* [warp tasks, team tasks, error, spare] */
-    void *bufs[10];
+    size_t scratch_bytes, colsave_bytes;
+    void *bufs[4];
 };
 
 static void sw16_release(Sw16Prep *pr, cudaStream_t st)
@@ -641,39 +651,70 @@ static void wave_set_smem(int bytes)
             pb_raise_smem((const void *)wave_kernel(ge != 0, rl), bytes);
 }
 
-static int sw16_prepare(const pb_batch *b, pb_pair_out *d_out_all, size_t prof_bytes, cudaStream_t st,
-                        Sw16Prep *pr)
+/* The length order of a batch's targets, shared by the launches of one
+ * search: targets by descending length (device), their lengths (host). */
+struct Sw16Sort {
+    int *order = nullptr;
+    std::vector<int> hlen;
+    void *bufs[4] = {nullptr, nullptr, nullptr, nullptr};
+};
+
+static void sw16_sort_release(Sw16Sort *so, cudaStream_t st)
+{
+    for (void *&x : so->bufs) { if (x) cudaFreeAsync(x, st); x = nullptr; }
+}
+
+/* synchronises st */
+static int sw16_sort(const pb_batch *b, cudaStream_t st, Sw16Sort *so)
+{
+    const int n = b->npairs;
+    int *keys_sorted = nullptr, *idx = nullptr, *order = nullptr;
+    void *tmp = nullptr;
+    size_t tmp_sort = 0;
+    cub::DeviceRadixSort::SortPairsDescending(nullptr, tmp_sort, b->d_tlen, keys_sorted, idx, order, n, 0, 32, st);
+    /* an allocation that fails ends the call before anything writes
+     * through it, releasing what was allocated */
+    if (cudaMallocAsync((void **)&keys_sorted, sizeof(int) * n, st) == cudaSuccess) so->bufs[0] = keys_sorted;
+    if (cudaMallocAsync((void **)&idx, sizeof(int) * n, st) == cudaSuccess) so->bufs[1] = idx;
+    if (cudaMallocAsync((void **)&order, sizeof(int) * n, st) == cudaSuccess) so->bufs[2] = order;
+    if (cudaMallocAsync(&tmp, tmp_sort, st) == cudaSuccess) so->bufs[3] = tmp;
+    for (void *x : so->bufs)
+        if (!x) {
+            sw16_sort_release(so, st);
+            cudaGetLastError();
+            return -1;
+        }
+    so->order = order;
+    k_iota<<<(n + 255) / 256, 256, 0, st>>>(idx, n);
+    cub::DeviceRadixSort::SortPairsDescending(tmp, tmp_sort, b->d_tlen, keys_sorted, idx, order, n, 0, 32, st);
+    so->hlen.resize(n);
+    cudaMemcpyAsync(so->hlen.data(), keys_sorted, sizeof(int) * n, cudaMemcpyDeviceToHost, st);
+    return cudaStreamSynchronize(st) == cudaSuccess ? 0 : -1;
+}
+
+/* b's profiles against its targets in the order of `so` (which outlives the
+ * launch) */
+static int sw16_prepare(const pb_batch *b, pb_pair_out *d_out_all, size_t prof_bytes, const Sw16Sort &so,
+                        cudaStream_t st, Sw16Prep *pr)
 {
     const int n = b->npairs, nq = b->nprofs;
     memset(pr, 0, sizeof *pr);
     pr->prof_bytes = prof_bytes;
-    /* targets sorted by length, descending */
-    int *keys_sorted = nullptr, *idx = nullptr, *order = nullptr, *counter = nullptr;
-    void *tmp = nullptr;
+    const std::vector<int> &hlen = so.hlen;
+    int *counter = nullptr;
     int8_t *prof_all = nullptr;
     pb::Sw16Task *d_tasks = nullptr;
     pb::Sw16Query *d_q = nullptr;
-    size_t tmp_sort = 0;
     /* an allocation that fails ends the call before anything writes
      * through it, releasing what was allocated */
     auto give_up = [&]() {
-        void *owned[10] = {keys_sorted, idx, order, counter, tmp, prof_all, d_tasks, d_q, nullptr, nullptr};
+        void *owned[4] = {counter, prof_all, d_tasks, d_q};
         memcpy(pr->bufs, owned, sizeof owned);
         sw16_release(pr, st);
         cudaGetLastError();
         return -1;
     };
-    if (cudaMallocAsync((void **)&keys_sorted, sizeof(int) * n, st) != cudaSuccess ||
-        cudaMallocAsync((void **)&idx, sizeof(int) * n, st) != cudaSuccess ||
-        cudaMallocAsync((void **)&order, sizeof(int) * n, st) != cudaSuccess ||
-        cudaMallocAsync((void **)&counter, sizeof(int) * 4, st) != cudaSuccess)
-        return give_up();
-    k_iota<<<(n + 255) / 256, 256, 0, st>>>(idx, n);
-    cub::DeviceRadixSort::SortPairsDescending(nullptr, tmp_sort, b->d_tlen, keys_sorted, idx, order, n, 0, 32, st);
-    if (cudaMallocAsync(&tmp, tmp_sort, st) != cudaSuccess) return give_up();
-    cub::DeviceRadixSort::SortPairsDescending(tmp, tmp_sort, b->d_tlen, keys_sorted, idx, order, n, 0, 32, st);
-    std::vector<int> hlen(n);
-    cudaMemcpyAsync(hlen.data(), keys_sorted, sizeof(int) * n, cudaMemcpyDeviceToHost, st);
+    if (cudaMallocAsync((void **)&counter, sizeof(int) * 4, st) != cudaSuccess) return give_up();
     cudaMemsetAsync(counter, 0, sizeof(int) * 4, st);   /* warp tasks, team tasks, error */
     /* concatenated int8 profiles */
     std::vector<pb::Sw16Query> hq(nq);
@@ -691,7 +732,6 @@ static int sw16_prepare(const pb_batch *b, pb_pair_out *d_out_all, size_t prof_b
             off += bytes;
         }
     }
-    cudaStreamSynchronize(st);
     /* tasks: (query, block of 32 sorted targets), most cells first */
     const int nblk = (n + 31) / 32;
     std::vector<pb::Sw16Task> tasks((size_t)nq * nblk);
@@ -766,16 +806,10 @@ static int sw16_prepare(const pb_batch *b, pb_pair_out *d_out_all, size_t prof_b
         const long long want = (items + pb::SW16_WARPS - 1) / pb::SW16_WARPS;
         blocks = (int)std::min<long long>(want, (long long)wper * nsm);
     }
-    uint32_t *scratch = nullptr;
-    const size_t scratch_bytes = few ? sizeof(int2) * (size_t)maxlen * blocks * pb::SW16_WARPS
-                                     : sizeof(uint32_t) * (size_t)maxlen * 32 * blocks * pb::SW16_WARPS;
-    if (cudaMallocAsync((void **)&scratch, scratch_bytes, st) != cudaSuccess)
-        scratch = nullptr;
+    pr->scratch_bytes = few ? sizeof(int2) * (size_t)maxlen * blocks * pb::SW16_WARPS
+                            : sizeof(uint32_t) * (size_t)maxlen * 32 * blocks * pb::SW16_WARPS;
     /* k_sw16: per thread, the two strips' best columns (2 x 16 words) */
-    uint4 *colsave = nullptr;
-    if (!few && cudaMallocAsync((void **)&colsave, sizeof(uint4) * (pb::SW16_R / 2) * (size_t)blocks * pb::SW16_WARPS * 32,
-                                st) != cudaSuccess)
-        colsave = nullptr;
+    pr->colsave_bytes = few ? 0 : sizeof(uint4) * (pb::SW16_R / 2) * (size_t)blocks * pb::SW16_WARPS * 32;
     /* team tasks: those above a fair share of the work per warp, which one
      * warp alone would finish last */
     int nteam = few ? (int)sorted_tasks.size() : 0;
@@ -792,18 +826,57 @@ static int sw16_prepare(const pb_batch *b, pb_pair_out *d_out_all, size_t prof_b
     p.bias = bias ? 1 : 0;
     p.ntasks = (int)sorted_tasks.size(); p.maxlen = maxlen; p.nteam = nteam;
     p.queries = d_q; p.prof_all = prof_all; p.prof_bytes = (int)prof_bytes;
-    p.order = order; p.tasks = d_tasks;
+    p.order = so.order; p.tasks = d_tasks;
     p.targets = b->d_targets; p.toff = b->d_toff; p.tlen = b->d_tlen;
-    p.scratch = scratch; p.out = d_out_all; p.colsave = colsave;
+    p.scratch = nullptr; p.colsave = nullptr;      /* sw16_workspace */
+    p.out = d_out_all;
     pr->blocks = blocks;
     pr->counter = counter;
-    void *owned[10] = {keys_sorted, idx, order, counter, tmp, prof_all, d_tasks, d_q, scratch, colsave};
+    void *owned[4] = {counter, prof_all, d_tasks, d_q};
     memcpy(pr->bufs, owned, sizeof owned);
-    if (!keys_sorted || !idx || !order || !counter || !tmp || !prof_all || !d_tasks || !d_q || !scratch ||
-        (!few && !colsave) ||
-        cudaGetLastError() != cudaSuccess) {
+    if (cudaGetLastError() != cudaSuccess) {
         sw16_release(pr, st);
         return -1;
+    }
+    return 0;
+}
+
+/* The pass buffers of launches that run one after another on one stream:
+ * one set of the largest size any of them needs. */
+struct Sw16Work {
+    uint32_t *scratch = nullptr;
+    uint4 *colsave = nullptr;
+};
+
+static void sw16_work_release(Sw16Work *w, cudaStream_t st)
+{
+    if (w->scratch) cudaFreeAsync(w->scratch, st);
+    if (w->colsave) cudaFreeAsync(w->colsave, st);
+    w->scratch = nullptr;
+    w->colsave = nullptr;
+}
+
+/* preps[first], preps[first + step], ... on st's memory */
+static int sw16_workspace(Sw16Prep *preps, size_t n, size_t first, size_t step, cudaStream_t st, Sw16Work *w)
+{
+    size_t sb = 0, cb = 0;
+    for (size_t k = first; k < n; k += step) {
+        sb = std::max(sb, preps[k].scratch_bytes);
+        cb = std::max(cb, preps[k].colsave_bytes);
+    }
+    if (sb && cudaMallocAsync((void **)&w->scratch, sb, st) != cudaSuccess) {
+        w->scratch = nullptr;
+        cudaGetLastError();
+        return -1;
+    }
+    if (cb && cudaMallocAsync((void **)&w->colsave, cb, st) != cudaSuccess) {
+        w->colsave = nullptr;
+        cudaGetLastError();
+        return -1;
+    }
+    for (size_t k = first; k < n; k += step) {
+        preps[k].p.scratch = w->scratch;
+        preps[k].p.colsave = w->colsave;
     }
     return 0;
 }
@@ -823,7 +896,33 @@ static void sw16_launch(const Sw16Prep &pr, cudaStream_t st)
     }
 }
 
-/* nq profiles against the same targets; out[q * npairs + i]. */
+/* One launch's share of the queries: as many consecutive profiles as fit
+ * `limit` bytes of shared memory (at least one). */
+static int sw16_group(const pb_batch *b, int q0, size_t limit, size_t *bytes)
+{
+    int q = q0;
+    *bytes = 0;
+    while (q < b->nprofs) {
+        const size_t one = (size_t)b->profs[q]->size * b->profs[q]->lp;
+        if (q > q0 && *bytes + one > limit) break;
+        *bytes += one;
+        ++q;
+    }
+    return q - q0;
+}
+
+/* nq profiles against the same targets; out[q * npairs + i]. Profiles past
+ * one launch's shared memory run in groups of consecutive queries, their
+ * launches on two streams in turn, so that a group's first blocks take the
+ * SMs that the last group's longest tasks leave idle. A group holds at most
+ * SW16_GROUP bytes, which keeps two blocks on an SM: 40 queries (median 270)
+ * x 10,000 targets from host memory took 508 ms on the exact kernel, one
+ * query at a time, and 37.3 ms in four groups. Up to
+ * 200 KB one launch of one block per SM stays: it holds every query of a
+ * small search, and its tasks in one queue. */
+static constexpr size_t SW16_SMEM_MAX = 200 * 1024;
+static constexpr size_t SW16_GROUP = 104 * 1024;
+
 extern "C" int pb_cuda_align_sw16_multi(const pb_batch *b, pb_pair_out *d_out_all)
 {
     if (pb_cuda_init() != 0) return -1;
@@ -833,10 +932,11 @@ extern "C" int pb_cuda_align_sw16_multi(const pb_batch *b, pb_pair_out *d_out_al
     size_t prof_bytes = 0;
     for (int q = 0; q < nq && ok; ++q) {
         const pb_device_profile *dp = b->profs[q];
-        ok = dp->fits8 && dp->size == b->profs[0]->size;
-        prof_bytes += (size_t)dp->size * dp->lp;
+        const size_t bytes = (size_t)dp->size * dp->lp;
+        ok = dp->fits8 && dp->size == b->profs[0]->size && bytes <= SW16_SMEM_MAX;
+        prof_bytes += bytes;
     }
-    if (!ok || prof_bytes > 200 * 1024) {
+    if (!ok) {
         /* outside this kernel's domain: the exact kernel, one profile at a time */
         for (int q = 0; q < nq; ++q) {
             pb_batch one = *b;
@@ -847,57 +947,92 @@ extern "C" int pb_cuda_align_sw16_multi(const pb_batch *b, pb_pair_out *d_out_al
         }
         return 0;
     }
-    cudaStream_t st = 0;
-    cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    cudaStream_t st = nullptr, st2 = nullptr;
+    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return -1;
     int rc = 0;
-    Sw16Prep prep;
-    if (sw16_prepare(b, d_out_all, prof_bytes, st, &prep) != 0) {
+    Sw16Sort sort;
+    if (sw16_sort(b, st, &sort) != 0) {
         cudaStreamSynchronize(st);
         cudaStreamDestroy(st);
         return -1;
     }
-    int *counter = prep.counter;
-    cudaEvent_t ev0, ev1;
-    cudaEventCreate(&ev0);
-    cudaEventCreate(&ev1);
-    cudaEventRecord(ev0, st);
-    sw16_launch(prep, st);
-    cudaEventRecord(ev1, st);
-    if (cudaGetLastError() != cudaSuccess) rc = -1;
-    pb_diag_count_launch(2);   /* k_iota, k_sw16 */
-    {
-        int herr = 0;
-        cudaMemcpyAsync(&herr, counter + 2, sizeof(int), cudaMemcpyDeviceToHost, st);
-        cudaStreamSynchronize(st);
-        if (herr) {
+    std::vector<Sw16Prep> preps;
+    const size_t limit = prof_bytes > SW16_SMEM_MAX ? SW16_GROUP : SW16_SMEM_MAX;
+    for (int q0 = 0; q0 < nq && rc == 0;) {
+        size_t bytes = 0;
+        const int k = sw16_group(b, q0, limit, &bytes);
+        pb_batch g = *b;
+        g.profs = b->profs + q0;
+        g.nprofs = k;
+        Sw16Prep prep;
+        if (sw16_prepare(&g, d_out_all + (size_t)q0 * n, bytes, sort, st, &prep) != 0) rc = -1;
+        else preps.push_back(prep);
+        q0 += k;
+    }
+    Sw16Work work[2];
+    if (rc == 0 && (sw16_workspace(preps.data(), preps.size(), 0, 2, st, &work[0]) != 0 ||
+                    sw16_workspace(preps.data(), preps.size(), 1, 2, st, &work[1]) != 0))
+        rc = -1;
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    if (rc == 0 && (cudaEventCreate(&ev0) != cudaSuccess || cudaEventCreate(&ev1) != cudaSuccess ||
+                    (preps.size() > 1 && cudaStreamCreateWithFlags(&st2, cudaStreamNonBlocking) != cudaSuccess)))
+        rc = -1;
+    if (rc == 0) {
+        cudaEventRecord(ev0, st);
+        if (st2) cudaStreamWaitEvent(st2, ev0, 0);
+        for (size_t k = 0; k < preps.size(); ++k) sw16_launch(preps[k], k & 1 ? st2 : st);
+        if (st2) {
+            cudaEventRecord(ev1, st2);
+            cudaStreamWaitEvent(st, ev1, 0);
+        }
+        cudaEventRecord(ev1, st);
+        if (cudaGetLastError() != cudaSuccess) rc = -1;
+        pb_diag_count_launch(1 + (int)preps.size());   /* k_iota, the score kernels */
+    }
+    /* the launches' error flags, and the pairs that left the 16-bit range */
+    std::vector<int> herr(preps.size(), 0);
+    int *over = nullptr, nover_all = 0;
+    const size_t N = (size_t)n * nq;
+    if (rc == 0 && cudaMallocAsync((void **)&over, sizeof(int), st) != cudaSuccess) rc = -1;
+    if (rc == 0) {
+        cudaMemsetAsync(over, 0, sizeof(int), st);
+        k_count_overflow<<<148, 256, 0, st>>>(d_out_all, N, over);
+        pb_diag_count_launch(1);
+        cudaMemcpyAsync(&nover_all, over, sizeof(int), cudaMemcpyDeviceToHost, st);
+        for (size_t k = 0; k < preps.size(); ++k)
+            cudaMemcpyAsync(&herr[k], preps[k].counter + 2, sizeof(int), cudaMemcpyDeviceToHost, st);
+    }
+    if (cudaStreamSynchronize(st) != cudaSuccess) rc = -1;
+    for (int e : herr)
+        if (e) {
             fprintf(stderr, "pb_cuda_align_sw16_multi: a pass wait exceeded its bound\n");
             rc = -1;
         }
-    }
-    {
+    if (rc == 0) {
         float ms = 0.f;
         cudaEventElapsedTime(&ms, ev0, ev1);
         pb_diag_sw16_time(ms);
-        cudaEventDestroy(ev0);
-        cudaEventDestroy(ev1);
     }
+    if (ev0) cudaEventDestroy(ev0);
+    if (ev1) cudaEventDestroy(ev1);
     /* pairs that left the 16-bit range: the exact kernel, per query */
     int *list = nullptr, *otlen = nullptr;
     int64_t *otoff = nullptr;
-    if (cudaMallocAsync((void **)&list, sizeof(int) * n, st) != cudaSuccess ||
-        cudaMallocAsync((void **)&otlen, sizeof(int) * n, st) != cudaSuccess ||
-        cudaMallocAsync((void **)&otoff, sizeof(int64_t) * n, st) != cudaSuccess) {
+    if (rc == 0 && nover_all > 0 &&
+        (cudaMallocAsync((void **)&list, sizeof(int) * n, st) != cudaSuccess ||
+         cudaMallocAsync((void **)&otlen, sizeof(int) * n, st) != cudaSuccess ||
+         cudaMallocAsync((void **)&otoff, sizeof(int64_t) * n, st) != cudaSuccess)) {
         cudaGetLastError();
         rc = -1;   /* nothing below runs; the buffers that exist are freed */
     }
-    for (int q = 0; q < nq && rc == 0; ++q) {
+    for (int q = 0; q < nq && rc == 0 && nover_all > 0; ++q) {
         int nover = 0;
         pb_pair_out *oq = d_out_all + (size_t)q * n;
-        cudaMemsetAsync(counter + 1, 0, sizeof(int), st);
-        k_collect_overflow<<<(n + 255) / 256, 256, 0, st>>>(oq, n, list, counter + 1, b->d_toff,
+        cudaMemsetAsync(over, 0, sizeof(int), st);
+        k_collect_overflow<<<(n + 255) / 256, 256, 0, st>>>(oq, n, list, over, b->d_toff,
                                                             b->d_tlen, otoff, otlen);
         pb_diag_count_launch(1);
-        cudaMemcpyAsync(&nover, counter + 1, sizeof(int), cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(&nover, over, sizeof(int), cudaMemcpyDeviceToHost, st);
         cudaStreamSynchronize(st);
         if (nover > 0) {
             pb_pair_out *tmpo = nullptr;
@@ -924,8 +1059,12 @@ extern "C" int pb_cuda_align_sw16_multi(const pb_batch *b, pb_pair_out *d_out_al
     if (list) cudaFreeAsync(list, st);
     if (otlen) cudaFreeAsync(otlen, st);
     if (otoff) cudaFreeAsync(otoff, st);
-    sw16_release(&prep, st);
+    if (over) cudaFreeAsync(over, st);
+    for (Sw16Prep &prep : preps) sw16_release(&prep, st);
+    for (Sw16Work &w : work) sw16_work_release(&w, st);
+    sw16_sort_release(&sort, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) rc = -1;
+    if (st2) cudaStreamDestroy(st2);
     cudaStreamDestroy(st);
     return rc;
 }
@@ -1018,20 +1157,13 @@ extern "C" int pb_cuda_align_sw16(const pb_batch *b)
 
 namespace {
 
-__global__ void k_count_overflow(const pb_pair_out *__restrict__ out, int n, int *__restrict__ count)
-{
-    int c = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        c += (out[i].status & PB_ST_OVERFLOW16) != 0;
-    for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, c);
-}
-
 struct DbPlan {
     cudaStream_t st = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    Sw16Sort sort;
     Sw16Prep prep;
+    Sw16Work work;
     bool prepared = false;
     pb_pair_out *o1 = nullptr;
     int *need = nullptr, *counts = nullptr;   /* counts[0..2] lane lists (unused), [4] overflow */
@@ -1048,6 +1180,8 @@ void plan_destroy(DbPlan *pl)
     if (pl->graph) cudaGraphDestroy(pl->graph);
     if (pl->st) {
         if (pl->prepared) sw16_release(&pl->prep, pl->st);
+        sw16_work_release(&pl->work, pl->st);
+        sw16_sort_release(&pl->sort, pl->st);
         if (pl->o1) cudaFreeAsync(pl->o1, pl->st);
         if (pl->need) cudaFreeAsync(pl->need, pl->st);
         if (pl->counts) cudaFreeAsync(pl->counts, pl->st);
@@ -1084,7 +1218,7 @@ extern "C" int pb_cuda_db_plan_create(const pb_job *job, const pb_batch *b, pb_r
         if (!dp->fits8 || dp->size != b->profs[0]->size) return -1;
         prof_bytes += (size_t)dp->size * dp->lp;
     }
-    if (prof_bytes > 200 * 1024) return -1;
+    if (prof_bytes > SW16_SMEM_MAX) return -1;
     DbPlan *pl = new DbPlan();
     pl->job = *job;
     pl->profs.assign(b->profs, b->profs + nq);
@@ -1101,15 +1235,17 @@ extern "C" int pb_cuda_db_plan_create(const pb_job *job, const pb_batch *b, pb_r
     if (rc == 0) {
         pb_batch bb = pl->b;
         bb.stats = 0; bb.pad_rows = 0; bb.d_qlim = nullptr; bb.d_tlim = nullptr;
-        rc = sw16_prepare(&bb, pl->o1, prof_bytes, pl->st, &pl->prep);
+        rc = sw16_sort(&bb, pl->st, &pl->sort);
+        if (rc == 0) rc = sw16_prepare(&bb, pl->o1, prof_bytes, pl->sort, pl->st, &pl->prep);
         pl->prepared = rc == 0;
+        if (rc == 0) rc = sw16_workspace(&pl->prep, 1, 0, 1, pl->st, &pl->work);
     }
     if (rc == 0 && cudaStreamSynchronize(pl->st) != cudaSuccess) rc = -1;
     if (rc == 0 && cudaStreamBeginCapture(pl->st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) rc = -1;
     if (rc == 0) {
         sw16_launch(pl->prep, pl->st);
         cudaMemsetAsync(pl->counts, 0, sizeof(int) * 8, pl->st);
-        k_count_overflow<<<148, 256, 0, pl->st>>>(pl->o1, (int)N, pl->counts + 4);
+        k_count_overflow<<<148, 256, 0, pl->st>>>(pl->o1, N, pl->counts + 4);
         for (int q = 0; q < nq; ++q)
             pb::launch_resolve_plain(pl->job, pl->o1 + (size_t)q * n, pl->profs[q]->qlen, b->d_tlen, n,
                                      d_rec + (size_t)q * n, pl->need, pl->counts, pl->st);
