@@ -56,7 +56,8 @@ void launch_exact_warp(const ExactParams &p, int alg, bool stats, int nitems, cu
 int exact_warp_pass_rows(bool stats);
 
 struct Sw16Query {
-    int prof_off;            /* byte offset of the query's int8 profile in shared memory */
+    const int8_t *prof8;     /* the query's int8 profile, [size][lp] */
+    int prof_off;            /* k_sw_wave: byte offset of the profile in shared memory */
     int qlen, lp, posmax;
 };
 
@@ -71,7 +72,7 @@ struct Sw16Params {
     int nletters;            /* profile alphabet size */
     int bias;                /* k_sw16<true>: H - open in the registers, scores + open */
     const Sw16Query *queries;
-    const int8_t *prof_all;  /* concatenated [size][lp] int8 profiles */
+    const int8_t *prof_all;  /* k_sw_wave: concatenated [size][lp] int8 profiles */
     int prof_bytes;
     const int *order;        /* target ids sorted by length (desc) */
     const Sw16Task *tasks;   /* most cells first */

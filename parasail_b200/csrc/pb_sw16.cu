@@ -11,8 +11,8 @@
  * halves of one DPX instruction always do useful, independent work. A pass
  * hands its bottom row (H and the vertical-gap value F, 16 bits each) to the
  * next pass through a per-warp buffer laid out [column][lane]: one
- * contiguous 128-byte transaction per warp access. The int8 query profiles
- * of all the batch's queries live in shared memory; a column's 16 + 16
+ * contiguous 128-byte transaction per warp access. Each warp stages the
+ * int8 scores of its pass's 32 rows in shared memory; a column's 16 + 16
  * scores are two 16-byte loads expanded to int16x2 words by sign-extending
  * byte permutes. The recurrence is written so that two DPX operations per
  * row sit on the column's dependency chain (F = viaddmax(H_up, -open,
@@ -49,6 +49,7 @@ namespace pb {
 
 static constexpr int SW16_R = 16;          /* query rows per strip (two strips per pass) */
 static constexpr int SW16_WARPS = 8;       /* warps per block */
+static constexpr int SW16_ROW = 48;        /* bytes between two letters' scores in a warp's slice */
 
 /* Packs two signed bytes (byte k of a and of b) into one int16x2 word:
  * low half from a, high half from b, each sign-extended (prmt sign mode). */
@@ -76,71 +77,106 @@ struct Sw16Best {
     int score, i, j;
 };
 
-__device__ __forceinline__ void fold_best(Sw16Best &best, bool &have, const Sw16Best &s)
-{
-    /* higher score, then smaller column; an equal column keeps the earlier
-     * (smaller) row, which was folded first */
-    if (s.j >= 0 && (!have || s.score > best.score || (s.score == best.score && s.j < best.j))) {
-        best = s;
-        have = true;
+/* A lane's target residues, four columns at a time. One byte load per
+ * column and lane touches 32 different lines; here the lane reads the
+ * aligned 32-bit words that hold its residues, two words ahead, and shifts
+ * them together. Only words that hold at least one byte of the sequence
+ * are read; columns past its end are letter 0. */
+struct ResidueWords {
+    const uint32_t *w;
+    int shift, last, len;
+    uint32_t a, b, c;        /* words k, k + 1, k + 2 of the next four columns */
+    __device__ __forceinline__ uint32_t word(int k) const { return k <= last ? __ldg(w + k) : 0u; }
+    __device__ __forceinline__ void start(const uint8_t *seq, int n)
+    {
+        const uintptr_t p = reinterpret_cast<uintptr_t>(seq);
+        w = reinterpret_cast<const uint32_t *>(p & ~(uintptr_t)3);
+        shift = (int)(p & 3) * 8;
+        len = n;
+        last = n > 0 ? ((int)(p & 3) + n - 1) >> 2 : -1;
+        a = word(0);
+        b = word(1);
+        c = word(2);
     }
+    /* the residues of columns j .. j + 3 (j a multiple of 4), one per byte */
+    __device__ __forceinline__ uint32_t next(int j)
+    {
+        uint32_t v = __funnelshift_r(a, b, shift);
+        const int left = len - j;
+        if (left < 4) v = left <= 0 ? 0u : v & (0xffffffffu >> (32 - 8 * left));
+        a = b;
+        b = c;
+        c = word((j >> 2) + 3);
+        return v;
+    }
+};
+
+/* higher score, then smaller column; an equal column keeps the earlier
+ * (smaller) row, which was folded first (scores are positive, a best of 0
+ * is none) */
+__device__ __forceinline__ void fold_best(Sw16Best &best, const Sw16Best &s)
+{
+    if (s.j >= 0 && (s.score > best.score || (s.score == best.score && s.j < best.j))) best = s;
 }
 
+/*
+ * What bounds it: the ALU pipe, which takes the DPX operations and byte
+ * permutes at half rate (64 lanes per SM and cycle): 5.5 per row of two
+ * cells (byte permute, E, A, F, H and half a three-way maximum; the add of
+ * -open issues on the FMA pipe beside them). So the column loop carries
+ * little else: four columns per iteration without a branch for each (the
+ * columns past the longest target, three at most, meet letter 0 and count
+ * for nothing), targets read by words, pass boundaries at pointers that
+ * advance by constants with the first pass reading none.
+ * The pass's 32 rows of scores are staged per warp as [letter][48 bytes]:
+ * 16-byte loads at an odd multiple of 16 bytes fall on all eight bank
+ * groups (at the profiles' own stride, a multiple of 64, the kernel took
+ * 1.07 to 1.17 times as long), and the launch holds any number of queries of
+ * any length, where whole profiles in shared memory ended at 200 KB.
+ * 5 queries (100-2000) x 200,000 targets (2.7e11 cells): 102.0 -> 55.6 ms,
+ * 4,900 GCUPS, ALU pipe 84% busy; 40 queries (median 270) x 10,000 targets:
+ * 28 ms in four launches of whole profiles -> 12.1 ms in one.
+ */
 template <bool BIAS>
 __global__ void __launch_bounds__(SW16_WARPS * 32, 2)
 k_sw16(Sw16Params p, int *task_counter)
 {
-    extern __shared__ __align__(16) int8_t s_prof[];
-    {
-        const int4 *src = reinterpret_cast<const int4 *>(p.prof_all);
-        int4 *dst = reinterpret_cast<int4 *>(s_prof);
-        const int n16 = p.prof_bytes / 16;
-        /* BIAS: every score + open (the host checked that it stays in int8) */
-        const uint32_t b4 = BIAS ? 0x01010101u * (uint32_t)(uint8_t)p.open : 0u;
-        for (int k = threadIdx.x; k < n16; k += blockDim.x) {
-            int4 v = src[k];
-            if (BIAS) {
-                v.x = (int)__vadd4((uint32_t)v.x, b4); v.y = (int)__vadd4((uint32_t)v.y, b4);
-                v.z = (int)__vadd4((uint32_t)v.z, b4); v.w = (int)__vadd4((uint32_t)v.w, b4);
-            }
-            dst[k] = v;
-        }
-    }
-    __syncthreads();
-
+    extern __shared__ __align__(16) int8_t s_slices[];
     const int lane = threadIdx.x & 31;
     const int wid = threadIdx.x >> 5;
+    int8_t *slice = s_slices + (size_t)wid * p.nletters * SW16_ROW;
     /* the block's SW16_WARPS buffers: warp w's is team_buf + w * maxlen * 32;
-     * an entry is strip B's bottom row at one column, H in the low and F in
+     * entry c + 1 is strip B's bottom row at column c, H in the low and F in
      * the high 16 bits */
-    uint32_t *team_buf = p.scratch + (size_t)blockIdx.x * SW16_WARPS * p.maxlen * 32;
+    uint32_t *team_buf = p.scratch + (size_t)blockIdx.x * SW16_WARPS * p.maxlen * 32 + lane;
     const uint32_t gapO = splat16(-p.open);
     const uint32_t gapE = splat16(-p.gap);
     /* BIAS: the H registers, the pass buffer, the column maxima and the
      * best-so-far hold H - open, so "H = 0" reads as -open */
     const uint32_t zeroH = BIAS ? gapO : 0u;
     const int bias = BIAS ? p.open : 0;
-    /* team tasks: the tasks at the front of the list (the most expensive,
-     * each more than a fair share of the work per warp) are run by all
-     * warps of a block together, pass k of the task on warp k % SW16_WARPS;
-     * a pass reads the previous one's bottom row from that warp's buffer,
-     * published every 32 columns through s_prog (generation-tagged, so that
-     * it only grows) */
+    const uint32_t b4 = BIAS ? 0x01010101u * (uint32_t)(uint8_t)p.open : 0u;
+    /* team tasks: the tasks at the front of the list (those that one warp
+     * alone would finish last) are run by all warps of a block together,
+     * pass k of the task on warp k % SW16_WARPS; a pass reads the previous
+     * one's bottom row from that warp's buffer, published every 8 columns
+     * through s_prog (generation-tagged, so that it only grows). A pass then
+     * runs 11 to 18 columns behind its predecessor; at 32 columns the lag of
+     * 64 left the eight warps waiting on targets of less than 512 residues. */
     __shared__ volatile long long s_prog[SW16_WARPS];
     __shared__ int s_task;
     __shared__ Sw16Best s_best[SW16_WARPS][32];
-    __shared__ int s_have[SW16_WARPS][32];
-    __shared__ int s_status[SW16_WARPS][32];
     volatile int *verr = task_counter + 2;
     /* this thread's copies of its strips' best columns: A's 16 words, then B's */
     uint4 *save = p.colsave + ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * (SW16_R / 2);
     bool team = p.nteam > 0;
 
-    /* warp tasks: the first of each warp block-strided, so that the largest
-     * ones (the list is sorted by cost) are spread one per block instead of
-     * landing on the first blocks' SMs; then from the shared counter */
-    const int nwarps_total = gridDim.x * SW16_WARPS;
-    bool first = true;
+    /* warp tasks: without team tasks the first of each warp block-strided,
+     * so that the largest ones (the list is sorted by cost) are spread one
+     * per block instead of landing on the first blocks' SMs; then from the
+     * shared counter */
+    const int nstatic = p.nteam > 0 ? 0 : gridDim.x * SW16_WARPS;
+    bool first = nstatic > 0;
     for (;;) {
         int task = 0, trank = 0, tsize = 1;
         if (team) {
@@ -154,10 +190,10 @@ k_sw16(Sw16Params p, int *task_counter)
             tsize = SW16_WARPS;
         } else {
             if (first) {
-                task = p.nteam + blockIdx.x + gridDim.x * wid;
+                task = blockIdx.x + gridDim.x * wid;
                 first = false;
             } else {
-                if (lane == 0) task = p.nteam + nwarps_total + atomicAdd(task_counter, 1);
+                if (lane == 0) task = p.nteam + nstatic + atomicAdd(task_counter, 1);
                 task = __shfl_sync(0xffffffffu, task, 0);
             }
             if (task >= p.ntasks) break;
@@ -174,16 +210,25 @@ k_sw16(Sw16Params p, int *task_counter)
         int wmax = len;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) wmax = max(wmax, __shfl_xor_sync(0xffffffffu, wmax, o));
-        const int8_t *prof = s_prof + Q.prof_off;
-        const int lp = Q.lp, ql = Q.qlen;
+        const int ql = Q.qlen;
 
         Sw16Best best = {0, 0, 0};
-        bool have = false;
-        int status = 0;
 
         const long long stride = (long long)wmax + 1;
         for (int r0 = 2 * SW16_R * trank; r0 < ql; r0 += 2 * SW16_R * tsize) {
             const int sp = r0 / (2 * SW16_R);            /* pass index */
+            /* the pass's scores of every letter (BIAS: + open; the host
+             * checked that it stays in int8) */
+            __syncwarp();
+            for (int x = lane; x < 2 * p.nletters; x += 32) {
+                int4 v = __ldg(reinterpret_cast<const int4 *>(Q.prof8 + (size_t)(x >> 1) * Q.lp + r0) + (x & 1));
+                if (BIAS) {
+                    v.x = (int)__vadd4((uint32_t)v.x, b4); v.y = (int)__vadd4((uint32_t)v.y, b4);
+                    v.z = (int)__vadd4((uint32_t)v.z, b4); v.w = (int)__vadd4((uint32_t)v.w, b4);
+                }
+                *reinterpret_cast<int4 *>(slice + (x >> 1) * SW16_ROW + (x & 1) * 16) = v;
+            }
+            __syncwarp();
             /* team: the previous pass (warp trank-1) must have published
              * column c before it is read */
             const long long in_base = (long long)((sp - 1) / tsize) * stride + 1;
@@ -204,151 +249,156 @@ k_sw16(Sw16Params p, int *task_counter)
                 __syncwarp();
                 return ok;
             };
-            if (!wait_for(33)) break;
+            /* columns [c0, c0 + 8) read the boundary up to column c0 + 11 */
+            if (!wait_for(11)) break;
             uint32_t H[SW16_R], E[SW16_R];
 #pragma unroll
             for (int r = 0; r < SW16_R; ++r) { H[r] = zeroH; E[r] = gapO; }
             uint32_t dg = zeroH;            /* lo: H(r0-1, j-1); hi: H(r0+15, j-2) */
             uint32_t prev_h = zeroH, prev_f = gapO;   /* lo halves: strip A bottom at j-1 */
             Sw16Best sa = {0, -1, -1}, sb = {0, -1, -1};
-            uint32_t sbest = zeroH;
-            int cb = 0;                     /* residue of column j-1 (strip B) */
-            const int8_t *pa_base = prof + r0;
-            const int8_t *pb_base = prof + r0 + SW16_R;
+            /* what a column maximum has to pass (each half's own): the half's
+             * best of this pass, and one less than the best of the other half
+             * and of the passes before, whose equal in an earlier column
+             * would win */
+            uint32_t sbest = splat16(max(best.score - 1, 0) - bias);
             const bool more = r0 + 2 * SW16_R < ql;
-            /* the residue and the previous pass's boundary of a column are
-             * loaded two and three columns ahead: both come from L2 or DRAM,
-             * and the chain of one column is too short to cover that latency
-             * (this pass overwrites buf[j-1] at column j, never buf[j+3]) */
+            const int8_t *pb_at = slice + SW16_R;     /* strip B's scores of column j-1 */
+            /* the pass boundary of a column is loaded four columns ahead: it
+             * comes from L2 or DRAM, and the chain of one column is too short
+             * to cover that latency (this pass overwrites entry j at column
+             * j, never entry j+5). The first pass reads none: row -1 is H = 0,
+             * F = -inf. */
             const uint32_t vnone = prmt(zeroH, gapO, 0x5410u);
-            int c_n1 = 0 < len ? tseq[0] : 0;
-            int c_n2 = 1 < len ? tseq[1] : 0;
-            uint32_t v_n1 = vnone, v_n2 = vnone, v_n3 = vnone;
-            if (r0 != 0) {
-                if (0 < wmax) v_n1 = __ldcg(&in_buf[lane]);
-                if (1 < wmax) v_n2 = __ldcg(&in_buf[32 + lane]);
-                if (2 < wmax) v_n3 = __ldcg(&in_buf[64 + lane]);
-            }
-            bool aborted = false;
-            /* unrolled by two: the prefetch registers then rotate by renaming
-             * instead of by moves, which would wait for the loads */
-#pragma unroll 2
-            for (int j = 0; j <= wmax; ++j) {
-                if (team && j > 0 && (j & 31) == 0 && !wait_for(j + 33)) { aborted = true; break; }
-                const int ca = c_n1;
-                c_n1 = c_n2;
-                c_n2 = j + 2 < len ? tseq[j + 2] : 0;
-                uint32_t hu, fu;
-                if (r0 == 0) {
-                    hu = prmt(zeroH, prev_h, 0x5410u);      /* top row H = 0 */
-                    fu = prmt(gapO, prev_f, 0x5410u);       /* top row F = -inf */
-                } else {
-                    const uint32_t v = v_n1;
-                    v_n1 = v_n2;
-                    v_n2 = v_n3;
-                    v_n3 = j + 3 < wmax ? __ldcg(&in_buf[(size_t)(j + 3) * 32 + lane]) : vnone;
-                    hu = prmt(v, prev_h, 0x5410u);          /* lo <- previous pass's strip B bottom */
-                    fu = prmt(v, prev_f, 0x5432u);
-                }
-                const uint4 pa4 = *reinterpret_cast<const uint4 *>(pa_base + (size_t)ca * lp);
-                const uint4 pb4 = *reinterpret_cast<const uint4 *>(pb_base + (size_t)cb * lp);
-                uint32_t hd = dg;
-                dg = hu;
-                uint32_t cmax = zeroH;
-                uint32_t aop = 0u;          /* BIAS: the previous row's max(H_diag + s, E, 0) - open */
+            const int rd = r0 != 0 ? wmax : 0;
+            uint32_t v_n[4];
 #pragma unroll
-                for (int r = 0; r < SW16_R; ++r) {
-                    const uint32_t wa = r < 4 ? pa4.x : r < 8 ? pa4.y : r < 12 ? pa4.z : pa4.w;
-                    const uint32_t wb = r < 4 ? pb4.x : r < 8 ? pb4.y : r < 12 ? pb4.z : pb4.w;
-                    uint32_t sc;
-                    switch (r & 3) {
-                        case 0: sc = pack_pair<0>(wa, wb); break;
-                        case 1: sc = pack_pair<1>(wa, wb); break;
-                        case 2: sc = pack_pair<2>(wa, wb); break;
-                        default: sc = pack_pair<3>(wa, wb); break;
-                    }
-                    if (BIAS) {
-                        /* registers hold HO = H - open and the profile s + open:
-                         *   E(i,j) = max(E(i,j-1) - gap, HO(i,j-1))
-                         *   a      = max(HO(i-1,j-1) + (s + open), E, 0)
-                         *   F(i,j) = max(F(i-1,j) - gap, HO(i-1,j))
-                         *          = max(F(i-1,j) - gap, a(i-1) - open)  (open >= gap)
-                         *   HO     = max(a - open, F - open)
-                         * so one DPX operation per row sits on the chain */
-                        const uint32_t e = __viaddmax_s16x2(E[r], gapE, H[r]);
-                        const uint32_t a = __viaddmax_s16x2_relu(hd, sc, e);
-                        const uint32_t ao = __vadd2(a, gapO);
-                        const uint32_t f = __viaddmax_s16x2(fu, gapE, r == 0 ? hu : aop);
-                        const uint32_t ho = __viaddmax_s16x2(f, gapO, ao);
-                        E[r] = e;
-                        hd = H[r];
-                        H[r] = ho;
-                        hu = ho;
-                        fu = f;
-                        aop = ao;
-                        if (r & 1) cmax = __vimax3_s16x2(cmax, H[r - 1], ho);
-                    } else {
-                        /* E(i,j) = max(E(i,j-1) - gap, H(i,j-1) - open): off the chain */
-                        const uint32_t e = __viaddmax_s16x2(E[r], gapE, __vadd2(H[r], gapO));
-                        const uint32_t a = __viaddmax_s16x2_relu(hd, sc, e);
-                        /* F(i,j) = max(H(i-1,j) - open, F(i-1,j) - gap): on the chain */
-                        const uint32_t f = __viaddmax_s16x2(hu, gapO, __vadd2(fu, gapE));
-                        const uint32_t h = __vmaxs2(a, f);
-                        E[r] = e;
-                        hd = H[r];
-                        H[r] = h;
-                        hu = h;
-                        fu = f;
-                        if (r & 1) cmax = __vimax3_s16x2(cmax, H[r - 1], h);
-                    }
-                }
-                if (j >= 1 && more) {
-                    out_buf[(size_t)(j - 1) * 32 + lane] = prmt(hu, fu, 0x7632u);
-                    /* team: publish every 32 columns and the last one */
-                    if (team && (((j - 1) & 31) == 31 || j - 1 == wmax - 1)) {
-                        __threadfence_block();
-                        __syncwarp();
-                        if (lane == 0) s_prog[trank] = out_base + (j - 1);
-                    }
-                }
-                prev_h = hu;
-                prev_f = fu;
-                cb = ca;
-                if (j == 0) {
-                    /* the high half computed column -1: restore strip B's
-                     * left boundary (H = 0, E = -inf) */
+            for (int k = 0; k < 4; ++k) v_n[k] = k < rd ? __ldcg(in_buf + (k + 1) * 32) : vnone;
+            const uint32_t *in_at = in_buf + 5 * 32;
+            uint32_t *out_at = out_buf;
+            ResidueWords tw;
+            tw.start(tseq, len);
+            bool aborted = false;
+            for (int j0 = 0; j0 <= wmax; j0 += 4, in_at += 4 * 32, out_at += 4 * 32) {
+                if (team && j0 > 0 && (j0 & 7) == 0 && !wait_for(j0 + 11)) { aborted = true; break; }
+                const uint32_t codes = tw.next(j0);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int j = j0 + u;
+                    const uint32_t v = v_n[u];
+                    v_n[u] = j + 4 < rd ? __ldcg(in_at + u * 32) : vnone;
+                    uint32_t hu = prmt(v, prev_h, 0x5410u);     /* lo <- previous pass's strip B bottom */
+                    uint32_t fu = prmt(v, prev_f, 0x5432u);
+                    const int8_t *pa_at = slice + ((codes >> (8 * u)) & 0xffu) * SW16_ROW;
+                    const uint4 pa4 = *reinterpret_cast<const uint4 *>(pa_at);
+                    const uint4 pb4 = *reinterpret_cast<const uint4 *>(pb_at);
+                    pb_at = pa_at + SW16_R;
+                    uint32_t hd = dg;
+                    dg = hu;
+                    uint32_t cmax = zeroH;
+                    uint32_t aop = 0u;          /* BIAS: the previous row's max(H_diag + s, E, 0) - open */
 #pragma unroll
                     for (int r = 0; r < SW16_R; ++r) {
-                        H[r] = (H[r] & 0xffffu) | (zeroH & 0xffff0000u);
-                        E[r] = (E[r] & 0xffffu) | (gapO & 0xffff0000u);
+                        const uint32_t wa = r < 4 ? pa4.x : r < 8 ? pa4.y : r < 12 ? pa4.z : pa4.w;
+                        const uint32_t wb = r < 4 ? pb4.x : r < 8 ? pb4.y : r < 12 ? pb4.z : pb4.w;
+                        uint32_t sc;
+                        switch (r & 3) {
+                            case 0: sc = pack_pair<0>(wa, wb); break;
+                            case 1: sc = pack_pair<1>(wa, wb); break;
+                            case 2: sc = pack_pair<2>(wa, wb); break;
+                            default: sc = pack_pair<3>(wa, wb); break;
+                        }
+                        if (BIAS) {
+                            /* registers hold HO = H - open and the profile s + open:
+                             *   E(i,j) = max(E(i,j-1) - gap, HO(i,j-1))
+                             *   a      = max(HO(i-1,j-1) + (s + open), E, 0)
+                             *   F(i,j) = max(F(i-1,j) - gap, HO(i-1,j))
+                             *          = max(F(i-1,j) - gap, a(i-1) - open)  (open >= gap)
+                             *   HO     = max(a - open, F - open)
+                             * so one DPX operation per row sits on the chain */
+                            const uint32_t e = __viaddmax_s16x2(E[r], gapE, H[r]);
+                            const uint32_t a = __viaddmax_s16x2_relu(hd, sc, e);
+                            const uint32_t ao = __vadd2(a, gapO);
+                            const uint32_t f = __viaddmax_s16x2(fu, gapE, r == 0 ? hu : aop);
+                            const uint32_t ho = __viaddmax_s16x2(f, gapO, ao);
+                            E[r] = e;
+                            hd = H[r];
+                            H[r] = ho;
+                            hu = ho;
+                            fu = f;
+                            aop = ao;
+                            if (r & 1) cmax = __vimax3_s16x2(cmax, H[r - 1], ho);
+                        } else {
+                            /* E(i,j) = max(E(i,j-1) - gap, H(i,j-1) - open): off the chain */
+                            const uint32_t e = __viaddmax_s16x2(E[r], gapE, __vadd2(H[r], gapO));
+                            const uint32_t a = __viaddmax_s16x2_relu(hd, sc, e);
+                            /* F(i,j) = max(H(i-1,j) - open, F(i-1,j) - gap): on the chain */
+                            const uint32_t f = __viaddmax_s16x2(hu, gapO, __vadd2(fu, gapE));
+                            const uint32_t h = __vmaxs2(a, f);
+                            E[r] = e;
+                            hd = H[r];
+                            H[r] = h;
+                            hu = h;
+                            fu = f;
+                            if (r & 1) cmax = __vimax3_s16x2(cmax, H[r - 1], h);
+                        }
+                    }
+                    if (more) out_at[u * 32] = prmt(hu, fu, 0x7632u);     /* column j - 1 */
+                    prev_h = hu;
+                    prev_f = fu;
+                    if (u == 0 && j0 == 0) {
+                        /* the high half computed column -1: restore strip B's
+                         * left boundary (H = 0, E = -inf) */
+#pragma unroll
+                        for (int r = 0; r < SW16_R; ++r) {
+                            H[r] = (H[r] & 0xffffu) | (zeroH & 0xffff0000u);
+                            E[r] = (E[r] & 0xffffu) | (gapO & 0xffff0000u);
+                        }
+                    }
+                    bool ge_lo, ge_hi;
+                    (void)__vibmax_s16x2(sbest, cmax, &ge_hi, &ge_lo);
+                    if (!ge_lo || !ge_hi) {
+                        /* past its half's bound: keep the column (the warp
+                         * takes this branch whenever any lane does, so the row
+                         * is looked up once per pass, from the saved column).
+                         * Columns outside the target only raise the bound, and
+                         * the high half's column -1 counts for nothing. */
+                        int ba = s16lo(sbest), bb = s16hi(sbest);
+                        if (!ge_lo) {
+                            ba = s16lo(cmax);
+                            if (j < len) {
+#pragma unroll
+                                for (int k = 0; k < SW16_R / 4; ++k)
+                                    save[k] = make_uint4(H[4 * k], H[4 * k + 1], H[4 * k + 2], H[4 * k + 3]);
+                                sa.score = ba + bias; sa.j = j;
+                                bb = max(bb, ba - 1);
+                            }
+                        }
+                        if (!ge_hi && j >= 1) {
+                            const int c = s16hi(cmax);
+                            bb = max(bb, c);
+                            if (j <= len) {
+#pragma unroll
+                                for (int k = 0; k < SW16_R / 4; ++k)
+                                    save[SW16_R / 4 + k] = make_uint4(H[4 * k], H[4 * k + 1], H[4 * k + 2], H[4 * k + 3]);
+                                sb.score = c + bias; sb.j = j - 1;
+                                ba = max(ba, c - 1);
+                            }
+                        }
+                        sbest = (uint32_t)(uint16_t)ba | ((uint32_t)(uint16_t)bb << 16);
                     }
                 }
-                bool ge_lo, ge_hi;
-                (void)__vibmax_s16x2(sbest, cmax, &ge_hi, &ge_lo);
-                const bool up_a = !ge_lo && j < len;
-                const bool up_b = !ge_hi && j >= 1 && j <= len;
-                if (up_a || up_b) {
-                    /* a new strip maximum: keep the column (the warp takes
-                     * this branch whenever any lane improves, so the row is
-                     * looked up once per pass, from the saved column) */
-                    if (up_a) {
-                        const int c = s16lo(cmax);
-#pragma unroll
-                        for (int k = 0; k < SW16_R / 4; ++k)
-                            save[k] = make_uint4(H[4 * k], H[4 * k + 1], H[4 * k + 2], H[4 * k + 3]);
-                        sa.score = c + bias; sa.j = j;
-                        if (c + bias >= Q.posmax) status |= PB_ST_OVERFLOW16;
-                    }
-                    if (up_b) {
-                        const int c = s16hi(cmax);
-#pragma unroll
-                        for (int k = 0; k < SW16_R / 4; ++k)
-                            save[SW16_R / 4 + k] = make_uint4(H[4 * k], H[4 * k + 1], H[4 * k + 2], H[4 * k + 3]);
-                        sb.score = c + bias; sb.j = j - 1;
-                        if (c + bias >= Q.posmax) status |= PB_ST_OVERFLOW16;
-                    }
-                    sbest = (uint32_t)(uint16_t)(sa.score - bias) | ((uint32_t)(uint16_t)(sb.score - bias) << 16);
+                /* team: columns up to j0 + 2 are out */
+                if (team && more && (j0 & 4)) {
+                    __threadfence_block();
+                    __syncwarp();
+                    if (lane == 0) s_prog[trank] = out_base + min(j0 + 2, wmax - 1);
                 }
+            }
+            if (team && more && !aborted) {
+                __threadfence_block();
+                __syncwarp();
+                if (lane == 0) s_prog[trank] = out_base + wmax - 1;
             }
             if (aborted) break;
             /* the first row of each strip's best column reaching its maximum */
@@ -374,38 +424,30 @@ k_sw16(Sw16Params p, int *task_counter)
                 }
                 sb.i = r0 + SW16_R + rr;
             }
-            fold_best(best, have, sa);
-            fold_best(best, have, sb);
+            fold_best(best, sa);
+            fold_best(best, sb);
         }
         if (team) {
             /* merge the warps' per-lane bests: highest score, then smallest
              * column, then smallest row (the reference's first maximum) */
             s_best[wid][lane] = best;
-            s_have[wid][lane] = have ? 1 : 0;
-            s_status[wid][lane] = status;
             __syncthreads();
             if (wid != 0) continue;
-            have = false;
-            status = 0;
-            for (int w = 0; w < SW16_WARPS; ++w) {
-                status |= s_status[w][lane];
-                if (!s_have[w][lane]) continue;
+            for (int w = 1; w < SW16_WARPS; ++w) {
                 const Sw16Best c = s_best[w][lane];
-                if (!have || c.score > best.score || (c.score == best.score && (c.j < best.j ||
-                                                        (c.j == best.j && c.i < best.i)))) {
+                if (c.score > best.score || (c.score == best.score && (c.j < best.j ||
+                                                                        (c.j == best.j && c.i < best.i))))
                     best = c;
-                    have = true;
-                }
             }
         }
         /* no positive cell: score 0 at (0, 0), the first cell (src/sw.c:150-158) */
         if (valid) {
             pb_pair_out o = {};
-            o.score = have ? best.score : 0;
-            o.end_query = have ? best.i : 0;
-            o.end_ref = have ? best.j : 0;
+            o.score = best.score;
+            o.end_query = best.i;
+            o.end_ref = best.j;
             o.max_h = o.score;
-            o.status = status;
+            o.status = best.score >= Q.posmax ? PB_ST_OVERFLOW16 : 0;
             p.out[(size_t)T.q * p.npairs + pid] = o;
         }
     }
@@ -601,6 +643,10 @@ __global__ void k_scatter(const pb_pair_out *src, const int *list, int n, pb_pai
 
 }  // namespace
 
+/* the largest profiles k_sw_wave takes into shared memory; also the limit
+ * of a plan */
+static constexpr size_t SW16_WAVE_SMEM = 200 * 1024;
+
 /* Everything the score kernel needs for a batch that depends only on the
  * profiles and the target lengths: the task list (most cells first, team
  * tasks at the front), the concatenated int8 profiles and the sizes of the
@@ -611,7 +657,7 @@ struct Sw16Prep {
     int blocks;
     bool wave;                    /* few tasks: the intra-task wavefront k_sw_wave */
     int wave_rl;                  /* its rows per lane */
-    size_t prof_bytes;
+    size_t smem;                  /* dynamic shared memory of its kernel */
     int *counter;                 /* [warp tasks, team tasks, error, spare] */
     size_t scratch_bytes, colsave_bytes;
     void *bufs[4];
@@ -694,12 +740,10 @@ static int sw16_sort(const pb_batch *b, cudaStream_t st, Sw16Sort *so)
 
 /* b's profiles against its targets in the order of `so` (which outlives the
  * launch) */
-static int sw16_prepare(const pb_batch *b, pb_pair_out *d_out_all, size_t prof_bytes, const Sw16Sort &so,
-                        cudaStream_t st, Sw16Prep *pr)
+static int sw16_prepare(const pb_batch *b, pb_pair_out *d_out_all, const Sw16Sort &so, cudaStream_t st, Sw16Prep *pr)
 {
     const int n = b->npairs, nq = b->nprofs;
     memset(pr, 0, sizeof *pr);
-    pr->prof_bytes = prof_bytes;
     const std::vector<int> &hlen = so.hlen;
     int *counter = nullptr;
     int8_t *prof_all = nullptr;
@@ -714,76 +758,114 @@ static int sw16_prepare(const pb_batch *b, pb_pair_out *d_out_all, size_t prof_b
         cudaGetLastError();
         return -1;
     };
-    if (cudaMallocAsync((void **)&counter, sizeof(int) * 4, st) != cudaSuccess) return give_up();
-    cudaMemsetAsync(counter, 0, sizeof(int) * 4, st);   /* warp tasks, team tasks, error */
-    /* concatenated int8 profiles */
+    int nsm = 0, dev = 0, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    /* the biased kernel (one DPX operation per row on the dependency
+     * chain) needs open >= gap and every score + open inside int8 */
+    bool bias = b->open >= b->gap;
+    size_t prof_bytes = 0;
+    for (int q = 0; q < nq; ++q) {
+        if (b->profs[q]->mmax + b->open > 127 || b->profs[q]->mmin + b->open < -128) bias = false;
+        prof_bytes += (size_t)b->profs[q]->size * b->profs[q]->lp;
+    }
+    pr->smem = (size_t)pb::SW16_WARPS * b->profs[0]->size * pb::SW16_ROW;
+    const void *kern = bias ? (const void *)pb::k_sw16<true> : (const void *)pb::k_sw16<false>;
+    pb_raise_smem(kern, (int)pr->smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, pb::SW16_WARPS * 32, pr->smem);
+    if (per_sm < 1) per_sm = 1;
+    int blocks = per_sm * nsm;
+    const int nblk = (n + 31) / 32;
+    const size_t ntasks = (size_t)nq * nblk;
+    /* few tasks (a small database, e.g. one query against 1,000 targets)
+     * whose profiles fit its shared memory: the intra-task wavefront, a warp
+     * per pair, as many warps as pairs (up to the resident warps) */
+    const bool few = ntasks <= (size_t)blocks && prof_bytes <= SW16_WAVE_SMEM;
+    if ((size_t)blocks > ntasks) blocks = (int)ntasks;
+    pr->wave = few;
+    /* the queries; for the wavefront their profiles side by side */
     std::vector<pb::Sw16Query> hq(nq);
-    if (cudaMallocAsync((void **)&prof_all, prof_bytes, st) != cudaSuccess) return give_up();
+    if (few && cudaMallocAsync((void **)&prof_all, prof_bytes, st) != cudaSuccess) return give_up();
     {
         size_t off = 0;
         for (int q = 0; q < nq; ++q) {
             const pb_device_profile *dp = b->profs[q];
             const size_t bytes = (size_t)dp->size * dp->lp;
-            cudaMemcpyAsync(prof_all + off, dp->d_prof8, bytes, cudaMemcpyDeviceToDevice, st);
-            hq[q].prof_off = (int)off;
+            if (few) cudaMemcpyAsync(prof_all + off, dp->d_prof8, bytes, cudaMemcpyDeviceToDevice, st);
+            hq[q].prof8 = dp->d_prof8;
+            hq[q].prof_off = few ? (int)off : 0;
             hq[q].qlen = dp->qlen;
             hq[q].lp = dp->lp;
             hq[q].posmax = 32767 - dp->mmax - 1;
             off += bytes;
         }
     }
-    /* tasks: (query, block of 32 sorted targets), most cells first */
-    const int nblk = (n + 31) / 32;
-    std::vector<pb::Sw16Task> tasks((size_t)nq * nblk);
-    std::vector<int64_t> cost((size_t)nq * nblk);
-    for (int q = 0; q < nq; ++q)
-        for (int k = 0; k < nblk; ++k) {
-            tasks[(size_t)q * nblk + k].q = q;
-            tasks[(size_t)q * nblk + k].first = 32 * k;
+    /* tasks: (query, block of 32 sorted targets), most columns (passes x
+     * target length) first: every query's are in that order already, so the
+     * queries' lists are merged */
+    std::vector<pb::Sw16Task> tasks;
+    std::vector<int64_t> cost;
+    tasks.reserve(ntasks);
+    cost.reserve(ntasks);
+    {
+        typedef std::pair<int64_t, int> Head;                 /* cost, query */
+        std::vector<Head> heap;
+        std::vector<int> at(nq, 0);
+        auto cost_of = [&](int q, int k) {
+            return (int64_t)((hq[q].qlen + 2 * pb::SW16_R - 1) / (2 * pb::SW16_R)) * (hlen[32 * (size_t)k] + 1);
+        };
+        for (int q = 0; q < nq; ++q) heap.push_back(Head(cost_of(q, 0), q));
+        std::make_heap(heap.begin(), heap.end());
+        while (!heap.empty()) {
+            std::pop_heap(heap.begin(), heap.end());
+            const Head h = heap.back();
+            heap.pop_back();
+            pb::Sw16Task t;
+            t.q = h.second;
+            t.first = 32 * at[h.second]++;
+            tasks.push_back(t);
+            cost.push_back(h.first);
+            if (at[h.second] < nblk) {
+                heap.push_back(Head(cost_of(h.second, at[h.second]), h.second));
+                std::push_heap(heap.begin(), heap.end());
+            }
         }
-    std::vector<int> perm(tasks.size());
-    for (size_t k = 0; k < perm.size(); ++k) perm[k] = (int)k;
-    std::sort(perm.begin(), perm.end(), [&](int x, int y) {
-        const int64_t cx = (int64_t)hq[tasks[x].q].qlen * hlen[tasks[x].first];
-        const int64_t cy = (int64_t)hq[tasks[y].q].qlen * hlen[tasks[y].first];
-        return cx > cy;
-    });
-    std::vector<pb::Sw16Task> sorted_tasks(tasks.size());
-    for (size_t k = 0; k < perm.size(); ++k) sorted_tasks[k] = tasks[perm[k]];
-    if (cudaMallocAsync((void **)&d_tasks, sizeof(pb::Sw16Task) * sorted_tasks.size(), st) != cudaSuccess ||
+    }
+    /* Team tasks, listed first: those that would hold up the end of the
+     * launch on one warp. The warp tasks that follow end at most one task
+     * after their fair share of the remaining work; a task above half of
+     * that share therefore goes to a team (above the whole share where its
+     * passes, fewer than a multiple of the team, would leave warps idle). */
+    int nteam = 0;
+    if (!few) {
+        double rest = 0.0;
+        for (int64_t c : cost) rest += (double)c;
+        const double warps = (double)blocks * pb::SW16_WARPS;
+        std::vector<pb::Sw16Task> lone;
+        lone.reserve(ntasks);
+        for (size_t k = 0; k < ntasks; ++k) {
+            const int np = (hq[tasks[k].q].qlen + 2 * pb::SW16_R - 1) / (2 * pb::SW16_R);
+            const int rounds = (np + pb::SW16_WARPS - 1) / pb::SW16_WARPS;
+            const double part = np >= 0.7 * rounds * pb::SW16_WARPS ? 0.5 : 1.0;
+            if (np > 1 && (double)cost[k] > part * rest / warps) {
+                rest -= (double)cost[k];
+                tasks[nteam++] = tasks[k];
+            } else {
+                lone.push_back(tasks[k]);
+            }
+        }
+        std::copy(lone.begin(), lone.end(), tasks.begin() + nteam);
+    }
+    if (cudaMallocAsync((void **)&counter, sizeof(int) * 4, st) != cudaSuccess ||
+        cudaMallocAsync((void **)&d_tasks, sizeof(pb::Sw16Task) * ntasks, st) != cudaSuccess ||
         cudaMallocAsync((void **)&d_q, sizeof(pb::Sw16Query) * nq, st) != cudaSuccess)
         return give_up();
-    cudaMemcpyAsync(d_tasks, sorted_tasks.data(), sizeof(pb::Sw16Task) * sorted_tasks.size(), cudaMemcpyHostToDevice, st);
+    cudaMemsetAsync(counter, 0, sizeof(int) * 4, st);   /* warp tasks, team tasks, error */
+    cudaMemcpyAsync(d_tasks, tasks.data(), sizeof(pb::Sw16Task) * ntasks, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(d_q, hq.data(), sizeof(pb::Sw16Query) * nq, cudaMemcpyHostToDevice, st);
-
-    int per_sm = 0, nsm = 0, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    /* the biased kernel (one DPX operation per row on the dependency
-     * chain) needs open >= gap and every score + open inside int8 */
-    bool bias = b->open >= b->gap;
-    for (int q = 0; q < nq; ++q)
-        if (b->profs[q]->mmax + b->open > 127 || b->profs[q]->mmin + b->open < -128) bias = false;
-    pb_raise_smem((const void *)pb::k_sw16<true>, (int)prof_bytes);
-    pb_raise_smem((const void *)pb::k_sw16<false>, (int)prof_bytes);
-    if (bias)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pb::k_sw16<true>, pb::SW16_WARPS * 32, prof_bytes);
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pb::k_sw16<false>, pb::SW16_WARPS * 32, prof_bytes);
-    if (per_sm < 1) per_sm = 1;
-    int blocks = per_sm * nsm;
-    const int need = (int)((sorted_tasks.size() + pb::SW16_WARPS - 1) / pb::SW16_WARPS);
-    /* few tasks (a small database, e.g. one query against 1,000 targets):
-     * every task gets a block of its own and is run as a team task, its
-     * passes spread over the block's warps, instead of leaving most SMs
-     * idle with one warp per task */
-    const bool few = (int)sorted_tasks.size() <= blocks;
-    if (few) blocks = (int)sorted_tasks.size();
-    else if (blocks > need) blocks = need;
-    const int maxlen = hlen[0] + 1;
-    /* few tasks: the intra-task wavefront, a warp per pair, as many warps
-     * as pairs (up to the resident warps) */
-    pr->wave = few;
+    /* entry c + 1 of a pass buffer is column c; a pass writes up to four
+     * past the longest target */
+    const int maxlen = hlen[0] + 8;
     if (few) {
         /* rows per lane: the fewest row-steps over the batch's queries,
          * npass * (RL + 4) per column, the 4 standing for the per-column
@@ -798,6 +880,7 @@ static int sw16_prepare(const pb_batch *b, pb_pair_out *d_out_all, size_t prof_b
         }
         pr->wave_rl = best_rl;
         int wper = 0;
+        pr->smem = prof_bytes;
         wave_set_smem((int)prof_bytes);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wper, wave_kernel(b->open >= b->gap, best_rl),
                                                       pb::SW16_WARPS * 32, prof_bytes);
@@ -810,21 +893,10 @@ static int sw16_prepare(const pb_batch *b, pb_pair_out *d_out_all, size_t prof_b
                             : sizeof(uint32_t) * (size_t)maxlen * 32 * blocks * pb::SW16_WARPS;
     /* k_sw16: per thread, the two strips' best columns (2 x 16 words) */
     pr->colsave_bytes = few ? 0 : sizeof(uint4) * (pb::SW16_R / 2) * (size_t)blocks * pb::SW16_WARPS * 32;
-    /* team tasks: those above a fair share of the work per warp, which one
-     * warp alone would finish last */
-    int nteam = few ? (int)sorted_tasks.size() : 0;
-    if (!few) {
-        double total = 0.0;
-        for (const auto &t : sorted_tasks) total += (double)hq[t.q].qlen * hlen[t.first];
-        const double fair = total / ((double)blocks * pb::SW16_WARPS);
-        while (nteam < (int)sorted_tasks.size() &&
-               (double)hq[sorted_tasks[nteam].q].qlen * hlen[sorted_tasks[nteam].first] > fair)
-            ++nteam;
-    }
     pb::Sw16Params &p = pr->p;
     p.open = b->open; p.gap = b->gap; p.npairs = n; p.nq = nq; p.nletters = b->profs[0]->size;
     p.bias = bias ? 1 : 0;
-    p.ntasks = (int)sorted_tasks.size(); p.maxlen = maxlen; p.nteam = nteam;
+    p.ntasks = (int)ntasks; p.maxlen = maxlen; p.nteam = nteam;
     p.queries = d_q; p.prof_all = prof_all; p.prof_bytes = (int)prof_bytes;
     p.order = so.order; p.tasks = d_tasks;
     p.targets = b->d_targets; p.toff = b->d_toff; p.tlen = b->d_tlen;
@@ -841,8 +913,7 @@ static int sw16_prepare(const pb_batch *b, pb_pair_out *d_out_all, size_t prof_b
     return 0;
 }
 
-/* The pass buffers of launches that run one after another on one stream:
- * one set of the largest size any of them needs. */
+/* The pass buffers of a prepared batch. */
 struct Sw16Work {
     uint32_t *scratch = nullptr;
     uint4 *colsave = nullptr;
@@ -856,29 +927,16 @@ static void sw16_work_release(Sw16Work *w, cudaStream_t st)
     w->colsave = nullptr;
 }
 
-/* preps[first], preps[first + step], ... on st's memory */
-static int sw16_workspace(Sw16Prep *preps, size_t n, size_t first, size_t step, cudaStream_t st, Sw16Work *w)
+static int sw16_workspace(Sw16Prep *pr, cudaStream_t st, Sw16Work *w)
 {
-    size_t sb = 0, cb = 0;
-    for (size_t k = first; k < n; k += step) {
-        sb = std::max(sb, preps[k].scratch_bytes);
-        cb = std::max(cb, preps[k].colsave_bytes);
-    }
-    if (sb && cudaMallocAsync((void **)&w->scratch, sb, st) != cudaSuccess) {
-        w->scratch = nullptr;
-        cudaGetLastError();
-        return -1;
-    }
-    if (cb && cudaMallocAsync((void **)&w->colsave, cb, st) != cudaSuccess) {
+    if (cudaMallocAsync((void **)&w->scratch, pr->scratch_bytes, st) != cudaSuccess) w->scratch = nullptr;
+    if (pr->colsave_bytes && cudaMallocAsync((void **)&w->colsave, pr->colsave_bytes, st) != cudaSuccess)
         w->colsave = nullptr;
-        cudaGetLastError();
-        return -1;
-    }
-    for (size_t k = first; k < n; k += step) {
-        preps[k].p.scratch = w->scratch;
-        preps[k].p.colsave = w->colsave;
-    }
-    return 0;
+    pr->p.scratch = w->scratch;
+    pr->p.colsave = w->colsave;
+    if (w->scratch && (w->colsave || !pr->colsave_bytes)) return 0;
+    cudaGetLastError();
+    return -1;
 }
 
 /* the kernel on a prepared batch (its counters zeroed first) */
@@ -886,56 +944,25 @@ static void sw16_launch(const Sw16Prep &pr, cudaStream_t st)
 {
     cudaMemsetAsync(pr.counter, 0, sizeof(int) * 4, st);
     if (pr.wave) {
-        wave_kernel(pr.p.open >= pr.p.gap, pr.wave_rl)<<<pr.blocks, pb::SW16_WARPS * 32, pr.prof_bytes, st>>>(
+        wave_kernel(pr.p.open >= pr.p.gap, pr.wave_rl)<<<pr.blocks, pb::SW16_WARPS * 32, pr.smem, st>>>(
             pr.p, pr.counter);
     } else {
         if (pr.p.bias)
-            pb::k_sw16<true><<<pr.blocks, pb::SW16_WARPS * 32, pr.prof_bytes, st>>>(pr.p, pr.counter);
+            pb::k_sw16<true><<<pr.blocks, pb::SW16_WARPS * 32, pr.smem, st>>>(pr.p, pr.counter);
         else
-            pb::k_sw16<false><<<pr.blocks, pb::SW16_WARPS * 32, pr.prof_bytes, st>>>(pr.p, pr.counter);
+            pb::k_sw16<false><<<pr.blocks, pb::SW16_WARPS * 32, pr.smem, st>>>(pr.p, pr.counter);
     }
 }
 
-/* One launch's share of the queries: as many consecutive profiles as fit
- * `limit` bytes of shared memory (at least one). */
-static int sw16_group(const pb_batch *b, int q0, size_t limit, size_t *bytes)
-{
-    int q = q0;
-    *bytes = 0;
-    while (q < b->nprofs) {
-        const size_t one = (size_t)b->profs[q]->size * b->profs[q]->lp;
-        if (q > q0 && *bytes + one > limit) break;
-        *bytes += one;
-        ++q;
-    }
-    return q - q0;
-}
-
-/* nq profiles against the same targets; out[q * npairs + i]. Profiles past
- * one launch's shared memory run in groups of consecutive queries, their
- * launches on two streams in turn, so that a group's first blocks take the
- * SMs that the last group's longest tasks leave idle. A group holds at most
- * SW16_GROUP bytes, which keeps two blocks on an SM: 40 queries (median 270)
- * x 10,000 targets from host memory took 508 ms on the exact kernel, one
- * query at a time, and 37.3 ms in four groups. Up to
- * 200 KB one launch of one block per SM stays: it holds every query of a
- * small search, and its tasks in one queue. */
-static constexpr size_t SW16_SMEM_MAX = 200 * 1024;
-static constexpr size_t SW16_GROUP = 104 * 1024;
-
+/* nq profiles against the same targets; out[q * npairs + i]: one launch for
+ * every query. */
 extern "C" int pb_cuda_align_sw16_multi(const pb_batch *b, pb_pair_out *d_out_all)
 {
     if (pb_cuda_init() != 0) return -1;
     const int n = b->npairs, nq = b->nprofs;
     if (n <= 0 || nq <= 0) return 0;
     bool ok = b->alg == PB_SW && !b->stats && !b->d_qlim && !b->d_tlim && b->open + b->gap <= 30000;
-    size_t prof_bytes = 0;
-    for (int q = 0; q < nq && ok; ++q) {
-        const pb_device_profile *dp = b->profs[q];
-        const size_t bytes = (size_t)dp->size * dp->lp;
-        ok = dp->fits8 && dp->size == b->profs[0]->size && bytes <= SW16_SMEM_MAX;
-        prof_bytes += bytes;
-    }
+    for (int q = 0; q < nq && ok; ++q) ok = b->profs[q]->fits8 && b->profs[q]->size == b->profs[0]->size;
     if (!ok) {
         /* outside this kernel's domain: the exact kernel, one profile at a time */
         for (int q = 0; q < nq; ++q) {
@@ -947,51 +974,27 @@ extern "C" int pb_cuda_align_sw16_multi(const pb_batch *b, pb_pair_out *d_out_al
         }
         return 0;
     }
-    cudaStream_t st = nullptr, st2 = nullptr;
+    cudaStream_t st = nullptr;
     if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return -1;
-    int rc = 0;
     Sw16Sort sort;
-    if (sw16_sort(b, st, &sort) != 0) {
-        cudaStreamSynchronize(st);
-        cudaStreamDestroy(st);
-        return -1;
-    }
-    std::vector<Sw16Prep> preps;
-    const size_t limit = prof_bytes > SW16_SMEM_MAX ? SW16_GROUP : SW16_SMEM_MAX;
-    for (int q0 = 0; q0 < nq && rc == 0;) {
-        size_t bytes = 0;
-        const int k = sw16_group(b, q0, limit, &bytes);
-        pb_batch g = *b;
-        g.profs = b->profs + q0;
-        g.nprofs = k;
-        Sw16Prep prep;
-        if (sw16_prepare(&g, d_out_all + (size_t)q0 * n, bytes, sort, st, &prep) != 0) rc = -1;
-        else preps.push_back(prep);
-        q0 += k;
-    }
-    Sw16Work work[2];
-    if (rc == 0 && (sw16_workspace(preps.data(), preps.size(), 0, 2, st, &work[0]) != 0 ||
-                    sw16_workspace(preps.data(), preps.size(), 1, 2, st, &work[1]) != 0))
-        rc = -1;
+    Sw16Prep prep;
+    Sw16Work work;
+    memset(&prep, 0, sizeof prep);
+    int rc = sw16_sort(b, st, &sort);
+    if (rc == 0) rc = sw16_prepare(b, d_out_all, sort, st, &prep);
+    if (rc == 0) rc = sw16_workspace(&prep, st, &work);
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    if (rc == 0 && (cudaEventCreate(&ev0) != cudaSuccess || cudaEventCreate(&ev1) != cudaSuccess ||
-                    (preps.size() > 1 && cudaStreamCreateWithFlags(&st2, cudaStreamNonBlocking) != cudaSuccess)))
-        rc = -1;
+    if (rc == 0 && (cudaEventCreate(&ev0) != cudaSuccess || cudaEventCreate(&ev1) != cudaSuccess)) rc = -1;
     if (rc == 0) {
         cudaEventRecord(ev0, st);
-        if (st2) cudaStreamWaitEvent(st2, ev0, 0);
-        for (size_t k = 0; k < preps.size(); ++k) sw16_launch(preps[k], k & 1 ? st2 : st);
-        if (st2) {
-            cudaEventRecord(ev1, st2);
-            cudaStreamWaitEvent(st, ev1, 0);
-        }
+        sw16_launch(prep, st);
         cudaEventRecord(ev1, st);
         if (cudaGetLastError() != cudaSuccess) rc = -1;
-        pb_diag_count_launch(1 + (int)preps.size());   /* k_iota, the score kernels */
+        pb_diag_count_launch(2);   /* k_iota, the score kernel */
     }
-    /* the launches' error flags, and the pairs that left the 16-bit range */
-    std::vector<int> herr(preps.size(), 0);
-    int *over = nullptr, nover_all = 0;
+    /* the launch's error flag, and the pairs that left the 16-bit range */
+    int herr = 0, nover_all = 0;
+    int *over = nullptr;
     const size_t N = (size_t)n * nq;
     if (rc == 0 && cudaMallocAsync((void **)&over, sizeof(int), st) != cudaSuccess) rc = -1;
     if (rc == 0) {
@@ -999,15 +1002,13 @@ extern "C" int pb_cuda_align_sw16_multi(const pb_batch *b, pb_pair_out *d_out_al
         k_count_overflow<<<148, 256, 0, st>>>(d_out_all, N, over);
         pb_diag_count_launch(1);
         cudaMemcpyAsync(&nover_all, over, sizeof(int), cudaMemcpyDeviceToHost, st);
-        for (size_t k = 0; k < preps.size(); ++k)
-            cudaMemcpyAsync(&herr[k], preps[k].counter + 2, sizeof(int), cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(&herr, prep.counter + 2, sizeof(int), cudaMemcpyDeviceToHost, st);
     }
     if (cudaStreamSynchronize(st) != cudaSuccess) rc = -1;
-    for (int e : herr)
-        if (e) {
-            fprintf(stderr, "pb_cuda_align_sw16_multi: a pass wait exceeded its bound\n");
-            rc = -1;
-        }
+    if (herr) {
+        fprintf(stderr, "pb_cuda_align_sw16_multi: a pass wait exceeded its bound\n");
+        rc = -1;
+    }
     if (rc == 0) {
         float ms = 0.f;
         cudaEventElapsedTime(&ms, ev0, ev1);
@@ -1060,11 +1061,10 @@ extern "C" int pb_cuda_align_sw16_multi(const pb_batch *b, pb_pair_out *d_out_al
     if (otlen) cudaFreeAsync(otlen, st);
     if (otoff) cudaFreeAsync(otoff, st);
     if (over) cudaFreeAsync(over, st);
-    for (Sw16Prep &prep : preps) sw16_release(&prep, st);
-    for (Sw16Work &w : work) sw16_work_release(&w, st);
+    sw16_release(&prep, st);
+    sw16_work_release(&work, st);
     sw16_sort_release(&sort, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) rc = -1;
-    if (st2) cudaStreamDestroy(st2);
     cudaStreamDestroy(st);
     return rc;
 }
@@ -1093,7 +1093,7 @@ extern "C" int pb_cuda_sw_single(const pb_device_profile *dp, int open, int gap,
         }
     }
     /* [Sw16Query][toff int64][order, tlen, counter x4: int][out][codes] then the scratch of 8 warps */
-    const size_t o_q = 0, o_toff = 16, o_ints = 24, o_out = 48;
+    const size_t o_q = 0, o_toff = 32, o_ints = 40, o_out = 64;
     const size_t o_codes = (o_out + sizeof(pb_pair_out) + 15) & ~(size_t)15;
     const size_t up = (o_codes + (size_t)tlen + 16 + 15) & ~(size_t)15;
     const size_t total = up + sizeof(int2) * (size_t)(tlen + 1) * pb::SW16_WARPS;
@@ -1101,7 +1101,7 @@ extern "C" int pb_cuda_sw_single(const pb_device_profile *dp, int open, int gap,
     char *d = pb_single_arena(total, up, &h);
     if (!d) { pb_cuda_set_error("single-pair arena", "allocation failed"); return -1; }
     pb::Sw16Query q;
-    q.prof_off = 0; q.qlen = dp->qlen; q.lp = dp->lp; q.posmax = 32767 - dp->mmax - 1;
+    q.prof8 = dp->d_prof8; q.prof_off = 0; q.qlen = dp->qlen; q.lp = dp->lp; q.posmax = 32767 - dp->mmax - 1;
     memcpy(h + o_q, &q, sizeof q);
     const int ints[6] = {0, tlen, 0, 0, 0, 0};
     memcpy(h + o_ints, ints, sizeof ints);
@@ -1218,7 +1218,7 @@ extern "C" int pb_cuda_db_plan_create(const pb_job *job, const pb_batch *b, pb_r
         if (!dp->fits8 || dp->size != b->profs[0]->size) return -1;
         prof_bytes += (size_t)dp->size * dp->lp;
     }
-    if (prof_bytes > SW16_SMEM_MAX) return -1;
+    if (prof_bytes > SW16_WAVE_SMEM) return -1;
     DbPlan *pl = new DbPlan();
     pl->job = *job;
     pl->profs.assign(b->profs, b->profs + nq);
@@ -1236,9 +1236,9 @@ extern "C" int pb_cuda_db_plan_create(const pb_job *job, const pb_batch *b, pb_r
         pb_batch bb = pl->b;
         bb.stats = 0; bb.pad_rows = 0; bb.d_qlim = nullptr; bb.d_tlim = nullptr;
         rc = sw16_sort(&bb, pl->st, &pl->sort);
-        if (rc == 0) rc = sw16_prepare(&bb, pl->o1, prof_bytes, pl->sort, pl->st, &pl->prep);
+        if (rc == 0) rc = sw16_prepare(&bb, pl->o1, pl->sort, pl->st, &pl->prep);
         pl->prepared = rc == 0;
-        if (rc == 0) rc = sw16_workspace(&pl->prep, 1, 0, 1, pl->st, &pl->work);
+        if (rc == 0) rc = sw16_workspace(&pl->prep, pl->st, &pl->work);
     }
     if (rc == 0 && cudaStreamSynchronize(pl->st) != cudaSuccess) rc = -1;
     if (rc == 0 && cudaStreamBeginCapture(pl->st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) rc = -1;

@@ -1,7 +1,7 @@
 """Database searches over the sizes at which the Smith-Waterman score path
-changes its kernel or its split of the work: more queries than one launch's
-shared memory holds (groups of queries on two streams), few and many
-targets, and pairs past the 16-bit range among them."""
+changes its kernel or its split of the work: more queries than fit the
+shared memory of the few-pairs kernel, few and many targets, teams and
+single warps, and pairs past the 16-bit range among them."""
 import random
 
 import numpy as np
@@ -38,7 +38,7 @@ def _check_db(queries, targets, name, open_, gap, sample, seed):
 
 
 @pytest.mark.parametrize("n_targets,t_hi", [(3, 400), (300, 400), (12000, 60)])
-def test_more_queries_than_one_launch_holds(n_targets, t_hi):
+def test_many_queries(n_targets, t_hi):
     rng = random.Random(n_targets)
     queries = [rand_seq(rng, L, AA) for L in (1, 31, 32, 33, 500, 777, 1000, 1500, 2000, 2500, 2990, 64)]
     queries[10] = "W" * 2990
