@@ -49,6 +49,7 @@ namespace pb {
 
 static constexpr int SW16_R = 16;          /* query rows per strip (two strips per pass) */
 static constexpr int SW16_WARPS = 8;       /* warps per block */
+static constexpr int WAVE16_WARPS = 4;     /* warps per block of k_sw_wave16 */
 static constexpr int SW16_ROW = 48;        /* bytes between two letters' scores in a warp's slice */
 
 /* Packs two signed bytes (byte k of a and of b) into one int16x2 word:
@@ -603,6 +604,266 @@ k_sw_wave(Sw16Params p, int *counter)
     }
 }
 
+/*
+ * The wavefront of small searches and single pairs in int16x2, where no
+ * pair can leave 16 bits (the host's bound, wave16_ok): one warp per pair,
+ * lane k holding 2R query rows as two strips of R rows in the halves of its
+ * registers, strip B one column behind strip A as in k_sw16. Lane k works on
+ * column t - 2k at iteration t (strip B on t - 2k - 1), so the row above its
+ * strip A is lane k-1's strip B bottom of the iteration before: one shuffle
+ * of (H, F) packed in a word.
+ * What bounds it is the latency of one iteration -- the shuffle, R dependent
+ * F steps, the hand-over -- with at most a few warps per scheduler, so the
+ * rows per lane follow the query length (R = 5 for 300 rows: one pass), and
+ * nothing is predicated: columns outside the target meet the letter after
+ * the alphabet, whose scores of -128 leave the zero boundary before column 0
+ * as it is and cannot raise a maximum after the last. Scores are staged per
+ * block as [pass][letter][strip][lane], so that the lanes' loads fall on
+ * different banks whatever their letters. One pair (300 x 350) takes 163 ->
+ * 85 us per call, 1 query (300) x 1,000 targets 253 -> 128 us per plan run,
+ * against the exact 32-bit wavefront (k_sw_wave), which stays for pairs that
+ * may pass 16 bits. Up to a task per resident block (9,472 targets) it beats
+ * k_sw16's teams: 300 rows x 1,000 / 4,000 / 9,000 targets 128 / 203 / 381 us
+ * against 316 / 314 / 475.
+ */
+template <bool BIAS, int R>
+__global__ void __launch_bounds__(WAVE16_WARPS * 32, 4)
+k_sw_wave16(Sw16Params p, int *counter)
+{
+    constexpr int W = (R + 3) / 4;                 /* score words per strip */
+    constexpr int LETTER = 2 * 32 * W;             /* words per letter */
+    extern __shared__ __align__(16) uint32_t s_sc[];
+    __shared__ int s_chunk;
+    __shared__ uint16_t s_ring[WAVE16_WARPS][128];
+    const int lane = threadIdx.x & 31;
+    const int wid = threadIdx.x >> 5;
+    uint16_t *ring = s_ring[wid];
+    const int L = p.nletters;
+    uint32_t *buf = p.scratch + (size_t)(blockIdx.x * WAVE16_WARPS + wid) * p.maxlen;
+    const uint32_t gapO = splat16(-p.open);
+    const uint32_t gapE = splat16(-p.gap);
+    const uint32_t zeroH = BIAS ? gapO : 0u;
+    const int bias = BIAS ? p.open : 0;
+    const uint32_t vnone = prmt(zeroH, gapO, 0x5410u);
+    const int per_q = (p.npairs + WAVE16_WARPS - 1) / WAVE16_WARPS;
+    const int nchunks = per_q * p.nq;
+    int staged = -1;
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) s_chunk = atomicAdd(counter, 1);
+        __syncthreads();
+        const int chunk = s_chunk;
+        if (chunk >= nchunks) break;
+        const int q = chunk / per_q;
+        const Sw16Query Q = p.queries[q];
+        const int n = Q.qlen;
+        const int npass = (n + 64 * R - 1) / (64 * R);
+        if (q != staged) {
+            /* a thread stages one (strip, lane) of every second letter: R
+             * bytes of the profile each, + open in the biased form */
+            const int slot = threadIdx.x & 63;
+            for (int pass = 0; pass < npass; ++pass) {
+                const int row = (pass * 32 + (slot & 31)) * 2 * R + (slot >> 5) * R;
+                uint32_t *d = s_sc + (size_t)pass * (L + 1) * LETTER + (slot >> 5) * 32 * W + (slot & 31) * W;
+#pragma unroll 4
+                for (int a = threadIdx.x >> 6; a <= L; a += WAVE16_WARPS / 2) {
+                    uint32_t w[W];
+#pragma unroll
+                    for (int k = 0; k < W; ++k) w[k] = 0u;
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        int v = -128;
+                        if (a < L) v = (row + r < Q.lp ? (int)__ldg(Q.prof8 + (size_t)a * Q.lp + row + r) : 0) + bias;
+                        w[r >> 2] |= (uint32_t)(uint8_t)(int8_t)v << (8 * (r & 3));
+                    }
+#pragma unroll
+                    for (int k = 0; k < W; ++k) d[(size_t)a * LETTER + k] = w[k];
+                }
+            }
+            staged = q;
+            __syncthreads();
+        }
+        const int item = (chunk - q * per_q) * WAVE16_WARPS + wid;
+        if (item >= p.npairs) continue;
+        const int pid = p.order[item];
+        const int m = p.tlen[pid];
+        const uint8_t *ts = p.targets + p.toff[pid];
+        Sw16Best best = {0, 0, 0};
+        int status = 0;
+        for (int pass = 0; pass < npass; ++pass) {
+            const uint32_t *sc_pass = s_sc + (size_t)pass * (L + 1) * LETTER + lane * W;
+            const int R0 = (pass * 32 + lane) * 2 * R;
+            const bool more = pass + 1 < npass;
+            uint32_t H[R], E[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) { H[r] = zeroH; E[r] = gapO; }
+            uint32_t dg = zeroH, prev_h = zeroH, prev_f = gapO, cur = vnone;
+            /* as in k_sw16: a half's own best of this pass, and one less than
+             * any other known score (every 32 columns, the warp's) */
+            uint32_t sbest = splat16(max(best.score - 1, 0) - bias);
+            Sw16Best sa = {0, -1, -1}, sb = {0, -1, -1};
+            uint32_t SA[R], SB[R];                 /* the strips' best columns */
+#pragma unroll
+            for (int r = 0; r < R; ++r) { SA[r] = 0u; SB[r] = 0u; }
+            /* Letters by column in the warp's ring of four 32-column chunks, as
+             * word offsets of their scores: a chunk is checked and stored once
+             * by the whole warp, one chunk before lane 0 needs it (a load per
+             * lane and column waited for its check in every iteration). */
+            auto fetch = [&](int c) -> int { return c < m ? (int)__ldg(ts + c) : L; };
+            auto put = [&](int c, int v) {
+                if (c < m && v >= L) { v = 0; status |= PB_ST_BADCODE; }
+                ring[c & 127] = (uint16_t)(v * LETTER);
+            };
+            __syncwarp();
+            put(lane, fetch(lane));
+            ring[64 + lane] = ring[96 + lane] = (uint16_t)(L * LETTER);
+            int pre = fetch(32 + lane);
+            __syncwarp();
+            /* A column's scores are loaded, and the row above handed down,
+             * right when the column before allows it, before that column's
+             * check for a new best: issue is in order, and a branch between
+             * would add its latency to the chain. */
+            auto load = [&](uint32_t (&w)[W], const uint32_t *at) {
+                if (W == 2) {
+                    const uint2 x = *reinterpret_cast<const uint2 *>(at);
+                    w[0] = x.x; w[W - 1] = x.y;
+                } else {
+                    w[0] = *at;
+                }
+            };
+            const uint32_t *pa_at = sc_pass + (lane == 0 ? ring[0] : L * LETTER);
+            uint32_t wa[W], wb4[W], v = vnone;
+            load(wa, pa_at);
+            load(wb4, sc_pass + L * LETTER + 32 * W);
+            const int iters = m + 63;
+            for (int t0 = 0; t0 < iters; t0 += 32) {
+                if (pass > 0) {
+                    cur = t0 + lane < m ? __ldcg(&buf[t0 + lane]) : vnone;
+                    const uint32_t vin = __shfl_sync(0xffffffffu, cur, 0);
+                    if (lane == 0) v = vin;
+                }
+                put(t0 + 32 + lane, pre);
+                pre = fetch(t0 + 64 + lane);
+                const int wb = __reduce_max_sync(0xffffffffu, max(best.score, max(sa.score, sb.score)));
+                sbest = __vmaxs2(sbest, splat16(max(wb - 1, 0) - bias));
+                __syncwarp();
+                const int n_it = min(32, iters - t0);
+                /* strip A's column j = t0 + it - 2 * lane */
+                int off = ring[(t0 - 2 * lane + 1) & 127];
+#pragma unroll 2
+                for (int it = 0; it < n_it; ++it) {
+                    const int j = t0 + it - 2 * lane;
+                    uint32_t na[W], nb[W];
+                    load(nb, pa_at + 32 * W);
+                    pa_at = sc_pass + off;
+                    load(na, pa_at);
+                    off = ring[(j + 2) & 127];
+                    uint32_t hu = prmt(v, prev_h, 0x5410u);
+                    uint32_t fu = prmt(v, prev_f, 0x5432u);
+                    uint32_t hd = dg;
+                    dg = hu;
+                    uint32_t cmax = zeroH, aop = 0u;
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        uint32_t sc;
+                        switch (r & 3) {
+                            case 0: sc = pack_pair<0>(wa[r >> 2], wb4[r >> 2]); break;
+                            case 1: sc = pack_pair<1>(wa[r >> 2], wb4[r >> 2]); break;
+                            case 2: sc = pack_pair<2>(wa[r >> 2], wb4[r >> 2]); break;
+                            default: sc = pack_pair<3>(wa[r >> 2], wb4[r >> 2]); break;
+                        }
+                        uint32_t e, a, f, h;
+                        if (BIAS) {
+                            e = __viaddmax_s16x2(E[r], gapE, H[r]);
+                            a = __viaddmax_s16x2_relu(hd, sc, e);
+                            const uint32_t ao = __vadd2(a, gapO);
+                            f = __viaddmax_s16x2(fu, gapE, r == 0 ? hu : aop);
+                            h = __viaddmax_s16x2(f, gapO, ao);
+                            aop = ao;
+                        } else {
+                            e = __viaddmax_s16x2(E[r], gapE, __vadd2(H[r], gapO));
+                            a = __viaddmax_s16x2_relu(hd, sc, e);
+                            f = __viaddmax_s16x2(hu, gapO, __vadd2(fu, gapE));
+                            h = __vmaxs2(a, f);
+                        }
+                        E[r] = e;
+                        hd = H[r];
+                        H[r] = h;
+                        hu = h;
+                        fu = f;
+                        if (r & 1) cmax = __vimax3_s16x2(cmax, H[r - 1], h);
+                        else if (r == R - 1) cmax = __vmaxs2(cmax, h);
+                    }
+                    const uint32_t out = prmt(hu, fu, 0x7632u);
+                    v = __shfl_up_sync(0xffffffffu, out, 1);
+                    const uint32_t vin = pass > 0 ? __shfl_sync(0xffffffffu, cur, (it + 1) & 31) : vnone;
+                    if (lane == 0) v = vin;
+                    prev_h = hu;
+                    prev_f = fu;
+#pragma unroll
+                    for (int k = 0; k < W; ++k) { wa[k] = na[k]; wb4[k] = nb[k]; }
+                    if (more && lane == 31 && (unsigned)(j - 1) < (unsigned)m) buf[j - 1] = out;
+                    if (__vmaxs2(sbest, cmax) != sbest) {
+                        const int ca = s16lo(cmax), cb = s16hi(cmax);
+                        int ba = s16lo(sbest), bb = s16hi(sbest);
+                        const bool up_a = ca > ba, up_b = cb > bb;
+                        if (up_a) {
+#pragma unroll
+                            for (int r = 0; r < R; ++r) SA[r] = H[r];
+                            sa.score = ca + bias; sa.j = j;
+                            ba = ca;
+                        }
+                        if (up_b) {
+#pragma unroll
+                            for (int r = 0; r < R; ++r) SB[r] = H[r];
+                            sb.score = cb + bias; sb.j = j - 1;
+                            bb = cb;
+                        }
+                        if (up_a) bb = max(bb, ca - 1);
+                        if (up_b) ba = max(ba, cb - 1);
+                        sbest = (uint32_t)(uint16_t)ba | ((uint32_t)(uint16_t)bb << 16);
+                    }
+                }
+            }
+            /* the first row of each strip's best column reaching its maximum */
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const Sw16Best c = h ? sb : sa;
+                if (c.j < 0) continue;
+                int rr = R - 1;
+#pragma unroll
+                for (int r = R - 2; r >= 0; --r) if ((h ? s16hi(SB[r]) : s16lo(SA[r])) == c.score - bias) rr = r;
+                const int ci = R0 + h * R + rr;
+                if (c.score > best.score || (c.score == best.score && (c.j < best.j || (c.j == best.j && ci < best.i)))) {
+                    best.score = c.score; best.j = c.j; best.i = ci;
+                }
+            }
+            __syncwarp();
+        }
+        /* the lanes' bests in the reference's order: higher score, then
+         * smaller column, then smaller row */
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const int os = __shfl_xor_sync(0xffffffffu, best.score, o);
+            const int oj = __shfl_xor_sync(0xffffffffu, best.j, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, best.i, o);
+            if (os > best.score || (os == best.score && (oj < best.j || (oj == best.j && oi < best.i)))) {
+                best.score = os; best.j = oj; best.i = oi;
+            }
+        }
+        status = __reduce_or_sync(0xffffffffu, status);
+        if (lane == 0) {
+            pb_pair_out o = {};
+            o.score = best.score;
+            o.end_query = best.i;
+            o.end_ref = best.j;
+            o.max_h = o.score;
+            o.status = status;
+            p.out[(size_t)q * p.npairs + pid] = o;
+        }
+    }
+}
+
 }  // namespace pb
 
 namespace {
@@ -657,6 +918,7 @@ struct Sw16Prep {
     int blocks;
     bool wave;                    /* few tasks: the intra-task wavefront k_sw_wave */
     int wave_rl;                  /* its rows per lane */
+    int wave16;                   /* > 0: k_sw_wave16 with that many rows per strip instead */
     size_t smem;                  /* dynamic shared memory of its kernel */
     int *counter;                 /* [warp tasks, team tasks, error, spare] */
     size_t scratch_bytes, colsave_bytes;
@@ -688,6 +950,60 @@ static WaveKernel wave_kernel(bool ge, int rl)
         case 16: return pb::k_sw_wave<false, 16>;
         default: return pb::k_sw_wave<false, 8>;
     }
+}
+
+/* k_sw_wave16 for (biased, rows per strip) */
+template <bool BIAS>
+static WaveKernel wave16_kernel_of(int r)
+{
+    switch (r) {
+        case 1: return pb::k_sw_wave16<BIAS, 1>;
+        case 2: return pb::k_sw_wave16<BIAS, 2>;
+        case 3: return pb::k_sw_wave16<BIAS, 3>;
+        case 4: return pb::k_sw_wave16<BIAS, 4>;
+        case 5: return pb::k_sw_wave16<BIAS, 5>;
+        case 6: return pb::k_sw_wave16<BIAS, 6>;
+        case 7: return pb::k_sw_wave16<BIAS, 7>;
+        default: return pb::k_sw_wave16<BIAS, 8>;
+    }
+}
+
+static WaveKernel wave16_kernel(bool bias, int r) { return bias ? wave16_kernel_of<true>(r) : wave16_kernel_of<false>(r); }
+
+/* every score + open inside int8, open >= gap: the biased kernels */
+static bool sw16_bias_ok(const pb_device_profile *dp, int open, int gap)
+{
+    return open >= gap && dp->mmax + open <= 127 && dp->mmin + open >= -128;
+}
+
+/* Can no pair of this profile with a target of at most maxlen residues leave
+ * k_sw_wave16's lanes? Every H is at most max(matrix) per aligned pair (below
+ * the same bound as k_sw16's overflow check), and E, F are at least -open -
+ * gap. */
+static bool wave16_ok(const pb_device_profile *dp, int maxlen, int open, int gap)
+{
+    const long long top = (long long)std::max(dp->mmax, 0) * (std::min(dp->qlen, maxlen) + 1);
+    return dp->fits8 && open + gap <= 30000 && top < 32767 - std::max(dp->mmax, 0) - 1;
+}
+
+/* rows per strip: the fewest row-steps over the queries, npass * (R + 3) per
+ * column, the 3 standing for an iteration's shuffles, loads and checks */
+static int wave16_rows(const pb_device_profile *const *profs, int nq)
+{
+    int best_r = 8;
+    double best = -1.0;
+    for (int r = 1; r <= 8; ++r) {
+        double cost = 0.0;
+        for (int q = 0; q < nq; ++q) cost += (double)((profs[q]->qlen + 64 * r - 1) / (64 * r)) * (r + 3);
+        if (best < 0.0 || cost < best) { best = cost; best_r = r; }
+    }
+    return best_r;
+}
+
+/* bytes of one query's staged scores */
+static size_t wave16_smem(const pb_device_profile *dp, int r)
+{
+    return (size_t)((dp->qlen + 64 * r - 1) / (64 * r)) * (dp->size + 1) * 64 * 4 * ((r + 3) / 4);
 }
 
 static void wave_set_smem(int bytes)
@@ -766,7 +1082,7 @@ static int sw16_prepare(const pb_batch *b, pb_pair_out *d_out_all, const Sw16Sor
     bool bias = b->open >= b->gap;
     size_t prof_bytes = 0;
     for (int q = 0; q < nq; ++q) {
-        if (b->profs[q]->mmax + b->open > 127 || b->profs[q]->mmin + b->open < -128) bias = false;
+        bias = bias && sw16_bias_ok(b->profs[q], b->open, b->gap);
         prof_bytes += (size_t)b->profs[q]->size * b->profs[q]->lp;
     }
     pr->smem = (size_t)pb::SW16_WARPS * b->profs[0]->size * pb::SW16_ROW;
@@ -780,20 +1096,27 @@ static int sw16_prepare(const pb_batch *b, pb_pair_out *d_out_all, const Sw16Sor
     /* few tasks (a small database, e.g. one query against 1,000 targets)
      * whose profiles fit its shared memory: the intra-task wavefront, a warp
      * per pair, as many warps as pairs (up to the resident warps) */
-    const bool few = ntasks <= (size_t)blocks && prof_bytes <= SW16_WAVE_SMEM;
+    int wave16 = wave16_rows(b->profs, nq);
+    size_t smem16 = 0;
+    for (int q = 0; q < nq; ++q) {
+        if (!wave16_ok(b->profs[q], hlen[0], b->open, b->gap)) wave16 = 0;
+        if (wave16) smem16 = std::max(smem16, wave16_smem(b->profs[q], wave16));
+    }
+    if (smem16 > SW16_WAVE_SMEM) wave16 = 0;
+    const bool few = ntasks <= (size_t)blocks && (wave16 || prof_bytes <= SW16_WAVE_SMEM);
     if ((size_t)blocks > ntasks) blocks = (int)ntasks;
     pr->wave = few;
     /* the queries; for the wavefront their profiles side by side */
     std::vector<pb::Sw16Query> hq(nq);
-    if (few && cudaMallocAsync((void **)&prof_all, prof_bytes, st) != cudaSuccess) return give_up();
+    if (few && !wave16 && cudaMallocAsync((void **)&prof_all, prof_bytes, st) != cudaSuccess) return give_up();
     {
         size_t off = 0;
         for (int q = 0; q < nq; ++q) {
             const pb_device_profile *dp = b->profs[q];
             const size_t bytes = (size_t)dp->size * dp->lp;
-            if (few) cudaMemcpyAsync(prof_all + off, dp->d_prof8, bytes, cudaMemcpyDeviceToDevice, st);
+            if (few && !wave16) cudaMemcpyAsync(prof_all + off, dp->d_prof8, bytes, cudaMemcpyDeviceToDevice, st);
             hq[q].prof8 = dp->d_prof8;
-            hq[q].prof_off = few ? (int)off : 0;
+            hq[q].prof_off = few && !wave16 ? (int)off : 0;
             hq[q].qlen = dp->qlen;
             hq[q].lp = dp->lp;
             hq[q].posmax = 32767 - dp->mmax - 1;
@@ -866,7 +1189,17 @@ static int sw16_prepare(const pb_batch *b, pb_pair_out *d_out_all, const Sw16Sor
     /* entry c + 1 of a pass buffer is column c; a pass writes up to four
      * past the longest target */
     const int maxlen = hlen[0] + 8;
-    if (few) {
+    if (few && wave16) {
+        pr->wave16 = wave16;
+        pr->smem = smem16;
+        const WaveKernel k16 = wave16_kernel(bias, wave16);
+        int wper = 0;
+        pb_raise_smem((const void *)k16, (int)smem16);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wper, k16, pb::WAVE16_WARPS * 32, smem16);
+        if (wper < 1) wper = 1;
+        const long long want = (long long)nq * ((n + pb::WAVE16_WARPS - 1) / pb::WAVE16_WARPS);
+        blocks = (int)std::min<long long>(want, (long long)wper * nsm);
+    } else if (few) {
         /* rows per lane: the fewest row-steps over the batch's queries,
          * npass * (RL + 4) per column, the 4 standing for the per-column
          * shuffles and loads (one query of 300 rows: one pass of 12 rows
@@ -943,7 +1276,9 @@ static int sw16_workspace(Sw16Prep *pr, cudaStream_t st, Sw16Work *w)
 static void sw16_launch(const Sw16Prep &pr, cudaStream_t st)
 {
     cudaMemsetAsync(pr.counter, 0, sizeof(int) * 4, st);
-    if (pr.wave) {
+    if (pr.wave16) {
+        wave16_kernel(pr.p.bias != 0, pr.wave16)<<<pr.blocks, pb::WAVE16_WARPS * 32, pr.smem, st>>>(pr.p, pr.counter);
+    } else if (pr.wave) {
         wave_kernel(pr.p.open >= pr.p.gap, pr.wave_rl)<<<pr.blocks, pb::SW16_WARPS * 32, pr.smem, st>>>(
             pr.p, pr.counter);
     } else {
@@ -1079,13 +1414,19 @@ extern "C" int pb_cuda_sw_single(const pb_device_profile *dp, int open, int gap,
     if (!dp->fits8 || !dp->d_prof8 || tlen <= 0 || open + gap > 30000) return -2;
     cudaGetLastError();   /* a launch error below is this call's own */
     const size_t prof_bytes = (size_t)dp->size * dp->lp;
+    const bool bias = sw16_bias_ok(dp, open, gap);
+    const int rows16 = wave16_rows(&dp, 1);
+    const size_t smem16 = wave16_smem(dp, rows16);
+    const bool use16 = wave16_ok(dp, tlen, open, gap) && smem16 <= SW16_WAVE_SMEM;
+    const size_t smem = use16 ? smem16 : prof_bytes;
     /* the kernels' shared-memory limit raised to this profile (never lowered) */
     {
         int dev = 0, optin = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        if ((long long)prof_bytes > optin) return -2;
-        wave_set_smem((int)prof_bytes);
+        if ((long long)smem > optin) return -2;
+        if (use16) pb_raise_smem((const void *)wave16_kernel(bias, rows16), (int)smem);
+        else wave_set_smem((int)smem);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) {
             pb_cuda_set_error("single-pair SW shared memory", cudaGetErrorString(e));
@@ -1130,7 +1471,8 @@ extern "C" int pb_cuda_sw_single(const pb_device_profile *dp, int open, int gap,
         if (best < 0.0 || c < best) { best = c; rl = r; }
     }
     int *counter = reinterpret_cast<int *>(d + o_ints) + 2;
-    wave_kernel(open >= gap, rl)<<<1, pb::SW16_WARPS * 32, prof_bytes, st>>>(p, counter);
+    if (use16) wave16_kernel(bias, rows16)<<<1, pb::WAVE16_WARPS * 32, smem, st>>>(p, counter);
+    else wave_kernel(open >= gap, rl)<<<1, pb::SW16_WARPS * 32, smem, st>>>(p, counter);
     pb_diag_count_launch(1);
     {
         const cudaError_t e = cudaGetLastError();

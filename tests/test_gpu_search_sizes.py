@@ -47,3 +47,30 @@ def test_many_queries(n_targets, t_hi):
     targets[1] = "W" * 2995        # 32890 against the query of 2990: past 16 bits
     _check_db(queries, targets, "sw_striped_profile_sat", 11, 1, 60, 1)
     _check_db(queries[4:9] + queries, targets, "sw_scan_profile_32", 10, 2, 20, 2)
+
+
+@pytest.mark.parametrize("open_,gap", [(11, 1), (120, 2)])
+def test_few_pairs_wavefront(open_, gap):
+    """Small searches and single calls: queries at the edges of the rows a
+    lane and a pass hold, targets of one residue and more; (120, 2) is past
+    the biased form. Every pair against the oracle."""
+    rng = random.Random(open_)
+    b62 = pb.matrix_lookup("blosum62")
+    om = O.Matrix.from_struct(b62)
+    lengths = [1, 2, 63, 64, 65, 127, 128, 129, 191, 193, 300, 319, 320, 321, 385, 448, 512, 513, 577, 1100]
+    for k, L in enumerate(lengths):
+        q = rand_seq(rng, L, AA)
+        targets = [rand_seq(rng, 1, AA), rand_seq(rng, 2, AA), q, mutate(rng, q, AA, 0.3, 0.05) + rand_seq(rng, 40, AA)]
+        targets += [rand_seq(rng, rng.randint(1, 700), AA) for _ in range(3)]
+        prof = pb.ProfileHandle("parasail_profile_create_16", q, b62)
+        recs = pb.batch_profile("sw_striped_profile_16", prof, targets, open_, gap)
+        for i, t in enumerate(targets):
+            e = O.align(O.SW, 0, 0, q, t, open_, gap, om)
+            exp = (e["score"], e["end_query"], e["end_ref"])
+            assert tuple(int(recs[i][f]) for f in FIELDS[:3]) == exp, (L, i)
+            got = pb.align_profile("parasail_sw_striped_profile_16", prof, t, open_, gap)
+            assert (got["score"], got["end_query"], got["end_ref"]) == exp, (L, i)
+        prof.close()
+    queries = [rand_seq(rng, L, AA) for L in (40, 300, 700)]
+    _check_db(queries, [rand_seq(rng, rng.randint(1, 500), AA) for _ in range(130)], "sw_striped_profile_16",
+              open_, gap, 130, 3)
