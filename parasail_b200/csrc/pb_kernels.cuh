@@ -84,6 +84,40 @@ struct Sw16Params {
     pb_pair_out *out;        /* [nq][npairs] */
 };
 
+/* A lane's target residues, four columns at a time. One byte load per
+ * column and lane touches 32 different lines; here the lane reads the
+ * aligned 32-bit words that hold its residues, two words ahead, and shifts
+ * them together. Only words that hold at least one byte of the sequence
+ * are read; columns past its end are letter 0. */
+struct ResidueWords {
+    const uint32_t *w;
+    int shift, last, len;
+    uint32_t a, b, c;        /* words k, k + 1, k + 2 of the next four columns */
+    __device__ __forceinline__ uint32_t word(int k) const { return k <= last ? __ldg(w + k) : 0u; }
+    __device__ __forceinline__ void start(const uint8_t *seq, int n)
+    {
+        const uintptr_t p = reinterpret_cast<uintptr_t>(seq);
+        w = reinterpret_cast<const uint32_t *>(p & ~(uintptr_t)3);
+        shift = (int)(p & 3) * 8;
+        len = n;
+        last = n > 0 ? ((int)(p & 3) + n - 1) >> 2 : -1;
+        a = word(0);
+        b = word(1);
+        c = word(2);
+    }
+    /* the residues of columns j .. j + 3 (j a multiple of 4), one per byte */
+    __device__ __forceinline__ uint32_t next(int j)
+    {
+        uint32_t v = __funnelshift_r(a, b, shift);
+        const int left = len - j;
+        if (left < 4) v = left <= 0 ? 0u : v & (0xffffffffu >> (32 - 8 * left));
+        a = b;
+        b = c;
+        c = word((j >> 2) + 3);
+        return v;
+    }
+};
+
 /* The int16x2 pair kernels (pb_pair16.cu). Items are pairs (pairs mode:
  * query codes per item scored through an int8 matrix) or query x target
  * products (db mode: item = query * nt + target, int8 profiles). */
@@ -104,7 +138,7 @@ struct P16Params {
     int nt;                       /* db mode: targets per query; 0 in pairs mode */
     const uint8_t *targets;
     const int64_t *toff;
-    uint32_t *scratch;            /* per resident warp [maxlen + 1][32] pass boundaries (H, F int16) */
+    uint32_t *scratch;            /* per resident warp [maxlen + 8][32] pass boundaries (H, F int16) */
     uint4 *colsave;               /* SW ends, per resident thread: its strips' best columns (8 x 16 bytes) */
     int maxlen;
     pb_pair_out *out;
@@ -127,6 +161,11 @@ struct P16Setup {
      * to the intra-task kernel instead (bit b set); 0: none */
     unsigned intra_mask;
 };
+
+/* columns that a pass of the pair kernels runs (and stores bits for) over a
+ * task whose widest target has wmax columns: strip B ends one column behind
+ * strip A, and four columns go together */
+__host__ __device__ inline int p16_cols(int wmax) { return (wmax + 4) & ~3; }
 
 /* length bucket of a pair for the schedule table */
 __host__ __device__ inline int p16_bucket(int rows, int cols)

@@ -44,9 +44,8 @@
  * cells carry 0. Those counts are the counts along that path. With
  * statistics the kernel stores, per cell, the four decisions that define
  * the path: not-diagonal (H > H_diag + s), not-F (H > F), E opened and F
- * opened -- each the sign bit of an int16 difference, shifted into per-row
- * bit accumulators: bit r (low half, strip A) and 16 + r (high half, strip
- * B) of four words stored as one uint4 per lane per iteration. The walk
+ * opened -- each the sign bit of an int16 difference, gathered into per-row
+ * bits (p16_bit) of four words stored as one uint4 per lane per iteration. The walk
  * (k_p16_walk) then follows the path back from the end cell, adding 1 to
  * length per step and, on diagonal steps, the match and positive-score
  * indicators; in SW it stops where the running H value (the end score
@@ -75,6 +74,11 @@ namespace pb {
 
 static constexpr int P16_R = 16;              /* rows per strip; two strips per pass */
 static constexpr int P16_PASS = 2 * P16_R;
+static constexpr int P16_ROW = 48;            /* bytes between two letters' scores in a shared slice */
+
+/* the bit of query row i of a task's direction bits (row i of its pass): the
+ * byte by the row's parity and strip, the bit by its pair of rows */
+__device__ __forceinline__ int p16_bit(int i) { return ((i & 1) * 2 + ((i >> 4) & 1)) * 8 + ((i & 15) >> 1); }
 
 __device__ __forceinline__ uint32_t p16_prmt(uint32_t a, uint32_t b, uint32_t sel)
 {
@@ -140,33 +144,53 @@ struct P16Best {
  * One task (32 items) per warp at a time. SHARED: every lane of a task has
  * the same query (its scores are staged once per warp); else every lane
  * stages its own. BITS: store the direction bits. ENDS: compute score and
- * ends (off for the FASTSTATS prefix pass, whose ends are known).
+ * ends (off for the FASTSTATS prefix pass, whose ends are known). BIAS (open
+ * >= gap, every score + open inside int8): H registers and boundaries hold
+ * H - open, staged scores s + open, so the gap sources need no add, and F of
+ * the next row is max(F - gap, max(H_diag + s, E) - open).
+ *
+ * What bounds it: the ALU pipe at half rate (maxima, three-operand DPX, byte
+ * permutes, logic), with the packed adds and differences on the FMA pipe
+ * beside it. Per row of two cells, score only: 5 ALU and 1 FMA operations;
+ * with bits: 8 and 8 -- the four decisions are signs of differences, and one
+ * permute gathers (and spreads over their bytes) the signs of two rows, of
+ * which a mask keeps the pair's bit (2 per decision and row before, by
+ * shifted accumulators). As in k_sw16, four columns run without a branch
+ * each, targets are read by words (the code check of a byte load waited
+ * for the load in every column), and the staged scores are laid out so
+ * that 16-byte loads fall on all bank groups: [letter][48 bytes] per warp,
+ * or [letter][strip][lane] x 16 bytes. 1 M DNA reads, NW statistics (bits):
+ * 29.3 -> 23.0 ms; 524 k protein pairs all against all: score pass 93.5 ->
+ * 65.7 ms (4,800 GCUPS), prefix bits pass 158 -> 115 ms.
  */
-template <int ALG, bool BITS, bool ENDS, bool SHARED, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, (WARPS == 8 ? 2 : 4))
+template <int ALG, bool BITS, bool ENDS, bool SHARED, int WARPS, bool BIAS>
+__global__ void __launch_bounds__(WARPS * 32, (WARPS == 8 ? 2 : 3))
 k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
 {
     extern __shared__ __align__(16) int8_t s_mem[];
+    constexpr int LETTER = SHARED ? P16_ROW : 1024, STRIP = SHARED ? 16 : 512;
     const int L = p.nletters;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int open = p.open, gap = p.gap, sgf = p.sgflags;
+    const int bias = BIAS ? open : 0;
     /* shared memory: [matrix L x L int8, padded to 16] [per-warp score slices] */
     const int mat_bytes = p.mat8 ? ((L * L + 15) & ~15) : 0;
-    const int lane_stride = SHARED ? 0 : L * P16_PASS + 16;
-    const int warp_bytes = SHARED ? L * P16_PASS : 32 * lane_stride;
     int8_t *s_mat = s_mem;
-    int8_t *wslice = s_mem + mat_bytes + wid * warp_bytes;
-    int8_t *myslice = wslice + lane * lane_stride;
+    int8_t *wslice = s_mem + mat_bytes + wid * L * LETTER;
+    int8_t *sl = wslice + (SHARED ? 0 : lane * 16);
     if (p.mat8)
-        for (int k = threadIdx.x; k < L * L; k += blockDim.x) s_mat[k] = p.mat8[k];
+        for (int k = threadIdx.x; k < L * L; k += blockDim.x) s_mat[k] = (int8_t)(p.mat8[k] + bias);
     __syncthreads();
 
-    /* pass boundary: strip B's bottom row per column, H low and F high */
-    uint32_t *buf = p.scratch + (size_t)(blockIdx.x * WARPS + wid) * (size_t)(p.maxlen + 1) * 32;
+    /* pass boundary: entry c + 1 is strip B's bottom row at column c, H low
+     * and F high */
+    uint32_t *buf = p.scratch + (size_t)(blockIdx.x * WARPS + wid) * (size_t)(p.maxlen + 8) * 32 + lane;
     /* SW ends: this thread's copies of its strips' best columns */
     uint4 *save = ENDS && ALG == PB_SW ? p.colsave + ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * (P16_R / 2)
                                        : nullptr;
-    const int open = p.open, gap = p.gap, sgf = p.sgflags;
     const uint32_t gO = p16_splat(-open), gE = p16_splat(-gap);
+    const uint32_t b4 = 0x01010101u * (uint32_t)(uint8_t)bias;
+    const uint32_t big4 = 0x01010101u * (uint32_t)(0x80 - L);
     const int nwarps_total = gridDim.x * WARPS;
     bool first = true;
     for (;;) {
@@ -211,12 +235,11 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
         const P16Bounds bd = p16_bounds(ALG, rows, cols, open, gap, p.mmax, p.mmin);
         const int negv = bd.lb - open - 1;
         const uint32_t NEG = p16_splat(negv);
-        uint4 *tbits = BITS ? p.bits + p.task_bits[task] : nullptr;
+        uint4 *tbits = BITS ? p.bits + p.task_bits[task] + lane : nullptr;
         int status = 0;
 
         /* end tracking */
         P16Best best = {0, 0, 0};
-        bool have = false;
         int lc_h = INT_MIN, lc_i = -1;       /* SG: last column over rows < rows - 1 */
         int lr_h = INT_MIN, lr_j = -1;       /* SG: last row */
         int corner = 0;
@@ -225,9 +248,9 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
 
         for (int pass = 0; pass < npass; ++pass) {
             const int r0 = pass * P16_PASS;
-            /* scores of this pass's 32 rows against every letter: once per
-             * warp (shared query) or once per lane; rows past the query
-             * (past the task's longest in shared pairs mode) score 0 */
+            /* scores (BIAS: + open) of this pass's 32 rows against every
+             * letter: once per warp (shared query) or once per lane; rows past
+             * the query (past the task's longest in shared pairs mode) score 0 */
             if (SHARED) {
                 __syncwarp();
                 if (p.mat8) {
@@ -235,12 +258,16 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
                     uint32_t c = i < rmax ? qseq0[i] : 255u;
                     if (c != 255u && c >= (uint32_t)L) { c = 0; status |= PB_ST_BADCODE; }
                     for (int a = 0; a < L; ++a)
-                        wslice[a * P16_PASS + lane] = c == 255u ? (int8_t)0 : s_mat[a * L + c];
+                        wslice[a * LETTER + lane] = c == 255u ? (int8_t)bias : s_mat[a * L + c];
                 } else {
                     for (int x = lane; x < 2 * L; x += 32) {
                         const int a = x >> 1, h = x & 1;
-                        const int4 v = *reinterpret_cast<const int4 *>(prof8 + (size_t)a * lp + r0 + 16 * h);
-                        *reinterpret_cast<int4 *>(wslice + a * P16_PASS + 16 * h) = v;
+                        int4 v = *reinterpret_cast<const int4 *>(prof8 + (size_t)a * lp + r0 + 16 * h);
+                        if (BIAS) {
+                            v.x = (int)__vadd4((uint32_t)v.x, b4); v.y = (int)__vadd4((uint32_t)v.y, b4);
+                            v.z = (int)__vadd4((uint32_t)v.z, b4); v.w = (int)__vadd4((uint32_t)v.w, b4);
+                        }
+                        *reinterpret_cast<int4 *>(wslice + a * LETTER + 16 * h) = v;
                     }
                 }
             } else if (p.mat8) {
@@ -259,15 +286,21 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
                 }
                 for (int a = 0; a < L; ++a) {
 #pragma unroll
-                    for (int w = 0; w < 8; ++w) {
-                        uint32_t word = 0;
+                    for (int h = 0; h < 2; ++h) {
+                        uint32_t word[4];
 #pragma unroll
-                        for (int b = 0; b < 4; ++b) {
-                            const uint32_t c = (qc[w] >> (8 * b)) & 0xffu;
-                            const uint32_t v = c == 255u ? 0u : (uint32_t)(uint8_t)s_mat[a * L + c];
-                            word |= v << (8 * b);
+                        for (int w = 0; w < 4; ++w) {
+                            word[w] = 0;
+#pragma unroll
+                            for (int b = 0; b < 4; ++b) {
+                                const uint32_t c = (qc[4 * h + w] >> (8 * b)) & 0xffu;
+                                const uint32_t v = c == 255u ? (uint32_t)(uint8_t)bias
+                                                             : (uint32_t)(uint8_t)s_mat[a * L + c];
+                                word[w] |= v << (8 * b);
+                            }
                         }
-                        *reinterpret_cast<uint32_t *>(myslice + a * P16_PASS + 4 * w) = word;
+                        *reinterpret_cast<uint4 *>(sl + a * LETTER + h * STRIP) =
+                            make_uint4(word[0], word[1], word[2], word[3]);
                     }
                 }
             } else {
@@ -276,163 +309,203 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
                  * beyond its query: zeros) */
                 const bool in = r0 + P16_PASS <= lp;
                 for (int a = 0; a < L; ++a) {
-                    const int4 z = make_int4(0, 0, 0, 0);
                     const int4 *src = reinterpret_cast<const int4 *>(prof8 + (size_t)a * lp + (in ? r0 : 0));
-                    *reinterpret_cast<int4 *>(myslice + a * P16_PASS) = in ? src[0] : z;
-                    *reinterpret_cast<int4 *>(myslice + a * P16_PASS + 16) = in ? src[1] : z;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        int4 v = in ? src[h] : make_int4(0, 0, 0, 0);
+                        if (BIAS) {
+                            v.x = (int)__vadd4((uint32_t)v.x, b4); v.y = (int)__vadd4((uint32_t)v.y, b4);
+                            v.z = (int)__vadd4((uint32_t)v.z, b4); v.w = (int)__vadd4((uint32_t)v.w, b4);
+                        }
+                        *reinterpret_cast<int4 *>(sl + a * LETTER + h * STRIP) = v;
+                    }
                 }
             }
             __syncwarp();
-            const int8_t *sl = SHARED ? wslice : myslice;
 
             /* initial state: column -1 */
             uint32_t H[P16_R], E[P16_R];
 #pragma unroll
             for (int r = 0; r < P16_R; ++r) {
-                const int la = p16_left(ALG, sgf, r0 + r, open, gap);
-                const int lb2 = p16_left(ALG, sgf, r0 + P16_R + r, open, gap);
+                const int la = p16_left(ALG, sgf, r0 + r, open, gap) - bias;
+                const int lb2 = p16_left(ALG, sgf, r0 + P16_R + r, open, gap) - bias;
                 H[r] = (uint32_t)(uint16_t)la | ((uint32_t)(uint16_t)lb2 << 16);
                 E[r] = NEG;
             }
-            uint32_t dg = (uint32_t)(uint16_t)p16_left(ALG, sgf, r0 - 1, open, gap);
-            uint32_t prev_h = (uint32_t)(uint16_t)p16_left(ALG, sgf, r0 + P16_R - 1, open, gap);
+            uint32_t dg = (uint32_t)(uint16_t)(p16_left(ALG, sgf, r0 - 1, open, gap) - bias);
+            uint32_t prev_h = (uint32_t)(uint16_t)(p16_left(ALG, sgf, r0 + P16_R - 1, open, gap) - bias);
             uint32_t prev_f = NEG & 0xffffu;
-            int top = p16_top(ALG, sgf, 0, open, gap);
-            const int top_step = (ALG == PB_SW || (ALG == PB_SG && (sgf & PB_S2_BEG))) ? 0 : gap;
+            /* the row above: row -1 (H by the boundary, F = -inf) in the first
+             * pass, else the previous pass's bottom row, loaded four columns
+             * ahead (this pass overwrites entry j at column j) */
+            const bool top = pass == 0;
+            uint32_t vtop = p16_prmt((uint32_t)(uint16_t)(p16_top(ALG, sgf, 0, open, gap) - bias), NEG, 0x5410u);
+            const uint32_t top_step = (ALG == PB_SW || (ALG == PB_SG && (sgf & PB_S2_BEG))) ? 0u
+                                                                                           : (uint32_t)(uint16_t)(-gap);
+            const uint32_t vnone = p16_prmt(0u, NEG, 0x5410u);
+            const int rd = top ? 0 : wmax;
+            uint32_t v_n[4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) v_n[x] = x < rd ? __ldcg(buf + (x + 1) * 32) : vnone;
+            const uint32_t *in_at = buf + 5 * 32;
+            uint32_t *out_at = buf;
             P16Best sa = {0, -1, -1}, sb = {0, -1, -1};
-            int cb = 0;
+            /* SW: what a column maximum has to pass, as in k_sw16 */
+            uint32_t sbest = p16_splat(max(best.score - 1, 0) - bias);
             const bool more = pass + 1 < npass;
             const bool lastpass = ENDS && ALG != PB_SW && pass == p_last;
-            const uint32_t vnone = p16_prmt(0u, NEG, 0x5410u);
-            auto code_at = [&](int j) -> int {
-                int c = j < cols ? tseq[j] : 0;
-                if (c >= L) { c = 0; status |= PB_ST_BADCODE; }
-                return c;
-            };
-            int c_n1 = code_at(0);
-            int c_n2 = code_at(1);
-            uint32_t v_n1 = vnone, v_n2 = vnone;
-            if (pass != 0) {
-                if (0 <= wmax) v_n1 = __ldcg(&buf[lane]);
-                if (1 <= wmax) v_n2 = __ldcg(&buf[32 + lane]);
-            }
-            /* unrolled by two: the prefetch registers then rotate by renaming
-             * instead of by moves, which would wait for the loads */
-#pragma unroll 2
-            for (int j = 0; j <= wmax; ++j) {
-                const int ca = c_n1;
-                c_n1 = c_n2;
-                c_n2 = code_at(j + 2);
-                uint32_t hu, fu;
-                if (pass == 0) {
-                    hu = p16_prmt((uint32_t)(uint16_t)top, prev_h, 0x5410u);
-                    fu = p16_prmt(NEG, prev_f, 0x5410u);
-                    top -= top_step;
-                } else {
-                    const uint32_t v = v_n1;
-                    v_n1 = v_n2;
-                    v_n2 = j + 2 <= wmax ? __ldcg(&buf[(size_t)(j + 2) * 32 + lane]) : vnone;
-                    hu = p16_prmt(v, prev_h, 0x5410u);       /* lo <- previous pass's strip B bottom */
-                    fu = p16_prmt(v, prev_f, 0x5432u);
-                }
-                const uint4 pa4 = *reinterpret_cast<const uint4 *>(sl + ca * P16_PASS);
-                const uint4 pb4 = *reinterpret_cast<const uint4 *>(sl + cb * P16_PASS + P16_R);
-                uint32_t hd = dg;
-                dg = hu;
-                uint32_t cmax = 0u;
-                uint32_t aD = 0u, aF = 0u, aE = 0u, aV = 0u;
-                uint32_t lastv = 0u;
+            const int8_t *pb_at = sl + STRIP;         /* strip B's scores of column j - 1 */
+            ResidueWords tw;
+            tw.start(tseq, cols);
+            for (int j0 = 0; j0 <= wmax; j0 += 4, in_at += 4 * 32, out_at += 4 * 32) {
+                uint32_t codes = tw.next(j0);
+                if ((codes | (codes + big4)) & 0x80808080u) {
+                    /* codes outside the alphabet read as letter 0 */
 #pragma unroll
-                for (int r = 0; r < P16_R; ++r) {
-                    const uint32_t wa = r < 4 ? pa4.x : r < 8 ? pa4.y : r < 12 ? pa4.z : pa4.w;
-                    const uint32_t wb = r < 4 ? pb4.x : r < 8 ? pb4.y : r < 12 ? pb4.z : pb4.w;
-                    uint32_t sc;
-                    switch (r & 3) {
-                        case 0: sc = p16_pair<0>(wa, wb); break;
-                        case 1: sc = p16_pair<1>(wa, wb); break;
-                        case 2: sc = p16_pair<2>(wa, wb); break;
-                        default: sc = p16_pair<3>(wa, wb); break;
-                    }
-                    uint32_t e, f, h;
-                    if (BITS) {
-                        const uint32_t ho = __vadd2(H[r], gO), ee = __vadd2(E[r], gE);
-                        e = __vmaxs2(ho, ee);
-                        const uint32_t fo = __vadd2(hu, gO), fe = __vadd2(fu, gE);
-                        f = __vmaxs2(fo, fe);
-                        const uint32_t hdg = __vadd2(hd, sc);
-                        h = ALG == PB_SW ? __vimax3_s16x2_relu(hdg, e, f) : __vimax3_s16x2(hdg, e, f);
-                        /* decision bits: sign of the difference of each half */
-                        aD = (aD >> 1) | (__vsub2(hdg, h) & 0x80008000u);
-                        aF = (aF >> 1) | (__vsub2(f, h) & 0x80008000u);
-                        aE = (aE >> 1) | (__vsub2(ee, ho) & 0x80008000u);
-                        aV = (aV >> 1) | (__vsub2(fe, fo) & 0x80008000u);
-                    } else {
-                        e = __viaddmax_s16x2(E[r], gE, __vadd2(H[r], gO));
-                        f = __viaddmax_s16x2(hu, gO, __vadd2(fu, gE));
-                        if (ALG == PB_SW) h = __vmaxs2(__viaddmax_s16x2_relu(hd, sc, e), f);
-                        else h = __vmaxs2(__viaddmax_s16x2(hd, sc, e), f);
-                    }
-                    E[r] = e;
-                    hd = H[r];
-                    H[r] = h;
-                    hu = h;
-                    fu = f;
-                    if (ENDS && ALG == PB_SW && (r & 1)) cmax = __vimax3_s16x2(cmax, H[r - 1], h);
-                    if (lastpass && (sgf & PB_S2_END) && r == r_last) lastv = h;
+                    for (int b = 0; b < 4; ++b)
+                        if (((codes >> (8 * b)) & 0xffu) >= (uint32_t)L) {
+                            codes &= ~(0xffu << (8 * b));
+                            status |= PB_ST_BADCODE;
+                        }
                 }
-                if (BITS) tbits[((size_t)pass * (wmax + 1) + j) * 32 + lane] = make_uint4(aD, aF, aE, aV);
-                if (j >= 1 && more) buf[(size_t)(j - 1) * 32 + lane] = p16_prmt(hu, fu, 0x7632u);
-                prev_h = hu;
-                prev_f = fu;
-                cb = ca;
-                if (j == 0) {
-                    /* the high half computed column -1: restore strip B's
-                     * left boundary (H(i,-1), E = -inf) */
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int j = j0 + u;
+                    const uint32_t v = top ? vtop : v_n[u];
+                    vtop = __vadd2(vtop, top_step);
+                    v_n[u] = j + 4 < rd ? __ldcg(in_at + u * 32) : vnone;
+                    uint32_t hu = p16_prmt(v, prev_h, 0x5410u);      /* lo <- the row above */
+                    uint32_t fu = p16_prmt(v, prev_f, 0x5432u);
+                    const int8_t *pa_at = sl + ((codes >> (8 * u)) & 0xffu) * LETTER;
+                    const uint4 pa4 = *reinterpret_cast<const uint4 *>(pa_at);
+                    const uint4 pb4 = *reinterpret_cast<const uint4 *>(pb_at);
+                    pb_at = pa_at + STRIP;
+                    uint32_t hd = dg;
+                    dg = hu;
+                    uint32_t cmax = p16_splat(-bias);
+                    uint32_t aop = 0u;               /* BIAS: the previous row's max(H_diag + s, E) - open */
+                    uint32_t aD = 0u, aF = 0u, aE = 0u, aV = 0u;
+                    uint32_t dD = 0u, dF = 0u, dE = 0u, dV = 0u;
 #pragma unroll
                     for (int r = 0; r < P16_R; ++r) {
-                        const int lb2 = p16_left(ALG, sgf, r0 + P16_R + r, open, gap);
-                        H[r] = (H[r] & 0xffffu) | ((uint32_t)(uint16_t)lb2 << 16);
-                        E[r] = (E[r] & 0xffffu) | (NEG & 0xffff0000u);
+                        const uint32_t wa = r < 4 ? pa4.x : r < 8 ? pa4.y : r < 12 ? pa4.z : pa4.w;
+                        const uint32_t wb = r < 4 ? pb4.x : r < 8 ? pb4.y : r < 12 ? pb4.z : pb4.w;
+                        uint32_t sc;
+                        switch (r & 3) {
+                            case 0: sc = p16_pair<0>(wa, wb); break;
+                            case 1: sc = p16_pair<1>(wa, wb); break;
+                            case 2: sc = p16_pair<2>(wa, wb); break;
+                            default: sc = p16_pair<3>(wa, wb); break;
+                        }
+                        uint32_t e, f, hn;           /* hn: H, or H - open */
+                        if (BITS) {
+                            const uint32_t ho = BIAS ? H[r] : __vadd2(H[r], gO);
+                            const uint32_t fo = BIAS ? hu : __vadd2(hu, gO);
+                            const uint32_t ee = __vadd2(E[r], gE), fe = __vadd2(fu, gE);
+                            e = __vmaxs2(ho, ee);
+                            f = __vmaxs2(fo, fe);
+                            const uint32_t hdg = __vadd2(hd, sc);
+                            const uint32_t h = ALG == PB_SW ? __vimax3_s16x2_relu(hdg, e, f) : __vimax3_s16x2(hdg, e, f);
+                            hn = BIAS ? __vadd2(h, gO) : h;
+                            /* the decisions of this row; of two rows, their signs
+                             * as four bytes: strips A and B of the even row, then
+                             * of the odd one; bit r / 2 of each byte is kept */
+                            const uint32_t nD = __vsub2(hdg, h), nF = __vsub2(f, h);
+                            const uint32_t nE = __vsub2(ee, ho), nV = __vsub2(fe, fo);
+                            if (r & 1) {
+                                const uint32_t m = 0x01010101u << (r >> 1);
+                                aD |= p16_prmt(dD, nD, 0xfdb9u) & m;
+                                aF |= p16_prmt(dF, nF, 0xfdb9u) & m;
+                                aE |= p16_prmt(dE, nE, 0xfdb9u) & m;
+                                aV |= p16_prmt(dV, nV, 0xfdb9u) & m;
+                            }
+                            dD = nD; dF = nF; dE = nE; dV = nV;
+                        } else if (BIAS) {
+                            e = __viaddmax_s16x2(E[r], gE, H[r]);
+                            const uint32_t a = ALG == PB_SW ? __viaddmax_s16x2_relu(hd, sc, e) : __viaddmax_s16x2(hd, sc, e);
+                            const uint32_t ao = __vadd2(a, gO);
+                            f = __viaddmax_s16x2(fu, gE, r == 0 ? hu : aop);
+                            hn = __viaddmax_s16x2(f, gO, ao);
+                            aop = ao;
+                        } else {
+                            e = __viaddmax_s16x2(E[r], gE, __vadd2(H[r], gO));
+                            f = __viaddmax_s16x2(hu, gO, __vadd2(fu, gE));
+                            hn = __vmaxs2(ALG == PB_SW ? __viaddmax_s16x2_relu(hd, sc, e)
+                                                       : __viaddmax_s16x2(hd, sc, e), f);
+                        }
+                        E[r] = e;
+                        hd = H[r];
+                        H[r] = hn;
+                        hu = hn;
+                        fu = f;
+                        if (ENDS && ALG == PB_SW && (r & 1)) cmax = __vimax3_s16x2(cmax, H[r - 1], hn);
                     }
-                }
-                if (ENDS && ALG == PB_SW) {
-                    /* a strictly higher column maximum than the strip's best
-                     * so far: the first column reaching it, kept whole (the
-                     * warp takes this branch whenever any lane improves; the
-                     * smallest row is looked up once per pass) */
-                    const int c_lo = p16_lo(cmax), c_hi = p16_hi(cmax);
-                    if (c_lo > sa.score && j < cols) {
-#pragma unroll
-                        for (int k = 0; k < P16_R / 4; ++k)
-                            save[k] = make_uint4(H[4 * k], H[4 * k + 1], H[4 * k + 2], H[4 * k + 3]);
-                        sa.score = c_lo; sa.j = j;
-                    }
-                    if (c_hi > sb.score && j >= 1 && j <= cols) {
-#pragma unroll
-                        for (int k = 0; k < P16_R / 4; ++k)
-                            save[P16_R / 4 + k] = make_uint4(H[4 * k], H[4 * k + 1], H[4 * k + 2], H[4 * k + 3]);
-                        sb.score = c_hi; sb.j = j - 1;
-                    }
-                }
-                if (ENDS && ALG != PB_SW) {
-                    /* last column (strip A at j = cols - 1, strip B one
-                     * iteration later): SG's last-column maximum over rows
-                     * below rows - 1 (smallest row on ties), and the corner */
-                    if (j == cols - 1 || j == cols) {
-                        const int hsel = j == cols - 1 ? 0 : 1;
-                        const int ib = r0 + hsel * P16_R;
+                    if (BITS) tbits[((size_t)pass * p16_cols(wmax) + j) * 32] = make_uint4(aD, aF, aE, aV);
+                    if (more) out_at[u * 32] = p16_prmt(hu, fu, 0x7632u);     /* column j - 1 */
+                    prev_h = hu;
+                    prev_f = fu;
+                    if (u == 0 && j0 == 0) {
+                        /* the high half computed column -1: restore strip B's
+                         * left boundary (H(i,-1), E = -inf) */
 #pragma unroll
                         for (int r = 0; r < P16_R; ++r) {
-                            const int v = hsel ? p16_hi(H[r]) : p16_lo(H[r]);
-                            const int i = ib + r;
-                            if (ALG == PB_SG && (sgf & PB_S1_END) && i < ilast && v > lc_h) { lc_h = v; lc_i = i; }
-                            if (i == ilast) corner = v;
+                            const int lb2 = p16_left(ALG, sgf, r0 + P16_R + r, open, gap) - bias;
+                            H[r] = (H[r] & 0xffffu) | ((uint32_t)(uint16_t)lb2 << 16);
+                            E[r] = (E[r] & 0xffffu) | (NEG & 0xffff0000u);
                         }
                     }
-                    if (lastpass && (sgf & PB_S2_END)) {
-                        const int jj = j - half_last;
-                        const int v = half_last ? p16_hi(lastv) : p16_lo(lastv);
-                        if (jj >= 0 && jj < cols && v > lr_h) { lr_h = v; lr_j = jj; }
+                    if (ENDS && ALG == PB_SW && __vmaxs2(sbest, cmax) != sbest) {
+                        /* past its half's bound: the column kept whole (the
+                         * smallest row is looked up once per pass); columns
+                         * outside the target only raise the bound */
+                        const int c_lo = p16_lo(cmax), c_hi = p16_hi(cmax);
+                        int ba = p16_lo(sbest), bb = p16_hi(sbest);
+                        const bool up_a = c_lo > ba, up_b = c_hi > bb && j >= 1;
+                        if (up_a) {
+                            ba = c_lo;
+                            if (j < cols) {
+#pragma unroll
+                                for (int x = 0; x < P16_R / 4; ++x)
+                                    save[x] = make_uint4(H[4 * x], H[4 * x + 1], H[4 * x + 2], H[4 * x + 3]);
+                                sa.score = c_lo + bias; sa.j = j;
+                                bb = max(bb, c_lo - 1);
+                            }
+                        }
+                        if (up_b) {
+                            bb = max(bb, c_hi);
+                            if (j <= cols) {
+#pragma unroll
+                                for (int x = 0; x < P16_R / 4; ++x)
+                                    save[P16_R / 4 + x] = make_uint4(H[4 * x], H[4 * x + 1], H[4 * x + 2], H[4 * x + 3]);
+                                sb.score = c_hi + bias; sb.j = j - 1;
+                                ba = max(ba, c_hi - 1);
+                            }
+                        }
+                        sbest = (uint32_t)(uint16_t)ba | ((uint32_t)(uint16_t)bb << 16);
+                    }
+                    if (ENDS && ALG != PB_SW) {
+                        /* last column (strip A at j = cols - 1, strip B one
+                         * iteration later): SG's last-column maximum over rows
+                         * below rows - 1 (smallest row on ties), and the corner */
+                        if ((unsigned)(j - (cols - 1)) <= 1u && (ALG == PB_SG || lastpass)) {
+                            const int hsel = j == cols - 1 ? 0 : 1;
+                            const int ib = r0 + hsel * P16_R;
+#pragma unroll
+                            for (int r = 0; r < P16_R; ++r) {
+                                const int hv = (hsel ? p16_hi(H[r]) : p16_lo(H[r])) + bias;
+                                const int i = ib + r;
+                                if (ALG == PB_SG && (sgf & PB_S1_END) && i < ilast && hv > lc_h) { lc_h = hv; lc_i = i; }
+                                if (i == ilast) corner = hv;
+                            }
+                        }
+                        if (ALG == PB_SG && (sgf & PB_S2_END) && lastpass) {
+                            const int jj = j - half_last;
+                            uint32_t lastv = 0u;
+#pragma unroll
+                            for (int r = 0; r < P16_R; ++r) if (r == r_last) lastv = H[r];
+                            const int hv = (half_last ? p16_hi(lastv) : p16_lo(lastv)) + bias;
+                            if (jj >= 0 && jj < cols && hv > lr_h) { lr_h = hv; lr_j = jj; }
+                        }
                     }
                 }
             }
@@ -440,22 +513,22 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
                 if (sa.j >= 0) {
                     int rr = P16_R - 1;
 #pragma unroll
-                    for (int k = P16_R / 4 - 1; k >= 0; --k) {
-                        const uint4 w = save[k];
+                    for (int x = P16_R / 4 - 1; x >= 0; --x) {
+                        const uint4 w = save[x];
                         const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-                        for (int x = 3; x >= 0; --x) if (p16_lo(ws[x]) == sa.score) rr = 4 * k + x;
+                        for (int y = 3; y >= 0; --y) if (p16_lo(ws[y]) == sa.score - bias) rr = 4 * x + y;
                     }
                     sa.i = r0 + rr;
                 }
                 if (sb.j >= 0) {
                     int rr = P16_R - 1;
 #pragma unroll
-                    for (int k = P16_R / 4 - 1; k >= 0; --k) {
-                        const uint4 w = save[P16_R / 4 + k];
+                    for (int x = P16_R / 4 - 1; x >= 0; --x) {
+                        const uint4 w = save[P16_R / 4 + x];
                         const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-                        for (int x = 3; x >= 0; --x) if (p16_hi(ws[x]) == sb.score) rr = 4 * k + x;
+                        for (int y = 3; y >= 0; --y) if (p16_hi(ws[y]) == sb.score - bias) rr = 4 * x + y;
                     }
                     sb.i = r0 + P16_R + rr;
                 }
@@ -463,10 +536,7 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
                     const P16Best c = cand[x];
-                    if (c.j >= 0 && (!have || c.score > best.score || (c.score == best.score && c.j < best.j))) {
-                        best = c;
-                        have = true;
-                    }
+                    if (c.j >= 0 && (c.score > best.score || (c.score == best.score && c.j < best.j))) best = c;
                 }
             }
         }
@@ -475,7 +545,7 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
             if (ENDS) {
                 int sc, eq, er;
                 if (ALG == PB_SW) {
-                    sc = have ? best.score : 0; eq = have ? best.i : 0; er = have ? best.j : 0;
+                    sc = best.score; eq = best.i; er = best.j;
                 } else if (ALG == PB_NW) {
                     sc = corner; eq = ilast; er = cols - 1;
                 } else {
@@ -562,8 +632,8 @@ __global__ void k_p16_walk(P16Params p, const int *__restrict__ tlist, int ntl, 
     for (int step = 0; step <= 2 * limit; ++step) {
         if (i < 0 || j < 0) break;
         if (ALG == PB_SW && state == 0 && v <= 0) break;
-        const int half = (i >> 4) & 1, bit = half * 16 + (i & 15);
-        const uint4 w = tb[((size_t)(i >> 5) * (wmax + 1) + j + half) * 32 + lane];
+        const int half = (i >> 4) & 1, bit = p16_bit(i);
+        const uint4 w = tb[((size_t)(i >> 5) * p16_cols(wmax) + j + half) * 32 + lane];
         if (state == 0) {
             if (!((w.x >> bit) & 1u)) {
                 int qc = qseq[i], tc = tseq[j];
@@ -647,8 +717,8 @@ __global__ void k_p16_path(P16Params p, const int *__restrict__ tlist, int ntl, 
     for (int step = 0; step <= 2 * cap + 2 && n < cap; ++step) {
         if (i < 0 || j < 0) break;
         if (ALG == PB_SW && state == 0 && v <= 0) break;
-        const int half = (i >> 4) & 1, bit = half * 16 + (i & 15);
-        const uint4 w = tb[((size_t)(i >> 5) * (wmax + 1) + j + half) * 32 + lane];
+        const int half = (i >> 4) & 1, bit = p16_bit(i);
+        const uint4 w = tb[((size_t)(i >> 5) * p16_cols(wmax) + j + half) * 32 + lane];
         if (state == 0) {
             if (!((w.x >> bit) & 1u)) {
                 int qc = qseq[i], tc = tseq[j];
@@ -733,7 +803,7 @@ __global__ void k_p16_tasks(P16Params p, int ntasks, const int *__restrict__ gro
         twmax[task] = c;
         tnpass[task] = np;
         tshared[task] = p.mat8 ? (same && group != nullptr) : 1;
-        tbits[task] = bits ? (long long)np * (c + 1) * 32 : 0;
+        tbits[task] = bits ? (long long)np * p16_cols(c) * 32 : 0;
     }
 }
 
@@ -855,27 +925,29 @@ int p16_warps(bool shared, int L) { return shared || L <= 8 ? 8 : 4; }
 size_t p16_smem(bool shared, int L, bool mat)
 {
     const size_t mat_bytes = mat ? ((size_t)(L * L + 15) & ~(size_t)15) : 0;
-    const size_t warp_bytes = shared ? (size_t)L * P16_PASS : 32 * ((size_t)L * P16_PASS + 16);
+    const size_t warp_bytes = (size_t)L * (shared ? P16_ROW : 32 * P16_PASS);
     return mat_bytes + warp_bytes * p16_warps(shared, L);
 }
 
 typedef void (*p16_kernel_t)(P16Params, const int *, int, int *);
 
-template <int ALG, bool BITS, bool ENDS>
+template <int ALG, bool BITS, bool ENDS, bool BIAS>
 p16_kernel_t pick3(bool shared, int warps)
 {
-    if (shared) return k_p16<ALG, BITS, ENDS, true, 8>;
-    return warps == 8 ? k_p16<ALG, BITS, ENDS, false, 8> : k_p16<ALG, BITS, ENDS, false, 4>;
+    if (shared) return k_p16<ALG, BITS, ENDS, true, 8, BIAS>;
+    return warps == 8 ? k_p16<ALG, BITS, ENDS, false, 8, BIAS> : k_p16<ALG, BITS, ENDS, false, 4, BIAS>;
 }
 
+template <bool BIAS>
 p16_kernel_t pick(int alg, bool bits, bool ends, bool shared, int warps)
 {
     if (alg == PB_SW) {
-        if (!ends) return pick3<PB_SW, true, false>(shared, warps);
-        return bits ? pick3<PB_SW, true, true>(shared, warps) : pick3<PB_SW, false, true>(shared, warps);
+        if (!ends) return pick3<PB_SW, true, false, BIAS>(shared, warps);
+        return bits ? pick3<PB_SW, true, true, BIAS>(shared, warps) : pick3<PB_SW, false, true, BIAS>(shared, warps);
     }
-    if (alg == PB_NW) return bits ? pick3<PB_NW, true, true>(shared, warps) : pick3<PB_NW, false, true>(shared, warps);
-    return bits ? pick3<PB_SG, true, true>(shared, warps) : pick3<PB_SG, false, true>(shared, warps);
+    if (alg == PB_NW)
+        return bits ? pick3<PB_NW, true, true, BIAS>(shared, warps) : pick3<PB_NW, false, true, BIAS>(shared, warps);
+    return bits ? pick3<PB_SG, true, true, BIAS>(shared, warps) : pick3<PB_SG, false, true, BIAS>(shared, warps);
 }
 
 }  // namespace
@@ -1071,13 +1143,15 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
         int dev = 0, nsm = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+        const bool bias = m->open >= m->gap && mmax + m->open <= 127 && mmin + m->open >= -128;
         int grid[2] = {0, 0}, warps[2] = {0, 0};
         size_t smem[2] = {0, 0};
         p16_kernel_t kern[2];
         for (int sh = 0; sh < 2; ++sh) {
             warps[sh] = p16_warps(sh == 1, L);
             smem[sh] = p16_smem(sh == 1, L, d_mat8 != nullptr);
-            kern[sh] = pick(m->alg, bits, ends_on, sh == 1, warps[sh]);
+            kern[sh] = bias ? pick<true>(m->alg, bits, ends_on, sh == 1, warps[sh])
+                            : pick<false>(m->alg, bits, ends_on, sh == 1, warps[sh]);
             int per_sm = 0;
             pb_raise_smem((const void *)kern[sh], (int)smem[sh]);
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern[sh], warps[sh] * 32, smem[sh]);
@@ -1085,7 +1159,7 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
         }
         const size_t rwarps = (size_t)std::max(grid[0] * warps[0], grid[1] * warps[1]);
         uint32_t *scratch = nullptr;
-        P16_CK(cudaMallocAsync((void **)&scratch, sizeof(uint32_t) * (size_t)(maxlen + 1) * 32 * rwarps, st));
+        P16_CK(cudaMallocAsync((void **)&scratch, sizeof(uint32_t) * (size_t)(maxlen + 8) * 32 * rwarps, st));
         frees.add(scratch);
         p.scratch = scratch;
         p.colsave = nullptr;

@@ -78,40 +78,6 @@ struct Sw16Best {
     int score, i, j;
 };
 
-/* A lane's target residues, four columns at a time. One byte load per
- * column and lane touches 32 different lines; here the lane reads the
- * aligned 32-bit words that hold its residues, two words ahead, and shifts
- * them together. Only words that hold at least one byte of the sequence
- * are read; columns past its end are letter 0. */
-struct ResidueWords {
-    const uint32_t *w;
-    int shift, last, len;
-    uint32_t a, b, c;        /* words k, k + 1, k + 2 of the next four columns */
-    __device__ __forceinline__ uint32_t word(int k) const { return k <= last ? __ldg(w + k) : 0u; }
-    __device__ __forceinline__ void start(const uint8_t *seq, int n)
-    {
-        const uintptr_t p = reinterpret_cast<uintptr_t>(seq);
-        w = reinterpret_cast<const uint32_t *>(p & ~(uintptr_t)3);
-        shift = (int)(p & 3) * 8;
-        len = n;
-        last = n > 0 ? ((int)(p & 3) + n - 1) >> 2 : -1;
-        a = word(0);
-        b = word(1);
-        c = word(2);
-    }
-    /* the residues of columns j .. j + 3 (j a multiple of 4), one per byte */
-    __device__ __forceinline__ uint32_t next(int j)
-    {
-        uint32_t v = __funnelshift_r(a, b, shift);
-        const int left = len - j;
-        if (left < 4) v = left <= 0 ? 0u : v & (0xffffffffu >> (32 - 8 * left));
-        a = b;
-        b = c;
-        c = word((j >> 2) + 3);
-        return v;
-    }
-};
-
 /* higher score, then smaller column; an equal column keeps the earlier
  * (smaller) row, which was folded first (scores are positive, a best of 0
  * is none) */
