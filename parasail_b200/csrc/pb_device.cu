@@ -615,8 +615,9 @@ char *pb_single_arena(size_t bytes, size_t host_bytes, char **host)
     return g_single.d;
 }
 
-/* One pair on the exact kernel from host target codes: the warp kernel for a
- * pair of 32 rows or more (or of 8 rows and 2^14 cells), else one thread.
+/* One pair on the exact kernel from host target codes: on one block, or, where
+ * it does not fit one, the warp kernel for a pair of 32 rows or more (or of 8
+ * rows and 2^14 cells), else one thread.
  * qlim/tlim > 0 limit the pair to a prefix (the FASTSTATS pass). */
 int pb_cuda_exact_single(const pb_batch *tmpl, const uint8_t *h_codes, int tlen, int qlim, int tlim,
                          pb_pair_out *h_out)
@@ -661,8 +662,10 @@ int pb_cuda_exact_single(const pb_batch *tmpl, const uint8_t *h_codes, int tlen,
     p.nt = 0;
     p.scan_vgap = tmpl->scan_vgap;
     const long long cells = (long long)ql * tl;
-    if (ql >= 32 || (ql >= 8 && cells >= (1LL << 14))) pb::launch_exact_warp(p, tmpl->alg, tmpl->stats != 0, 1, st);
-    else pb::launch_exact(p, tmpl->alg, tmpl->stats != 0, st);
+    if (!pb::launch_exact_block(p, tmpl->alg, tmpl->stats != 0, dp, ql, tl, st)) {
+        if (ql >= 32 || (ql >= 8 && cells >= (1LL << 14))) pb::launch_exact_warp(p, tmpl->alg, tmpl->stats != 0, 1, st);
+        else pb::launch_exact(p, tmpl->alg, tmpl->stats != 0, st);
+    }
     pb_diag_count_launch(1);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(h_out, d + o_out, sizeof(pb_pair_out), cudaMemcpyDeviceToHost, st));

@@ -50,6 +50,35 @@ __device__ __forceinline__ EwCell ew_shfl(const EwCell &c, int src)
                   __shfl_sync(0xffffffffu, c.s, src), __shfl_sync(0xffffffffu, c.l, src)};
 }
 
+/* the end rules: SW's best, the NW corner, SG's by src/sg.c:160-242 */
+template <int ALG>
+__device__ __forceinline__ void ew_ends(const EwCell &best, int best_i, int best_j, const EwCell &lc, int lc_i,
+                                        const EwCell &lr, int lr_j, const EwCell &corner, int ql, int tl, int sgf,
+                                        EwCell *out, int *out_q, int *out_r)
+{
+    EwCell res;
+    int eq, er;
+    if (ALG == PB_SW) {
+        res = best; eq = best_i; er = best_j;
+    } else if (ALG == PB_NW) {
+        res = corner; eq = ql - 1; er = tl - 1;
+    } else {
+        const bool s1e = sgf & PB_S1_END, s2e = sgf & PB_S2_END;
+        res = EwCell{NEG_INF, 0, 0, 0};
+        eq = ql; er = tl;
+        if (s1e && lc_i >= 0) { res = lc; eq = lc_i; er = tl - 1; }
+        if (s1e && s2e) {
+            if (lr.h > res.h || (lr.h == res.h && lr_j < er)) { res = lr; eq = ql - 1; er = lr_j; }
+        } else if (s2e) {
+            if (lr.h > res.h) { res = lr; eq = ql - 1; er = lr_j; }
+        }
+        if ((s1e && corner.h > res.h) || (!s1e && !s2e)) { res = corner; eq = ql - 1; er = tl - 1; }
+    }
+    *out = res;
+    *out_q = eq;
+    *out_r = er;
+}
+
 /* PAIRS: pair k has its own query codes (qall + qoff[k], qlen[k]) scored
  * through the square matrix mat[target letter * msize + query letter];
  * else profiles: every query of profs against the same nt targets, or
@@ -290,23 +319,7 @@ k_exact_warp(ExactParams p, int nitems)
 
     EwCell res;
     int eq, er;
-    if (ALG == PB_SW) {
-        res = best; eq = best_i; er = best_j;
-    } else if (ALG == PB_NW) {
-        res = corner; eq = ql - 1; er = tl - 1;
-    } else {
-        /* src/sg.c:160-242 */
-        const bool s1e = sgf & PB_S1_END, s2e = sgf & PB_S2_END;
-        res = EwCell{NEG_INF, 0, 0, 0};
-        eq = ql; er = tl;
-        if (s1e && lc_i >= 0) { res = lc; eq = lc_i; er = tl - 1; }
-        if (s1e && s2e) {
-            if (lr.h > res.h || (lr.h == res.h && lr_j < er)) { res = lr; eq = ql - 1; er = lr_j; }
-        } else if (s2e) {
-            if (lr.h > res.h) { res = lr; eq = ql - 1; er = lr_j; }
-        }
-        if ((s1e && corner.h > res.h) || (!s1e && !s2e)) { res = corner; eq = ql - 1; er = tl - 1; }
-    }
+    ew_ends<ALG>(best, best_i, best_j, lc, lc_i, lr, lr_j, corner, ql, tl, sgf, &res, &eq, &er);
     pb_pair_out o;
     o.score = res.h; o.end_query = eq; o.end_ref = er;
     o.matches = res.m; o.similar = res.s; o.length = res.l;
@@ -317,6 +330,294 @@ k_exact_warp(ExactParams p, int nitems)
     o.min_f_pad[0] = min_f_pad0; o.min_f_pad[1] = min_f_pad1; o.min_f_pad[2] = min_f_pad2;
     o.status = status;
     p.out[pid] = o;
+}
+
+/*
+ * One pair on one block: the latency path of the single calls. Thread g of
+ * the block holds rows g * R .. g * R + R - 1 and computes column t - g at
+ * iteration t, so the whole query is one pass (the warp kernel above runs
+ * 512 or 256 rows a pass on one warp, 16 or 8 rows deep per iteration: 3,100
+ * cycles per column of 300 rows with statistics). The row above comes from
+ * the lane before by shuffle; the last lane of a warp leaves it in shared
+ * memory for the next warp, double-buffered, with one barrier per iteration.
+ * Bound by the latency of an iteration (shuffles, barrier, R rows), so R is
+ * the smallest that keeps the block at 512 threads, matches and similar
+ * share a word (rows + columns below 65,536), the scores are int8 in shared
+ * memory, loaded one column ahead, and the extremes are kept per row and
+ * sorted into the row regions once, at the end. One sg_qx statistics pair of
+ * 300 x 332: 1,174 -> 233 us per call.
+ * Every cell and end rule is k_exact_warp's (without SCANF).
+ */
+static constexpr int EB_THREADS = 512;
+
+/* a column's bottom row handed to the next warp: H, F, then with statistics
+ * their (matches | similar << 16) and length */
+struct EbRow { int h, f; uint32_t hms, fms; int hl, fl; };
+
+template <int ALG, bool STATS, int R>
+__global__ void __launch_bounds__(EB_THREADS)
+k_exact_block(ExactParams p, int stride)
+{
+    extern __shared__ __align__(16) int8_t s_sc[];        /* [letter][stride] */
+    __shared__ EbRow s_row[2][EB_THREADS / 32];
+    __shared__ EwCell s_best[2][EB_THREADS / 32];          /* SW best, SG last column */
+    __shared__ int s_pos[3][EB_THREADS / 32], s_ext[13][EB_THREADS / 32], s_status[EB_THREADS / 32];
+    __shared__ EwCell s_corner, s_lr;
+    __shared__ int s_lrj;
+    const int g = threadIdx.x, lane = g & 31, warp = g >> 5;
+    const ProfDesc pd = p.profs[0];
+    const uint8_t *tseq = p.targets + p.toff[0];
+    const int ql = p.qlim ? p.qlim[0] : pd.qlen;
+    const int tl = p.tlim ? p.tlim[0] : p.tlen[0];
+    const int open = p.open, gap = p.gap, sgf = p.sgflags;
+    const int c8 = (ql + 7) & ~7, c16 = (ql + 15) & ~15, c32 = (ql + 31) & ~31;
+    const int nrows = p.pad_rows == 0 ? ql : (p.pad_rows == 8 ? c8 : (p.pad_rows == 16 ? c16 : c32));
+    /* the scores of the query's rows; rows past it (padding) score 0 */
+    for (int a = warp; a < pd.size; a += blockDim.x >> 5)
+        for (int i = lane; i < stride; i += 32)
+            s_sc[a * stride + i] = i < ql ? pd.prof8[(size_t)a * pd.lp + i] : (int8_t)0;
+    __syncthreads();
+
+    const int i0 = g * R;
+    const bool mine = i0 < nrows;
+    int H[R], E[R], HL[R], EL[R], qc[R], min_h[R], min_f[R], max_st[R], max_h = INT32_MIN;
+    uint32_t HMS[R], EMS[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        H[r] = left_h<ALG>(i0 + r, open, gap, sgf);
+        E[r] = NEG_INF;
+        HMS[r] = EMS[r] = 0u;
+        HL[r] = EL[r] = 0;
+        qc[r] = i0 + r < ql ? (int)pd.qcodes[i0 + r] : -1;
+        min_h[r] = min_f[r] = INT32_MAX;
+        max_st[r] = INT32_MIN;
+    }
+    int dg = i0 == 0 ? 0 : left_h<ALG>(i0 - 1, open, gap, sgf);
+    uint32_t dgMS = 0u;
+    int dgL = 0;
+    EbRow sh = {NEG_INF, NEG_INF, 0u, 0u, 0, 0};
+    EwCell best = {NEG_INF, 0, 0, 0}, lc = {NEG_INF, 0, 0, 0}, lr = {NEG_INF, 0, 0, 0}, corner = {0, 0, 0, 0};
+    int best_i = ql, best_j = tl, lc_i = -1, lr_j = -1, status = 0;
+    /* the code two columns ahead, the scores one column ahead */
+    auto code_at = [&](int j) -> int { return mine && j >= 0 && j < tl ? (int)tseq[j] : 0; };
+    int c_cur = code_at(-g), c_nxt = code_at(1 - g);
+    int sc_nxt[R];
+    auto scores = [&](int code) {
+        const int cs = code < pd.size ? code : 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) sc_nxt[r] = mine ? (int)s_sc[cs * stride + i0 + r] : 0;
+    };
+    scores(c_cur);
+    const int iters = tl + (nrows + R - 1) / R - 1;
+    for (int it = 0; it < iters; ++it) {
+        const int j = it - g;
+        int sc[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) sc[r] = sc_nxt[r];
+        const int code = c_cur;
+        c_cur = c_nxt;
+        c_nxt = code_at(j + 2);
+        scores(c_cur);
+        EbRow up;
+        up.h = __shfl_up_sync(0xffffffffu, sh.h, 1);
+        up.f = __shfl_up_sync(0xffffffffu, sh.f, 1);
+        if (STATS) {
+            up.hms = __shfl_up_sync(0xffffffffu, sh.hms, 1);
+            up.fms = __shfl_up_sync(0xffffffffu, sh.fms, 1);
+            up.hl = __shfl_up_sync(0xffffffffu, sh.hl, 1);
+            up.fl = __shfl_up_sync(0xffffffffu, sh.fl, 1);
+        }
+        if (lane == 0 && warp > 0) up = s_row[(it + 1) & 1][warp - 1];
+        if (mine && j >= 0 && j < tl) {
+            if (g == 0) {
+                up.h = top_h<ALG>(j, open, gap, sgf); up.f = NEG_INF;
+                up.hms = up.fms = 0u; up.hl = up.fl = 0;
+            }
+            if (code >= pd.size) status |= PB_ST_BADCODE;
+            int hd = dg, hdL = dgL;
+            uint32_t hdMS = dgMS;
+            dg = up.h;
+            if (STATS) { dgMS = up.hms; dgL = up.hl; }
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int i = i0 + r;
+                const int f_opn = up.h - open, f_ext = up.f - gap;
+                const int fn = max(f_opn, f_ext);
+                const int e_opn = H[r] - open, e_ext = E[r] - gap;
+                const int en = max(e_opn, e_ext);
+                const int hdag = hd + sc[r];
+                const int gp = max(en, fn);
+                const int h0 = max(hdag, gp);
+                /* SW: max(h0, 0) */
+                const int hn = ALG == PB_SW ? h0 & ~(h0 >> 31) : h0;
+                uint32_t hMS = 0u, fMS = 0u;
+                int hL = 0, fL = 0;
+                if (STATS) {
+                    /* gap-source choice by strict >, then cell choice diagonal
+                     * > F > E, SW resets at H <= 0 (src/sw_stats.c:205-237) */
+                    const bool fo = f_opn > f_ext;
+                    fMS = fo ? up.hms : up.fms;
+                    fL = (fo ? up.hl : up.fl) + 1;
+                    const bool eo = e_opn > e_ext;
+                    const uint32_t eMS = eo ? HMS[r] : EMS[r];
+                    const int eL = (eo ? HL[r] : EL[r]) + 1;
+                    EMS[r] = eMS; EL[r] = eL;
+                    /* the choices from the operands: a maximum compared with
+                     * its own operand lost resets in this kernel's SW form
+                     * (right scores, counts that no path gives) */
+                    const bool isd = (int)((unsigned)hdag - (unsigned)gp) >= 0;
+                    const bool isf = (int)((unsigned)fn - (unsigned)en) >= 0;
+                    const uint32_t dMS = hdMS + (qc[r] == code ? 1u : 0u) + (sc[r] > 0 ? 0x10000u : 0u);
+                    hMS = isd ? dMS : (isf ? fMS : eMS);
+                    hL = isd ? hdL + 1 : (isf ? fL : eL);
+                    if (ALG == PB_SW && h0 <= 0) { hMS = 0u; hL = 0; }
+                }
+                E[r] = en;
+                if (i < nrows) {
+                    max_h = max(max_h, hn);
+                    min_h[r] = min(min_h[r], hn);
+                    min_f[r] = min(min_f[r], fn);
+                    if (STATS) max_st[r] = max(max_st[r], hL);
+                }
+                if (i < ql) {
+                    if (ALG == PB_SW) {
+                        if (hn > best.h) {
+                            best = EwCell{hn, (int)(hMS & 0xffffu), (int)(hMS >> 16), hL};
+                            best_i = i; best_j = j;
+                        }
+                    } else if (i == ql - 1) {
+                        const EwCell c = {hn, (int)(hMS & 0xffffu), (int)(hMS >> 16), hL};
+                        if (hn > lr.h) { lr = c; lr_j = j; }
+                        if (j == tl - 1) corner = c;
+                    } else if (ALG == PB_SG && j == tl - 1) {
+                        if (hn > lc.h) { lc = EwCell{hn, (int)(hMS & 0xffffu), (int)(hMS >> 16), hL}; lc_i = i; }
+                    }
+                }
+                hd = H[r];
+                H[r] = hn;
+                up.h = hn;
+                up.f = fn;
+                if (STATS) {
+                    hdMS = HMS[r]; hdL = HL[r];
+                    HMS[r] = hMS; HL[r] = hL;
+                    up.hms = hMS; up.hl = hL; up.fms = fMS; up.fl = fL;
+                }
+            }
+            sh = up;
+        }
+        if (lane == 31) s_row[it & 1][warp] = sh;
+        __syncthreads();
+    }
+
+    /* merge the lanes, then the warps */
+    int ext[13];         /* minima: real H, F, padded H x 3, F x 3; maxima: H, real statistic, padded x 3 */
+#pragma unroll
+    for (int x = 0; x < 13; ++x) ext[x] = x < 8 ? INT32_MAX : INT32_MIN;
+    ext[8] = max_h;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = i0 + r;
+        const int reg = i < ql ? 0 : i < c8 ? 1 : i < c16 ? 2 : 3;
+        if (i >= nrows) continue;
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+            if (reg == x) {
+                const int mh = x == 0 ? 0 : 1 + x, mf = x == 0 ? 1 : 4 + x;
+                ext[mh] = min(ext[mh], min_h[r]);
+                ext[mf] = min(ext[mf], min_f[r]);
+                ext[9 + x] = max(ext[9 + x], max_st[r]);
+            }
+    }
+#pragma unroll
+    for (int x = 0; x < 13; ++x)
+        ext[x] = x < 8 ? __reduce_min_sync(0xffffffffu, ext[x]) : __reduce_max_sync(0xffffffffu, ext[x]);
+    status = __reduce_or_sync(0xffffffffu, status);
+    for (int o = 16; o; o >>= 1) {
+        const EwCell bc = ew_shfl_xor(best, o);
+        const int bi = __shfl_xor_sync(0xffffffffu, best_i, o);
+        const int bj = __shfl_xor_sync(0xffffffffu, best_j, o);
+        if (ew_better(bc.h, bj, bi, best.h, best_j, best_i)) { best = bc; best_i = bi; best_j = bj; }
+        const EwCell cc = ew_shfl_xor(lc, o);
+        const int ci = __shfl_xor_sync(0xffffffffu, lc_i, o);
+        if (ci >= 0 && (lc_i < 0 || cc.h > lc.h || (cc.h == lc.h && ci < lc_i))) { lc = cc; lc_i = ci; }
+    }
+    if (mine && i0 <= ql - 1 && ql - 1 < i0 + R) { s_lr = lr; s_lrj = lr_j; s_corner = corner; }
+    if (lane == 0) {
+        s_best[0][warp] = best; s_best[1][warp] = lc;
+        s_pos[0][warp] = best_i; s_pos[1][warp] = best_j; s_pos[2][warp] = lc_i;
+        s_status[warp] = status;
+#pragma unroll
+        for (int x = 0; x < 13; ++x) s_ext[x][warp] = ext[x];
+    }
+    __syncthreads();
+    if (g != 0) return;
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
+        status |= s_status[w];
+#pragma unroll
+        for (int x = 0; x < 13; ++x) ext[x] = x < 8 ? min(ext[x], s_ext[x][w]) : max(ext[x], s_ext[x][w]);
+        const EwCell bc = s_best[0][w], cc = s_best[1][w];
+        if (ew_better(bc.h, s_pos[1][w], s_pos[0][w], best.h, best_j, best_i)) {
+            best = bc; best_i = s_pos[0][w]; best_j = s_pos[1][w];
+        }
+        const int ci = s_pos[2][w];
+        if (ci >= 0 && (lc_i < 0 || cc.h > lc.h || (cc.h == lc.h && ci < lc_i))) { lc = cc; lc_i = ci; }
+    }
+    lr = s_lr; lr_j = s_lrj; corner = s_corner;
+    EwCell res;
+    int eq, er;
+    ew_ends<ALG>(best, best_i, best_j, lc, lc_i, lr, lr_j, corner, ql, tl, sgf, &res, &eq, &er);
+    pb_pair_out o;
+    o.score = res.h; o.end_query = eq; o.end_ref = er;
+    o.matches = res.m; o.similar = res.s; o.length = res.l;
+    o.max_h = ext[8]; o.min_h_real = ext[0]; o.min_f_real = ext[1]; o.max_stat_real = ext[9];
+    for (int x = 0; x < 3; ++x) {
+        o.min_h_pad[x] = ext[2 + x];
+        o.min_f_pad[x] = ext[5 + x];
+        o.max_stat_pad[x] = ext[10 + x];
+    }
+    o.status = status;
+    p.out[0] = o;
+}
+
+template <bool STATS, int R>
+static void launch_eb(const ExactParams &p, int alg, int threads, int smem, int stride, cudaStream_t st)
+{
+    if (alg == PB_SW) {
+        pb_raise_smem((const void *)k_exact_block<PB_SW, STATS, R>, smem);
+        k_exact_block<PB_SW, STATS, R><<<1, threads, smem, st>>>(p, stride);
+    } else if (alg == PB_NW) {
+        pb_raise_smem((const void *)k_exact_block<PB_NW, STATS, R>, smem);
+        k_exact_block<PB_NW, STATS, R><<<1, threads, smem, st>>>(p, stride);
+    } else {
+        pb_raise_smem((const void *)k_exact_block<PB_SG, STATS, R>, smem);
+        k_exact_block<PB_SG, STATS, R><<<1, threads, smem, st>>>(p, stride);
+    }
+}
+
+/* The pair of p (one profile, descriptors at index 0) on one block; rows:
+ * its query rows padded to 32, cols its columns, prof its profile on the
+ * host. false when it does not fit the block: more than 4 rows a thread,
+ * counts past 16 bits, scores past int8 or past shared memory, the serial
+ * scan forms. */
+bool launch_exact_block(const ExactParams &p, int alg, bool stats, const pb_device_profile *prof, int rows, int cols,
+                        cudaStream_t st)
+{
+    const int r32 = (rows + 31) & ~31;
+    if (p.scan_vgap || !prof->fits8 || !prof->d_prof8 || r32 > 4 * EB_THREADS || r32 + cols >= 65536) return false;
+    /* an odd number of words between letters */
+    const int stride = ((r32 + 4 + 3) / 4 | 1) * 4;
+    const size_t smem = (size_t)prof->size * stride;
+    if (smem > 160 * 1024) return false;
+    const int R = r32 <= 2 * EB_THREADS ? 2 : 4;
+    const int threads = ((r32 + R - 1) / R + 31) & ~31;
+    if (R == 2) {
+        if (stats) launch_eb<true, 2>(p, alg, threads, (int)smem, stride, st);
+        else launch_eb<false, 2>(p, alg, threads, (int)smem, stride, st);
+    } else {
+        if (stats) launch_eb<true, 4>(p, alg, threads, (int)smem, stride, st);
+        else launch_eb<false, 4>(p, alg, threads, (int)smem, stride, st);
+    }
+    return true;
 }
 
 template <bool STATS, bool PAIRS, bool SCANF = false>

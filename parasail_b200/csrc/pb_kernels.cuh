@@ -52,6 +52,9 @@ struct ExactParams {
 /* the exact kernel with one warp per pair (pb_exact_warp.cu): items
  * order[0..nitems) of p, which uses p.nt query-major pairs */
 void launch_exact_warp(const ExactParams &p, int alg, bool stats, int nitems, cudaStream_t st);
+/* one pair on one block (the single calls); false when it does not fit */
+bool launch_exact_block(const ExactParams &p, int alg, bool stats, const pb_device_profile *prof, int rows, int cols,
+                        cudaStream_t st);
 /* query rows of one of its passes */
 int exact_warp_pass_rows(bool stats);
 

@@ -56,3 +56,47 @@ def test_all_against_all_at_edges(open_, gap):
     targets = [seqs[j] for i in range(len(seqs)) for j in range(i + 1, len(seqs))]
     for name in ("nw_stats_scan_32", "sg_qx_striped_32", "sw_striped_32", "sw_stats_striped_32"):
         _check(name, pb.batch_all(name, m, seqs, open_, gap), queries, targets, open_, gap, om)
+
+
+@pytest.mark.parametrize("qlen", [1, 2, 31, 33, 64, 65, 300, 1023, 1024, 1025, 2047, 2048, 2049])
+def test_single_calls_on_one_block(qlen):
+    """One pair per call: queries at the edges of warps, of 2 and 4 rows a
+    thread and past the block; every statistic against the oracle, and the
+    16-bit forms (whose verdicts read the extremes of the padded rows)
+    against the 32-bit ones."""
+    rng = random.Random(qlen)
+    b62 = pb.matrix_lookup("blosum62")
+    om = O.Matrix.from_struct(b62)
+    q = rand_seq(rng, qlen, AA)
+    targets = [rand_seq(rng, 1, AA), mutate(rng, q, AA, 0.3, 0.05)[:400] or "A", rand_seq(rng, rng.randint(2, 300), AA)]
+    prof = pb.ProfileHandle("parasail_profile_create_stats_32", q, b62)
+    prof16 = pb.ProfileHandle("parasail_profile_create_stats_16", q, b62)
+    for name in ("nw_stats_striped", "sg_qx_stats_scan", "sg_stats_striped", "sw_stats_scan", "nw_scan", "sg_de_striped"):
+        stats = "_stats" in name
+        alg, sgf = O.alg_of(name.split("_striped")[0].split("_scan")[0].replace("_stats", ""))
+        keys = ("score", "end_query", "end_ref") + (("matches", "similar", "length") if stats else ())
+        for t in targets:
+            e = O.align(alg, sgf, int(stats), q, t, 11, 1, om)
+            got = pb.align_profile("parasail_%s_profile_32" % name, prof, t, 11, 1)
+            assert all(got[f] == e[f] for f in keys), (name, len(t))
+            g16 = pb.align_profile("parasail_%s_profile_16" % name, prof16, t, 11, 1)
+            assert not g16["flag"] & pb.FLAG_SATURATED and all(g16[f] == e[f] for f in keys), (name, len(t))
+
+
+@pytest.mark.parametrize("alg", ["sw", "nw", "sg", "sg_qx", "sg_de"])
+def test_batch_cigars_equal_single_ones(alg):
+    """CIGARs built on the device against parasail_result_get_cigar on the
+    single trace results: mixed case, gaps to the edges, end gaps, pairs of
+    one residue, a saturated 8-bit pair."""
+    rng = random.Random(len(alg))
+    m = pb.matrix_lookup("blosum62")
+    qs, ts = ["A", "W", "ARNDW", "W" * 40], ["A", "GGGW", "W", "W" * 40]
+    for _ in range(60):
+        q = rand_seq(rng, rng.randint(1, 120), AA)
+        t = rand_seq(rng, rng.randint(0, 30), AA) + mutate(rng, q, AA, 0.2, 0.1) + rand_seq(rng, rng.randint(0, 30), AA)
+        qs.append("".join(c.lower() if rng.random() < 0.3 else c for c in q))
+        ts.append("".join(c.lower() if rng.random() < 0.3 else c for c in t) or "A")
+    for form in ("", "_striped_8", "_scan_sat"):
+        got = pb.batch_pairs_cigar("%s_trace%s" % (alg, form), m, qs, ts, 11, 1)
+        for q, t, g in zip(qs, ts, got):
+            assert g == pb.trace("parasail_%s_trace%s" % (alg, form), q, t, 11, 1, m), (alg, form, q, t)
