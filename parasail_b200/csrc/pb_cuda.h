@@ -181,6 +181,13 @@ int pb_cuda_trace_pairs_host(const struct pb_job *job, const pb_batch *tmpl, con
                              const char *h_t, const int64_t *h_toff, const int *h_tlen, int n,
                              int *h_ends, uint8_t *h_ops, const int64_t *h_ops_off, int *h_info);
 
+/* The same with CIGARs instead of paths (see the definition). */
+int pb_cuda_trace_cigars_host(const struct pb_job *job, const pb_batch *tmpl, const uint8_t *mapper256,
+                              const uint8_t *upper256, const char *h_q, const int64_t *h_qoff, const int *h_qlen,
+                              const char *h_t, const int64_t *h_toff, const int *h_tlen, int n,
+                              int *h_ends, const int64_t *h_ops_off, int *h_info, int *h_len, int *h_beg,
+                              uint32_t **h_elems);
+
 /* Lane-exact emulation of the reference's 8/16-bit striped kernels
  * (pb_lane.cu) for the pairs listed in d_list. kind: 0 nw/sg score-only,
  * 1 nw/sg with statistics, 2 the SW statistics kernel on the FASTSTATS prefix

@@ -521,12 +521,12 @@ static void mapper_of(const parasail_matrix_t *m, uint8_t *out)
 }
 
 /* Paths of n pairs (host characters). ends[3k..] score, end_query,
- * end_ref; paths[k] allocated here (NULL when the pair has no path: it is
+ * end_ref; info[3k..] steps (-1: no path) and the stop cell; paths[k] allocated here (NULL when the pair has no path: it is
  * outside the 16-bit bounds of the pair kernels). */
 static int trace_pairs(int alg, int sgflags, const parasail_matrix_t *matrix, int open, int gap,
                        const char *q, const int64_t *qoff, const int *qlen,
                        const char *t, const int64_t *toff, const int *tlen, int n,
-                       int *ends, pb_trace_path **paths)
+                       int *ends, int *info, pb_trace_path **paths)
 {
     pb_job job;
     pb_batch b;
@@ -534,18 +534,16 @@ static int trace_pairs(int alg, int sgflags, const parasail_matrix_t *matrix, in
     int32_t *d_mat;
     int64_t *ooff;
     uint8_t *ops;
-    int *info;
     int64_t total = 0;
     int k, rc;
     if (matrix->type != PARASAIL_MATRIX_TYPE_SQUARE) return -2;
     trace_job(alg, sgflags, matrix, open, gap, &job);
     ooff = (int64_t *)malloc(sizeof(int64_t) * (size_t)n);
-    info = (int *)malloc(sizeof(int) * 3 * (size_t)n);
-    if (!ooff || !info) { free(ooff); free(info); return -1; }
+    if (!ooff) return -1;
     for (k = 0; k < n; ++k) { ooff[k] = total; total += (int64_t)qlen[k] + tlen[k]; }
     ops = (uint8_t *)malloc((size_t)total + 16);
     d_mat = (int32_t *)pb_cuda_malloc(sizeof(int32_t) * (size_t)matrix->size * matrix->size);
-    if (!ops || !d_mat) { free(ooff); free(info); free(ops); pb_cuda_free(d_mat); return -1; }
+    if (!ops || !d_mat) { free(ooff); free(ops); pb_cuda_free(d_mat); return -1; }
     rc = pb_cuda_h2d(d_mat, matrix->matrix, sizeof(int32_t) * (size_t)matrix->size * matrix->size);
     pb_cuda_sync();
     memset(&b, 0, sizeof b);
@@ -571,7 +569,6 @@ static int trace_pairs(int alg, int sgflags, const parasail_matrix_t *matrix, in
         paths[k] = p;
     }
     free(ooff);
-    free(info);
     free(ops);
     return rc;
 }
@@ -642,12 +639,13 @@ static int nwsg_clean(int w, int qlen, int tlen, int open, int gap, int mmax, in
  * sw_trace_striped_avx2_256_8.c:398-418, sw_trace_scan_avx2_256_8.c:
  * 352-359) saturate exactly when the alignment score exceeds
  * INT_MAX_w - max(matrix) - 1 (penalties that wrap in the lane are taken
- * as saturating). NW/SG: clean by nwsg_clean, else the lane-exact
+ * as saturating; info[3k] is the pair's number of steps, -1 for no path).
+ * NW/SG: clean by nwsg_clean, else the lane-exact
  * emulation of the kernel on the GPU decides (pb_lane.cuh). sat[k] is -1
  * for a SW pair with no path: its score, and so its width, is unknown. */
 static int trace_widths(const trace_form *f, const parasail_matrix_t *matrix, int open, int gap, const char *q,
                         const int64_t *qoff, const int *qlen, const char *t, const int64_t *toff, const int *tlen,
-                        int n, const int *ends, pb_trace_path *const *paths, int *width, int *sat)
+                        int n, const int *ends, const int *info, int *width, int *sat)
 {
     static const int chain[3] = {8, 16, 32};
     const int first = f->bits == 16 ? 1 : f->bits == 32 ? 2 : 0;
@@ -671,7 +669,7 @@ static int trace_widths(const trace_form *f, const parasail_matrix_t *matrix, in
             if (w == 32) continue;
             if (f->alg == PB_SW) {
                 if (open > imax || gap > imax) sat[k] = 1;
-                else if (!paths[k]) sat[k] = -1;
+                else if (info[3 * k] < 0) sat[k] = -1;
                 else sat[k] = ends[3 * k] > imax - matrix->max - 1;
             } else if (!nwsg_clean(w, qlen[k], tlen[k], open, gap, matrix->max, matrix->min)) {
                 list[nl++] = k;
@@ -702,16 +700,20 @@ static int trace_results(const char *who, const trace_form *f, const parasail_ma
     int *ends = (int *)malloc(sizeof(int) * 3 * (size_t)n);
     int *width = (int *)malloc(sizeof(int) * (size_t)n);
     int *sat = (int *)malloc(sizeof(int) * (size_t)n);
+    int *info = (int *)malloc(sizeof(int) * 3 * (size_t)n);
     pb_trace_path **paths = (pb_trace_path **)calloc((size_t)n, sizeof *paths);
     int k, rc;
     for (k = 0; k < n; ++k) results[k] = NULL;
-    if (!ends || !width || !sat || !paths) { free(ends); free(width); free(sat); free(paths); return -1; }
-    rc = trace_pairs(f->alg, f->sgf, matrix, open, gap, q, qoff, qlen, t, toff, tlen, n, ends, paths);
+    if (!ends || !width || !sat || !info || !paths) {
+        free(ends); free(width); free(sat); free(info); free(paths);
+        return -1;
+    }
+    rc = trace_pairs(f->alg, f->sgf, matrix, open, gap, q, qoff, qlen, t, toff, tlen, n, ends, info, paths);
     if (rc == -2) fprintf(stderr, "%s: traceback needs a square matrix\n", who);
     else if (rc != 0) fprintf(stderr, "%s: GPU alignment failed: %s\n", who, pb_cuda_last_error());
     for (k = 0; k < n; ++k) { width[k] = 32; sat[k] = 0; }
     if (rc == 0 && f->kind >= 2 && f->bits != 32) {
-        rc = trace_widths(f, matrix, open, gap, q, qoff, qlen, t, toff, tlen, n, ends, paths, width, sat);
+        rc = trace_widths(f, matrix, open, gap, q, qoff, qlen, t, toff, tlen, n, ends, info, width, sat);
         if (rc != 0) fprintf(stderr, "%s: GPU alignment failed: %s\n", who, pb_cuda_last_error());
     }
     for (k = 0; rc == 0 && k < n; ++k) {
@@ -740,6 +742,7 @@ static int trace_results(const char *who, const trace_form *f, const parasail_ma
     free(ends);
     free(width);
     free(sat);
+    free(info);
     free(paths);
     return rc;
 }
@@ -910,9 +913,14 @@ int parasail_b200_batch_pairs_cigar(const char *funcname, const parasail_matrix_
                                     int *cigar_lengths, int *beg_query, int *beg_ref)
 {
     trace_form f;
-    parasail_result_t **res;
-    int64_t off = 0;
-    int k, rc;
+    pb_job job;
+    pb_batch b;
+    uint8_t map[256], upper[256];
+    int32_t *d_mat = NULL;
+    uint32_t *elems = NULL;
+    int *buf, *ends, *info, *width, *sat, *len, *beg;
+    int64_t *ooff, at = 0, off = 0;
+    int c, k, rc;
     if (!matrix || !queries || !qoffsets || !qlengths || !targets || !toffsets || !tlengths || !records || !cigars ||
         !cigar_lengths || !beg_query || !beg_ref || !funcname) {
         fprintf(stderr, "%s: missing arguments\n", __func__);
@@ -927,31 +935,61 @@ int parasail_b200_batch_pairs_cigar(const char *funcname, const parasail_matrix_
     for (k = 0; k < n; ++k)
         if (qlengths[k] <= 0 || tlengths[k] <= 0) { fprintf(stderr, "%s: pair %d has an empty sequence\n", __func__, k); return -1; }
     if (!pb_gpu_ready(__func__)) return -1;
-    res = (parasail_result_t **)calloc((size_t)n, sizeof *res);
-    if (!res) return -1;
-    rc = trace_results(__func__, &f, matrix, open, gap, queries, qoffsets, qlengths, targets, toffsets, tlengths, n,
-                       res);
-    for (k = 0; rc == 0 && k < n; off += (int64_t)qlengths[k] + tlengths[k], ++k) {
+    if (matrix->type != PARASAIL_MATRIX_TYPE_SQUARE) {
+        fprintf(stderr, "%s: traceback needs a square matrix\n", __func__);
+        return -1;
+    }
+    /* ends, info: 3 ints a pair; begins: 2; width, verdict, length: 1 */
+    buf = (int *)malloc(sizeof(int) * 11 * (size_t)n);
+    ooff = (int64_t *)malloc(sizeof(int64_t) * (size_t)n);
+    d_mat = (int32_t *)pb_cuda_malloc(sizeof(int32_t) * (size_t)matrix->size * matrix->size);
+    if (!buf || !ooff || !d_mat) { free(buf); free(ooff); pb_cuda_free(d_mat); return -1; }
+    ends = buf; info = buf + 3 * (size_t)n; beg = buf + 6 * (size_t)n;
+    width = buf + 8 * (size_t)n; sat = buf + 9 * (size_t)n; len = buf + 10 * (size_t)n;
+    for (k = 0; k < n; ++k) { ooff[k] = off; off += (int64_t)qlengths[k] + tlengths[k]; width[k] = 32; sat[k] = 0; }
+    trace_job(f.alg, f.sgf, matrix, open, gap, &job);
+    memset(&b, 0, sizeof b);
+    b.alg = f.alg; b.sgflags = f.sgf; b.open = open; b.gap = gap;
+    b.d_mat = d_mat; b.msize = matrix->size; b.mmax = matrix->max; b.mmin = matrix->min;
+    mapper_of(matrix, map);
+    for (c = 0; c < 256; ++c) upper[c] = (uint8_t)toupper(c);
+    rc = pb_cuda_h2d(d_mat, matrix->matrix, sizeof(int32_t) * (size_t)matrix->size * matrix->size);
+    pb_cuda_sync();
+    if (rc == 0)
+        rc = pb_cuda_trace_cigars_host(&job, &b, map, upper, queries, qoffsets, qlengths, targets, toffsets, tlengths, n,
+                                       ends, ooff, info, len, beg, &elems);
+    pb_cuda_free(d_mat);
+    pb_cuda_sync();
+    if (rc == 0 && f.kind >= 2 && f.bits != 32)
+        rc = trace_widths(&f, matrix, open, gap, queries, qoffsets, qlengths, targets, toffsets, tlengths, n, ends, info,
+                          width, sat);
+    if (rc != 0) fprintf(stderr, "%s: GPU alignment failed: %s\n", __func__, pb_cuda_last_error());
+    for (k = 0; rc == 0 && k < n; ++k) {
         parasail_b200_record_t *rec = &records[k];
-        parasail_cigar_t *c;
+        const uint32_t *e = elems + at;
+        if (len[k] > 0) at += len[k];
         memset(rec, 0, sizeof *rec);
         cigar_lengths[k] = -1;
         beg_query[k] = beg_ref[k] = 0;
-        if (!res[k]) continue;
-        rec->score = res[k]->score; rec->end_query = res[k]->end_query; rec->end_ref = res[k]->end_ref;
-        rec->flag = res[k]->flag;
-        if (!res[k]->extra) continue;    /* saturated: no alignment */
-        c = parasail_result_get_cigar(res[k], queries + qoffsets[k], qlengths[k], targets + toffsets[k], tlengths[k],
-                                      matrix);
-        if (c) {
-            memcpy(cigars + off, c->seq, sizeof(uint32_t) * (size_t)c->len);
-            cigar_lengths[k] = c->len;
-            beg_query[k] = c->beg_query;
-            beg_ref[k] = c->beg_ref;
-            parasail_cigar_free(c);
+        if (sat[k] != 1 && info[3 * k] < 0) {
+            fprintf(stderr, "%s: pair %d leaves the range of the traceback kernel (int16)\n", __func__, k);
+            continue;
         }
+        rec->flag = form_flags(&f, width[k]);
+        if (sat[k] == 1) {
+            /* saturated: no alignment */
+            rec->flag |= PARASAIL_FLAG_SATURATED;
+            continue;
+        }
+        rec->score = ends[3 * k]; rec->end_query = ends[3 * k + 1]; rec->end_ref = ends[3 * k + 2];
+        if (len[k] < 0) continue;
+        memcpy(cigars + ooff[k], e, sizeof(uint32_t) * (size_t)len[k]);
+        cigar_lengths[k] = len[k];
+        beg_query[k] = beg[2 * k];
+        beg_ref[k] = beg[2 * k + 1];
     }
-    for (k = 0; k < n; ++k) if (res[k]) parasail_result_free(res[k]);
-    free(res);
+    free(elems);
+    free(buf);
+    free(ooff);
     return rc;
 }
