@@ -66,6 +66,7 @@ struct NwWaveParams {
     long long *prog;              /* per warp slot: publication progress of its ring */
     int maxlen;
     int *score;                   /* per pair */
+    int solo;                     /* k_nw_wave16: a pair per warp */
 };
 
 static constexpr unsigned long long NWL_COOP_BIT = 1ull << 62;
@@ -77,6 +78,16 @@ __device__ __forceinline__ int sext_byte(uint32_t lo, uint32_t hi, int k)
     uint32_t d;
     asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(lo), "r"(hi), "r"(sel));
     return (int)d;
+}
+
+/* byte K of a (low half) and of b (high half), sign-extended to int16x2 */
+template <int K>
+__device__ __forceinline__ uint32_t nw_pair(uint32_t a, uint32_t b)
+{
+    constexpr uint32_t sel = (K) | ((K | 8) << 4) | ((4 + K) << 8) | (((4 + K) | 8) << 12);
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+    return d;
 }
 
 /*
@@ -392,6 +403,304 @@ k_nw_wave(NwWaveParams p, int *counter, int *error)
     if (coop) cluster.sync();
 }
 
+/*
+ * The unbanded kernel in int16x2: the same teams, passes and rings, with
+ * lane k of a warp holding 2R rows as two strips of R rows in the halves of
+ * its registers, strip B one column behind strip A, on column t - 2k at
+ * iteration t (as k_sw_wave16, pb_sw16.cu). A pass covers 64R rows and costs
+ * 6.5 R + about 40 instructions per column for them; the 32-bit form spends
+ * about 120 on 256 rows.
+ *
+ * Values are relative to a base of the warp, moved every 32 iterations to
+ * lane 16's top row. Neighbouring cells differ by at most max(matrix) + open
+ * (H(i,j) >= H(i-1,j) - open by a gap; H(i,j) <= H(i-1,j) + max(matrix) +
+ * open by dropping residue i and gapping what it was aligned to; the same
+ * along columns and on the boundaries), so everything a warp holds lies
+ * within (max(matrix) + open) x (64R rows + its skew and 32 columns of
+ * drift) of its base; the host takes this kernel where that fits 16 bits
+ * (nw16_ok). E(i,-1) and F(-1,j) start at H - open, which no gap opened from
+ * the boundary can tie. A ring entry is the packed (H, F) and its base.
+ *
+ * p.solo: pairs that are less than half a warp's fair share of the launch run
+ * on one warp each, pass after pass, so that no warp waits for another (a
+ * CTA of eight warps per pair of three passes leaves five idle).
+ *
+ * 64 DNA pairs of 5-50 kbp (5.9e10 cells): 104.5 -> 31.0 ms; the 18,000 pairs
+ * above 512 residues of 100,000 protein pairs: 17.4 -> 5.8 ms. Bound by the
+ * ALU pipe while all warps run, by the largest pairs' passes at the end.
+ */
+template <int R>
+__global__ void __launch_bounds__(NWL_WARPS * 32, 2)
+k_nw_wave16(NwWaveParams p, int *counter, int *error)
+{
+    namespace cg = cooperative_groups;
+    constexpr int W = (R + 3) / 4;                 /* score words per strip */
+    constexpr int LETTER = 2 * 32 * W;             /* words per letter */
+    constexpr int ROWS = 64 * R;
+    extern __shared__ __align__(16) uint32_t s_sc[];
+    __shared__ __align__(16) int8_t s_mat[32 * 32];
+    __shared__ uint16_t s_ring[NWL_WARPS][128];
+    __shared__ int s_pair;
+    const int L = p.msize;
+    for (int k = threadIdx.x; k < L * L; k += blockDim.x) s_mat[(k / L) * 32 + k % L] = p.mat[k];   /* s + open */
+    __syncthreads();
+    cg::cluster_group cluster = cg::this_cluster();
+    const int C = (int)cluster.num_blocks();
+    const int crank = (int)cluster.block_rank();
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    const int open = p.open, gap = p.gap;
+    const uint32_t gO = 0x10001u * (uint32_t)(uint16_t)(-open), gE = 0x10001u * (uint32_t)(uint16_t)(-gap);
+    uint32_t *sc_pass = s_sc + (size_t)warp * L * LETTER + lane * W;
+    uint16_t *ring = s_ring[warp];
+    volatile int *verr = error;
+    bool coop = C > 1;
+    auto pack = [](int lo, int hi) -> uint32_t { return (uint32_t)(uint16_t)lo | ((uint32_t)(uint16_t)hi << 16); };
+
+    for (;;) {
+        int w;
+        if (p.solo) {
+            w = 0;
+            if (lane == 0) w = atomicAdd(counter, 1);
+            w = __shfl_sync(0xffffffffu, w, 0);
+        } else if (coop) {
+            cluster.sync();
+            if (crank == 0 && threadIdx.x == 0) s_pair = atomicAdd(counter, 1);
+            cluster.sync();
+            w = *cluster.map_shared_rank(&s_pair, 0);
+            /* every CTA has read rank 0's pair before it is overwritten */
+            cluster.sync();
+        } else {
+            __syncthreads();
+            if (threadIdx.x == 0) s_pair = atomicAdd(counter, 1);
+            __syncthreads();
+            w = s_pair;
+        }
+        if (w >= p.npairs) break;
+        const int T = p.solo ? 1 : coop ? C * NWL_WARPS : NWL_WARPS;           /* warps of the team */
+        const int tw = p.solo ? 0 : coop ? crank * NWL_WARPS + warp : warp;    /* this warp in the team */
+        const long long slot0 = p.solo ? (long long)blockIdx.x * NWL_WARPS + warp
+                              : coop ? (long long)(blockIdx.x / C) * C * NWL_WARPS
+                                     : (long long)blockIdx.x * NWL_WARPS;
+        const int pid = p.order[w];
+        const int n = p.qlen[pid], m = p.tlen[pid];
+        const uint8_t *qs = p.q + p.qoff[pid];
+        const uint8_t *ts = p.t + p.toff[pid];
+        const int npass = (n + ROWS - 1) / ROWS;
+        if (!p.solo) {
+            /* this CTA's slots start the pair unpublished */
+            if (threadIdx.x < NWL_WARPS)
+                cuda::atomic_ref<long long, cuda::thread_scope_device>(p.prog[(long long)blockIdx.x * NWL_WARPS + threadIdx.x])
+                    .store(0, cuda::memory_order_relaxed);
+            if (coop) cluster.sync(); else __syncthreads();
+        }
+        for (int pass = tw; pass < npass; pass += T) {
+            const int R0 = pass * ROWS + lane * 2 * R;
+            const long long in_slot = slot0 + (pass + T - 1) % T, out_slot = slot0 + pass % T;
+            const int2 *in_buf = p.scratch + in_slot * p.maxlen;
+            int2 *out_buf = p.scratch + out_slot * p.maxlen;
+            const long long stride = (long long)m + 1;
+            cuda::atomic_ref<long long, cuda::thread_scope_device> in_prog(p.prog[in_slot]);
+            cuda::atomic_ref<long long, cuda::thread_scope_device> out_prog(p.prog[out_slot]);
+            const long long in_base = pass > 0 ? (long long)((pass - 1) / T) * stride + 1 : 0;
+            const long long out_base = (long long)(pass / T) * stride + 1;
+            const bool more = pass + 1 < npass;
+            /* the previous pass must have published column c before it is read */
+            auto wait_for = [&](int c) -> bool {
+                if (pass == 0 || p.solo) return true;
+                const int need = min(c, m - 1);
+                const long long t0 = clock64();
+                unsigned ns = 32;
+                while (in_prog.load(cuda::memory_order_acquire) < in_base + need) {
+                    if (*verr) return false;
+                    if (clock64() - t0 > NWL_SPIN_CYCLES) { atomicExch(error, 1); return false; }
+                    /* back off, so that waiting warps leave the memory
+                     * system and the issue slots to the producers */
+                    __nanosleep(ns);
+                    if (ns < 1024) ns <<= 1;
+                }
+                return true;
+            };
+            /* this lane's scores against every letter; rows past the query
+             * take letter 0 (nothing above depends on them) */
+            __syncwarp();
+            {
+                int qc[2 * R];
+#pragma unroll
+                for (int r = 0; r < 2 * R; ++r) {
+                    const int c = R0 + r < n ? (int)qs[R0 + r] : 0;
+                    qc[r] = c < L ? c : 0;
+                }
+                for (int a = 0; a < L; ++a)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int k = 0; k < W; ++k) {
+                            uint32_t word = 0u;
+#pragma unroll
+                            for (int b = 0; b < 4 && 4 * k + b < R; ++b)
+                                word |= (uint32_t)(uint8_t)s_mat[a * 32 + qc[h * R + 4 * k + b]] << (8 * b);
+                            sc_pass[a * LETTER + h * 32 * W + k] = word;
+                        }
+            }
+            /* letters by column, as word offsets of their scores (the ring of
+             * k_sw_wave16); columns outside the target take letter 0 */
+            auto fetch = [&](int c) -> int { return c < m ? (int)__ldg(ts + c) : 0; };
+            auto put = [&](int c, int v) { ring[c & 127] = (uint16_t)((v < L ? v : 0) * LETTER); };
+            put(lane, fetch(lane));
+            ring[64 + lane] = ring[96 + lane] = 0;
+            int pre = fetch(32 + lane);
+            __syncwarp();
+            /* registers hold H - open relative to base */
+            auto left = [&](int i) -> int { return (i < 0 ? 0 : -open - i * gap) - open; };
+            int base = left(pass * ROWS + ROWS / 2);
+            uint32_t H[R], E[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                H[r] = pack(left(R0 + r) - base, left(R0 + R + r) - base);
+                E[r] = H[r];
+            }
+            uint32_t dg = pack(left(R0 - 1) - base, 0);
+            uint32_t prev_h = pack(left(R0 + R - 1) - base, 0), prev_f = prev_h;
+            uint32_t v = 0u, cur = 0u;
+            auto load = [&](uint32_t (&x)[W], const uint32_t *at) {
+                if (W == 2) {
+                    const uint2 y = *reinterpret_cast<const uint2 *>(at);
+                    x[0] = y.x; x[W - 1] = y.y;
+                } else {
+                    x[0] = *at;
+                }
+            };
+            const uint32_t *pa_at = sc_pass + (lane == 0 ? ring[0] : 0);
+            uint32_t wa[W], wb[W];
+            load(wa, pa_at);
+            load(wb, sc_pass + 32 * W);
+            /* the row above at column c, relative to this warp's base: row -1
+             * in the first pass, else the ring's entry */
+            auto above = [&](int c) -> uint32_t {
+                if (pass == 0) {
+                    const int h = -open - c * gap - open - base;
+                    return pack(h, h);
+                }
+                if (c >= m) return 0u;
+                const int2 x = __ldcg(&in_buf[c]);
+                return __vadd2((uint32_t)x.x, 0x10001u * (uint32_t)(uint16_t)(x.y - base));
+            };
+            const int iters = m + 63;
+            const int ra = n - 1 - R0;               /* the corner's row among this lane's */
+            int result = 0;
+            bool have_result = false, aborted = false;
+            for (int t0 = 0; t0 < iters; t0 += 32) {
+                bool ok = true;
+                if (lane == 0) ok = wait_for(t0 + 31);
+                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                if (!ok) { aborted = true; break; }
+                if (t0 > 0) {
+                    /* rebase */
+                    const int shift = __shfl_sync(0xffffffffu, (int)(int16_t)(H[0] & 0xffffu), 16);
+                    const uint32_t sh2 = 0x10001u * (uint32_t)(uint16_t)shift;
+                    base += shift;
+#pragma unroll
+                    for (int r = 0; r < R; ++r) { H[r] = __vsub2(H[r], sh2); E[r] = __vsub2(E[r], sh2); }
+                    dg = __vsub2(dg, sh2);
+                    prev_h = __vsub2(prev_h, sh2);
+                    prev_f = __vsub2(prev_f, sh2);
+                    v = __vsub2(v, sh2);
+                }
+                cur = above(t0 + lane);
+                const uint32_t vin0 = __shfl_sync(0xffffffffu, cur, 0);
+                if (lane == 0) v = vin0;
+                put(t0 + 32 + lane, pre);
+                pre = fetch(t0 + 64 + lane);
+                __syncwarp();
+                const int n_it = min(32, iters - t0);
+                int off = ring[(t0 - 2 * lane + 1) & 127];
+#pragma unroll 2
+                for (int it = 0; it < n_it; ++it) {
+                    /* strip A's column; strip B is on column j - 1 */
+                    const int j = t0 + it - 2 * lane;
+                    uint32_t na[W], nb[W];
+                    load(nb, pa_at + 32 * W);
+                    pa_at = sc_pass + off;
+                    load(na, pa_at);
+                    off = ring[(j + 2) & 127];
+                    uint32_t hu = __byte_perm(v, prev_h, 0x5410);
+                    uint32_t fu = __byte_perm(v, prev_f, 0x5432);
+                    uint32_t out = 0u;
+                    if (j >= 0 && j <= m) {
+                        uint32_t hd = dg, aop = 0u;
+                        dg = hu;
+#pragma unroll
+                        for (int r = 0; r < R; ++r) {
+                            uint32_t sc;
+                            /* byte r of both strips, sign-extended */
+                            switch (r & 3) {
+                                case 0: sc = nw_pair<0>(wa[r >> 2], wb[r >> 2]); break;
+                                case 1: sc = nw_pair<1>(wa[r >> 2], wb[r >> 2]); break;
+                                case 2: sc = nw_pair<2>(wa[r >> 2], wb[r >> 2]); break;
+                                default: sc = nw_pair<3>(wa[r >> 2], wb[r >> 2]); break;
+                            }
+                            const uint32_t e = __viaddmax_s16x2(E[r], gE, H[r]);
+                            const uint32_t a = __viaddmax_s16x2(hd, sc, e);
+                            const uint32_t ao = __vadd2(a, gO);
+                            const uint32_t f = __viaddmax_s16x2(fu, gE, r == 0 ? hu : aop);
+                            const uint32_t h = __viaddmax_s16x2(f, gO, ao);
+                            E[r] = e;
+                            hd = H[r];
+                            H[r] = h;
+                            hu = h;
+                            fu = f;
+                            aop = ao;
+                        }
+                        out = __byte_perm(hu, fu, 0x7632);
+                        prev_h = hu;
+                        prev_f = fu;
+                        if (j == 0) {
+                            /* strip B has not begun: its left boundary again */
+#pragma unroll
+                            for (int r = 0; r < R; ++r) {
+                                const uint32_t lb = (uint32_t)(uint16_t)(left(R0 + R + r) - base) << 16;
+                                H[r] = (H[r] & 0xffffu) | lb;
+                                E[r] = (E[r] & 0xffffu) | lb;
+                            }
+                        }
+                    }
+                    v = __shfl_up_sync(0xffffffffu, out, 1);
+                    const uint32_t vin = __shfl_sync(0xffffffffu, cur, (it + 1) & 31);
+                    if (lane == 0) v = vin;
+#pragma unroll
+                    for (int k = 0; k < W; ++k) { wa[k] = na[k]; wb[k] = nb[k]; }
+                    if (more) {
+                        if (lane == 31 && (unsigned)(j - 1) < (unsigned)m) out_buf[j - 1] = make_int2((int)out, base);
+                    } else if ((unsigned)(j - (m - 1)) <= 1u && (unsigned)ra < 2u * R) {
+                        /* the corner: strip A at j = m - 1, strip B at j = m */
+                        const int h = ra >= R ? 1 : 0;
+                        if (j - (m - 1) == h) {
+#pragma unroll
+                            for (int r = 0; r < R; ++r)
+                                if (ra == h * R + r) {
+                                    result = (int)(int16_t)(h ? H[r] >> 16 : H[r] & 0xffffu) + base + open;
+                                    have_result = true;
+                                }
+                        }
+                    }
+                }
+                /* columns up to t0 - 32 are out */
+                if (more && !p.solo && lane == 31 && t0 >= 32)
+                    out_prog.store(out_base + min(t0 - 32, m - 1), cuda::memory_order_release);
+            }
+            if (aborted) break;
+            if (more && !p.solo && lane == 31) out_prog.store(out_base + m - 1, cuda::memory_order_release);
+            if (p.solo) __threadfence_block();
+            __syncwarp();
+            /* the corner's owner publishes the result */
+            if (have_result) p.score[pid] = result;
+        }
+    }
+    /* no CTA leaves while another of its cluster may still read its pair */
+    if (coop) cluster.sync();
+}
+
 __global__ void k_iota_nw(int *v, int n)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -399,12 +708,13 @@ __global__ void k_iota_nw(int *v, int n)
 }
 
 /* sort key: the pair's work (cells, or for a band its rows x the columns
- * its passes sweep); the total goes to *total for k_team_class */
+ * its passes sweep); the total goes to total[0] for k_team_class, the rows'
+ * to total[1] */
 __global__ void k_cells(const int *ql, const int *tl, const int *lo, const int *hi, int n,
                         unsigned long long *keys, unsigned long long *total)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned long long k = 0;
+    unsigned long long k = 0, rows = i < n ? (unsigned long long)ql[i] : 0ull;
     if (i < n) {
         const unsigned long long cols = lo ? (unsigned long long)min((long long)tl[i],
                                                   (long long)hi[i] - lo[i] + 32 * NWL_RL)
@@ -412,8 +722,14 @@ __global__ void k_cells(const int *ql, const int *tl, const int *lo, const int *
         k = (unsigned long long)ql[i] * cols;
         keys[i] = k;
     }
-    for (int o = 16; o; o >>= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
-    if ((threadIdx.x & 31) == 0 && k) atomicAdd(total, k);
+    for (int o = 16; o; o >>= 1) {
+        k += __shfl_xor_sync(0xffffffffu, k, o);
+        rows += __shfl_xor_sync(0xffffffffu, rows, o);
+    }
+    if ((threadIdx.x & 31) == 0 && k) {
+        atomicAdd(total, k);
+        atomicAdd(total + 1, rows);
+    }
 }
 
 /*
@@ -428,19 +744,24 @@ __global__ void k_cells(const int *ql, const int *tl, const int *lo, const int *
  * smaller, and every warp of the team gets a pass.
  */
 __global__ void k_team_class(const int *ql, const int *tl, const int *lo, const int *hi, int n, int nwarps,
-                             TeamPolicy pol, const unsigned long long *total, unsigned long long *keys,
-                             int *count)
+                             TeamPolicy pol, int pass_rows, float solo, const unsigned long long *total,
+                             unsigned long long *keys, int *count)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const unsigned long long k = keys[i];
-    const int npass = (ql[i] + 32 * NWL_RL - 1) / (32 * NWL_RL);
+    const int npass = (ql[i] + pass_rows - 1) / pass_rows;
     const long long m = tl[i];
     const bool narrow = lo && (long long)hi[i] - lo[i] + 32 * NWL_RL < m;
     const double cols = narrow ? (double)((long long)hi[i] - lo[i] + 32 * NWL_RL) : (double)m;
     const double kappa = (cols + 31.0) / (narrow ? 32.0 * NWL_RL + 94.0 : 94.0);
     const double share = (double)k * nwarps / ((double)*total * pol.share);
     int c = 0;
+    if (share < solo) {
+        /* a pair per warp: the smallest pairs, sorted last */
+        atomicAdd(&count[NWL_CLASSES], 1);
+        return;
+    }
     if (pol.jump) {
         if (share > NWL_WARPS && npass >= NWL_WARPS * (pol.max_class + 1)) c = pol.max_class;
     } else {
@@ -452,6 +773,16 @@ __global__ void k_team_class(const int *ql, const int *tl, const int *lo, const 
 }
 
 }  // namespace pb
+
+/* Does everything a warp of k_nw_wave16 holds lie within 16 bits of its
+ * base? (See there; 64 x 8 rows, 64 columns of skew, 32 of drift and 32 of
+ * the chunk ahead, twice for the columns at the target's end; a few values
+ * of open, gap and score beside H.) */
+static bool nw16_ok(int mmax, int open, int gap)
+{
+    const long long step = (long long)mmax + open;
+    return step * (512 + 256) + 4LL * (open + gap + 128) <= 32000;
+}
 
 /* Global alignment scores of npairs device-resident pairs (codes), query i =
  * q[qoff[i] ..+qlen[i]), target i likewise, scored through the square matrix
@@ -486,46 +817,14 @@ static int nw_long_impl(int npairs, int open, int gap, const int32_t *h_mat, int
      * score + open inside int8 */
     const bool ge = open >= gap;
     bool bias = ge;
-    for (int k = 0; k < msize * msize; ++k)
+    int mmax = 0;
+    for (int k = 0; k < msize * msize; ++k) {
         if (h_mat[k] + open > 127 || h_mat[k] + open < -128) bias = false;
+        mmax = std::max(mmax, h_mat[k]);
+    }
     if (bias)
         for (int k = 0; k < msize * msize; ++k) hm[k] = (int8_t)(h_mat[k] + open);
-    void (*kern)(pb::NwWaveParams, int *, int *) =
-        d_lo ? (bias ? pb::k_nw_wave<true, true, true> : ge ? pb::k_nw_wave<true, true, false>
-                                                            : pb::k_nw_wave<true, false, false>)
-             : (bias ? pb::k_nw_wave<false, true, true> : ge ? pb::k_nw_wave<false, true, false>
-                                                             : pb::k_nw_wave<false, false, false>);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, pb::NWL_WARPS * 32, 0);
-    if (per_sm < 1) per_sm = 1;
-    const int plain_max = per_sm * nsm;
-    /* the largest cluster class the device runs, and how many clusters of
-     * each class fit at once */
-    /* full DP: kappa is in the hundreds, the largest pairs take 8-CTA teams;
-     * banded: teams as large as the pair's share, bounded by what its band
-     * keeps busy, and by 4 CTAs (larger teams leave fewer slots to the other
-     * pairs than they gain: 0.064 vs 0.073 s for 300 long pairs on their
-     * certified bands) */
-    pb::TeamPolicy pol = d_lo ? pb::TeamPolicy{3, 1.0f, 0} : pb::TeamPolicy{7, 1.0f, 1};
-    int maxclusters[pb::NWL_CLASSES] = {plain_max, 0, 0, 0, 0, 0, 0, 0};
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.blockDim = dim3(pb::NWL_WARPS * 32);
-    cfg.dynamicSmemBytes = 0;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    for (int c = 1; c <= pol.max_class; ++c) {
-        attr[0].val.clusterDim.x = c + 1;
-        cfg.gridDim = dim3((c + 1) * nsm);
-        if (cudaOccupancyMaxActiveClusters(&maxclusters[c], (const void *)kern, &cfg) != cudaSuccess ||
-            maxclusters[c] < 1) {
-            cudaGetLastError();
-            pol.max_class = c - 1;
-            break;
-        }
-    }
+    const bool use16 = !d_lo && bias && nw16_ok(mmax, open, gap);
     /* the work-queue buffers, each checked before any launch writes
      * through it; a failure frees what was allocated and ends the call */
     auto give_up = [&]() {
@@ -550,21 +849,69 @@ static int nw_long_impl(int npairs, int open, int gap, const int32_t *h_mat, int
         return give_up();
     cudaMemcpyAsync(d_mat, hm.data(), hm.size(), cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(counter, 0, sizeof(int) * 32, st);
-    /* counter[0..7]: pair counters of the class launches; [8..9]: total
-     * work; [16..23]: pairs per class */
+    /* counter[0..7]: pair counters of the class launches; [8..11]: total
+     * work and rows; [12]: the solo launch's counter; [16..24]: pairs per
+     * class, solo ones last */
     unsigned long long *total = reinterpret_cast<unsigned long long *>(counter + 8);
     pb::k_iota_nw<<<(npairs + 255) / 256, 256, 0, st>>>(idx, npairs);
     pb::k_cells<<<(npairs + 255) / 256, 256, 0, st>>>(d_qlen, d_tlen, d_lo, d_hi, npairs, keys, total);
+    /* rows per strip in 16 bits: 8 (the fewest instructions per cell), or 4
+     * where passes of 512 rows are fewer than the resident warps */
+    unsigned long long tot[2] = {0, 0};
+    cudaMemcpyAsync(tot, total, sizeof tot, cudaMemcpyDeviceToHost, st);
+    cudaStreamSynchronize(st);
+    const int r16 = tot[1] / 512 + (unsigned long long)npairs / 2 >= (unsigned long long)nsm * 16 ? 8 : 4;
+    void (*kern)(pb::NwWaveParams, int *, int *) =
+        use16 ? (r16 == 8 ? pb::k_nw_wave16<8> : pb::k_nw_wave16<4>) :
+        d_lo ? (bias ? pb::k_nw_wave<true, true, true> : ge ? pb::k_nw_wave<true, true, false>
+                                                            : pb::k_nw_wave<true, false, false>)
+             : (bias ? pb::k_nw_wave<false, true, true> : ge ? pb::k_nw_wave<false, true, false>
+                                                             : pb::k_nw_wave<false, false, false>);
+    const int pass_rows = use16 ? 64 * r16 : 32 * pb::NWL_RL;
+    const size_t smem = use16 ? (size_t)pb::NWL_WARPS * msize * 2 * 32 * ((r16 + 3) / 4) * 4 : 0;
+    if (use16) pb_raise_smem((const void *)kern, (int)smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, pb::NWL_WARPS * 32, smem);
+    if (per_sm < 1) per_sm = 1;
+    const int plain_max = per_sm * nsm;
+    /* the largest cluster class the device runs, and how many clusters of
+     * each class fit at once */
+    /* full DP: kappa is in the hundreds; in 32 bits the largest pairs take
+     * 8-CTA teams, in 16 bits (half the passes) each pair a team of its share;
+     * banded: teams as large as the pair's share, bounded by what its band
+     * keeps busy, and by 4 CTAs (larger teams leave fewer slots to the other
+     * pairs than they gain: 0.064 vs 0.073 s for 300 long pairs on their
+     * certified bands) */
+    pb::TeamPolicy pol = d_lo ? pb::TeamPolicy{3, 1.0f, 0} : pb::TeamPolicy{7, 1.0f, use16 ? 0 : 1};
+    int maxclusters[pb::NWL_CLASSES] = {plain_max, 0, 0, 0, 0, 0, 0, 0};
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.blockDim = dim3(pb::NWL_WARPS * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    for (int c = 1; c <= pol.max_class; ++c) {
+        attr[0].val.clusterDim.x = c + 1;
+        cfg.gridDim = dim3((c + 1) * nsm);
+        if (cudaOccupancyMaxActiveClusters(&maxclusters[c], (const void *)kern, &cfg) != cudaSuccess ||
+            maxclusters[c] < 1) {
+            cudaGetLastError();
+            pol.max_class = c - 1;
+            break;
+        }
+    }
     pb::k_team_class<<<(npairs + 255) / 256, 256, 0, st>>>(d_qlen, d_tlen, d_lo, d_hi, npairs,
-                                                           plain_max * pb::NWL_WARPS, pol, total, keys,
-                                                           counter + 16);
+                                                           plain_max * pb::NWL_WARPS, pol, pass_rows,
+                                                           use16 ? 0.5f : 0.0f, total, keys, counter + 16);
     pb_diag_count_launch(3);
     cub::DeviceRadixSort::SortPairsDescending(nullptr, tmpb, keys, keys_sorted, idx, order, npairs, 0, 64, st);
     if (cudaMallocAsync(&tmp, tmpb, st) != cudaSuccess) return give_up();
     cub::DeviceRadixSort::SortPairsDescending(tmp, tmpb, keys, keys_sorted, idx, order, npairs, 0, 64, st);
     /* pairs sorted by class, largest first; one launch per class, each on
      * its own stream, the largest teams first; they never wait on each other */
-    int ncls[pb::NWL_CLASSES] = {0, 0, 0, 0, 0, 0, 0, 0};
+    int ncls[pb::NWL_CLASSES + 1] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     cudaMemcpyAsync(ncls, counter + 16, sizeof ncls, cudaMemcpyDeviceToHost, st);
     cudaStreamSynchronize(st);
     /* Each launch gets as many teams as fit at once (or as it has pairs);
@@ -594,20 +941,24 @@ static int nw_long_impl(int npairs, int open, int gap, const int32_t *h_mat, int
         before += ncls[c];
         blocks += cblocks[c];
     }
+    /* the pairs of one warp each */
+    const int nsolo = ncls[pb::NWL_CLASSES];
+    const int sblocks = std::min(plain_max, (nsolo + pb::NWL_WARPS - 1) / pb::NWL_WARPS);
+    blocks += sblocks;
     int2 *scratch = nullptr;
     long long *prog = nullptr;
     int *d_err = nullptr;
     int rc = 0, herr = 0;
-    cudaStream_t sc[pb::NWL_CLASSES] = {};
-    cudaEvent_t ev = nullptr, evc[pb::NWL_CLASSES] = {};
+    cudaStream_t sc[pb::NWL_CLASSES + 1] = {};
+    cudaEvent_t ev = nullptr, evc[pb::NWL_CLASSES + 1] = {};
     if (cudaMallocAsync((void **)&d_err, sizeof(int), st) != cudaSuccess) rc = -1;
     else cudaMemsetAsync(d_err, 0, sizeof(int), st);
     if (rc != 0 || cudaMallocAsync((void **)&scratch, sizeof(int2) * (size_t)(maxlen + 1) * blocks * pb::NWL_WARPS, st) != cudaSuccess ||
         cudaMallocAsync((void **)&prog, sizeof(long long) * (size_t)blocks * pb::NWL_WARPS, st) != cudaSuccess ||
         cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess)
         rc = -1;
-    for (int c = 0; c < pb::NWL_CLASSES && rc == 0; ++c)
-        if (cblocks[c] > 0 &&
+    for (int c = 0; c <= pb::NWL_CLASSES && rc == 0; ++c)
+        if ((c < pb::NWL_CLASSES ? cblocks[c] : sblocks) > 0 &&
             (cudaStreamCreateWithFlags(&sc[c], cudaStreamNonBlocking) != cudaSuccess ||
              cudaEventCreateWithFlags(&evc[c], cudaEventDisableTiming) != cudaSuccess))
             rc = -1;
@@ -622,6 +973,7 @@ static int nw_long_impl(int npairs, int open, int gap, const int32_t *h_mat, int
         p.cert = d_lo && d_rounds ? 1 : 0;
         p.cm.a = cert_a; p.cm.open = open; p.cm.ext = gap;
         p.lo_out = d_lo_out; p.hi_out = d_hi_out; p.rounds = d_rounds;
+        p.solo = 0;
         size_t slot = 0;
         int nlaunch = 0;
         for (int c = pb::NWL_CLASSES - 1; c >= 0; --c) {
@@ -638,11 +990,24 @@ static int nw_long_impl(int npairs, int open, int gap, const int32_t *h_mat, int
                 cfg.stream = sc[c];
                 if (cudaLaunchKernelEx(&cfg, kern, pc, counter + c, d_err) != cudaSuccess) rc = -1;
             } else {
-                kern<<<cblocks[c], pb::NWL_WARPS * 32, 0, sc[c]>>>(pc, counter + c, d_err);
+                kern<<<cblocks[c], pb::NWL_WARPS * 32, smem, sc[c]>>>(pc, counter + c, d_err);
             }
             ++nlaunch;
             cudaEventRecord(evc[c], sc[c]);
             cudaStreamWaitEvent(st, evc[c], 0);
+        }
+        if (sblocks > 0) {
+            cudaStream_t ss = sc[pb::NWL_CLASSES];
+            cudaStreamWaitEvent(ss, ev, 0);
+            pb::NwWaveParams ps = p;
+            ps.solo = 1;
+            ps.npairs = nsolo; ps.order = order + before; ps.keys = keys_sorted + before;
+            ps.scratch = scratch + slot * p.maxlen;
+            ps.prog = prog + slot;
+            kern<<<sblocks, pb::NWL_WARPS * 32, smem, ss>>>(ps, counter + 12, d_err);
+            ++nlaunch;
+            cudaEventRecord(evc[pb::NWL_CLASSES], ss);
+            cudaStreamWaitEvent(st, evc[pb::NWL_CLASSES], 0);
         }
         pb_diag_count_launch(nlaunch);
         if (cudaGetLastError() != cudaSuccess) rc = -1;
@@ -655,7 +1020,7 @@ static int nw_long_impl(int npairs, int open, int gap, const int32_t *h_mat, int
     if (prog) cudaFreeAsync(prog, st);
     if (d_err) cudaFreeAsync(d_err, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) rc = -1;
-    for (int c = 0; c < pb::NWL_CLASSES; ++c) {
+    for (int c = 0; c <= pb::NWL_CLASSES; ++c) {
         if (sc[c]) cudaStreamDestroy(sc[c]);
         if (evc[c]) cudaEventDestroy(evc[c]);
     }

@@ -1,0 +1,57 @@
+"""Global scores of long pairs at the sizes where the int16x2 wavefront
+changes: rows at the edges of strips, lanes and passes, targets shorter than
+the skew of a warp and at the edges of 32-column chunks, pairs of one warp
+and of teams, and the 32-bit wavefront for scores whose steps do not fit 16
+bits. Every score against the oracle."""
+import random
+
+import numpy as np
+import pytest
+
+import oracle as O
+from conftest import AA, DNA, rand_seq, mutate
+
+pb = pytest.importorskip("parasail_b200")
+pytestmark = pytest.mark.gpu
+
+
+def _check(m, queries, targets, open_, gap):
+    om = O.Matrix.from_struct(m)
+    qb, qo, ql = pb.pack(queries)
+    tb, to, tl = pb.pack(targets)
+    got = pb.nw_long(m, qb, qo, ql, tb, to, tl, open_, gap)
+    exp = np.array([O.align(O.NW, 0, 0, q, t, open_, gap, om)["score"] for q, t in zip(queries, targets)], np.int32)
+    bad = np.nonzero(got != exp)[0]
+    assert len(bad) == 0, [(len(queries[k]), len(targets[k]), int(got[k]), int(exp[k])) for k in bad[:5]]
+
+
+@pytest.mark.parametrize("alphabet,match,mismatch,open_,gap", [(DNA, 1, -2, 4, 1), (DNA, 2, -3, 5, 5), (AA, 0, 0, 11, 1),
+                                                               (AA, 0, 0, 60, 2)])
+def test_nw_long_edges(alphabet, match, mismatch, open_, gap):
+    rng = random.Random(open_)
+    m = pb.matrix_create("ACGT", match, mismatch) if alphabet is DNA else pb.matrix_lookup("blosum62")
+    rows = (1, 4, 5, 8, 9, 15, 16, 17, 255, 256, 257, 511, 512, 513, 1023, 1025, 1600)
+    cols = (1, 2, 31, 32, 33, 62, 63, 64, 65, 95, 96, 97, 500)
+    queries, targets = [], []
+    for k, a in enumerate(rows):
+        for b in cols[k % 2::2]:
+            q = rand_seq(rng, a, alphabet)
+            t = mutate(rng, q, alphabet, 0.1, 0.05) if b == 500 else rand_seq(rng, b, alphabet)
+            queries.append(q)
+            targets.append(t or rand_seq(rng, b, alphabet))
+    _check(m, queries, targets, open_, gap)                    # one warp each, and teams for the largest
+    for k in (0, len(queries) // 2, len(queries) - 1):
+        _check(m, queries[k:k + 1], targets[k:k + 1], open_, gap)
+
+
+def test_nw_long_drift():
+    """Scores far outside 16 bits in both directions, teams of several
+    blocks, and a set of unequal pairs."""
+    rng = random.Random(5)
+    m = pb.matrix_create("ACGT", 3, -4)
+    a = rand_seq(rng, 15000, DNA)
+    pairs = [(a, a), (a, mutate(rng, a, DNA, 0.1, 0.02)), ("A" * 14000, "C" * 15000), (a, rand_seq(rng, 40, DNA)),
+             (rand_seq(rng, 30, DNA), a)]
+    _check(m, [p[0] for p in pairs], [p[1] for p in pairs], 8, 2)
+    pairs += [(rand_seq(rng, rng.randint(1, 900), DNA), rand_seq(rng, rng.randint(1, 900), DNA)) for _ in range(300)]
+    _check(m, [p[0] for p in pairs], [p[1] for p in pairs], 8, 2)
