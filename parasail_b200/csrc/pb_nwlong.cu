@@ -43,6 +43,9 @@ static constexpr int NWL_WARPS = 8;       /* warps per CTA */
  * one CTA); one launch per class */
 static constexpr int NWL_CLASSES = 8;
 static constexpr int NWL_NEG = INT32_MIN / 4;
+/* k_nw_wave16's -infinity in a band, and what its values in the band stay
+ * above (nw16_ok) */
+static constexpr int NW16_NEG = -31000, NW16_OUT = -28000;
 
 /* How large a team a pair gets (k_team_class). `share`: a pair gets the
  * smallest team whose warps hold its share of the work (its cells over the
@@ -87,6 +90,14 @@ __device__ __forceinline__ uint32_t nw_pair(uint32_t a, uint32_t b)
     constexpr uint32_t sel = (K) | ((K | 8) << 4) | ((4 + K) << 8) | (((4 + K) | 8) << 12);
     uint32_t d;
     asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+    return d;
+}
+
+/* 0xffff in each half whose sign bit is set, else 0 */
+__device__ __forceinline__ uint32_t nw_signs(uint32_t a)
+{
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %1, %2;" : "=r"(d) : "r"(a), "r"(0xbb99u));
     return d;
 }
 
@@ -429,7 +440,7 @@ k_nw_wave(NwWaveParams p, int *counter, int *error)
  * above 512 residues of 100,000 protein pairs: 17.4 -> 5.8 ms. Bound by the
  * ALU pipe while all warps run, by the largest pairs' passes at the end.
  */
-template <int R>
+template <int R, bool BANDED>
 __global__ void __launch_bounds__(NWL_WARPS * 32, 2)
 k_nw_wave16(NwWaveParams p, int *counter, int *error)
 {
@@ -456,6 +467,7 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
     volatile int *verr = error;
     bool coop = C > 1;
     auto pack = [](int lo, int hi) -> uint32_t { return (uint32_t)(uint16_t)lo | ((uint32_t)(uint16_t)hi << 16); };
+    constexpr uint32_t NEG2 = 0x10001u * (uint32_t)(uint16_t)NW16_NEG;
 
     for (;;) {
         int w;
@@ -487,6 +499,9 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
         const uint8_t *qs = p.q + p.qoff[pid];
         const uint8_t *ts = p.t + p.toff[pid];
         const int npass = (n + ROWS - 1) / ROWS;
+        int lo = BANDED ? p.lo[pid] : 0, hi = BANDED ? p.hi[pid] : 0;
+        /* the certificate's second round, as in k_nw_wave */
+        for (int round = 0; round < (BANDED && p.cert ? 2 : 1); ++round) {
         if (!p.solo) {
             /* this CTA's slots start the pair unpublished */
             if (threadIdx.x < NWL_WARPS)
@@ -505,10 +520,17 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
             const long long in_base = pass > 0 ? (long long)((pass - 1) / T) * stride + 1 : 0;
             const long long out_base = (long long)(pass / T) * stride + 1;
             const bool more = pass + 1 < npass;
+            /* this pass's and the previous one's columns */
+            const int r0 = pass * ROWS;
+            const int jlo = BANDED ? max(0, r0 - hi) : 0;
+            const int jhi = BANDED ? min(m - 1, r0 + ROWS - 1 - lo) : m - 1;
+            const int prev_jlo = BANDED ? max(0, r0 - ROWS - hi) : 0;
+            const int prev_jhi = BANDED ? min(m - 1, r0 - 1 - lo) : m - 1;
             /* the previous pass must have published column c before it is read */
             auto wait_for = [&](int c) -> bool {
                 if (pass == 0 || p.solo) return true;
-                const int need = min(c, m - 1);
+                const int need = min(c, prev_jhi);
+                if (BANDED && need < 0) return true;
                 const long long t0 = clock64();
                 unsigned ns = 32;
                 while (in_prog.load(cuda::memory_order_acquire) < in_base + need) {
@@ -547,22 +569,54 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
              * k_sw_wave16); columns outside the target take letter 0 */
             auto fetch = [&](int c) -> int { return c < m ? (int)__ldg(ts + c) : 0; };
             auto put = [&](int c, int v) { ring[c & 127] = (uint16_t)((v < L ? v : 0) * LETTER); };
-            put(lane, fetch(lane));
-            ring[64 + lane] = ring[96 + lane] = 0;
-            int pre = fetch(32 + lane);
+            put(jlo + lane, fetch(jlo + lane));
+            ring[(jlo - 32 + lane) & 127] = ring[(jlo - 64 + lane) & 127] = 0;
+            int pre = fetch(jlo + 32 + lane);
             __syncwarp();
             /* registers hold H - open relative to base */
             auto left = [&](int i) -> int { return (i < 0 ? 0 : -open - i * gap) - open; };
-            int base = left(pass * ROWS + ROWS / 2);
+            int base = left(r0 + ROWS / 2);
+            const bool corner_above = BANDED && jlo > 0 && lane == 0 && jlo - 1 >= prev_jlo && jlo - 1 <= prev_jhi;
+            int dg_abs = INT_MIN;
+            if (BANDED) {
+                /* the largest value above the first columns, or row -1's */
+                bool ok = true;
+                if (lane == 0) ok = wait_for(jlo + 31);
+                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                if (!ok) break;
+                int top = INT_MIN;
+                if (pass == 0) {
+                    top = left(0);
+                } else if (jlo + lane <= prev_jhi) {
+                    const int2 x = __ldcg(&in_buf[jlo + lane]);
+                    if ((int)(int16_t)(x.x & 0xffff) > NW16_OUT) top = (int)(int16_t)(x.x & 0xffff) + x.y;
+                }
+                if (corner_above) {
+                    /* H(r0 - 1, jlo - 1) */
+                    const int2 x = __ldcg(&in_buf[jlo - 1]);
+                    if ((int)(int16_t)(x.x & 0xffff) > NW16_OUT) {
+                        dg_abs = (int)(int16_t)(x.x & 0xffff) + x.y;
+                        top = max(top, dg_abs);
+                    }
+                }
+                base = __reduce_max_sync(0xffffffffu, top);
+                if (base == INT_MIN) base = 0;
+            }
+            /* H(i,-1) - open relative to base; NW16_NEG where it lies outside
+             * the band, or column jlo - 1 does (every row here) */
+            auto left_rel = [&](int i) -> int {
+                return BANDED && (jlo > 0 || i + 1 < lo || i + 1 > hi) ? NW16_NEG : left(i) - base;
+            };
             uint32_t H[R], E[R];
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                H[r] = pack(left(R0 + r) - base, left(R0 + R + r) - base);
-                E[r] = H[r];
+                H[r] = pack(left_rel(R0 + r), left_rel(R0 + R + r));
+                E[r] = BANDED ? NEG2 : H[r];
             }
-            uint32_t dg = pack(left(R0 - 1) - base, 0);
-            uint32_t prev_h = pack(left(R0 + R - 1) - base, 0), prev_f = prev_h;
-            uint32_t v = 0u, cur = 0u;
+            const int none = BANDED ? NW16_NEG : 0;
+            uint32_t dg = pack(BANDED && dg_abs != INT_MIN ? dg_abs - base : left_rel(R0 - 1), none);
+            uint32_t prev_h = pack(left_rel(R0 + R - 1), none), prev_f = BANDED ? NEG2 : prev_h;
+            uint32_t v = BANDED ? NEG2 : 0u, cur = 0u;
             auto load = [&](uint32_t (&x)[W], const uint32_t *at) {
                 if (W == 2) {
                     const uint2 y = *reinterpret_cast<const uint2 *>(at);
@@ -571,7 +625,7 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
                     x[0] = *at;
                 }
             };
-            const uint32_t *pa_at = sc_pass + (lane == 0 ? ring[0] : 0);
+            const uint32_t *pa_at = sc_pass + (lane == 0 ? ring[jlo & 127] : 0);
             uint32_t wa[W], wb[W];
             load(wa, pa_at);
             load(wb, sc_pass + 32 * W);
@@ -580,22 +634,47 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
             auto above = [&](int c) -> uint32_t {
                 if (pass == 0) {
                     const int h = -open - c * gap - open - base;
+                    if (BANDED) return -1 - c >= lo && -1 - c <= hi ? pack(h, NW16_NEG) : NEG2;
                     return pack(h, h);
                 }
-                if (c >= m) return 0u;
+                if (c > prev_jhi || (BANDED && c < prev_jlo)) return BANDED ? NEG2 : 0u;
                 const int2 x = __ldcg(&in_buf[c]);
+                if (BANDED) {
+                    const int h = (int)(int16_t)(x.x & 0xffff), f = (int)(int16_t)((uint32_t)x.x >> 16);
+                    return pack(h > NW16_OUT ? h + x.y - base : NW16_NEG, f > NW16_OUT ? f + x.y - base : NW16_NEG);
+                }
                 return __vadd2((uint32_t)x.x, 0x10001u * (uint32_t)(uint16_t)(x.y - base));
             };
-            const int iters = m + 63;
+            const int tend = jhi + 64;               /* iterations jlo .. tend - 1 */
             const int ra = n - 1 - R0;               /* the corner's row among this lane's */
             int result = 0;
             bool have_result = false, aborted = false;
-            for (int t0 = 0; t0 < iters; t0 += 32) {
+            for (int t0 = jlo; t0 < tend; t0 += 32) {
                 bool ok = true;
                 if (lane == 0) ok = wait_for(t0 + 31);
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
                 if (!ok) { aborted = true; break; }
-                if (t0 > 0) {
+                if (BANDED && t0 > jlo) {
+                    /* rebase to the largest value held; what lies outside the
+                     * band stays where it is */
+                    uint32_t mx = __vimax3_s16x2(dg, prev_h, v);
+#pragma unroll
+                    for (int r = 0; r < R; ++r) mx = __vmaxs2(mx, H[r]);
+                    const int top = __reduce_max_sync(0xffffffffu, max((int)(int16_t)(mx & 0xffffu), (int)(int16_t)(mx >> 16)));
+                    const int shift = top > NW16_OUT ? top : 0;
+                    base += shift;
+                    auto move = [&](uint32_t x) -> uint32_t {
+                        const int a = (int)(int16_t)(x & 0xffffu), b = (int)(int16_t)(x >> 16);
+                        return pack(a > NW16_OUT ? a - shift : NW16_NEG, b > NW16_OUT ? b - shift : NW16_NEG);
+                    };
+#pragma unroll
+                    for (int r = 0; r < R; ++r) { H[r] = move(H[r]); E[r] = move(E[r]); }
+                    dg = move(dg);
+                    prev_h = move(prev_h);
+                    prev_f = move(prev_f);
+                    v = move(v);
+                }
+                if (!BANDED && t0 > 0) {
                     /* rebase */
                     const int shift = __shfl_sync(0xffffffffu, (int)(int16_t)(H[0] & 0xffffu), 16);
                     const uint32_t sh2 = 0x10001u * (uint32_t)(uint16_t)shift;
@@ -613,7 +692,7 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
                 put(t0 + 32 + lane, pre);
                 pre = fetch(t0 + 64 + lane);
                 __syncwarp();
-                const int n_it = min(32, iters - t0);
+                const int n_it = min(32, tend - t0);
                 int off = ring[(t0 - 2 * lane + 1) & 127];
 #pragma unroll 2
                 for (int it = 0; it < n_it; ++it) {
@@ -626,10 +705,25 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
                     off = ring[(j + 2) & 127];
                     uint32_t hu = __byte_perm(v, prev_h, 0x5410);
                     uint32_t fu = __byte_perm(v, prev_f, 0x5432);
-                    uint32_t out = 0u;
-                    if (j >= 0 && j <= m) {
+                    uint32_t out = BANDED ? NEG2 : 0u;
+                    /* the rows outside the band: bit r of mo for strip A, bit 16 +
+                     * r for strip B (whose column is j - 1) */
+                    uint32_t mo = 0u;
+                    if (BANDED) {
+                        const int d = R0 - j;
+                        const int a0 = min(max(lo - d, 0), R), a1 = min(max(hi - d + 1, 0), R);
+                        const int b0 = min(max(lo - d - R - 1, 0), R), b1 = min(max(hi - d - R, 0), R);
+                        const uint32_t ma = ~((1u << a1) - (1u << a0)), mb = ~((1u << b1) - (1u << b0));
+                        mo = (a1 > a0 ? ma & 0xffu : 0xffu) | ((b1 > b0 ? mb & 0xffu : 0xffu) << 16);
+                    }
+                    constexpr uint32_t rows_mask = 0x10001u * ((1u << R) - 1u);
+                    const bool active = j >= jlo && j <= jhi + 1;
+                    const bool masked = BANDED && __any_sync(0xffffffffu, active && (mo & rows_mask));
+                    if (active) {
                         uint32_t hd = dg, aop = 0u;
                         dg = hu;
+                        auto rows = [&](auto mask_tag) {
+                        constexpr bool MASK = decltype(mask_tag)::value;
 #pragma unroll
                         for (int r = 0; r < R; ++r) {
                             uint32_t sc;
@@ -642,9 +736,20 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
                             }
                             const uint32_t e = __viaddmax_s16x2(E[r], gE, H[r]);
                             const uint32_t a = __viaddmax_s16x2(hd, sc, e);
-                            const uint32_t ao = __vadd2(a, gO);
+                            uint32_t ao = __vadd2(a, gO);
                             const uint32_t f = __viaddmax_s16x2(fu, gE, r == 0 ? hu : aop);
-                            const uint32_t h = __viaddmax_s16x2(f, gO, ao);
+                            uint32_t fm = f;
+                            if (MASK) {
+                                /* 0xffff where the row is outside: its source of
+                                 * F and its H are -infinity. Its E and F need no
+                                 * mask: E leaves the band for good to the right
+                                 * and starts at -infinity on the left, F leaves it
+                                 * for good below and starts so above. */
+                                const uint32_t out2 = nw_signs(mo << (15 - r));
+                                ao = (ao & ~out2) | (NEG2 & out2);
+                                fm = (f & ~out2) | (NEG2 & out2);
+                            }
+                            const uint32_t h = __viaddmax_s16x2(fm, gO, ao);
                             E[r] = e;
                             hd = H[r];
                             H[r] = h;
@@ -652,16 +757,19 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
                             fu = f;
                             aop = ao;
                         }
+                        };
+                        if (BANDED && masked) rows(std::integral_constant<bool, true>());
+                        else rows(std::integral_constant<bool, false>());
                         out = __byte_perm(hu, fu, 0x7632);
                         prev_h = hu;
                         prev_f = fu;
-                        if (j == 0) {
+                        if (j == jlo) {
                             /* strip B has not begun: its left boundary again */
 #pragma unroll
                             for (int r = 0; r < R; ++r) {
-                                const uint32_t lb = (uint32_t)(uint16_t)(left(R0 + R + r) - base) << 16;
+                                const uint32_t lb = (uint32_t)(uint16_t)left_rel(R0 + R + r) << 16;
                                 H[r] = (H[r] & 0xffffu) | lb;
-                                E[r] = (E[r] & 0xffffu) | lb;
+                                E[r] = (E[r] & 0xffffu) | (BANDED ? NEG2 & 0xffff0000u : lb);
                             }
                         }
                     }
@@ -671,7 +779,7 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
 #pragma unroll
                     for (int k = 0; k < W; ++k) { wa[k] = na[k]; wb[k] = nb[k]; }
                     if (more) {
-                        if (lane == 31 && (unsigned)(j - 1) < (unsigned)m) out_buf[j - 1] = make_int2((int)out, base);
+                        if (lane == 31 && j - 1 >= jlo && j - 1 <= jhi) out_buf[j - 1] = make_int2((int)out, base);
                     } else if ((unsigned)(j - (m - 1)) <= 1u && (unsigned)ra < 2u * R) {
                         /* the corner: strip A at j = m - 1, strip B at j = m */
                         const int h = ra >= R ? 1 : 0;
@@ -686,16 +794,40 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
                     }
                 }
                 /* columns up to t0 - 32 are out */
-                if (more && !p.solo && lane == 31 && t0 >= 32)
-                    out_prog.store(out_base + min(t0 - 32, m - 1), cuda::memory_order_release);
+                if (more && !p.solo && lane == 31 && t0 - 32 >= jlo)
+                    out_prog.store(out_base + min(t0 - 32, jhi), cuda::memory_order_release);
             }
             if (aborted) break;
-            if (more && !p.solo && lane == 31) out_prog.store(out_base + m - 1, cuda::memory_order_release);
+            if (more && !p.solo && lane == 31) out_prog.store(out_base + jhi, cuda::memory_order_release);
             if (p.solo) __threadfence_block();
             __syncwarp();
             /* the corner's owner publishes the result */
             if (have_result) p.score[pid] = result;
         }
+        if (!(BANDED && p.cert)) break;
+        /* every thread of the team reads the one published score, so all
+         * take the same branch (and the same barriers) below */
+        if (coop) cluster.sync(); else __syncthreads();
+        const int sc = *(volatile int *)&p.score[pid];
+        const bool whole = lo <= -(m + 1) && hi >= n + 1;
+        bool ok = whole;
+        if (!whole && cert_valid(p.cm)) ok = cost2_of(p.cm, n, m, sc) <= exit_cost2(p.cm, n, m, lo, hi);
+        if (ok || round == 1) break;
+        if (cert_valid(p.cm)) {
+            int l2, h2;
+            label_band(p.cm, n, m, cost2_of(p.cm, n, m, sc), &l2, &h2);
+            lo = min(lo, l2);
+            hi = max(hi, h2);
+        } else {
+            lo = -(m + 1);
+            hi = n + 1;
+        }
+        if (threadIdx.x == 0 && (!coop || crank == 0)) {
+            p.lo_out[pid] = lo;
+            p.hi_out[pid] = hi;
+            p.rounds[pid] = 2;
+        }
+        }   /* rounds */
     }
     /* no CTA leaves while another of its cluster may still read its pair */
     if (coop) cluster.sync();
@@ -709,12 +841,14 @@ __global__ void k_iota_nw(int *v, int n)
 
 /* sort key: the pair's work (cells, or for a band its rows x the columns
  * its passes sweep); the total goes to total[0] for k_team_class, the rows'
- * to total[1] */
+ * to total[1]; total[2] is set when a band misses diagonal 0 or the
+ * corner's, so that cells inside it cannot be reached */
 __global__ void k_cells(const int *ql, const int *tl, const int *lo, const int *hi, int n,
                         unsigned long long *keys, unsigned long long *total)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long k = 0, rows = i < n ? (unsigned long long)ql[i] : 0ull;
+    if (i < n && lo && (lo[i] > 0 || hi[i] < 0 || ql[i] - tl[i] < lo[i] || ql[i] - tl[i] > hi[i])) total[2] = 1ull;
     if (i < n) {
         const unsigned long long cols = lo ? (unsigned long long)min((long long)tl[i],
                                                   (long long)hi[i] - lo[i] + 32 * NWL_RL)
@@ -778,10 +912,11 @@ __global__ void k_team_class(const int *ql, const int *tl, const int *lo, const 
  * base? (See there; 64 x 8 rows, 64 columns of skew, 32 of drift and 32 of
  * the chunk ahead, twice for the columns at the target's end; a few values
  * of open, gap and score beside H.) */
-static bool nw16_ok(int mmax, int open, int gap)
+static bool nw16_ok(int mmax, int open, int gap, bool banded)
 {
     const long long step = (long long)mmax + open;
-    return step * (512 + 256) + 4LL * (open + gap + 128) <= 32000;
+    return step * (512 + 256) + 4LL * (open + gap + 128) <= (banded ? -pb::NW16_OUT - 1000 : 32000) &&
+           open + gap + 128 <= 1700;
 }
 
 /* Global alignment scores of npairs device-resident pairs (codes), query i =
@@ -824,7 +959,6 @@ static int nw_long_impl(int npairs, int open, int gap, const int32_t *h_mat, int
     }
     if (bias)
         for (int k = 0; k < msize * msize; ++k) hm[k] = (int8_t)(h_mat[k] + open);
-    const bool use16 = !d_lo && bias && nw16_ok(mmax, open, gap);
     /* the work-queue buffers, each checked before any launch writes
      * through it; a failure frees what was allocated and ends the call */
     auto give_up = [&]() {
@@ -849,20 +983,23 @@ static int nw_long_impl(int npairs, int open, int gap, const int32_t *h_mat, int
         return give_up();
     cudaMemcpyAsync(d_mat, hm.data(), hm.size(), cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(counter, 0, sizeof(int) * 32, st);
-    /* counter[0..7]: pair counters of the class launches; [8..11]: total
-     * work and rows; [12]: the solo launch's counter; [16..24]: pairs per
+    /* counter[0..7]: pair counters of the class launches; [8..13]: total
+     * work, rows, bands; [14]: the solo launch's counter; [16..24]: pairs per
      * class, solo ones last */
     unsigned long long *total = reinterpret_cast<unsigned long long *>(counter + 8);
     pb::k_iota_nw<<<(npairs + 255) / 256, 256, 0, st>>>(idx, npairs);
     pb::k_cells<<<(npairs + 255) / 256, 256, 0, st>>>(d_qlen, d_tlen, d_lo, d_hi, npairs, keys, total);
     /* rows per strip in 16 bits: 8 (the fewest instructions per cell), or 4
      * where passes of 512 rows are fewer than the resident warps */
-    unsigned long long tot[2] = {0, 0};
+    unsigned long long tot[3] = {0, 0, 0};
     cudaMemcpyAsync(tot, total, sizeof tot, cudaMemcpyDeviceToHost, st);
     cudaStreamSynchronize(st);
-    const int r16 = tot[1] / 512 + (unsigned long long)npairs / 2 >= (unsigned long long)nsm * 16 ? 8 : 4;
+    const bool use16 = bias && nw16_ok(mmax, open, gap, d_lo != nullptr) && tot[2] == 0;
+    /* (in a band 4: passes of 256 rows keep more warps busy and fewer columns
+     * at its edges) */
+    const int r16 = d_lo ? 4 : tot[1] / 512 + (unsigned long long)npairs / 2 >= (unsigned long long)nsm * 16 ? 8 : 4;
     void (*kern)(pb::NwWaveParams, int *, int *) =
-        use16 ? (r16 == 8 ? pb::k_nw_wave16<8> : pb::k_nw_wave16<4>) :
+        use16 ? (d_lo ? pb::k_nw_wave16<4, true> : r16 == 8 ? pb::k_nw_wave16<8, false> : pb::k_nw_wave16<4, false>) :
         d_lo ? (bias ? pb::k_nw_wave<true, true, true> : ge ? pb::k_nw_wave<true, true, false>
                                                             : pb::k_nw_wave<true, false, false>)
              : (bias ? pb::k_nw_wave<false, true, true> : ge ? pb::k_nw_wave<false, true, false>
@@ -904,7 +1041,7 @@ static int nw_long_impl(int npairs, int open, int gap, const int32_t *h_mat, int
     }
     pb::k_team_class<<<(npairs + 255) / 256, 256, 0, st>>>(d_qlen, d_tlen, d_lo, d_hi, npairs,
                                                            plain_max * pb::NWL_WARPS, pol, pass_rows,
-                                                           use16 ? 0.5f : 0.0f, total, keys, counter + 16);
+                                                           use16 && !d_lo ? 0.5f : 0.0f, total, keys, counter + 16);
     pb_diag_count_launch(3);
     cub::DeviceRadixSort::SortPairsDescending(nullptr, tmpb, keys, keys_sorted, idx, order, npairs, 0, 64, st);
     if (cudaMallocAsync(&tmp, tmpb, st) != cudaSuccess) return give_up();
@@ -1004,7 +1141,7 @@ static int nw_long_impl(int npairs, int open, int gap, const int32_t *h_mat, int
             ps.npairs = nsolo; ps.order = order + before; ps.keys = keys_sorted + before;
             ps.scratch = scratch + slot * p.maxlen;
             ps.prog = prog + slot;
-            kern<<<sblocks, pb::NWL_WARPS * 32, smem, ss>>>(ps, counter + 12, d_err);
+            kern<<<sblocks, pb::NWL_WARPS * 32, smem, ss>>>(ps, counter + 14, d_err);
             ++nlaunch;
             cudaEventRecord(evc[pb::NWL_CLASSES], ss);
             cudaStreamWaitEvent(st, evc[pb::NWL_CLASSES], 0);

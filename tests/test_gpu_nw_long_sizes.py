@@ -55,3 +55,23 @@ def test_nw_long_drift():
     _check(m, [p[0] for p in pairs], [p[1] for p in pairs], 8, 2)
     pairs += [(rand_seq(rng, rng.randint(1, 900), DNA), rand_seq(rng, rng.randint(1, 900), DNA)) for _ in range(300)]
     _check(m, [p[0] for p in pairs], [p[1] for p in pairs], 8, 2)
+
+
+@pytest.mark.parametrize("alphabet,open_,gap", [(DNA, 5, 2), (AA, 11, 1)])
+def test_bands_of_long_pairs(alphabet, open_, gap):
+    """Bands over many passes: narrow ones that a lane leaves between two
+    checks of the base, ones as wide as a pass, scores outside 16 bits, and
+    targets much shorter and longer than the query."""
+    rng = random.Random(gap)
+    m = pb.matrix_create("ACGT", 2, -3) if alphabet is DNA else pb.matrix_lookup("blosum62")
+    om = O.Matrix.from_struct(m)
+    queries, targets = [], []
+    for n in (254, 256, 258, 1300, 2047, 6000):
+        q = rand_seq(rng, n, alphabet)
+        queries += [q, q, q]
+        targets += [mutate(rng, q, alphabet, 0.1, 0.02), rand_seq(rng, n // 2 + 1, alphabet),
+                    q + rand_seq(rng, 300, alphabet)]
+    for k in (1, 2, 3, 8, 33, 130, 257, 700):
+        got = pb.nw_banded_batch(m, queries, targets, open_, gap, k)
+        for q, t, g in zip(queries, targets, got):
+            assert g == O.nw_banded(q, t, open_, gap, k, om)["score"], (k, len(q), len(t))
