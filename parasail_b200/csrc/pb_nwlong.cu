@@ -646,6 +646,10 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
                 return __vadd2((uint32_t)x.x, 0x10001u * (uint32_t)(uint16_t)(x.y - base));
             };
             const int tend = jhi + 64;               /* iterations jlo .. tend - 1 */
+            /* iterations in which every lane works on columns past its first
+             * and before the last two, all its rows inside the band */
+            const int in_from = BANDED ? max(jlo, r0 + ROWS - hi) + 63 : 63;
+            const int in_to = BANDED ? min(r0 - lo, jhi - 1) : m - 2;
             const int ra = n - 1 - R0;               /* the corner's row among this lane's */
             int result = 0;
             bool have_result = false, aborted = false;
@@ -692,7 +696,12 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
                 put(t0 + 32 + lane, pre);
                 pre = fetch(t0 + 64 + lane);
                 __syncwarp();
-                const int n_it = min(32, tend - t0);
+                /* 32 iterations; EDGE: some lane has not begun or has ended, holds
+                 * rows outside the band, or meets the corner */
+                auto chunk = [&](auto edge_tag) {
+                constexpr bool EDGE = decltype(edge_tag)::value;
+                constexpr bool MASK = EDGE && BANDED;
+                const int n_it = EDGE ? min(32, tend - t0) : 32;
                 int off = ring[(t0 - 2 * lane + 1) & 127];
 #pragma unroll 2
                 for (int it = 0; it < n_it; ++it) {
@@ -707,23 +716,19 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
                     uint32_t fu = __byte_perm(v, prev_f, 0x5432);
                     uint32_t out = BANDED ? NEG2 : 0u;
                     /* the rows outside the band: bit r of mo for strip A, bit 16 +
-                     * r for strip B (whose column is j - 1) */
+                     * r for strip B. Strip B's row r lies R + 1 + r diagonals
+                     * below strip A's row 0 (its column is j - 1), so both are
+                     * bits of one interval. */
                     uint32_t mo = 0u;
-                    if (BANDED) {
+                    if (MASK) {
                         const int d = R0 - j;
-                        const int a0 = min(max(lo - d, 0), R), a1 = min(max(hi - d + 1, 0), R);
-                        const int b0 = min(max(lo - d - R - 1, 0), R), b1 = min(max(hi - d - R, 0), R);
-                        const uint32_t ma = ~((1u << a1) - (1u << a0)), mb = ~((1u << b1) - (1u << b0));
-                        mo = (a1 > a0 ? ma & 0xffu : 0xffu) | ((b1 > b0 ? mb & 0xffu : 0xffu) << 16);
+                        const int x0 = min(max(lo - d, 0), 2 * R + 1), x1 = min(max(hi - d + 1, 0), 2 * R + 1);
+                        const uint32_t ms = ~((1u << x1) - (1u << x0)) & ((2u << (2 * R)) - 1u);
+                        mo = ms | (ms << (15 - R));
                     }
-                    constexpr uint32_t rows_mask = 0x10001u * ((1u << R) - 1u);
-                    const bool active = j >= jlo && j <= jhi + 1;
-                    const bool masked = BANDED && __any_sync(0xffffffffu, active && (mo & rows_mask));
-                    if (active) {
+                    if (!EDGE || (j >= jlo && j <= jhi + 1)) {
                         uint32_t hd = dg, aop = 0u;
                         dg = hu;
-                        auto rows = [&](auto mask_tag) {
-                        constexpr bool MASK = decltype(mask_tag)::value;
 #pragma unroll
                         for (int r = 0; r < R; ++r) {
                             uint32_t sc;
@@ -757,13 +762,10 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
                             fu = f;
                             aop = ao;
                         }
-                        };
-                        if (BANDED && masked) rows(std::integral_constant<bool, true>());
-                        else rows(std::integral_constant<bool, false>());
                         out = __byte_perm(hu, fu, 0x7632);
                         prev_h = hu;
                         prev_f = fu;
-                        if (j == jlo) {
+                        if (EDGE && j == jlo) {
                             /* strip B has not begun: its left boundary again */
 #pragma unroll
                             for (int r = 0; r < R; ++r) {
@@ -779,8 +781,9 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
 #pragma unroll
                     for (int k = 0; k < W; ++k) { wa[k] = na[k]; wb[k] = nb[k]; }
                     if (more) {
-                        if (lane == 31 && j - 1 >= jlo && j - 1 <= jhi) out_buf[j - 1] = make_int2((int)out, base);
-                    } else if ((unsigned)(j - (m - 1)) <= 1u && (unsigned)ra < 2u * R) {
+                        if (lane == 31 && (!EDGE || (j - 1 >= jlo && j - 1 <= jhi)))
+                            out_buf[j - 1] = make_int2((int)out, base);
+                    } else if (EDGE && (unsigned)(j - (m - 1)) <= 1u && (unsigned)ra < 2u * R) {
                         /* the corner: strip A at j = m - 1, strip B at j = m */
                         const int h = ra >= R ? 1 : 0;
                         if (j - (m - 1) == h) {
@@ -793,6 +796,9 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
                         }
                     }
                 }
+                };
+                if (t0 >= in_from && t0 + 31 <= in_to) chunk(std::integral_constant<bool, false>());
+                else chunk(std::integral_constant<bool, true>());
                 /* columns up to t0 - 32 are out */
                 if (more && !p.solo && lane == 31 && t0 - 32 >= jlo)
                     out_prog.store(out_base + min(t0 - 32, jhi), cuda::memory_order_release);
