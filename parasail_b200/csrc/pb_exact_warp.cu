@@ -197,8 +197,9 @@ k_exact_warp(ExactParams p, int nitems)
                 const int en = max(e_opn, e_ext);
                 const int hdag = hd + sc;
                 const int ht = max(hdag, en);
-                int hn = max(ht, fn);
-                if (ALG == PB_SW) hn = max(hn, 0);
+                const int h0 = max(ht, fn);
+                /* SW: max(h0, 0) */
+                const int hn = ALG == PB_SW ? h0 & ~(h0 >> 31) : h0;
                 int hM = 0, hS = 0, hL = 0, fM = 0, fS = 0, fL = 0;
                 if (STATS) {
                     /* src/sw_stats.c:205-237: gap-source choice by strict >,
@@ -213,13 +214,17 @@ k_exact_warp(ExactParams p, int nitems)
                     const int eS = eo ? HlS[r] : ES[r];
                     const int eL = (eo ? HlL[r] : EL[r]) + 1;
                     EM[r] = eM; ES[r] = eS; EL[r] = eL;
-                    const bool isd = hn == hdag, isf = hn == fn;
+                    /* the choices from the operands: maxima compared with their
+                     * own operands lost SW's counts in the per-pair query form
+                     * (right scores, counts that no path gives) */
+                    const bool isd = (int)((unsigned)hdag - (unsigned)max(en, fn)) >= 0;
+                    const bool isf = (int)((unsigned)fn - (unsigned)en) >= 0;
                     const int mt = real ? ((PAIRS ? qc[r] : (int)pd.qcodes[i]) == code) : 0;
                     hM = isd ? hdM + mt : (isf ? fM : eM);
                     hS = isd ? hdS + (sc > 0) : (isf ? fS : eS);
                     hL = isd ? hdL + 1 : (isf ? fL : eL);
                     if (ALG == PB_SW) {
-                        const bool z = hn <= 0;
+                        const bool z = h0 <= 0;
                         hM = z ? 0 : hM;
                         hS = z ? 0 : hS;
                         hL = z ? 0 : hL;

@@ -100,3 +100,23 @@ def test_batch_cigars_equal_single_ones(alg):
         got = pb.batch_pairs_cigar("%s_trace%s" % (alg, form), m, qs, ts, 11, 1)
         for q, t, g in zip(qs, ts, got):
             assert g == pb.trace("parasail_%s_trace%s" % (alg, form), q, t, 11, 1, m), (alg, form, q, t)
+
+
+@pytest.mark.parametrize("name", ["sw_stats_striped_32", "sw_stats_striped_sat", "sw_stats_scan_32"])
+def test_local_statistics_with_pairs_past_16_bits(name):
+    """Local statistics in one pass: pairs that the 16-bit kernels take beside
+    pairs past their bounds (whose score runs on the exact kernel and whose
+    prefix pass follows alone), paths over many blocks and passes, scores of
+    0, and ends in the first row and column."""
+    rng = random.Random(7)
+    m = pb.matrix_lookup("blosum62")
+    om = O.Matrix.from_struct(m)
+    long_a, long_b = rand_seq(rng, 3100, AA), rand_seq(rng, 3050, AA)
+    queries = ["W" * 3000, long_a, long_a[:2950], "W", "A", "G" * 40]
+    targets = ["W" * 2990, mutate(rng, long_a, AA, 0.5, 0.02), long_b, "W", "W", "W" * 40]
+    for _ in range(60):
+        q = rand_seq(rng, rng.randint(1, 700), AA)
+        queries.append(q)
+        targets.append(rand_seq(rng, rng.randint(0, 200), AA) +
+                       (mutate(rng, q, AA, 0.4, 0.03) if rng.random() < 0.7 else rand_seq(rng, rng.randint(1, 700), AA)) or "A")
+    _check(name, pb.batch_pairs(name, m, queries, targets, 11, 1), queries, targets, 11, 1, om)
