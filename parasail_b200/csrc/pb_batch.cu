@@ -67,17 +67,31 @@ __global__ void k_max_int(const int *__restrict__ v, int n, int *__restrict__ ou
     if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
 
-/* prefix limits of the FASTSTATS stats pass; pairs that need none get a
- * 1x1 problem */
-__global__ void k_prefix_limits(pb_job job, const pb_pair_out *__restrict__ o1, int n,
+/* prefix limits of the FASTSTATS stats pass (of all pairs, or of the n
+ * listed); pairs that need none get a 1x1 problem */
+__global__ void k_prefix_limits(pb_job job, const pb_pair_out *__restrict__ o1, int n, const int *__restrict__ list,
                                 int *__restrict__ qlim, int *__restrict__ tlim)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const int i = list ? list[k] : k;
     const pb_pair_out a = o1[i];
     const bool need = pb_needs_pass2(&job, &a);
     qlim[i] = need ? a.end_query + 1 : 1;
     tlim[i] = need ? a.end_ref + 1 : 1;
+}
+
+__global__ void k_fill_int(int *__restrict__ v, size_t n, int x)
+{
+    const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (i < n) v[i] = x;
+}
+
+__global__ void k_copy_outs(const pb_pair_out *__restrict__ src, const int *__restrict__ list, int n,
+                            pb_pair_out *__restrict__ dst)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n) dst[list[k]] = src[list[k]];
 }
 
 /*
@@ -214,6 +228,9 @@ extern "C" int pb_cuda_batch_run(const pb_job *job, const pb_batch *tmpl, pb_rec
     if (cudaMallocAsync((void **)&o1, sizeof(pb_pair_out) * nitems, st) != cudaSuccess) rc = -1;
     const bool faststats = pb_job_is_faststats(job);
     int *rest = nullptr;      /* items the 16-bit pair kernels leave to the exact kernel */
+    /* FASTSTATS: items that still need the prefix pass (-1: all of them) */
+    int prefix_left = -1, *left = nullptr;
+    pb_pair_out *o2b = nullptr;
     if (rc == 0 && faststats &&
         (cudaMallocAsync((void **)&o2, sizeof(pb_pair_out) * nitems, st) != cudaSuccess ||
          cudaMallocAsync((void **)&qlim, sizeof(int) * nitems, st) != cudaSuccess ||
@@ -247,7 +264,16 @@ extern "C" int pb_cuda_batch_run(const pb_job *job, const pb_batch *tmpl, pb_rec
          * the pair kernels cannot take */
         const bool wave = pb::wave_ok(*job, &b);
         rc = pb::p16_pass(*job, &b, 0, nullptr, o1, group, rest, &nrest, st, nullptr, nullptr, nullptr,
-                          wave ? pb::pb_schedule_nw_mask() : 0u);
+                          wave ? pb::pb_schedule_nw_mask() : 0u, faststats ? o2 : nullptr);
+        if (rc == 0 && faststats) {
+            /* the prefix outputs are there already (the traceback runs from the
+             * score pass's own checkpoints), except those of the rest */
+            prefix_left = nrest;
+            if (nrest > 0 &&
+                (cudaMallocAsync((void **)&left, sizeof(int) * (size_t)nrest, st) != cudaSuccess ||
+                 cudaMemcpyAsync(left, rest, sizeof(int) * (size_t)nrest, cudaMemcpyDeviceToDevice, st) != cudaSuccess))
+                rc = -1;
+        }
         if (rc == 0 && wave && nrest > 0) {
             int *rest2 = nullptr, nrest2 = 0;
             if (cudaMallocAsync((void **)&rest2, sizeof(int) * (size_t)nrest, st) != cudaSuccess) rc = -1;
@@ -258,22 +284,42 @@ extern "C" int pb_cuda_batch_run(const pb_job *job, const pb_batch *tmpl, pb_rec
         }
         if (rc == 0 && nrest > 0) rc = pb::exact_subset(&b, rest, nrest, b.stats, b.pad_rows, o1, st);
     }
-    if (rc == 0 && faststats) {
-        /* the prefix statistics pass of every item: limits per (query,
-         * target) item, query-major like o1; statistics by the direction-bit
-         * walk from the score pass's ends */
-        pb::k_prefix_limits<<<(int)((nitems + 255) / 256), 256, 0, st>>>(*job, o1, (int)nitems, qlim, tlim);
-        pb_diag_count_launch(1);
-        if (cudaStreamSynchronize(st) != cudaSuccess) rc = -1;
+    if (rc == 0 && faststats && prefix_left != 0) {
+        /* the prefix statistics pass: of every item (after the database score
+         * kernel), or of those that the pair kernels left, the others then
+         * being problems of one cell. Limits per (query, target) item,
+         * query-major like o1; statistics by the traceback from the score
+         * pass's ends. */
+        const bool some = prefix_left > 0;
+        pb_pair_out *o = o2;
+        if (some) {
+            if (cudaMallocAsync((void **)&o2b, sizeof(pb_pair_out) * nitems, st) != cudaSuccess) rc = -1;
+            o = o2b;
+        }
+        if (rc == 0 && some) {
+            pb::k_fill_int<<<(unsigned)((nitems + 255) / 256), 256, 0, st>>>(qlim, nitems, 1);
+            pb::k_fill_int<<<(unsigned)((nitems + 255) / 256), 256, 0, st>>>(tlim, nitems, 1);
+            pb_diag_count_launch(2);
+        }
+        if (rc == 0) {
+            const int nl = some ? prefix_left : (int)nitems;
+            pb::k_prefix_limits<<<(nl + 255) / 256, 256, 0, st>>>(*job, o1, nl, some ? left : nullptr, qlim, tlim);
+            pb_diag_count_launch(1);
+            if (cudaStreamSynchronize(st) != cudaSuccess) rc = -1;
+        }
         pb_batch b2 = *tmpl;
         b2.stats = 1;
         b2.pad_rows = 32;
         b2.d_qlim = qlim;
         b2.d_tlim = tlim;
-        b2.d_out = o2;
+        b2.d_out = o;
         int nrest = 0;
-        if (rc == 0) rc = pb::p16_pass(*job, &b2, 1, o1, o2, group, rest, &nrest, st);
-        if (rc == 0 && nrest > 0) rc = pb::exact_subset(&b2, rest, nrest, 1, 32, o2, st);
+        if (rc == 0) rc = pb::p16_pass(*job, &b2, 1, o1, o, group, rest, &nrest, st);
+        if (rc == 0 && nrest > 0) rc = pb::exact_subset(&b2, rest, nrest, 1, 32, o, st);
+        if (rc == 0 && some) {
+            pb::k_copy_outs<<<(prefix_left + 255) / 256, 256, 0, st>>>(o2b, left, prefix_left, o2);
+            pb_diag_count_launch(1);
+        }
     }
     for (int q = 0; q < nq && rc == 0; ++q) {
         const int qall = tmpl->nprofs > 0 ? tmpl->profs[q]->qlen : 0;
@@ -285,6 +331,8 @@ extern "C" int pb_cuda_batch_run(const pb_job *job, const pb_batch *tmpl, pb_rec
     if (o1) cudaFreeAsync(o1, st);
     if (o2) cudaFreeAsync(o2, st);
     if (rest) cudaFreeAsync(rest, st);
+    if (left) cudaFreeAsync(left, st);
+    if (o2b) cudaFreeAsync(o2b, st);
     if (qlim) cudaFreeAsync(qlim, st);
     if (tlim) cudaFreeAsync(tlim, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) rc = -1;

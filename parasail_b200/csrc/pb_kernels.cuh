@@ -131,8 +131,8 @@ struct P16Params {
     const int *order;             /* sorted position -> item */
     const int *rows, *cols;       /* per item: query rows (or prefix limit) and target columns */
     const int *task_wmax, *task_npass;
-    const long long *task_bits;   /* per task: first uint4 of its direction bits in `bits` */
-    uint4 *bits;
+    const long long *task_ckpt;   /* per task: first uint4 of its checkpoints in `ckpt` */
+    uint4 *ckpt;
     const int8_t *mat8;           /* pairs mode: [target letter][query letter] int8, else nullptr */
     const int32_t *mat32;         /* pairs mode: the same in int32 (the statistics walk) */
     const uint8_t *qall;
@@ -145,6 +145,7 @@ struct P16Params {
     uint4 *colsave;               /* SW ends, per resident thread: its strips' best columns (8 x 16 bytes) */
     int maxlen;
     pb_pair_out *out;
+    pb_pair_out *out2;            /* FASTSTATS in one pass: the prefix outputs */
     /* traceback paths (optional): per item, steps written backwards into
      * ops[ops_off[item] .. + rows + cols), and path_info[3 * item] = steps,
      * the row and the column where the walk stopped */
@@ -165,7 +166,7 @@ struct P16Setup {
     unsigned intra_mask;
 };
 
-/* columns that a pass of the pair kernels runs (and stores bits for) over a
+/* columns that a pass of the pair kernels runs (and stores) over a
  * task whose widest target has wmax columns: strip B ends one column behind
  * strip A, and four columns go together */
 __host__ __device__ inline int p16_cols(int wmax) { return (wmax + 4) & ~3; }
@@ -179,8 +180,9 @@ __host__ __device__ inline int p16_bucket(int rows, int cols)
 }
 
 /* Runs the items of batch b that fit 16-bit lanes on the pair kernels:
- * scores and ends (prefix = 0), with statistics by the direction-bit walk
- * when the job has them; or (prefix = 1, the FASTSTATS prefix pass, b
+ * scores and ends (prefix = 0), with statistics by the traceback
+ * when the job has them; with out2 (a FASTSTATS job) also the prefix outputs,
+ * by the traceback from the same pass's ends; or (prefix = 1, the FASTSTATS prefix pass, b
  * carrying qlim/tlim) statistics only, walked from the ends in `ends`.
  * Items outside the 16-bit bounds, and items whose width verdicts need
  * exact extremes, are listed in d_rest (*n_rest of them, device memory of
@@ -189,7 +191,7 @@ __host__ __device__ inline int p16_bucket(int rows, int cols)
 int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out *ends, pb_pair_out *out,
              const int *group, int *d_rest, int *n_rest, cudaStream_t st,
              uint8_t *d_ops = nullptr, const int64_t *d_ops_off = nullptr, int *d_path_info = nullptr,
-             unsigned intra_mask = 0);
+             unsigned intra_mask = 0, pb_pair_out *out2 = nullptr);
 /* Global score-only pairs (pairs mode) on the intra-task wavefront kernel
  * (pb_nwlong.cu): the listed items of b, scores and ends into out with
  * sound bounds for the width verdicts; items whose verdicts need exact

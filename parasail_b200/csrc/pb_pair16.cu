@@ -1,7 +1,7 @@
 /*
  * pb_pair16.cu -- global (NW), semi-global (SG) and local (SW) alignment of
  * batches of independent pairs in packed int16x2 lanes, with statistics
- * (matches, similar, length) from a traceback walk over direction bits.
+ * (matches, similar, length) and paths from a traceback over checkpoints.
  *
  * Inter-task schedule: one thread aligns one pair; a warp takes a task of
  * 32 pairs of like size (items sorted by passes and columns); a persistent
@@ -11,7 +11,7 @@
  * A (rows r0..r0+15) at column j, the high half strip B (rows r0+16..r0+31)
  * at column j-1, so strip B reads strip A's bottom row from the previous
  * iteration. A pass hands its bottom row (H and F) to the next pass through
- * the warp's buffer laid out [column][lane] (one 256-byte transaction per
+ * the warp's buffer laid out [column][lane] (one 128-byte transaction per
  * warp access). Each lane (pairs mode) or each warp (all 32 pairs of the
  * task share a query) stages the scores of the pass's 32 rows against every
  * alphabet letter in shared memory as int8 (a column's 16 + 16 scores are
@@ -41,15 +41,15 @@
  * every H, E and F, the counts of the one path its tie rules select: the
  * gap source by strict > (open only when H - open > E - gap), the cell
  * source diagonal, then F, then E; SW restarts at H <= 0 and the boundary
- * cells carry 0. Those counts are the counts along that path. With
- * statistics the kernel stores, per cell, the four decisions that define
- * the path: not-diagonal (H > H_diag + s), not-F (H > F), E opened and F
- * opened -- each the sign bit of an int16 difference, gathered into per-row
- * bits (p16_bit) of four words stored as one uint4 per lane per iteration. The walk
- * (k_p16_walk) then follows the path back from the end cell, adding 1 to
- * length per step and, on diagonal steps, the match and positive-score
- * indicators; in SW it stops where the running H value (the end score
- * minus the steps walked) reaches 0, in NW/SG at the boundary.
+ * cells carry 0. Those counts are the counts along that path, which four
+ * decisions per cell define: not-diagonal (H > H_diag + s), not-F (H > F), E
+ * opened and F opened. The forward kernel leaves checkpoints instead of the
+ * decisions -- every pass's bottom row, and its column state every P16_CK
+ * columns -- and the traceback (k_p16_trace) recomputes only the blocks that
+ * the path from the end cell crosses, adding 1 to length per step and, on
+ * diagonal steps, the match and positive-score indicators; in SW it stops
+ * where the running H value (the end score minus the steps walked) reaches
+ * 0, in NW/SG at the boundary.
  */
 #include <cstdio>
 #include <cstdint>
@@ -76,7 +76,26 @@ static constexpr int P16_R = 16;              /* rows per strip; two strips per 
 static constexpr int P16_PASS = 2 * P16_R;
 static constexpr int P16_ROW = 48;            /* bytes between two letters' scores in a shared slice */
 
-/* the bit of query row i of a task's direction bits (row i of its pass): the
+static constexpr int P16_TR_WARPS = 2;        /* warps per block of the traceback */
+/* Checkpoints of a task (one lane's words 32 apart): per pass its bottom row,
+ * p16_cols words (entry c + 1: H low and F high at column c), and per pass
+ * and block of P16_CK columns after the first the state before the block's
+ * first iteration: H and E of the 16 register rows, F of the last one, and
+ * the next diagonal. */
+static constexpr int P16_CK = 32, P16_CK_U4 = P16_R / 2 + 1;
+__host__ __device__ __forceinline__ int p16_ck_blocks(int wmax) { return (p16_cols(wmax) - 1) / P16_CK; }
+/* in words */
+__device__ __forceinline__ size_t p16_ck_row(int wmax, int pass, int entry)
+{
+    return ((size_t)pass * p16_cols(wmax) + entry) * 32;
+}
+/* in uint4 from the task's first */
+__host__ __device__ __forceinline__ size_t p16_ck_col(int npass, int wmax, int pass, int block)
+{
+    return (size_t)npass * p16_cols(wmax) * 8 + ((size_t)pass * p16_ck_blocks(wmax) + block) * P16_CK_U4 * 32;
+}
+
+/* the bit of query row i of a block's direction bits (row i of its pass): the
  * byte by the row's parity and strip, the bit by its pair of rows */
 __device__ __forceinline__ int p16_bit(int i) { return ((i & 1) * 2 + ((i >> 4) & 1)) * 8 + ((i & 15) >> 1); }
 
@@ -143,27 +162,27 @@ struct P16Best {
 /*
  * One task (32 items) per warp at a time. SHARED: every lane of a task has
  * the same query (its scores are staged once per warp); else every lane
- * stages its own. BITS: store the direction bits. ENDS: compute score and
- * ends (off for the FASTSTATS prefix pass, whose ends are known). BIAS (open
- * >= gap, every score + open inside int8): H registers and boundaries hold
- * H - open, staged scores s + open, so the gap sources need no add, and F of
- * the next row is max(F - gap, max(H_diag + s, E) - open).
+ * stages its own. CKPT: leave the checkpoints that the traceback restarts
+ * from (p16_ck_row, p16_ck_col). ENDS: compute score and ends (off for the
+ * FASTSTATS prefix pass, whose ends are known). BIAS (open >= gap, every
+ * score + open inside int8): H registers and boundaries hold H - open, staged
+ * scores s + open, so the gap sources need no add, and F of the next row is
+ * max(F - gap, max(H_diag + s, E) - open).
  *
  * What bounds it: the ALU pipe at half rate (maxima, three-operand DPX, byte
- * permutes, logic), with the packed adds and differences on the FMA pipe
- * beside it. Per row of two cells, score only: 5 ALU and 1 FMA operations;
- * with bits: 8 and 8 -- the four decisions are signs of differences, and one
- * permute gathers (and spreads over their bytes) the signs of two rows, of
- * which a mask keeps the pair's bit (2 per decision and row before, by
- * shifted accumulators). As in k_sw16, four columns run without a branch
- * each, targets are read by words (the code check of a byte load waited
- * for the load in every column), and the staged scores are laid out so
- * that 16-byte loads fall on all bank groups: [letter][48 bytes] per warp,
- * or [letter][strip][lane] x 16 bytes. 1 M DNA reads, NW statistics (bits):
- * 29.3 -> 23.0 ms; 524 k protein pairs all against all: score pass 93.5 ->
- * 65.7 ms (4,800 GCUPS), prefix bits pass 158 -> 115 ms.
+ * permutes), with the packed adds on the FMA pipe beside it: 5 ALU and 1 FMA
+ * operations per row of two cells. As in k_sw16, four columns run without a
+ * branch each, targets are read by words (the code check of a byte load
+ * waited for the load in every column), and the staged scores are laid out
+ * so that 16-byte loads fall on all bank groups: [letter][48 bytes] per
+ * warp, or [letter][strip][lane] x 16 bytes. The checkpoints add 8.5 bytes
+ * per column and lane (0.27 per cell), where the direction bits of every
+ * cell took 0.5 bytes and twice the operations.
+ * 1 M DNA reads, NW: 29.3 ms with direction bits, now 10.3 ms with
+ * checkpoints; 524 k protein pairs all against all: score pass 93.5 -> 72.7
+ * ms with checkpoints (65.7 without).
  */
-template <int ALG, bool BITS, bool ENDS, bool SHARED, int WARPS, bool BIAS>
+template <int ALG, bool CKPT, bool ENDS, bool SHARED, int WARPS, bool BIAS>
 __global__ void __launch_bounds__(WARPS * 32, (WARPS == 8 ? 2 : 3))
 k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
 {
@@ -235,7 +254,10 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
         const P16Bounds bd = p16_bounds(ALG, rows, cols, open, gap, p.mmax, p.mmin);
         const int negv = bd.lb - open - 1;
         const uint32_t NEG = p16_splat(negv);
-        uint4 *tbits = BITS ? p.bits + p.task_bits[task] + lane : nullptr;
+        /* the task's checkpoints: rows (entry c + 1 of a pass: its bottom row at
+         * column c), then columns */
+        uint32_t *ckr = CKPT ? reinterpret_cast<uint32_t *>(p.ckpt + p.task_ckpt[task]) + lane : nullptr;
+        uint4 *ckc = CKPT ? p.ckpt + p.task_ckpt[task] + p16_ck_col(npass, wmax, 0, 0) + lane : nullptr;
         int status = 0;
 
         /* end tracking */
@@ -344,11 +366,12 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
                                                                                            : (uint32_t)(uint16_t)(-gap);
             const uint32_t vnone = p16_prmt(0u, NEG, 0x5410u);
             const int rd = top ? 0 : wmax;
+            const uint32_t *in_row = CKPT ? ckr + (top ? 0 : p16_ck_row(wmax, pass - 1, 0)) : buf;
             uint32_t v_n[4];
 #pragma unroll
-            for (int x = 0; x < 4; ++x) v_n[x] = x < rd ? __ldcg(buf + (x + 1) * 32) : vnone;
-            const uint32_t *in_at = buf + 5 * 32;
-            uint32_t *out_at = buf;
+            for (int x = 0; x < 4; ++x) v_n[x] = x < rd ? __ldcg(in_row + (x + 1) * 32) : vnone;
+            const uint32_t *in_at = in_row + 5 * 32;
+            uint32_t *out_at = CKPT ? ckr + p16_ck_row(wmax, pass, 0) : buf;
             P16Best sa = {0, -1, -1}, sb = {0, -1, -1};
             /* SW: what a column maximum has to pass, as in k_sw16 */
             uint32_t sbest = p16_splat(max(best.score - 1, 0) - bias);
@@ -358,6 +381,16 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
             ResidueWords tw;
             tw.start(tseq, cols);
             for (int j0 = 0; j0 <= wmax; j0 += 4, in_at += 4 * 32, out_at += 4 * 32) {
+                if (CKPT && j0 > 0 && j0 % P16_CK == 0) {
+                    /* the state before iteration j0 */
+                    uint4 *d = ckc + ((size_t)pass * p16_ck_blocks(wmax) + j0 / P16_CK - 1) * P16_CK_U4 * 32;
+#pragma unroll
+                    for (int x = 0; x < P16_R / 4; ++x) {
+                        d[x * 32] = make_uint4(H[4 * x], H[4 * x + 1], H[4 * x + 2], H[4 * x + 3]);
+                        d[(x + P16_R / 4) * 32] = make_uint4(E[4 * x], E[4 * x + 1], E[4 * x + 2], E[4 * x + 3]);
+                    }
+                    d[P16_R / 2 * 32] = make_uint4(prev_f, dg, 0u, 0u);
+                }
                 uint32_t codes = tw.next(j0);
                 if ((codes | (codes + big4)) & 0x80808080u) {
                     /* codes outside the alphabet read as letter 0 */
@@ -384,8 +417,6 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
                     dg = hu;
                     uint32_t cmax = p16_splat(-bias);
                     uint32_t aop = 0u;               /* BIAS: the previous row's max(H_diag + s, E) - open */
-                    uint32_t aD = 0u, aF = 0u, aE = 0u, aV = 0u;
-                    uint32_t dD = 0u, dF = 0u, dE = 0u, dV = 0u;
 #pragma unroll
                     for (int r = 0; r < P16_R; ++r) {
                         const uint32_t wa = r < 4 ? pa4.x : r < 8 ? pa4.y : r < 12 ? pa4.z : pa4.w;
@@ -398,29 +429,7 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
                             default: sc = p16_pair<3>(wa, wb); break;
                         }
                         uint32_t e, f, hn;           /* hn: H, or H - open */
-                        if (BITS) {
-                            const uint32_t ho = BIAS ? H[r] : __vadd2(H[r], gO);
-                            const uint32_t fo = BIAS ? hu : __vadd2(hu, gO);
-                            const uint32_t ee = __vadd2(E[r], gE), fe = __vadd2(fu, gE);
-                            e = __vmaxs2(ho, ee);
-                            f = __vmaxs2(fo, fe);
-                            const uint32_t hdg = __vadd2(hd, sc);
-                            const uint32_t h = ALG == PB_SW ? __vimax3_s16x2_relu(hdg, e, f) : __vimax3_s16x2(hdg, e, f);
-                            hn = BIAS ? __vadd2(h, gO) : h;
-                            /* the decisions of this row; of two rows, their signs
-                             * as four bytes: strips A and B of the even row, then
-                             * of the odd one; bit r / 2 of each byte is kept */
-                            const uint32_t nD = __vsub2(hdg, h), nF = __vsub2(f, h);
-                            const uint32_t nE = __vsub2(ee, ho), nV = __vsub2(fe, fo);
-                            if (r & 1) {
-                                const uint32_t m = 0x01010101u << (r >> 1);
-                                aD |= p16_prmt(dD, nD, 0xfdb9u) & m;
-                                aF |= p16_prmt(dF, nF, 0xfdb9u) & m;
-                                aE |= p16_prmt(dE, nE, 0xfdb9u) & m;
-                                aV |= p16_prmt(dV, nV, 0xfdb9u) & m;
-                            }
-                            dD = nD; dF = nF; dE = nE; dV = nV;
-                        } else if (BIAS) {
+                        if (BIAS) {
                             e = __viaddmax_s16x2(E[r], gE, H[r]);
                             const uint32_t a = ALG == PB_SW ? __viaddmax_s16x2_relu(hd, sc, e) : __viaddmax_s16x2(hd, sc, e);
                             const uint32_t ao = __vadd2(a, gO);
@@ -440,7 +449,6 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
                         fu = f;
                         if (ENDS && ALG == PB_SW && (r & 1)) cmax = __vimax3_s16x2(cmax, H[r - 1], hn);
                     }
-                    if (BITS) tbits[((size_t)pass * p16_cols(wmax) + j) * 32] = make_uint4(aD, aF, aE, aV);
                     if (more) out_at[u * 32] = p16_prmt(hu, fu, 0x7632u);     /* column j - 1 */
                     prev_h = hu;
                     prev_f = fu;
@@ -584,164 +592,347 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
 }
 
 /*
- * The statistics walk of one item: from its end cell back along the path
- * the reference's tie rules select, reading the direction bits of the
- * item's task (lane = its position in the task). Writes matches, similar
- * and length into out[item].
- */
-template <int ALG>
-__global__ void k_p16_walk(P16Params p, const int *__restrict__ tlist, int ntl, const pb_pair_out *__restrict__ ends,
-                           int open, int gap)
-{
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= ntl * 32) return;
-    const int task = tlist[g >> 5], lane = g & 31;
-    const int s = task * 32 + lane;
-    if (s >= p.nitems) return;
-    const int item = p.order[s];
-    if (item < 0) return;
-    const int wmax = p.task_wmax[task];
-    const uint4 *tb = p.bits + p.task_bits[task];
-    const pb_pair_out e = ends[item];
-    const int ti = p.nt ? item % p.nt : item;
-    const uint8_t *tseq = p.targets + p.toff[ti];
-    const uint8_t *qseq;
-    const int32_t *prof32 = nullptr;
-    int lp = 0;
-    if (p.mat8) {
-        qseq = p.qall + p.qoff[item];
-    } else {
-        const ProfDesc pd = p.profs[p.nt ? item / p.nt : 0];
-        qseq = pd.qcodes;
-        prof32 = pd.prof;
-        lp = pd.lp;
-    }
-    const int L = p.nletters;
-    int i = e.end_query, j = e.end_ref;
-    int v = e.score;
-    pb_pair_out *o = p.out + item;
-    if (i >= p.rows[item] || j >= p.cols[item]) {
-        /* the end lies outside the computed region (a FASTSTATS item
-         * whose prefix pass was not needed): nothing to walk */
-        o->matches = o->similar = o->length = 0;
-        return;
-    }
-    int M = 0, S = 0, Ln = 0;
-    int state = 0;                                  /* 0 H, 1 F, 2 E */
-    const int limit = p.rows[item] + p.cols[item] + 2;
-    for (int step = 0; step <= 2 * limit; ++step) {
-        if (i < 0 || j < 0) break;
-        if (ALG == PB_SW && state == 0 && v <= 0) break;
-        const int half = (i >> 4) & 1, bit = p16_bit(i);
-        const uint4 w = tb[((size_t)(i >> 5) * p16_cols(wmax) + j + half) * 32 + lane];
-        if (state == 0) {
-            if (!((w.x >> bit) & 1u)) {
-                int qc = qseq[i], tc = tseq[j];
-                if (qc >= L) qc = 0;
-                if (tc >= L) tc = 0;
-                const int sc = p.mat32 ? p.mat32[tc * L + qc] : prof32[(size_t)tc * lp + i];
-                M += qc == tc;
-                S += sc > 0;
-                Ln += 1;
-                v -= sc;
-                --i;
-                --j;
-            } else {
-                state = ((w.y >> bit) & 1u) ? 2 : 1;
-            }
-        } else if (state == 1) {
-            Ln += 1;
-            if ((w.w >> bit) & 1u) { v += open; state = 0; } else { v += gap; }
-            --i;
-        } else {
-            Ln += 1;
-            if ((w.z >> bit) & 1u) { v += open; state = 0; } else { v += gap; }
-            --j;
-        }
-    }
-    o->matches = M;
-    o->similar = S;
-    o->length = Ln;
-}
-
-/*
- * The traceback path of one item: the walk of k_p16_walk, recording its
- * steps instead of counting them -- 0 a diagonal step (query and target
+ * The traceback of one task's items, a lane each: from its end cell back
+ * along the path the reference's tie rules select. A lane restarts the
+ * dynamic program at the checkpoint before its cell -- the column state at
+ * the start of the cell's block of P16_CK columns, the bottom row of the
+ * pass above -- and recomputes the block up to the cell with the direction
+ * bits of its 32 rows in shared memory, walks until it leaves the block, and
+ * goes on with the next one. The lanes of a warp run their blocks in step,
+ * each its own pass and columns, so a task takes as many blocks as its
+ * longest path: two per pass for a global alignment, a handful for the local
+ * alignment of unrelated sequences, where direction bits had to be computed
+ * and stored for the whole prefix before the end cell. All against all, 524 k
+ * protein pairs: 158 ms of prefix pass and walk -> 7.5 ms; 1 M reads, NW: 3.2
+ * ms of walk over stored bits -> 8.7 ms, against 19 ms less in the forward
+ * pass. Bound by latency: shared memory (the block's bits and the lane's
+ * scores) holds ten warps an SM for DNA, four for proteins.
+ *
+ * The bits (the four decisions of the file comment) are signs of differences;
+ * of two rows, one permute spreads the signs over four bytes (strips A and B
+ * of the even row, then of the odd one) of which a mask keeps bit r / 2: 8 ALU
+ * and 8 FMA operations per row of two cells.
+ *
+ * MODE 0: matches, similar and length into out[item]; 1 (FASTSTATS in one
+ * pass): the whole prefix output into out2[item], the bounds being those of
+ * the prefix up to the end cell; 2: the path's steps, written backwards from
+ * the end of the item's op buffer -- 0 a diagonal step (query and target
  * residue aligned), 1 a step up a vertical gap (a query residue against a
  * gap), 2 a step left along a horizontal gap (a target residue against a
- * gap) -- written backwards from the end of the item's op buffer, with
- * the cell where the walk stopped. These are the decisions the reference's
- * trace tables hold (src/sw_trace.c:138-147: DIAG when H == H_diag, else
- * DEL when H == F, else INS; DIAG_F / DIAG_E when the gap opened by strict
- * >), followed as its CIGAR builder does (src/cigar_template.c:143-243).
+ * gap) -- with the cell where the walk stopped. The decisions are those the
+ * reference's trace tables hold (src/sw_trace.c:138-147: DIAG when H ==
+ * H_diag, else DEL when H == F, else INS; DIAG_F / DIAG_E when the gap opened
+ * by strict >), followed as its CIGAR builder does (src/cigar_template.c:
+ * 143-243).
  */
-template <int ALG>
-__global__ void k_p16_path(P16Params p, const int *__restrict__ tlist, int ntl, const pb_pair_out *__restrict__ ends,
-                           int open, int gap)
+template <int ALG, int MODE, bool BIAS>
+__global__ void __launch_bounds__(P16_TR_WARPS * 32, 5)
+k_p16_trace(pb_job job, P16Params p, const int *__restrict__ tlist, int ntl, const pb_pair_out *__restrict__ ends,
+            int *counter)
 {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= ntl * 32) return;
-    const int task = tlist[g >> 5], lane = g & 31;
-    const int s = task * 32 + lane;
-    if (s >= p.nitems) return;
-    const int item = p.order[s];
-    if (item < 0) return;
-    const int wmax = p.task_wmax[task];
-    const uint4 *tb = p.bits + p.task_bits[task];
-    const pb_pair_out e = ends[item];
-    const int rows = p.rows[item], cols = p.cols[item];
-    const int cap = rows + cols;
-    uint8_t *ops = p.ops + p.ops_off[item];
-    int *info = p.path_info + 3 * (size_t)item;
-    int i = e.end_query, j = e.end_ref;
-    int v = e.score;
-    if (i >= rows || j >= cols || i < 0 || j < 0) {
-        info[0] = -1; info[1] = i; info[2] = j;
-        return;
-    }
-    const int ti = p.nt ? item % p.nt : item;
-    const uint8_t *tseq = p.targets + p.toff[ti];
-    const uint8_t *qseq;
-    const int32_t *prof32 = nullptr;
-    int lp = 0;
-    if (p.mat8) {
-        qseq = p.qall + p.qoff[item];
-    } else {
-        const ProfDesc pd = p.profs[p.nt ? item / p.nt : 0];
-        qseq = pd.qcodes;
-        prof32 = pd.prof;
-        lp = pd.lp;
-    }
+    extern __shared__ __align__(16) int8_t s_mem[];
+    constexpr int LETTER = 1024, STRIP = 512;
     const int L = p.nletters;
-    int n = 0, state = 0;                       /* 0 H, 1 F, 2 E */
-    for (int step = 0; step <= 2 * cap + 2 && n < cap; ++step) {
-        if (i < 0 || j < 0) break;
-        if (ALG == PB_SW && state == 0 && v <= 0) break;
-        const int half = (i >> 4) & 1, bit = p16_bit(i);
-        const uint4 w = tb[((size_t)(i >> 5) * p16_cols(wmax) + j + half) * 32 + lane];
-        if (state == 0) {
-            if (!((w.x >> bit) & 1u)) {
-                int qc = qseq[i], tc = tseq[j];
-                if (qc >= L) qc = 0;
-                if (tc >= L) tc = 0;
-                v -= p.mat32 ? p.mat32[tc * L + qc] : prof32[(size_t)tc * lp + i];
-                ops[cap - 1 - n++] = 0;
-                --i;
-                --j;
-            } else {
-                state = ((w.y >> bit) & 1u) ? 2 : 1;
-            }
-        } else if (state == 1) {
-            ops[cap - 1 - n++] = 1;
-            if ((w.w >> bit) & 1u) { v += open; state = 0; } else { v += gap; }
-            --i;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int open = p.open, gap = p.gap, sgf = p.sgflags;
+    const int bias = BIAS ? open : 0;
+    /* shared memory: [matrix L x L int8, padded to 16] then per warp [bits of
+     * a block][scores] */
+    const int mat_bytes = p.mat8 ? ((L * L + 15) & ~15) : 0;
+    int8_t *s_mat = s_mem;
+    int8_t *wmem = s_mem + mat_bytes + (size_t)wid * (P16_CK * 512 + L * LETTER);
+    uint4 *tile = reinterpret_cast<uint4 *>(wmem) + lane;
+    int8_t *sl = wmem + P16_CK * 512 + lane * 16;
+    if (p.mat8)
+        for (int x = threadIdx.x; x < L * L; x += blockDim.x) s_mat[x] = (int8_t)(p.mat8[x] + bias);
+    __syncthreads();
+    const uint32_t gO = p16_splat(-open), gE = p16_splat(-gap);
+    const uint32_t b4 = 0x01010101u * (uint32_t)(uint8_t)bias;
+
+    for (;;) {
+        int k = 0;
+        if (lane == 0) k = atomicAdd(counter, 1);
+        k = __shfl_sync(0xffffffffu, k, 0);
+        if (k >= ntl) break;
+        const int task = tlist[k];
+        const int s = task * 32 + lane;
+        const bool valid = s < p.nitems && p.order[s] >= 0;
+        const int item = valid ? p.order[s] : 0;
+        const int rows = valid ? p.rows[item] : 0, cols = valid ? p.cols[item] : 0;
+        const int wmax = p.task_wmax[task], npass = p.task_npass[task];
+        const int stride = p16_cols(wmax);
+        const uint32_t *ckr = reinterpret_cast<const uint32_t *>(p.ckpt + p.task_ckpt[task]) + lane;
+        const uint4 *ckc = p.ckpt + p.task_ckpt[task] + p16_ck_col(npass, wmax, 0, 0) + lane;
+        const int ti = p.nt ? item % p.nt : item;
+        const uint8_t *tseq = p.targets + (valid ? p.toff[ti] : 0);
+        const uint8_t *qseq = nullptr;
+        const int8_t *prof8 = nullptr;
+        int lp = 0;
+        if (p.mat8) {
+            qseq = p.qall + (valid ? p.qoff[item] : 0);
         } else {
-            ops[cap - 1 - n++] = 2;
-            if ((w.z >> bit) & 1u) { v += open; state = 0; } else { v += gap; }
-            --j;
+            const ProfDesc pd = p.profs[p.nt ? item / p.nt : 0];
+            qseq = pd.qcodes;
+            prof8 = pd.prof8;
+            lp = pd.lp;
+        }
+        pb_pair_out e;
+        if (valid) e = ends[item];
+        else memset(&e, 0, sizeof e);
+        int i = e.end_query, j = e.end_ref, v = e.score;
+        /* an end outside the computed region (a FASTSTATS item whose prefix
+         * pass was not needed): nothing to walk */
+        bool active = valid && i >= 0 && j >= 0 && i < rows && j < cols;
+        bool need2 = true;
+        if (MODE == 1 && valid) {
+            need2 = pb_needs_pass2(&job, &e) != 0;
+            active = active && need2;
+        }
+        const P16Bounds bd = p16_bounds(ALG, rows, cols, open, gap, p.mmax, p.mmin);
+        const int negv = bd.lb - open - 1;
+        const uint32_t NEG = p16_splat(negv);
+        const int cap = rows + cols;
+        uint8_t *ops = MODE == 2 && valid ? p.ops + p.ops_off[item] : nullptr;
+        const bool started = active;
+        int M = 0, S = 0, n = 0, state = 0;                  /* state: 0 H, 1 F, 2 E */
+        int staged = -1;
+        if (ALG == PB_SW && v <= 0) active = false;
+        while (__any_sync(0xffffffffu, active)) {
+            const int pass = active ? i >> 5 : 0, r0 = pass * P16_PASS;
+            const int jt = active ? j + ((i >> 4) & 1) : 0;  /* the iteration of the cell */
+            const int jb = jt / P16_CK * P16_CK;
+            /* the scores (BIAS: + open) of this pass's rows */
+            if (active && pass != staged) {
+                staged = pass;
+                if (p.mat8) {
+                    uint32_t qc[8];
+#pragma unroll
+                    for (int w = 0; w < 8; ++w) {
+                        uint32_t word = 0;
+#pragma unroll
+                        for (int b = 0; b < 4; ++b) {
+                            const int x = r0 + 4 * w + b;
+                            uint32_t c = x < rows ? qseq[x] : 255u;
+                            if (c != 255u && c >= (uint32_t)L) c = 0;
+                            word |= c << (8 * b);
+                        }
+                        qc[w] = word;
+                    }
+                    for (int a = 0; a < L; ++a) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            uint32_t word[4];
+#pragma unroll
+                            for (int w = 0; w < 4; ++w) {
+                                word[w] = 0;
+#pragma unroll
+                                for (int b = 0; b < 4; ++b) {
+                                    const uint32_t c = (qc[4 * h + w] >> (8 * b)) & 0xffu;
+                                    const uint32_t x = c == 255u ? (uint32_t)(uint8_t)bias
+                                                                 : (uint32_t)(uint8_t)s_mat[a * L + c];
+                                    word[w] |= x << (8 * b);
+                                }
+                            }
+                            *reinterpret_cast<uint4 *>(sl + a * LETTER + h * STRIP) =
+                                make_uint4(word[0], word[1], word[2], word[3]);
+                        }
+                    }
+                } else {
+                    const bool in = r0 + P16_PASS <= lp;
+                    for (int a = 0; a < L; ++a) {
+                        const int4 *src = reinterpret_cast<const int4 *>(prof8 + (size_t)a * lp + (in ? r0 : 0));
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            int4 x = in ? src[h] : make_int4(0, 0, 0, 0);
+                            if (BIAS) {
+                                x.x = (int)__vadd4((uint32_t)x.x, b4); x.y = (int)__vadd4((uint32_t)x.y, b4);
+                                x.z = (int)__vadd4((uint32_t)x.z, b4); x.w = (int)__vadd4((uint32_t)x.w, b4);
+                            }
+                            *reinterpret_cast<int4 *>(sl + a * LETTER + h * STRIP) = x;
+                        }
+                    }
+                }
+            }
+            /* the state before iteration jb */
+            uint32_t H[P16_R], E[P16_R], dg, prev_h, prev_f;
+            if (jb == 0) {
+#pragma unroll
+                for (int r = 0; r < P16_R; ++r) {
+                    const int la = p16_left(ALG, sgf, r0 + r, open, gap) - bias;
+                    const int lb2 = p16_left(ALG, sgf, r0 + P16_R + r, open, gap) - bias;
+                    H[r] = (uint32_t)(uint16_t)la | ((uint32_t)(uint16_t)lb2 << 16);
+                    E[r] = NEG;
+                }
+                dg = (uint32_t)(uint16_t)(p16_left(ALG, sgf, r0 - 1, open, gap) - bias);
+                prev_h = (uint32_t)(uint16_t)(p16_left(ALG, sgf, r0 + P16_R - 1, open, gap) - bias);
+                prev_f = NEG & 0xffffu;
+            } else {
+                const uint4 *d = ckc + ((size_t)pass * p16_ck_blocks(wmax) + jb / P16_CK - 1) * P16_CK_U4 * 32;
+#pragma unroll
+                for (int x = 0; x < P16_R / 4; ++x) {
+                    const uint4 h4 = __ldcg(d + x * 32), e4 = __ldcg(d + (x + P16_R / 4) * 32);
+                    H[4 * x] = h4.x; H[4 * x + 1] = h4.y; H[4 * x + 2] = h4.z; H[4 * x + 3] = h4.w;
+                    E[4 * x] = e4.x; E[4 * x + 1] = e4.y; E[4 * x + 2] = e4.z; E[4 * x + 3] = e4.w;
+                }
+                const uint4 m4 = __ldcg(d + P16_R / 2 * 32);
+                prev_f = m4.x;
+                dg = m4.y;
+                prev_h = H[P16_R - 1];
+            }
+            /* the row above: row -1 (as the forward kernel steps it), or the
+             * pass above's bottom row */
+            const bool top = pass == 0;
+            const int tstep = (ALG == PB_SW || (ALG == PB_SG && (sgf & PB_S2_BEG))) ? 0 : gap;
+            uint32_t vtop = p16_prmt((uint32_t)(uint16_t)(p16_top(ALG, sgf, 0, open, gap) - bias - jb * tstep), NEG, 0x5410u);
+            const uint32_t top_step = (uint32_t)(uint16_t)(-tstep);
+            const uint32_t *in_row = ckr + (top ? 0 : p16_ck_row(wmax, pass - 1, 0)) + 32;
+            const int rd = top ? 0 : wmax;
+            const uint32_t vnone = p16_prmt(0u, NEG, 0x5410u);
+            uint32_t v_n[4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) v_n[x] = jb + x < rd ? __ldcg(in_row + (size_t)(jb + x) * 32) : vnone;
+            ResidueWords tw;
+            tw.start(tseq + jb, active ? cols - jb : 0);
+            int cb = active && jb > 0 ? tseq[jb - 1] : 0;
+            if (cb >= L) cb = 0;
+            const int8_t *pb_at = sl + cb * LETTER + STRIP;
+            const int cnt = __reduce_max_sync(0xffffffffu, active ? jt - jb + 1 : 0);
+            for (int x0 = 0; x0 < cnt; x0 += 4) {
+                uint32_t codes = tw.next(x0);
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+                    if (((codes >> (8 * b)) & 0xffu) >= (uint32_t)L) codes &= ~(0xffu << (8 * b));
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int x = x0 + u, jj = jb + x;
+                    const uint32_t vv = top ? vtop : v_n[u];
+                    vtop = __vadd2(vtop, top_step);
+                    v_n[u] = jj + 4 < rd ? __ldcg(in_row + (size_t)(jj + 4) * 32) : vnone;
+                    uint32_t hu = p16_prmt(vv, prev_h, 0x5410u);
+                    uint32_t fu = p16_prmt(vv, prev_f, 0x5432u);
+                    const int8_t *pa_at = sl + ((codes >> (8 * u)) & 0xffu) * LETTER;
+                    const uint4 pa4 = *reinterpret_cast<const uint4 *>(pa_at);
+                    const uint4 pb4 = *reinterpret_cast<const uint4 *>(pb_at);
+                    pb_at = pa_at + STRIP;
+                    uint32_t hd = dg;
+                    dg = hu;
+                    uint32_t aD = 0u, aF = 0u, aE = 0u, aV = 0u;
+                    uint32_t dD = 0u, dF = 0u, dE = 0u, dV = 0u;
+#pragma unroll
+                    for (int r = 0; r < P16_R; ++r) {
+                        const uint32_t wa = r < 4 ? pa4.x : r < 8 ? pa4.y : r < 12 ? pa4.z : pa4.w;
+                        const uint32_t wb = r < 4 ? pb4.x : r < 8 ? pb4.y : r < 12 ? pb4.z : pb4.w;
+                        uint32_t sc;
+                        switch (r & 3) {
+                            case 0: sc = p16_pair<0>(wa, wb); break;
+                            case 1: sc = p16_pair<1>(wa, wb); break;
+                            case 2: sc = p16_pair<2>(wa, wb); break;
+                            default: sc = p16_pair<3>(wa, wb); break;
+                        }
+                        const uint32_t ho = BIAS ? H[r] : __vadd2(H[r], gO);
+                        const uint32_t fo = BIAS ? hu : __vadd2(hu, gO);
+                        const uint32_t ee = __vadd2(E[r], gE), fe = __vadd2(fu, gE);
+                        const uint32_t en = __vmaxs2(ho, ee), fn = __vmaxs2(fo, fe);
+                        const uint32_t hdg = __vadd2(hd, sc);
+                        const uint32_t h = ALG == PB_SW ? __vimax3_s16x2_relu(hdg, en, fn) : __vimax3_s16x2(hdg, en, fn);
+                        const uint32_t hn = BIAS ? __vadd2(h, gO) : h;
+                        const uint32_t nD = __vsub2(hdg, h), nF = __vsub2(fn, h);
+                        const uint32_t nE = __vsub2(ee, ho), nV = __vsub2(fe, fo);
+                        if (r & 1) {
+                            const uint32_t m = 0x01010101u << (r >> 1);
+                            aD |= p16_prmt(dD, nD, 0xfdb9u) & m;
+                            aF |= p16_prmt(dF, nF, 0xfdb9u) & m;
+                            aE |= p16_prmt(dE, nE, 0xfdb9u) & m;
+                            aV |= p16_prmt(dV, nV, 0xfdb9u) & m;
+                        }
+                        dD = nD; dF = nF; dE = nE; dV = nV;
+                        E[r] = en;
+                        hd = H[r];
+                        H[r] = hn;
+                        hu = hn;
+                        fu = fn;
+                    }
+                    tile[x * 32] = make_uint4(aD, aF, aE, aV);
+                    prev_h = hu;
+                    prev_f = fu;
+                    if (u == 0 && jj == 0) {
+                        /* the high half computed column -1 */
+#pragma unroll
+                        for (int r = 0; r < P16_R; ++r) {
+                            const int lb2 = p16_left(ALG, sgf, r0 + P16_R + r, open, gap) - bias;
+                            H[r] = (H[r] & 0xffffu) | ((uint32_t)(uint16_t)lb2 << 16);
+                            E[r] = (E[r] & 0xffffu) | (NEG & 0xffff0000u);
+                        }
+                    }
+                }
+            }
+            /* the walk inside the block (each step moves up or left or changes
+             * from H to a gap, so it ends) */
+            while (active) {
+                const int half = (i >> 4) & 1, x = j + half - jb;
+                if ((i >> 5) != pass || x < 0) break;
+                const int bit = p16_bit(i);
+                const uint4 w = tile[x * 32];
+                if (state == 0) {
+                    if (!((w.x >> bit) & 1u)) {
+                        int qc = qseq[i], tc = tseq[j];
+                        if (qc >= L) qc = 0;
+                        if (tc >= L) tc = 0;
+                        /* the staged score of this cell */
+                        const int sc = (int)sl[tc * LETTER + half * STRIP + (i & 15)] - bias;
+                        M += qc == tc;
+                        S += sc > 0;
+                        v -= sc;
+                        if (MODE == 2 && n < cap) ops[cap - 1 - n] = 0;
+                        ++n;
+                        --i;
+                        --j;
+                    } else {
+                        state = ((w.y >> bit) & 1u) ? 2 : 1;
+                    }
+                } else if (state == 1) {
+                    if (MODE == 2 && n < cap) ops[cap - 1 - n] = 1;
+                    ++n;
+                    if ((w.w >> bit) & 1u) { v += open; state = 0; } else { v += gap; }
+                    --i;
+                } else {
+                    if (MODE == 2 && n < cap) ops[cap - 1 - n] = 2;
+                    ++n;
+                    if ((w.z >> bit) & 1u) { v += open; state = 0; } else { v += gap; }
+                    --j;
+                }
+                if (i < 0 || j < 0 || (ALG == PB_SW && state == 0 && v <= 0) || n >= cap) active = false;
+            }
+            __syncwarp();
+        }
+        if (!valid) continue;
+        if (MODE == 2) {
+            int *info = p.path_info + 3 * (size_t)item;
+            info[0] = started ? n : -1; info[1] = i; info[2] = j;
+        } else if (MODE == 0) {
+            pb_pair_out *o = p.out + item;
+            o->matches = M; o->similar = S; o->length = n;
+        } else {
+            /* as the prefix pass (ENDS off) writes it */
+            const int pr = need2 ? e.end_query + 1 : 1, pc = need2 ? e.end_ref + 1 : 1;
+            const P16Bounds b2 = p16_bounds(ALG, pr, pc, open, gap, p.mmax, p.mmin);
+            pb_pair_out o;
+            o.score = 0; o.end_query = 0; o.end_ref = 0;
+            o.max_h = b2.ub;
+            o.matches = M; o.similar = S; o.length = n;
+            o.min_h_real = b2.lb;
+            o.min_f_real = b2.lb - open;
+            o.max_stat_real = ((pr + 31) & ~31) + pc;
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                o.min_h_pad[x] = b2.lb;
+                o.max_stat_pad[x] = o.max_stat_real;
+                o.min_f_pad[x] = b2.lb - open;
+            }
+            o.status = e.status | PB_ST_BOUNDED;
+            p.out2[item] = o;
         }
     }
-    info[0] = n; info[1] = i; info[2] = j;
 }
 
 /* per item: rows, columns, eligibility and the sort key (eligible first,
@@ -774,10 +965,11 @@ __global__ void k_p16_setup(P16Setup q, int *__restrict__ rows, int *__restrict_
     }
 }
 
-/* per task (a warp each): widest target, passes, shared query, bits size */
+/* per task (a warp each): widest target, passes, shared query, uint4s of its
+ * checkpoints */
 __global__ void k_p16_tasks(P16Params p, int ntasks, const int *__restrict__ group, int *__restrict__ twmax,
-                            int *__restrict__ tnpass, int *__restrict__ tshared, long long *__restrict__ tbits,
-                            int bits)
+                            int *__restrict__ tnpass, int *__restrict__ tshared, long long *__restrict__ tckpt,
+                            int ckpt)
 {
     const int task = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -803,7 +995,7 @@ __global__ void k_p16_tasks(P16Params p, int ntasks, const int *__restrict__ gro
         twmax[task] = c;
         tnpass[task] = np;
         tshared[task] = p.mat8 ? (same && group != nullptr) : 1;
-        tbits[task] = bits ? (long long)np * p16_cols(c) * 32 : 0;
+        tckpt[task] = ckpt ? (long long)p16_ck_col(np, c, np, 0) : 0;
     }
 }
 
@@ -912,7 +1104,7 @@ struct P16Frees {
 
 namespace {
 
-#define P16_CK(call)                                           \
+#define PB_P16(call)                                           \
     do {                                                       \
         if ((call) != cudaSuccess) {                           \
             fprintf(stderr, "pb_pair16: %s failed\n", #call);  \
@@ -931,30 +1123,41 @@ size_t p16_smem(bool shared, int L, bool mat)
 
 typedef void (*p16_kernel_t)(P16Params, const int *, int, int *);
 
-template <int ALG, bool BITS, bool ENDS, bool BIAS>
+template <int ALG, bool CKPT, bool ENDS, bool BIAS>
 p16_kernel_t pick3(bool shared, int warps)
 {
-    if (shared) return k_p16<ALG, BITS, ENDS, true, 8, BIAS>;
-    return warps == 8 ? k_p16<ALG, BITS, ENDS, false, 8, BIAS> : k_p16<ALG, BITS, ENDS, false, 4, BIAS>;
+    if (shared) return k_p16<ALG, CKPT, ENDS, true, 8, BIAS>;
+    return warps == 8 ? k_p16<ALG, CKPT, ENDS, false, 8, BIAS> : k_p16<ALG, CKPT, ENDS, false, 4, BIAS>;
 }
 
 template <bool BIAS>
-p16_kernel_t pick(int alg, bool bits, bool ends, bool shared, int warps)
+p16_kernel_t pick(int alg, bool ckpt, bool ends, bool shared, int warps)
 {
     if (alg == PB_SW) {
         if (!ends) return pick3<PB_SW, true, false, BIAS>(shared, warps);
-        return bits ? pick3<PB_SW, true, true, BIAS>(shared, warps) : pick3<PB_SW, false, true, BIAS>(shared, warps);
+        return ckpt ? pick3<PB_SW, true, true, BIAS>(shared, warps) : pick3<PB_SW, false, true, BIAS>(shared, warps);
     }
     if (alg == PB_NW)
-        return bits ? pick3<PB_NW, true, true, BIAS>(shared, warps) : pick3<PB_NW, false, true, BIAS>(shared, warps);
-    return bits ? pick3<PB_SG, true, true, BIAS>(shared, warps) : pick3<PB_SG, false, true, BIAS>(shared, warps);
+        return ckpt ? pick3<PB_NW, true, true, BIAS>(shared, warps) : pick3<PB_NW, false, true, BIAS>(shared, warps);
+    return ckpt ? pick3<PB_SG, true, true, BIAS>(shared, warps) : pick3<PB_SG, false, true, BIAS>(shared, warps);
+}
+
+typedef void (*p16_trace_t)(pb_job, P16Params, const int *, int, const pb_pair_out *, int *);
+
+template <bool BIAS>
+p16_trace_t pick_trace(int alg, int mode)
+{
+    if (alg == PB_SW)
+        return mode == 0 ? k_p16_trace<PB_SW, 0, BIAS> : mode == 1 ? k_p16_trace<PB_SW, 1, BIAS> : k_p16_trace<PB_SW, 2, BIAS>;
+    if (alg == PB_NW) return mode == 2 ? k_p16_trace<PB_NW, 2, BIAS> : k_p16_trace<PB_NW, 0, BIAS>;
+    return mode == 2 ? k_p16_trace<PB_SG, 2, BIAS> : k_p16_trace<PB_SG, 0, BIAS>;
 }
 
 }  // namespace
 
 int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out *ends, pb_pair_out *out,
              const int *group, int *d_rest, int *n_rest, cudaStream_t st,
-             uint8_t *d_ops, const int64_t *d_ops_off, int *d_path_info, unsigned intra_mask)
+             uint8_t *d_ops, const int64_t *d_ops_off, int *d_path_info, unsigned intra_mask, pb_pair_out *out2)
 {
     const pb_mode *m = &job.mode;
     const bool dbmode = b->nprofs > 0;
@@ -963,8 +1166,8 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
     if (N <= 0) return 0;
     if ((long long)(dbmode ? (long long)b->npairs * b->nprofs : b->npairs) > INT32_MAX) return -1;
     const bool paths = d_ops != nullptr;
-    const bool bits = prefix || (m->stats && !pb_job_is_faststats(&job)) || paths;
-    const bool walk = prefix || (m->stats && !pb_job_is_faststats(&job));
+    const bool walk = prefix || out2 || (m->stats && !pb_job_is_faststats(&job));
+    const bool ckpt = walk || paths;
     const bool ends_on = !prefix;
     P16Frees frees(st);
     /* alphabet and score source; anything the kernels cannot take goes to the exact kernel */
@@ -988,19 +1191,19 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
             mmin = dp->mmin < mmin ? dp->mmin : mmin;
         }
         if (usable) {
-            P16_CK(cudaMallocAsync((void **)&d_profs, sizeof(ProfDesc) * b->nprofs, st));
+            PB_P16(cudaMallocAsync((void **)&d_profs, sizeof(ProfDesc) * b->nprofs, st));
             frees.add(d_profs);
-            P16_CK(cudaMallocAsync((void **)&d_pql, sizeof(int) * b->nprofs, st));
+            PB_P16(cudaMallocAsync((void **)&d_pql, sizeof(int) * b->nprofs, st));
             frees.add(d_pql);
-            P16_CK(cudaMemcpyAsync(d_profs, h.data(), sizeof(ProfDesc) * b->nprofs, cudaMemcpyHostToDevice, st));
-            P16_CK(cudaMemcpyAsync(d_pql, ql.data(), sizeof(int) * b->nprofs, cudaMemcpyHostToDevice, st));
-            P16_CK(cudaStreamSynchronize(st));      /* the host vectors die at return */
+            PB_P16(cudaMemcpyAsync(d_profs, h.data(), sizeof(ProfDesc) * b->nprofs, cudaMemcpyHostToDevice, st));
+            PB_P16(cudaMemcpyAsync(d_pql, ql.data(), sizeof(int) * b->nprofs, cudaMemcpyHostToDevice, st));
+            PB_P16(cudaStreamSynchronize(st));      /* the host vectors die at return */
         }
     } else {
         L = b->msize; mmax = b->mmax; mmin = b->mmin;
         usable = b->d_mat && b->mmin >= -128 && b->mmax <= 127;
         if (usable) {
-            P16_CK(cudaMallocAsync((void **)&d_mat8, (size_t)L * L, st));
+            PB_P16(cudaMallocAsync((void **)&d_mat8, (size_t)L * L, st));
             frees.add(d_mat8);
             k_mat_to_int8<<<(L * L + 255) / 256, 256, 0, st>>>(b->d_mat, L * L, d_mat8);
             pb_diag_count_launch(1);
@@ -1012,20 +1215,20 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
         k_iota_int<<<(N + 255) / 256, 256, 0, st>>>(d_rest, N);
         pb_diag_count_launch(1);
         *n_rest = N;
-        P16_CK(cudaStreamSynchronize(st));
+        PB_P16(cudaStreamSynchronize(st));
         return 0;
     }
     /* per item: rows, columns, eligibility, sort */
     int *rows = nullptr, *cols = nullptr, *idx = nullptr, *order = nullptr, *counts = nullptr;
     unsigned long long *keys = nullptr, *keys_sorted = nullptr;
-    P16_CK(cudaMallocAsync((void **)&rows, sizeof(int) * N, st)); frees.add(rows);
-    P16_CK(cudaMallocAsync((void **)&cols, sizeof(int) * N, st)); frees.add(cols);
-    P16_CK(cudaMallocAsync((void **)&idx, sizeof(int) * N, st)); frees.add(idx);
-    P16_CK(cudaMallocAsync((void **)&order, sizeof(int) * N, st)); frees.add(order);
-    P16_CK(cudaMallocAsync((void **)&counts, sizeof(int) * 4, st)); frees.add(counts);
-    P16_CK(cudaMallocAsync((void **)&keys, sizeof(unsigned long long) * N, st)); frees.add(keys);
-    P16_CK(cudaMallocAsync((void **)&keys_sorted, sizeof(unsigned long long) * N, st)); frees.add(keys_sorted);
-    P16_CK(cudaMemsetAsync(counts, 0, sizeof(int) * 4, st));
+    PB_P16(cudaMallocAsync((void **)&rows, sizeof(int) * N, st)); frees.add(rows);
+    PB_P16(cudaMallocAsync((void **)&cols, sizeof(int) * N, st)); frees.add(cols);
+    PB_P16(cudaMallocAsync((void **)&idx, sizeof(int) * N, st)); frees.add(idx);
+    PB_P16(cudaMallocAsync((void **)&order, sizeof(int) * N, st)); frees.add(order);
+    PB_P16(cudaMallocAsync((void **)&counts, sizeof(int) * 4, st)); frees.add(counts);
+    PB_P16(cudaMallocAsync((void **)&keys, sizeof(unsigned long long) * N, st)); frees.add(keys);
+    PB_P16(cudaMallocAsync((void **)&keys_sorted, sizeof(unsigned long long) * N, st)); frees.add(keys_sorted);
+    PB_P16(cudaMemsetAsync(counts, 0, sizeof(int) * 4, st));
     P16Setup q;
     memset(&q, 0, sizeof q);
     q.alg = m->alg; q.open = m->open; q.gap = m->gap; q.mmax = mmax; q.mmin = mmin; q.nitems = N;
@@ -1042,12 +1245,12 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
     size_t sort_bytes = 0;
     void *sort_tmp = nullptr;
     cub::DeviceRadixSort::SortPairsDescending(nullptr, sort_bytes, keys, keys_sorted, idx, order, N, 0, 64, st);
-    P16_CK(cudaMallocAsync(&sort_tmp, sort_bytes, st));
+    PB_P16(cudaMallocAsync(&sort_tmp, sort_bytes, st));
     frees.add(sort_tmp);
     cub::DeviceRadixSort::SortPairsDescending(sort_tmp, sort_bytes, keys, keys_sorted, idx, order, N, 0, 64, st);
     int nelig = 0;
-    P16_CK(cudaMemcpyAsync(&nelig, counts, sizeof(int), cudaMemcpyDeviceToHost, st));
-    P16_CK(cudaStreamSynchronize(st));
+    PB_P16(cudaMemcpyAsync(&nelig, counts, sizeof(int), cudaMemcpyDeviceToHost, st));
+    PB_P16(cudaStreamSynchronize(st));
     /* the ineligible items (sorted last) start the rest list */
     if (N - nelig > 0) {
         k_copy_int<<<(N - nelig + 255) / 256, 256, 0, st>>>(order + nelig, N - nelig, d_rest);
@@ -1060,38 +1263,38 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
     if (nelig > 0 && (dbmode || group)) {
         int *head = nullptr, *gid = nullptr, *gstart = nullptr, *pcount = nullptr, *pstart = nullptr, *iota = nullptr;
         int ng = 0, last_start = 0, last_count = 0;
-        P16_CK(cudaMallocAsync((void **)&head, sizeof(int) * nelig, st)); frees.add(head);
-        P16_CK(cudaMallocAsync((void **)&gid, sizeof(int) * nelig, st)); frees.add(gid);
-        P16_CK(cudaMallocAsync((void **)&gstart, sizeof(int) * nelig, st)); frees.add(gstart);
-        P16_CK(cudaMallocAsync((void **)&pcount, sizeof(int) * nelig, st)); frees.add(pcount);
-        P16_CK(cudaMallocAsync((void **)&pstart, sizeof(int) * nelig, st)); frees.add(pstart);
-        P16_CK(cudaMallocAsync((void **)&iota, sizeof(int) * nelig, st)); frees.add(iota);
+        PB_P16(cudaMallocAsync((void **)&head, sizeof(int) * nelig, st)); frees.add(head);
+        PB_P16(cudaMallocAsync((void **)&gid, sizeof(int) * nelig, st)); frees.add(gid);
+        PB_P16(cudaMallocAsync((void **)&gstart, sizeof(int) * nelig, st)); frees.add(gstart);
+        PB_P16(cudaMallocAsync((void **)&pcount, sizeof(int) * nelig, st)); frees.add(pcount);
+        PB_P16(cudaMallocAsync((void **)&pstart, sizeof(int) * nelig, st)); frees.add(pstart);
+        PB_P16(cudaMallocAsync((void **)&iota, sizeof(int) * nelig, st)); frees.add(iota);
         k_pad_heads<<<(nelig + 255) / 256, 256, 0, st>>>(keys_sorted, nelig, head);
         k_iota_int<<<(nelig + 255) / 256, 256, 0, st>>>(iota, nelig);
         pb_diag_count_launch(2);
         size_t b1 = 0, b2 = 0, b3 = 0;
         void *tmp = nullptr;
-        P16_CK(cub::DeviceScan::InclusiveSum(nullptr, b1, head, gid, nelig, st));
-        P16_CK(cub::DeviceSelect::Flagged(nullptr, b2, iota, head, gstart, counts + 2, nelig, st));
-        P16_CK(cub::DeviceScan::ExclusiveSum(nullptr, b3, pcount, pstart, nelig, st));
+        PB_P16(cub::DeviceScan::InclusiveSum(nullptr, b1, head, gid, nelig, st));
+        PB_P16(cub::DeviceSelect::Flagged(nullptr, b2, iota, head, gstart, counts + 2, nelig, st));
+        PB_P16(cub::DeviceScan::ExclusiveSum(nullptr, b3, pcount, pstart, nelig, st));
         const size_t tb = std::max(b1, std::max(b2, b3));
-        P16_CK(cudaMallocAsync(&tmp, tb, st)); frees.add(tmp);
+        PB_P16(cudaMallocAsync(&tmp, tb, st)); frees.add(tmp);
         size_t b = tb;
-        P16_CK(cub::DeviceScan::InclusiveSum(tmp, b, head, gid, nelig, st));
+        PB_P16(cub::DeviceScan::InclusiveSum(tmp, b, head, gid, nelig, st));
         b = tb;
-        P16_CK(cub::DeviceSelect::Flagged(tmp, b, iota, head, gstart, counts + 2, nelig, st));
-        P16_CK(cudaMemcpyAsync(&ng, counts + 2, sizeof(int), cudaMemcpyDeviceToHost, st));
-        P16_CK(cudaStreamSynchronize(st));
+        PB_P16(cub::DeviceSelect::Flagged(tmp, b, iota, head, gstart, counts + 2, nelig, st));
+        PB_P16(cudaMemcpyAsync(&ng, counts + 2, sizeof(int), cudaMemcpyDeviceToHost, st));
+        PB_P16(cudaStreamSynchronize(st));
         k_pad_counts<<<(ng + 255) / 256, 256, 0, st>>>(gstart, ng, nelig, pcount);
         pb_diag_count_launch(1);
         b = tb;
-        P16_CK(cub::DeviceScan::ExclusiveSum(tmp, b, pcount, pstart, ng, st));
-        P16_CK(cudaMemcpyAsync(&last_start, pstart + ng - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-        P16_CK(cudaMemcpyAsync(&last_count, pcount + ng - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-        P16_CK(cudaStreamSynchronize(st));
+        PB_P16(cub::DeviceScan::ExclusiveSum(tmp, b, pcount, pstart, ng, st));
+        PB_P16(cudaMemcpyAsync(&last_start, pstart + ng - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+        PB_P16(cudaMemcpyAsync(&last_count, pcount + ng - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+        PB_P16(cudaStreamSynchronize(st));
         nslots = last_start + last_count;
-        P16_CK(cudaMallocAsync((void **)&porder, sizeof(int) * (size_t)nslots, st)); frees.add(porder);
-        P16_CK(cudaMemsetAsync(porder, 0xff, sizeof(int) * (size_t)nslots, st));
+        PB_P16(cudaMallocAsync((void **)&porder, sizeof(int) * (size_t)nslots, st)); frees.add(porder);
+        PB_P16(cudaMemsetAsync(porder, 0xff, sizeof(int) * (size_t)nslots, st));
         k_pad_scatter<<<(nelig + 255) / 256, 256, 0, st>>>(order, nelig, gid, gstart, pstart, porder);
         pb_diag_count_launch(1);
     }
@@ -1107,21 +1310,21 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
         p.out = out;
         p.ops = d_ops; p.ops_off = d_ops_off; p.path_info = d_path_info;
         int *twmax = nullptr, *tnpass = nullptr, *tshared = nullptr;
-        long long *tbits = nullptr;
-        P16_CK(cudaMallocAsync((void **)&twmax, sizeof(int) * ntasks, st)); frees.add(twmax);
-        P16_CK(cudaMallocAsync((void **)&tnpass, sizeof(int) * ntasks, st)); frees.add(tnpass);
-        P16_CK(cudaMallocAsync((void **)&tshared, sizeof(int) * ntasks, st)); frees.add(tshared);
-        P16_CK(cudaMallocAsync((void **)&tbits, sizeof(long long) * ntasks, st)); frees.add(tbits);
+        long long *tckpt = nullptr;
+        PB_P16(cudaMallocAsync((void **)&twmax, sizeof(int) * ntasks, st)); frees.add(twmax);
+        PB_P16(cudaMallocAsync((void **)&tnpass, sizeof(int) * ntasks, st)); frees.add(tnpass);
+        PB_P16(cudaMallocAsync((void **)&tshared, sizeof(int) * ntasks, st)); frees.add(tshared);
+        PB_P16(cudaMallocAsync((void **)&tckpt, sizeof(long long) * ntasks, st)); frees.add(tckpt);
         k_p16_tasks<<<(ntasks * 32 + 255) / 256, 256, 0, st>>>(p, ntasks, dbmode ? nullptr : group, twmax, tnpass,
-                                                               tshared, tbits, bits ? 1 : 0);
+                                                               tshared, tckpt, ckpt ? 1 : 0);
         pb_diag_count_launch(1);
         std::vector<int> hw(ntasks), hn(ntasks), hs(ntasks);
         std::vector<long long> hb(ntasks);
-        P16_CK(cudaMemcpyAsync(hw.data(), twmax, sizeof(int) * ntasks, cudaMemcpyDeviceToHost, st));
-        P16_CK(cudaMemcpyAsync(hn.data(), tnpass, sizeof(int) * ntasks, cudaMemcpyDeviceToHost, st));
-        P16_CK(cudaMemcpyAsync(hs.data(), tshared, sizeof(int) * ntasks, cudaMemcpyDeviceToHost, st));
-        P16_CK(cudaMemcpyAsync(hb.data(), tbits, sizeof(long long) * ntasks, cudaMemcpyDeviceToHost, st));
-        P16_CK(cudaStreamSynchronize(st));
+        PB_P16(cudaMemcpyAsync(hw.data(), twmax, sizeof(int) * ntasks, cudaMemcpyDeviceToHost, st));
+        PB_P16(cudaMemcpyAsync(hn.data(), tnpass, sizeof(int) * ntasks, cudaMemcpyDeviceToHost, st));
+        PB_P16(cudaMemcpyAsync(hs.data(), tshared, sizeof(int) * ntasks, cudaMemcpyDeviceToHost, st));
+        PB_P16(cudaMemcpyAsync(hb.data(), tckpt, sizeof(long long) * ntasks, cudaMemcpyDeviceToHost, st));
+        PB_P16(cudaStreamSynchronize(st));
         int maxlen = 0;
         for (int t = 0; t < ntasks; ++t) maxlen = hw[t] > maxlen ? hw[t] : maxlen;
         /* task order: most work first */
@@ -1130,14 +1333,19 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
         std::stable_sort(torder.begin(), torder.end(), [&](int x, int y) {
             return (long long)hn[x] * (hw[x] + 1) > (long long)hn[y] * (hw[y] + 1);
         });
-        /* chunks of tasks whose direction bits fit the budget: half of the
-         * free device memory (at most 96 GiB), so that a chunk of the largest
-         * tasks (about 36 MB of bits each at 1500 x 1500) still fills the
-         * SMs; a budget of a few GiB left chunks of ~200 warps */
-        size_t free_b = 0, total_b = 0;
-        cudaMemGetInfo(&free_b, &total_b);
-        size_t budget = (size_t)96 << 30;
-        if (free_b / 2 < budget) budget = free_b / 2;
+        /* chunks of tasks whose checkpoints fit the budget: half of the free
+         * device memory (at most 96 GiB), so that a chunk of the largest tasks
+         * (about 20 MB each at 1500 x 1500) still fills the SMs. A batch of 1
+         * GiB or less takes what it needs without asking the device, which
+         * took 0.1 to 9 ms beside other copies. */
+        size_t all_u4 = 0;
+        for (int t = 0; t < ntasks; ++t) all_u4 += (size_t)hb[t];
+        size_t budget = (size_t)1 << 30;
+        if (all_u4 * sizeof(uint4) > budget) {
+            size_t free_b = 0, total_b = 0;
+            cudaMemGetInfo(&free_b, &total_b);
+            budget = std::max(budget, std::min((size_t)96 << 30, free_b / 2));
+        }
         const size_t budget_u4 = budget / sizeof(uint4);
         /* launch shapes and the pass-boundary buffers, sized for the larger grid */
         int dev = 0, nsm = 0;
@@ -1150,8 +1358,8 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
         for (int sh = 0; sh < 2; ++sh) {
             warps[sh] = p16_warps(sh == 1, L);
             smem[sh] = p16_smem(sh == 1, L, d_mat8 != nullptr);
-            kern[sh] = bias ? pick<true>(m->alg, bits, ends_on, sh == 1, warps[sh])
-                            : pick<false>(m->alg, bits, ends_on, sh == 1, warps[sh]);
+            kern[sh] = bias ? pick<true>(m->alg, ckpt, ends_on, sh == 1, warps[sh])
+                            : pick<false>(m->alg, ckpt, ends_on, sh == 1, warps[sh]);
             int per_sm = 0;
             pb_raise_smem((const void *)kern[sh], (int)smem[sh]);
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern[sh], warps[sh] * 32, smem[sh]);
@@ -1159,21 +1367,21 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
         }
         const size_t rwarps = (size_t)std::max(grid[0] * warps[0], grid[1] * warps[1]);
         uint32_t *scratch = nullptr;
-        P16_CK(cudaMallocAsync((void **)&scratch, sizeof(uint32_t) * (size_t)(maxlen + 8) * 32 * rwarps, st));
+        PB_P16(cudaMallocAsync((void **)&scratch, ckpt ? 256 : sizeof(uint32_t) * (size_t)(maxlen + 8) * 32 * rwarps, st));
         frees.add(scratch);
         p.scratch = scratch;
         p.colsave = nullptr;
         if (ends_on && m->alg == PB_SW) {
-            P16_CK(cudaMallocAsync((void **)&p.colsave, sizeof(uint4) * (P16_R / 2) * 32 * rwarps, st));
+            PB_P16(cudaMallocAsync((void **)&p.colsave, sizeof(uint4) * (P16_R / 2) * 32 * rwarps, st));
             frees.add(p.colsave);
         }
         p.maxlen = maxlen;
-        p.task_wmax = twmax; p.task_npass = tnpass; p.task_bits = tbits;
+        p.task_wmax = twmax; p.task_npass = tnpass; p.task_ckpt = tckpt; p.out2 = out2;
         int *d_tlist = nullptr, *d_counter = nullptr;
-        P16_CK(cudaMallocAsync((void **)&d_tlist, sizeof(int) * ntasks, st)); frees.add(d_tlist);
-        P16_CK(cudaMallocAsync((void **)&d_counter, sizeof(int) * 2, st)); frees.add(d_counter);
-        uint4 *bitsbuf = nullptr;
-        size_t bits_cap = 0;
+        PB_P16(cudaMallocAsync((void **)&d_tlist, sizeof(int) * ntasks, st)); frees.add(d_tlist);
+        PB_P16(cudaMallocAsync((void **)&d_counter, sizeof(int) * 2, st)); frees.add(d_counter);
+        uint4 *ckbuf = nullptr;
+        size_t ck_cap = 0;
         std::vector<long long> hoff(ntasks, 0);
         int t0 = 0;
         while (t0 < ntasks) {
@@ -1185,18 +1393,18 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
             for (int k = t0; k < t1; ++k) lst[hs[torder[k]] ? 1 : 0].push_back(torder[k]);
             size_t off = 0;
             for (int k = t0; k < t1; ++k) { hoff[torder[k]] = (long long)off; off += (size_t)hb[torder[k]]; }
-            if (bits && off > bits_cap) {
-                if (bitsbuf) cudaFreeAsync(bitsbuf, st);
-                bitsbuf = nullptr;
-                P16_CK(cudaMallocAsync((void **)&bitsbuf, sizeof(uint4) * (off + 1), st));
-                bits_cap = off;
+            if (ckpt && off > ck_cap) {
+                if (ckbuf) cudaFreeAsync(ckbuf, st);
+                ckbuf = nullptr;
+                PB_P16(cudaMallocAsync((void **)&ckbuf, sizeof(uint4) * (off + 1), st));
+                ck_cap = off;
             }
-            p.bits = bitsbuf;
-            P16_CK(cudaMemcpyAsync(tbits, hoff.data(), sizeof(long long) * ntasks, cudaMemcpyHostToDevice, st));
+            p.ckpt = ckbuf;
+            PB_P16(cudaMemcpyAsync(tckpt, hoff.data(), sizeof(long long) * ntasks, cudaMemcpyHostToDevice, st));
             const int n1 = (int)lst[1].size(), n0 = (int)lst[0].size();
             std::vector<int> all(lst[1]);
             all.insert(all.end(), lst[0].begin(), lst[0].end());
-            P16_CK(cudaMemcpyAsync(d_tlist, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice, st));
+            PB_P16(cudaMemcpyAsync(d_tlist, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice, st));
             for (int sh = 1; sh >= 0; --sh) {
                 const int nl = sh ? n1 : n0;
                 if (!nl) continue;
@@ -1204,46 +1412,44 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
                 int g = grid[sh];
                 const int need = (nl + warps[sh] - 1) / warps[sh];
                 if (g > need) g = need;
-                P16_CK(cudaMemsetAsync(d_counter, 0, sizeof(int), st));
+                PB_P16(cudaMemsetAsync(d_counter, 0, sizeof(int), st));
                 kern[sh]<<<g, warps[sh] * 32, smem[sh], st>>>(p, tl, nl, d_counter);
                 pb_diag_count_launch(1);
-                P16_CK(cudaGetLastError());
+                PB_P16(cudaGetLastError());
             }
-            if (paths) {
-                const int nw = (int)all.size() * 32;
-                if (m->alg == PB_SW) k_p16_path<PB_SW><<<(nw + 127) / 128, 128, 0, st>>>(p, d_tlist, (int)all.size(), out, m->open, m->gap);
-                else if (m->alg == PB_NW) k_p16_path<PB_NW><<<(nw + 127) / 128, 128, 0, st>>>(p, d_tlist, (int)all.size(), out, m->open, m->gap);
-                else k_p16_path<PB_SG><<<(nw + 127) / 128, 128, 0, st>>>(p, d_tlist, (int)all.size(), out, m->open, m->gap);
+            if (ckpt) {
+                const int mode = paths ? 2 : out2 ? 1 : 0;
+                const p16_trace_t tk = bias ? pick_trace<true>(m->alg, mode) : pick_trace<false>(m->alg, mode);
+                const size_t tsm = (d_mat8 ? (((size_t)L * L + 15) & ~(size_t)15) : 0) +
+                                   (size_t)P16_TR_WARPS * (P16_CK * 512 + (size_t)L * 1024);
+                int per_sm = 0;
+                pb_raise_smem((const void *)tk, (int)tsm);
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tk, P16_TR_WARPS * 32, tsm);
+                const int nl = (int)all.size();
+                const int g = std::min((per_sm < 1 ? 1 : per_sm) * nsm, (nl + P16_TR_WARPS - 1) / P16_TR_WARPS);
+                PB_P16(cudaMemsetAsync(d_counter, 0, sizeof(int), st));
+                tk<<<g, P16_TR_WARPS * 32, tsm, st>>>(job, p, d_tlist, nl, prefix ? ends : out, d_counter);
                 pb_diag_count_launch(1);
-                P16_CK(cudaGetLastError());
-            }
-            if (walk) {
-                const int nw = (int)all.size() * 32;
-                const pb_pair_out *e = prefix ? ends : out;
-                if (m->alg == PB_SW) k_p16_walk<PB_SW><<<(nw + 127) / 128, 128, 0, st>>>(p, d_tlist, (int)all.size(), e, m->open, m->gap);
-                else if (m->alg == PB_NW) k_p16_walk<PB_NW><<<(nw + 127) / 128, 128, 0, st>>>(p, d_tlist, (int)all.size(), e, m->open, m->gap);
-                else k_p16_walk<PB_SG><<<(nw + 127) / 128, 128, 0, st>>>(p, d_tlist, (int)all.size(), e, m->open, m->gap);
-                pb_diag_count_launch(1);
-                P16_CK(cudaGetLastError());
+                PB_P16(cudaGetLastError());
             }
             /* the host vectors handed to the copies above change next chunk */
-            P16_CK(cudaStreamSynchronize(st));
+            PB_P16(cudaStreamSynchronize(st));
             t0 = t1;
         }
-        if (bitsbuf) cudaFreeAsync(bitsbuf, st);
+        if (ckbuf) cudaFreeAsync(ckbuf, st);
         /* items whose width verdicts need exact extremes */
         if (!prefix) {
-            P16_CK(cudaMemsetAsync(counts + 1, 0, sizeof(int), st));
+            PB_P16(cudaMemsetAsync(counts + 1, 0, sizeof(int), st));
             k_p16_check<<<(nslots + 255) / 256, 256, 0, st>>>(job, p, d_rest + nrest, counts + 1);
             pb_diag_count_launch(1);
             int nx = 0;
-            P16_CK(cudaMemcpyAsync(&nx, counts + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-            P16_CK(cudaStreamSynchronize(st));
+            PB_P16(cudaMemcpyAsync(&nx, counts + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+            PB_P16(cudaStreamSynchronize(st));
             nrest += nx;
         }
     }
     *n_rest = nrest;
-    P16_CK(cudaStreamSynchronize(st));
+    PB_P16(cudaStreamSynchronize(st));
     return 0;
 }
 
@@ -1299,30 +1505,30 @@ int wave_subset(const pb_job &job, const pb_batch *b, const int *d_list, int n, 
     P16Frees frees(st);
     int64_t *gq = nullptr, *gt = nullptr;
     int *gql = nullptr, *gtl = nullptr, *sc = nullptr, *cnt = nullptr;
-    P16_CK(cudaMallocAsync((void **)&gq, sizeof(int64_t) * n, st)); frees.add(gq);
-    P16_CK(cudaMallocAsync((void **)&gt, sizeof(int64_t) * n, st)); frees.add(gt);
-    P16_CK(cudaMallocAsync((void **)&gql, sizeof(int) * n, st)); frees.add(gql);
-    P16_CK(cudaMallocAsync((void **)&gtl, sizeof(int) * n, st)); frees.add(gtl);
-    P16_CK(cudaMallocAsync((void **)&sc, sizeof(int) * n, st)); frees.add(sc);
-    P16_CK(cudaMallocAsync((void **)&cnt, sizeof(int), st)); frees.add(cnt);
+    PB_P16(cudaMallocAsync((void **)&gq, sizeof(int64_t) * n, st)); frees.add(gq);
+    PB_P16(cudaMallocAsync((void **)&gt, sizeof(int64_t) * n, st)); frees.add(gt);
+    PB_P16(cudaMallocAsync((void **)&gql, sizeof(int) * n, st)); frees.add(gql);
+    PB_P16(cudaMallocAsync((void **)&gtl, sizeof(int) * n, st)); frees.add(gtl);
+    PB_P16(cudaMallocAsync((void **)&sc, sizeof(int) * n, st)); frees.add(sc);
+    PB_P16(cudaMallocAsync((void **)&cnt, sizeof(int), st)); frees.add(cnt);
     k_gather_pairs<<<(n + 255) / 256, 256, 0, st>>>(d_list, n, b->d_qoff, b->d_qlen, b->d_toff, b->d_tlen, gq, gql,
                                                     gt, gtl);
     pb_diag_count_launch(1);
     std::vector<int> hl(n), hm((size_t)b->msize * b->msize);
-    P16_CK(cudaMemcpyAsync(hl.data(), gtl, sizeof(int) * n, cudaMemcpyDeviceToHost, st));
-    P16_CK(cudaMemcpyAsync(hm.data(), b->d_mat, sizeof(int) * hm.size(), cudaMemcpyDeviceToHost, st));
-    P16_CK(cudaMemsetAsync(cnt, 0, sizeof(int), st));
-    P16_CK(cudaStreamSynchronize(st));
+    PB_P16(cudaMemcpyAsync(hl.data(), gtl, sizeof(int) * n, cudaMemcpyDeviceToHost, st));
+    PB_P16(cudaMemcpyAsync(hm.data(), b->d_mat, sizeof(int) * hm.size(), cudaMemcpyDeviceToHost, st));
+    PB_P16(cudaMemsetAsync(cnt, 0, sizeof(int), st));
+    PB_P16(cudaStreamSynchronize(st));
     int maxlen = 0;
     for (int x : hl) maxlen = x > maxlen ? x : maxlen;
     if (pb_cuda_nw_long(n, job.mode.open, job.mode.gap, hm.data(), b->msize, b->d_qall, gq, gql, b->d_targets, gt,
                         gtl, nullptr, nullptr, maxlen, sc) != 0)
         return -1;
-    P16_CK(cudaDeviceSynchronize());
+    PB_P16(cudaDeviceSynchronize());
     k_wave_fill<<<(n + 255) / 256, 256, 0, st>>>(job, d_list, n, sc, gql, gtl, out, d_rest2, cnt);
     pb_diag_count_launch(1);
-    P16_CK(cudaMemcpyAsync(n_rest2, cnt, sizeof(int), cudaMemcpyDeviceToHost, st));
-    P16_CK(cudaStreamSynchronize(st));
+    PB_P16(cudaMemcpyAsync(n_rest2, cnt, sizeof(int), cudaMemcpyDeviceToHost, st));
+    PB_P16(cudaStreamSynchronize(st));
     return 0;
 }
 
@@ -1367,22 +1573,22 @@ int exact_subset(const pb_batch *b, const int *d_list, int n, int stats, int pad
     int64_t *g_toff = nullptr, *g_qoff = nullptr;
     int *g_tlen = nullptr, *g_qlen = nullptr, *g_pidx = nullptr, *g_qlim = nullptr, *g_tlim = nullptr;
     pb_pair_out *tmp = nullptr;
-    P16_CK(cudaMallocAsync((void **)&g_toff, sizeof(int64_t) * n, st)); frees.add(g_toff);
-    P16_CK(cudaMallocAsync((void **)&g_tlen, sizeof(int) * n, st)); frees.add(g_tlen);
-    P16_CK(cudaMallocAsync((void **)&tmp, sizeof(pb_pair_out) * n, st)); frees.add(tmp);
+    PB_P16(cudaMallocAsync((void **)&g_toff, sizeof(int64_t) * n, st)); frees.add(g_toff);
+    PB_P16(cudaMallocAsync((void **)&g_tlen, sizeof(int) * n, st)); frees.add(g_tlen);
+    PB_P16(cudaMallocAsync((void **)&tmp, sizeof(pb_pair_out) * n, st)); frees.add(tmp);
     if (dbmode) {
-        P16_CK(cudaMallocAsync((void **)&g_pidx, sizeof(int) * n, st)); frees.add(g_pidx);
+        PB_P16(cudaMallocAsync((void **)&g_pidx, sizeof(int) * n, st)); frees.add(g_pidx);
     } else {
-        P16_CK(cudaMallocAsync((void **)&g_qoff, sizeof(int64_t) * n, st)); frees.add(g_qoff);
-        P16_CK(cudaMallocAsync((void **)&g_qlen, sizeof(int) * n, st)); frees.add(g_qlen);
+        PB_P16(cudaMallocAsync((void **)&g_qoff, sizeof(int64_t) * n, st)); frees.add(g_qoff);
+        PB_P16(cudaMallocAsync((void **)&g_qlen, sizeof(int) * n, st)); frees.add(g_qlen);
     }
-    if (b->d_qlim) { P16_CK(cudaMallocAsync((void **)&g_qlim, sizeof(int) * n, st)); frees.add(g_qlim); }
-    if (b->d_tlim) { P16_CK(cudaMallocAsync((void **)&g_tlim, sizeof(int) * n, st)); frees.add(g_tlim); }
+    if (b->d_qlim) { PB_P16(cudaMallocAsync((void **)&g_qlim, sizeof(int) * n, st)); frees.add(g_qlim); }
+    if (b->d_tlim) { PB_P16(cudaMallocAsync((void **)&g_tlim, sizeof(int) * n, st)); frees.add(g_tlim); }
     k_gather_items<<<(n + 255) / 256, 256, 0, st>>>(d_list, n, dbmode ? b->npairs : 0, b->d_toff, b->d_tlen,
                                                     b->d_qoff, b->d_qlen, b->d_qlim, b->d_tlim, g_toff, g_tlen,
                                                     g_qoff, g_qlen, g_pidx, g_qlim, g_tlim);
     pb_diag_count_launch(1);
-    P16_CK(cudaStreamSynchronize(st));
+    PB_P16(cudaStreamSynchronize(st));
     pb_batch s = *b;
     s.npairs = n;
     s.stats = stats;
@@ -1395,7 +1601,7 @@ int exact_subset(const pb_batch *b, const int *d_list, int n, int stats, int pad
     if (pb_cuda_align_exact(&s) != 0) return -1;
     k_scatter_items<<<(n + 255) / 256, 256, 0, st>>>(tmp, d_list, n, out);
     pb_diag_count_launch(1);
-    P16_CK(cudaStreamSynchronize(st));
+    PB_P16(cudaStreamSynchronize(st));
     return 0;
 }
 
@@ -1523,7 +1729,7 @@ struct TraceCigars {
 
 /* Traceback paths of n pairs from host memory (pairs mode: tmpl carries the
  * matrix table on the device): characters copied and mapped on the device,
- * the pair kernels with direction bits and the path walk, then per pair
+ * the pair kernels with checkpoints and the traceback, then per pair
  * h_ends[3k..] = score, end_query, end_ref, the steps in
  * h_ops[h_ops_off[k] ..] (written backwards from the end of the pair's
  * qlen + tlen bytes) and h_info[3k..] = steps (-1: the pair is outside the
