@@ -44,7 +44,7 @@
  * cells carry 0. Those counts are the counts along that path, which four
  * decisions per cell define: not-diagonal (H > H_diag + s), not-F (H > F), E
  * opened and F opened. The forward kernel leaves checkpoints instead of the
- * decisions -- every pass's bottom row, and its column state every P16_CK
+ * decisions -- every pass's bottom row, and its column state every p16_ck
  * columns -- and the traceback (k_p16_trace) recomputes only the blocks that
  * the path from the end cell crosses, adding 1 to length per step and, on
  * diagonal steps, the match and positive-score indicators; in SW it stops
@@ -79,20 +79,26 @@ static constexpr int P16_ROW = 48;            /* bytes between two letters' scor
 static constexpr int P16_TR_WARPS = 2;        /* warps per block of the traceback */
 /* Checkpoints of a task (one lane's words 32 apart): per pass its bottom row,
  * p16_cols words (entry c + 1: H low and F high at column c), and per pass
- * and block of P16_CK columns after the first the state before the block's
+ * and block of p16_ck columns after the first the state before the block's
  * first iteration: H and E of the 16 register rows, F of the last one, and
  * the next diagonal. */
-static constexpr int P16_CK = 32, P16_CK_U4 = P16_R / 2 + 1;
-__host__ __device__ __forceinline__ int p16_ck_blocks(int wmax) { return (p16_cols(wmax) - 1) / P16_CK; }
+static constexpr int P16_CK_U4 = P16_R / 2 + 1;
+/* Columns per block. A path that crosses every pass recomputes blocks in step
+ * with the 31 others of its warp, a whole block each time: 16 (1 M reads, NW:
+ * traceback 8.7 -> 7.0 ms, forward pass 10.3 -> 10.4). Short local paths
+ * cross few blocks, and the column states' traffic counts: 32 (all against
+ * all: forward pass 72.7 ms, 78.2 with 16). */
+__host__ __device__ constexpr int p16_ck(int alg) { return alg == PB_SW ? 32 : 16; }
+__host__ __device__ __forceinline__ int p16_ck_blocks(int alg, int wmax) { return (p16_cols(wmax) - 1) / p16_ck(alg); }
 /* in words */
 __device__ __forceinline__ size_t p16_ck_row(int wmax, int pass, int entry)
 {
     return ((size_t)pass * p16_cols(wmax) + entry) * 32;
 }
 /* in uint4 from the task's first */
-__host__ __device__ __forceinline__ size_t p16_ck_col(int npass, int wmax, int pass, int block)
+__host__ __device__ __forceinline__ size_t p16_ck_col(int alg, int npass, int wmax, int pass, int block)
 {
-    return (size_t)npass * p16_cols(wmax) * 8 + ((size_t)pass * p16_ck_blocks(wmax) + block) * P16_CK_U4 * 32;
+    return (size_t)npass * p16_cols(wmax) * 8 + ((size_t)pass * p16_ck_blocks(alg, wmax) + block) * P16_CK_U4 * 32;
 }
 
 /* the bit of query row i of a block's direction bits (row i of its pass): the
@@ -257,7 +263,7 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
         /* the task's checkpoints: rows (entry c + 1 of a pass: its bottom row at
          * column c), then columns */
         uint32_t *ckr = CKPT ? reinterpret_cast<uint32_t *>(p.ckpt + p.task_ckpt[task]) + lane : nullptr;
-        uint4 *ckc = CKPT ? p.ckpt + p.task_ckpt[task] + p16_ck_col(npass, wmax, 0, 0) + lane : nullptr;
+        uint4 *ckc = CKPT ? p.ckpt + p.task_ckpt[task] + p16_ck_col(ALG, npass, wmax, 0, 0) + lane : nullptr;
         int status = 0;
 
         /* end tracking */
@@ -381,9 +387,9 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
             ResidueWords tw;
             tw.start(tseq, cols);
             for (int j0 = 0; j0 <= wmax; j0 += 4, in_at += 4 * 32, out_at += 4 * 32) {
-                if (CKPT && j0 > 0 && j0 % P16_CK == 0) {
+                if (CKPT && j0 > 0 && j0 % p16_ck(ALG) == 0) {
                     /* the state before iteration j0 */
-                    uint4 *d = ckc + ((size_t)pass * p16_ck_blocks(wmax) + j0 / P16_CK - 1) * P16_CK_U4 * 32;
+                    uint4 *d = ckc + ((size_t)pass * p16_ck_blocks(ALG, wmax) + j0 / p16_ck(ALG) - 1) * P16_CK_U4 * 32;
 #pragma unroll
                     for (int x = 0; x < P16_R / 4; ++x) {
                         d[x * 32] = make_uint4(H[4 * x], H[4 * x + 1], H[4 * x + 2], H[4 * x + 3]);
@@ -595,7 +601,7 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
  * The traceback of one task's items, a lane each: from its end cell back
  * along the path the reference's tie rules select. A lane restarts the
  * dynamic program at the checkpoint before its cell -- the column state at
- * the start of the cell's block of P16_CK columns, the bottom row of the
+ * the start of the cell's block of p16_ck columns, the bottom row of the
  * pass above -- and recomputes the block up to the cell with the direction
  * bits of its 32 rows in shared memory, walks until it leaves the block, and
  * goes on with the next one. The lanes of a warp run their blocks in step,
@@ -604,9 +610,9 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
  * alignment of unrelated sequences, where direction bits had to be computed
  * and stored for the whole prefix before the end cell. All against all, 524 k
  * protein pairs: 158 ms of prefix pass and walk -> 7.5 ms; 1 M reads, NW: 3.2
- * ms of walk over stored bits -> 8.7 ms, against 19 ms less in the forward
- * pass. Bound by latency: shared memory (the block's bits and the lane's
- * scores) holds ten warps an SM for DNA, four for proteins.
+ * ms of walk over stored bits -> 7.0 ms, against 19 ms less in the forward
+ * pass. Bound by the ALU and FMA pipes for DNA (58% each), by latency for
+ * proteins, whose scores leave room for four warps an SM.
  *
  * The bits (the four decisions of the file comment) are signs of differences;
  * of two rows, one permute spreads the signs over four bytes (strips A and B
@@ -626,12 +632,12 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
  * 143-243).
  */
 template <int ALG, int MODE, bool BIAS>
-__global__ void __launch_bounds__(P16_TR_WARPS * 32, 5)
+__global__ void __launch_bounds__(P16_TR_WARPS * 32, 7)
 k_p16_trace(pb_job job, P16Params p, const int *__restrict__ tlist, int ntl, const pb_pair_out *__restrict__ ends,
             int *counter)
 {
     extern __shared__ __align__(16) int8_t s_mem[];
-    constexpr int LETTER = 1024, STRIP = 512;
+    constexpr int LETTER = 1024, STRIP = 512, CK = p16_ck(ALG);
     const int L = p.nletters;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int open = p.open, gap = p.gap, sgf = p.sgflags;
@@ -640,9 +646,9 @@ k_p16_trace(pb_job job, P16Params p, const int *__restrict__ tlist, int ntl, con
      * a block][scores] */
     const int mat_bytes = p.mat8 ? ((L * L + 15) & ~15) : 0;
     int8_t *s_mat = s_mem;
-    int8_t *wmem = s_mem + mat_bytes + (size_t)wid * (P16_CK * 512 + L * LETTER);
+    int8_t *wmem = s_mem + mat_bytes + (size_t)wid * (CK * 512 + L * LETTER);
     uint4 *tile = reinterpret_cast<uint4 *>(wmem) + lane;
-    int8_t *sl = wmem + P16_CK * 512 + lane * 16;
+    int8_t *sl = wmem + CK * 512 + lane * 16;
     if (p.mat8)
         for (int x = threadIdx.x; x < L * L; x += blockDim.x) s_mat[x] = (int8_t)(p.mat8[x] + bias);
     __syncthreads();
@@ -662,7 +668,7 @@ k_p16_trace(pb_job job, P16Params p, const int *__restrict__ tlist, int ntl, con
         const int wmax = p.task_wmax[task], npass = p.task_npass[task];
         const int stride = p16_cols(wmax);
         const uint32_t *ckr = reinterpret_cast<const uint32_t *>(p.ckpt + p.task_ckpt[task]) + lane;
-        const uint4 *ckc = p.ckpt + p.task_ckpt[task] + p16_ck_col(npass, wmax, 0, 0) + lane;
+        const uint4 *ckc = p.ckpt + p.task_ckpt[task] + p16_ck_col(ALG, npass, wmax, 0, 0) + lane;
         const int ti = p.nt ? item % p.nt : item;
         const uint8_t *tseq = p.targets + (valid ? p.toff[ti] : 0);
         const uint8_t *qseq = nullptr;
@@ -700,7 +706,7 @@ k_p16_trace(pb_job job, P16Params p, const int *__restrict__ tlist, int ntl, con
         while (__any_sync(0xffffffffu, active)) {
             const int pass = active ? i >> 5 : 0, r0 = pass * P16_PASS;
             const int jt = active ? j + ((i >> 4) & 1) : 0;  /* the iteration of the cell */
-            const int jb = jt / P16_CK * P16_CK;
+            const int jb = jt / CK * CK;
             /* the scores (BIAS: + open) of this pass's rows */
             if (active && pass != staged) {
                 staged = pass;
@@ -767,7 +773,7 @@ k_p16_trace(pb_job job, P16Params p, const int *__restrict__ tlist, int ntl, con
                 prev_h = (uint32_t)(uint16_t)(p16_left(ALG, sgf, r0 + P16_R - 1, open, gap) - bias);
                 prev_f = NEG & 0xffffu;
             } else {
-                const uint4 *d = ckc + ((size_t)pass * p16_ck_blocks(wmax) + jb / P16_CK - 1) * P16_CK_U4 * 32;
+                const uint4 *d = ckc + ((size_t)pass * p16_ck_blocks(ALG, wmax) + jb / CK - 1) * P16_CK_U4 * 32;
 #pragma unroll
                 for (int x = 0; x < P16_R / 4; ++x) {
                     const uint4 h4 = __ldcg(d + x * 32), e4 = __ldcg(d + (x + P16_R / 4) * 32);
@@ -995,7 +1001,7 @@ __global__ void k_p16_tasks(P16Params p, int ntasks, const int *__restrict__ gro
         twmax[task] = c;
         tnpass[task] = np;
         tshared[task] = p.mat8 ? (same && group != nullptr) : 1;
-        tckpt[task] = ckpt ? (long long)p16_ck_col(np, c, np, 0) : 0;
+        tckpt[task] = ckpt ? (long long)p16_ck_col(p.alg, np, c, np, 0) : 0;
     }
 }
 
@@ -1421,7 +1427,7 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
                 const int mode = paths ? 2 : out2 ? 1 : 0;
                 const p16_trace_t tk = bias ? pick_trace<true>(m->alg, mode) : pick_trace<false>(m->alg, mode);
                 const size_t tsm = (d_mat8 ? (((size_t)L * L + 15) & ~(size_t)15) : 0) +
-                                   (size_t)P16_TR_WARPS * (P16_CK * 512 + (size_t)L * 1024);
+                                   (size_t)P16_TR_WARPS * (p16_ck(m->alg) * 512 + (size_t)L * 1024);
                 int per_sm = 0;
                 pb_raise_smem((const void *)tk, (int)tsm);
                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tk, P16_TR_WARPS * 32, tsm);
