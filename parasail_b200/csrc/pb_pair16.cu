@@ -1148,6 +1148,22 @@ p16_kernel_t pick(int alg, bool ckpt, bool ends, bool shared, int warps)
     return ckpt ? pick3<PB_SG, true, true, BIAS>(shared, warps) : pick3<PB_SG, false, true, BIAS>(shared, warps);
 }
 
+/* the current device's memory in bytes */
+size_t device_memory()
+{
+    static std::mutex mu;
+    static std::vector<size_t> seen;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(mu);
+    if ((size_t)dev >= seen.size()) seen.resize(dev + 1, 0);
+    if (!seen[dev]) {
+        size_t free_b = 0, total = 0;
+        seen[dev] = cudaMemGetInfo(&free_b, &total) == cudaSuccess && total ? total : (size_t)24 << 30;
+    }
+    return seen[dev];
+}
+
 typedef void (*p16_trace_t)(pb_job, P16Params, const int *, int, const pb_pair_out *, int *);
 
 template <bool BIAS>
@@ -1339,20 +1355,30 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
         std::stable_sort(torder.begin(), torder.end(), [&](int x, int y) {
             return (long long)hn[x] * (hw[x] + 1) > (long long)hn[y] * (hw[y] + 1);
         });
-        /* chunks of tasks whose checkpoints fit the budget: half of the free
-         * device memory (at most 96 GiB), so that a chunk of the largest tasks
-         * (about 20 MB each at 1500 x 1500) still fills the SMs. A batch of 1
-         * GiB or less takes what it needs without asking the device, which
-         * took 0.1 to 9 ms beside other copies. */
-        size_t all_u4 = 0;
+        /* chunks of tasks whose checkpoints fit the budget: a third of the
+         * device's memory, so that a chunk of the largest tasks (about 20 MB
+         * each at 1500 x 1500) still fills the SMs; halved when the allocation
+         * fails. The free memory is not asked for: on a shared host that call
+         * takes 0.1 to 90 ms, at random (18.9 ms passes of 1 M reads became
+         * 20-110 ms). */
+        size_t all_u4 = 0, budget_u4 = device_memory() / 3 / sizeof(uint4);
         for (int t = 0; t < ntasks; ++t) all_u4 += (size_t)hb[t];
-        size_t budget = (size_t)1 << 30;
-        if (all_u4 * sizeof(uint4) > budget) {
-            size_t free_b = 0, total_b = 0;
-            cudaMemGetInfo(&free_b, &total_b);
-            budget = std::max(budget, std::min((size_t)96 << 30, free_b / 2));
+        /* Chunks of like make-up: chunk c takes tasks c, c + nch, ... of the
+         * order, so that each ends on small tasks (524 k protein pairs in two
+         * chunks: 84.2 ms when the first took the largest tasks, 80.7 so). */
+        const int nch = (int)std::min<size_t>((size_t)ntasks, all_u4 / budget_u4 + 1);
+        std::vector<int> cut(nch + 1, 0);
+        if (nch > 1) {
+            std::vector<int> dealt;
+            dealt.reserve(ntasks);
+            for (int c = 0; c < nch; ++c) {
+                for (int t = c; t < ntasks; t += nch) dealt.push_back(torder[t]);
+                cut[c + 1] = (int)dealt.size();
+            }
+            torder.swap(dealt);
         }
-        const size_t budget_u4 = budget / sizeof(uint4);
+        cut[nch] = ntasks;
+        budget_u4 = all_u4 / nch + (size_t)*std::max_element(hb.begin(), hb.end()) * 2;
         /* launch shapes and the pass-boundary buffers, sized for the larger grid */
         int dev = 0, nsm = 0;
         cudaGetDevice(&dev);
@@ -1394,7 +1420,8 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
             /* the chunk [t0, t1) of torder, its tasks listed shared-first */
             int t1 = t0;
             size_t used = 0;
-            while (t1 < ntasks && (t1 == t0 || used + (size_t)hb[torder[t1]] <= budget_u4)) used += (size_t)hb[torder[t1++]];
+            const int t_end = *std::upper_bound(cut.begin(), cut.end(), t0);
+            while (t1 < t_end && (t1 == t0 || used + (size_t)hb[torder[t1]] <= budget_u4)) used += (size_t)hb[torder[t1++]];
             std::vector<int> lst[2];
             for (int k = t0; k < t1; ++k) lst[hs[torder[k]] ? 1 : 0].push_back(torder[k]);
             size_t off = 0;
@@ -1402,7 +1429,14 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
             if (ckpt && off > ck_cap) {
                 if (ckbuf) cudaFreeAsync(ckbuf, st);
                 ckbuf = nullptr;
-                PB_P16(cudaMallocAsync((void **)&ckbuf, sizeof(uint4) * (off + 1), st));
+                ck_cap = 0;
+                if (cudaMallocAsync((void **)&ckbuf, sizeof(uint4) * (off + 1), st) != cudaSuccess) {
+                    ckbuf = nullptr;
+                    cudaGetLastError();
+                    if (t1 - t0 > 1) { budget_u4 = off / 2; continue; }
+                    fprintf(stderr, "pb_pair16: checkpoints of %zu bytes failed\n", sizeof(uint4) * (off + 1));
+                    return -1;
+                }
                 ck_cap = off;
             }
             p.ckpt = ckbuf;
