@@ -100,8 +100,8 @@ __device__ __forceinline__ void fold_best(Sw16Best &best, const Sw16Best &s)
  * groups (at the profiles' own stride, a multiple of 64, the kernel took
  * 1.07 to 1.17 times as long), and the launch holds any number of queries of
  * any length, where whole profiles in shared memory ended at 200 KB.
- * 5 queries (100-2000) x 200,000 targets (2.7e11 cells): 102.0 -> 55.6 ms,
- * 4,900 GCUPS, ALU pipe 84% busy; 40 queries (median 270) x 10,000 targets:
+ * 5 queries (100-2000) x 200,000 targets (2.7e11 cells): 102.0 -> 54.9 ms,
+ * 4,950 GCUPS, ALU pipe 84% busy; 40 queries (median 270) x 10,000 targets:
  * 28 ms in four launches of whole profiles -> 12.1 ms in one.
  */
 template <bool BIAS>
@@ -256,7 +256,7 @@ k_sw16(Sw16Params p, int *task_counter)
                     v_n[u] = j + 4 < rd ? __ldcg(in_at + u * 32) : vnone;
                     uint32_t hu = prmt(v, prev_h, 0x5410u);     /* lo <- previous pass's strip B bottom */
                     uint32_t fu = prmt(v, prev_f, 0x5432u);
-                    const int8_t *pa_at = slice + ((codes >> (8 * u)) & 0xffu) * SW16_ROW;
+                    const int8_t *pa_at = slice + __byte_perm(codes, 0u, 0x4440u + u) * SW16_ROW;
                     const uint4 pa4 = *reinterpret_cast<const uint4 *>(pa_at);
                     const uint4 pb4 = *reinterpret_cast<const uint4 *>(pb_at);
                     pb_at = pa_at + SW16_R;
@@ -322,9 +322,8 @@ k_sw16(Sw16Params p, int *task_counter)
                             E[r] = (E[r] & 0xffffu) | (gapO & 0xffff0000u);
                         }
                     }
-                    bool ge_lo, ge_hi;
-                    (void)__vibmax_s16x2(sbest, cmax, &ge_hi, &ge_lo);
-                    if (!ge_lo || !ge_hi) {
+                    if (__vmaxs2(sbest, cmax) != sbest) {
+                        const bool ge_lo = s16lo(cmax) <= s16lo(sbest), ge_hi = s16hi(cmax) <= s16hi(sbest);
                         /* past its half's bound: keep the column (the warp
                          * takes this branch whenever any lane does, so the row
                          * is looked up once per pass, from the saved column).
