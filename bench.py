@@ -53,9 +53,10 @@ QUERY_LENGTHS = (100, 250, 500, 1000, 2000)
 N_TARGETS = 200_000
 OPS_PER_CELL = 6   # SW score-only algorithmic lane-operations per cell
 # DRAM bytes (read + write) per cell of k_sw16 on this workload, from one ncu
-# capture of a full-size launch (60.1 GB for 2.7213e11 cells)
-SW16_DRAM_BYTES_PER_CELL = 60.08e9 / 2.7213e11
+# capture of a launch on 100,000 targets (15.5 GB for 1.348e11 cells)
+SW16_DRAM_BYTES_PER_CELL = 15.54e9 / 1.348e11
 REF_DRIVER = os.path.join(ROOT, "oracle", "_ref", "ref_driver")
+REF_UNAVAILABLE = "oracle/_ref/ref_driver is not built"
 FIELDS = ("score", "end_query", "end_ref", "flag", "matches", "similar", "length")
 
 
@@ -171,7 +172,10 @@ def ref_run(family, width, mspec, open_, gap, mode, qfile, tfile, limit=None, st
             records=True, threads=None):
     """Runs the reference's AVX2 kernels through ref_driver. Returns a dict
     with pairs, cells, per-repetition seconds and (records=True) the
-    per-pair records as int32 [pairs, 8]."""
+    per-pair records as int32 [pairs, 8]; where the driver is not built, one
+    without records that cpu_block and compare report as such."""
+    if not os.path.exists(REF_DRIVER):
+        return {"unavailable": REF_UNAVAILABLE, "pairs": 0, "cells": 0.0, "records": None}
     threads = threads or os.cpu_count() or 1
     with tempfile.TemporaryDirectory() as td:
         rec = os.path.join(td, "rec.bin")
@@ -203,6 +207,8 @@ def cpu_model():
 
 def cpu_block(r, sample, kind="reference"):
     """cpu_baseline object from a ref_run result (median repetition)."""
+    if "unavailable" in r:
+        return {"unavailable": r["unavailable"]}
     sec = statistics.median(r["reps"]) if r["reps"] else r["seconds"]
     return {"value": r["cells"] / sec / 1e9, "unit": "GCUPS", "cores": r["threads"], "kind": kind,
             "pairs_per_s": r["pairs"] / sec, "sample": sample, "seconds_per_pass": sec,
@@ -212,6 +218,8 @@ def cpu_block(r, sample, kind="reference"):
 def compare(gpu, ref, fields=FIELDS):
     """Field-by-field mismatch counts of GPU records (int32 [n, 8] or the
     structured record array) against reference records (int32 [n, 8])."""
+    if ref is None:
+        return {"unavailable": REF_UNAVAILABLE}
     g = np.asarray(gpu)
     if g.dtype.names:
         g = np.stack([g[f] for f in FIELDS + ("reserved",)], axis=1)
@@ -491,7 +499,6 @@ def leg_config5(pb, args, td):
     write_lines(tf, te[3], te[4][:k], te[5][:k])
     r = ref_run("nw_scan", 32, "ACGT:1:-2", 4, 1, "pairs", qf, tf)
     pb.lib.parasail_matrix_free(dna)
-    ref_scores = r["records"][:, 0]
     return {"workload": "%d DNA pairs 5-50 kbp (1-15%% divergence, 30%% with a 50-500 bp indel), +1/-2, "
                         "open 4, extend 1; model trained on %d separate pairs" % (n_test, len(tr[2])),
             "cells_full_dp": cells, "generate_seconds": gen_s,
@@ -509,8 +516,9 @@ def leg_config5(pb, args, td):
             "scores_identical_to_full_dp": bool((sc == full).all()),
             "train": {"pairs": len(tr[2]), "epochs": 120, "final_loss": loss, "seconds": train_s},
             "cpu_baseline": cpu_block(r, "reference nw_scan_profile_32 on the first %d test pairs" % k),
-            "parity": {"full_dp_vs_reference_scores": {"pairs_compared": k,
-                                                       "mismatches": int((full[:k] != ref_scores).sum())},
+            "parity": {"full_dp_vs_reference_scores":
+                           {"pairs_compared": k, "mismatches": int((full[:k] != r["records"][:, 0]).sum())}
+                           if r["records"] is not None else {"unavailable": REF_UNAVAILABLE},
                        "learned_band_vs_full_dp_scores": {"pairs_compared": n_test,
                                                           "mismatches": int((sc != full).sum())}}}
 
@@ -529,7 +537,7 @@ def run_reference(args, rank, world):
     if rank != 0:
         return
     if not os.path.exists(REF_DRIVER):
-        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/ref_driver is not built"}))
+        print(json.dumps({"impl": "reference", "unavailable": REF_UNAVAILABLE}))
         return
     queries, buf, offs, lens = workload(0, args.n_targets)
     with tempfile.TemporaryDirectory() as td:
