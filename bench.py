@@ -676,7 +676,8 @@ def main():
     def pipe_roofline(gcups, ops):
         return {"bound": "int", "ops_per_cell": ops, "achieved": gcups * 1e9 * ops / 1e12,
                 "peak": peak / 1e12, "unit": "Tops/s", "frac": gcups * 1e9 * ops / peak if peak > 0 else None,
-                "note": "whole pipeline (every kernel of the call) against the live DPX peak"}
+                "note": "whole pipeline (every kernel of the call) against the live DPX peak; statistics "
+                        "counted as the recurrence's operations, of which a traceback needs fewer"}
     if isinstance(blocks.get("1"), dict) and "value" in blocks["1"]:
         blocks["1"]["roofline"] = pipe_roofline(blocks["1"]["value"], 6)
     if isinstance(blocks.get("3"), dict):

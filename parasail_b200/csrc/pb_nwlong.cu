@@ -436,8 +436,9 @@ k_nw_wave(NwWaveParams p, int *counter, int *error)
  * on one warp each, pass after pass, so that no warp waits for another (a
  * CTA of eight warps per pair of three passes leaves five idle).
  *
- * 64 DNA pairs of 5-50 kbp (5.9e10 cells): 104.5 -> 31.0 ms; the 18,000 pairs
- * above 512 residues of 100,000 protein pairs: 17.4 -> 5.8 ms. Bound by the
+ * 64 DNA pairs of 5-50 kbp (5.9e10 cells): 104.5 -> 25 ms; the 18,000 pairs
+ * above 512 residues of 100,000 protein pairs: 17.4 -> 4.9 ms; 256 pairs of
+ * 5-50 kbp in a band of 1,001 diagonals: 31.2 -> 17.4 ms. Bound by the
  * ALU pipe while all warps run, by the largest pairs' passes at the end.
  */
 template <int R, bool BANDED>

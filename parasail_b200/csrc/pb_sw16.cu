@@ -102,7 +102,7 @@ __device__ __forceinline__ void fold_best(Sw16Best &best, const Sw16Best &s)
  * any length, where whole profiles in shared memory ended at 200 KB.
  * 5 queries (100-2000) x 200,000 targets (2.7e11 cells): 102.0 -> 54.9 ms,
  * 4,950 GCUPS, ALU pipe 84% busy; 40 queries (median 270) x 10,000 targets:
- * 28 ms in four launches of whole profiles -> 12.1 ms in one.
+ * 28 ms in four launches of whole profiles -> 11.9 ms in one.
  */
 template <bool BIAS>
 __global__ void __launch_bounds__(SW16_WARPS * 32, 2)

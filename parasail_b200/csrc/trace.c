@@ -2,8 +2,8 @@
  * trace.c -- traceback entry points and CIGAR strings of parasail-b200.
  *
  * A trace result carries the alignment path the reference's trace tables
- * encode, computed on the GPU (pb_pair16.cu: direction bits per cell and a
- * walk from the end cell): the trace functions of the exact widths --
+ * encode, computed on the GPU (pb_pair16.cu: checkpoints and a traceback
+ * from the end cell): the trace functions of the exact widths --
  *   parasail_{alg}_trace, parasail_{alg}_trace_scan        (serial forms,
  *       src/sw_trace.c etc.: flags NOVEC / NOVEC_SCAN, 32 bits, 1 lane)
  *   parasail_{alg}_trace_{striped,scan}[_profile]_32       (the 32-bit
