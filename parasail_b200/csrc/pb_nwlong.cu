@@ -227,6 +227,16 @@ k_nw_wave(NwWaveParams p, int *counter, int *error)
                 }
                 return true;
             };
+            /* the whole warp: lane 0 acquires the counter, and the barrier
+             * orders every lane's ring loads after it (a shuffle orders no
+             * memory accesses) */
+            auto wait_warp = [&](int c) -> bool {
+                bool ok = true;
+                if (lane == 0) ok = wait_for(c);
+                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                __syncwarp();
+                return ok;
+            };
             int Hl[NWL_RL], E[NWL_RL];
 #pragma unroll
             for (int r = 0; r < NWL_RL; ++r) {
@@ -242,10 +252,7 @@ k_nw_wave(NwWaveParams p, int *counter, int *error)
                 if (BIAS && dg != NWL_NEG) dg -= open;
             } else {
                 dg = NWL_NEG;
-                bool ok = true;
-                if (lane == 0) ok = wait_for(jlo - 1);
-                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0);
-                if (!ok) break;
+                if (!wait_warp(jlo - 1)) break;
                 if (lane == 0 && jlo - 1 <= prev_jhi && jlo - 1 >= prev_jlo) dg = __ldcg(&in_buf[jlo - 1]).x;
             }
             int sh_h = NWL_NEG, sh_f = NWL_NEG;
@@ -273,10 +280,7 @@ k_nw_wave(NwWaveParams p, int *counter, int *error)
                 const int j = it - lane;
                 const int cpos = (it - jlo) & 31;
                 if (cpos == 0) {
-                    bool ok = true;
-                    if (lane == 0) ok = wait_for(it + 31);
-                    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0);
-                    if (!ok) { aborted = true; break; }
+                    if (!wait_warp(it + 31)) { aborted = true; break; }
                     cur_v = ring_at(it + lane);
                 }
                 const int vh = __shfl_sync(0xffffffffu, cur_v.x, cpos);
@@ -544,6 +548,15 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
                 }
                 return true;
             };
+            /* the whole warp: lane 0 acquires the counter, and the barrier
+             * orders every lane's ring loads after it, as in k_nw_wave */
+            auto wait_warp = [&](int c) -> bool {
+                bool ok = true;
+                if (lane == 0) ok = wait_for(c);
+                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                __syncwarp();
+                return ok;
+            };
             /* this lane's scores against every letter; rows past the query
              * take letter 0 (nothing above depends on them) */
             __syncwarp();
@@ -581,10 +594,7 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
             int dg_abs = INT_MIN;
             if (BANDED) {
                 /* the largest value above the first columns, or row -1's */
-                bool ok = true;
-                if (lane == 0) ok = wait_for(jlo + 31);
-                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-                if (!ok) break;
+                if (!wait_warp(jlo + 31)) break;
                 int top = INT_MIN;
                 if (pass == 0) {
                     top = left(0);
@@ -655,10 +665,7 @@ k_nw_wave16(NwWaveParams p, int *counter, int *error)
             int result = 0;
             bool have_result = false, aborted = false;
             for (int t0 = jlo; t0 < tend; t0 += 32) {
-                bool ok = true;
-                if (lane == 0) ok = wait_for(t0 + 31);
-                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-                if (!ok) { aborted = true; break; }
+                if (!wait_warp(t0 + 31)) { aborted = true; break; }
                 if (BANDED && t0 > jlo) {
                     /* rebase to the largest value held; what lies outside the
                      * band stays where it is */

@@ -75,3 +75,17 @@ def test_bands_of_long_pairs(alphabet, open_, gap):
         got = pb.nw_banded_batch(m, queries, targets, open_, gap, k)
         for q, t, g in zip(queries, targets, got):
             assert g == O.nw_banded(q, t, open_, gap, k, om)["score"], (k, len(q), len(t))
+
+
+@pytest.mark.parametrize("match,mismatch,open_,gap", [(100, -100, 20, 10), (3, -4, 8, 2)])
+def test_passes_read_what_the_pass_before_published(match, mismatch, open_, gap):
+    """Pairs of more passes than a team of several blocks has warps, so that
+    every ring is written over while the next block reads it: (100, -100) in
+    the 32-bit wavefront, (3, -4) in the 16-bit one. Insertions and deletions
+    make the lanes of one chunk read the ring at different times."""
+    rng = random.Random(match)
+    m = pb.matrix_create("ACGT", match, mismatch)
+    a = rand_seq(rng, 18700, DNA)
+    queries = [a, a[:18500], a[:600], a[:300]]
+    targets = [mutate(rng, a, DNA, 0.1, 0.04)[:9000], rand_seq(rng, 7000, DNA), mutate(rng, a[:600], DNA, 0.2, 0.1), a[:90]]
+    _check(m, queries, targets, open_, gap)
