@@ -74,3 +74,40 @@ def test_few_pairs_wavefront(open_, gap):
     queries = [rand_seq(rng, L, AA) for L in (40, 300, 700)]
     _check_db(queries, [rand_seq(rng, rng.randint(1, 500), AA) for _ in range(130)], "sw_striped_profile_16",
               open_, gap, 130, 3)
+
+
+@pytest.mark.parametrize("qlens,n", [((300,), 40), ((300,), 12000), ((60, 700, 1500), 5000), ((2000,), 10000)])
+def test_codes_outside_the_alphabet_read_as_letter_0(qlens, n):
+    """Caller-supplied device codes of the alphabet's size and more give the
+    records of the same targets with letter 0 there, whatever kernel the size
+    selects (the few-pairs kernel, warps, teams), also from a plan."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.RandomState(n)
+    b62 = pb.matrix_lookup("blosum62")
+    size = b62.contents.size
+    lens = rng.randint(1, 400, n).astype(np.int32)
+    offs = np.concatenate([[0], np.cumsum(lens[:-1], dtype=np.int64)]).astype(np.int64)
+    codes = rng.randint(0, size, int(lens.sum())).astype(np.uint8)
+    at = rng.randint(0, len(codes), len(codes) // 20)
+    codes[at] = rng.choice([size, size + 1, 31, 32, 127, 128, 200, 255], len(at)).astype(np.uint8)
+    clean = np.where(codes < size, codes, 0).astype(np.uint8)
+    profs = [pb.ProfileHandle("parasail_profile_create_sat", rand_seq(random.Random(L), L, AA), b62) for L in qlens]
+    parr = pb.ctypes.cast(pb.profile_array(profs), pb.ctypes.c_void_p)
+    d_offs, d_lens = torch.from_numpy(offs).cuda(), torch.from_numpy(lens).cuda()
+    recs = []
+    for c in (clean, codes):
+        d_codes = torch.from_numpy(c).cuda()
+        for plan in (False, True):
+            rec = torch.zeros((len(qlens), n, 8), dtype=torch.int32, device="cuda")
+            args = (b"sw_striped_profile_sat", parr, len(qlens), d_codes.data_ptr(), d_offs.data_ptr(), d_lens.data_ptr(),
+                    n, 11, 1, rec.data_ptr())
+            if plan:
+                h = pb.lib.parasail_b200_db_plan_create(*args)
+                assert h and pb.lib.parasail_b200_db_plan_run(h) == 0
+                pb.lib.parasail_b200_db_plan_free(h)
+            else:
+                assert pb.lib.parasail_b200_batch_db_device(*args) == 0
+            torch.cuda.synchronize()
+            recs.append(rec.cpu().numpy())
+    for r in recs[1:]:
+        assert np.array_equal(r, recs[0])
