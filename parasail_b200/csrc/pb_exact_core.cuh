@@ -152,7 +152,11 @@ __host__ __device__ __forceinline__ void exact_pair(const ExactParams &p, const 
             for (int r = 0; r < R; ++r) {
                 const int i = r0 + r;
                 const bool real = i < ql;
-                const int sc = real ? (matmode ? prow[pd.qcodes[i]] : prow[i]) : 0;
+                /* a query code outside the alphabet reads as letter 0 (a
+                 * profile was built from valid ones) */
+                int qc = real && (matmode || STATS) ? (int)pd.qcodes[i] : 0;
+                if (matmode && qc >= pd.size) { status |= PB_ST_BADCODE; qc = 0; }
+                const int sc = real ? (matmode ? prow[qc] : prow[i]) : 0;
                 /* F: vertical gap (along the query), E: horizontal gap */
                 const int f_opn = hu - open, f_ext = fu - gap;
                 const int fn = SCANF ? fu : max(f_opn, f_ext);
@@ -177,7 +181,7 @@ __host__ __device__ __forceinline__ void exact_pair(const ExactParams &p, const 
                     const int eL = (eo ? HlL[r] : EL[r]) + 1;
                     EM[r] = eM; ES[r] = eS; EL[r] = eL;
                     const bool isd = hn == hdag, isf = hn == fn;
-                    const int mt = real ? (pd.qcodes[i] == code) : 0;
+                    const int mt = real ? (qc == (matmode ? csafe : code)) : 0;
                     hM = isd ? DgM[r] + mt : (isf ? fM : eM);
                     hS = isd ? DgS[r] + (sc > 0) : (isf ? fS : eS);
                     hL = isd ? DgL[r] + 1 : (isf ? fL : eL);

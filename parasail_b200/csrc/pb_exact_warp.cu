@@ -219,7 +219,7 @@ k_exact_warp(ExactParams p, int nitems)
                      * (right scores, counts that no path gives) */
                     const bool isd = (int)((unsigned)hdag - (unsigned)max(en, fn)) >= 0;
                     const bool isf = (int)((unsigned)fn - (unsigned)en) >= 0;
-                    const int mt = real ? ((PAIRS ? qc[r] : (int)pd.qcodes[i]) == code) : 0;
+                    const int mt = real ? (PAIRS ? qc[r] == csafe : (int)pd.qcodes[i] == code) : 0;
                     hM = isd ? hdM + mt : (isf ? fM : eM);
                     hS = isd ? hdS + (sc > 0) : (isf ? fS : eS);
                     hL = isd ? hdL + 1 : (isf ? fL : eL);
