@@ -201,7 +201,10 @@ k_nw_wave(NwWaveParams p, int *counter, int *error)
             const long long out_base = (long long)(pass / T) * stride + 1;
             int qc[NWL_RL];
 #pragma unroll
-            for (int r = 0; r < NWL_RL; ++r) qc[r] = (R0 + r < n) ? qs[R0 + r] : 0;
+            for (int r = 0; r < NWL_RL; ++r) {
+                const int c = R0 + r < n ? (int)qs[R0 + r] : 0;
+                qc[r] = c < p.msize ? c : 0;
+            }
             int jlo = 0, jhi = m - 1, prev_jlo = 0, prev_jhi = m - 1;
             if (BANDED) {
                 jlo = max(0, r0 - hi);
@@ -288,7 +291,8 @@ k_nw_wave(NwWaveParams p, int *counter, int *error)
                 int up_h = __shfl_up_sync(0xffffffffu, sh_h, 1);
                 int up_f = __shfl_up_sync(0xffffffffu, sh_f, 1);
                 const bool active = j >= jlo && j <= jhi;
-                const int tc = tc_n1;
+                /* codes outside the alphabet read as letter 0 */
+                const int tc = tc_n1 < p.msize ? tc_n1 : 0;
                 tc_n1 = tc_n2;
                 tc_n2 = res_at(j + 2);
                 if (lane == 0 && active) {

@@ -89,3 +89,39 @@ def test_passes_read_what_the_pass_before_published(match, mismatch, open_, gap)
     queries = [a, a[:18500], a[:600], a[:300]]
     targets = [mutate(rng, a, DNA, 0.1, 0.04)[:9000], rand_seq(rng, 7000, DNA), mutate(rng, a[:600], DNA, 0.2, 0.1), a[:90]]
     _check(m, queries, targets, open_, gap)
+
+
+@pytest.mark.parametrize("match,open_,gap", [(2, 5, 2), (100, 200, 20), (100, 20, 10)])
+def test_codes_outside_the_alphabet_read_as_letter_0(match, open_, gap):
+    """Caller-supplied device codes of the alphabet's size and more, in
+    queries and targets, give the scores of letter 0 there: the 16-bit
+    wavefront, and the 32-bit one beside the biased form."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.RandomState(open_)
+    m = pb.matrix_create("ACGT", match, -match)
+    size = m.contents.size
+    rows = []
+    for outside in (False, True):
+        rng.seed(open_)
+        sets = []
+        for lo, hi in ((1, 900), (1, 700)):
+            lens = rng.randint(lo, hi, 40).astype(np.int32)
+            lens[:2] = (3000, 2600)
+            offs = np.concatenate([[0], np.cumsum(lens[:-1], dtype=np.int64)]).astype(np.int64)
+            codes = rng.randint(0, 4, int(lens.sum())).astype(np.uint8)
+            at = rng.randint(0, len(codes), len(codes) // 10)
+            bad = rng.choice([size, size + 1, 31, 32, 33, 128, 255], len(at)).astype(np.uint8)
+            codes[at] = bad if outside else 0
+            sets += [torch.from_numpy(x).cuda() for x in (codes, offs, lens)]
+        rec = torch.zeros((40, 8), dtype=torch.int32, device="cuda")
+        mask = pb.lib.parasail_b200_schedule_get()
+        pb.lib.parasail_b200_schedule_set(0xffffffff)        # every length to the wavefront
+        try:
+            rc = pb.lib.parasail_b200_batch_pairs_device(b"nw_striped_32", m, *[x.data_ptr() for x in sets], 40, open_, gap,
+                                                         rec.data_ptr())
+        finally:
+            pb.lib.parasail_b200_schedule_set(mask)
+        assert rc == 0
+        torch.cuda.synchronize()
+        rows.append(rec.cpu().numpy())
+    assert np.array_equal(rows[0], rows[1])
