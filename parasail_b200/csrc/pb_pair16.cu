@@ -283,8 +283,11 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
                 __syncwarp();
                 if (p.mat8) {
                     const int i = r0 + lane;
-                    uint32_t c = i < rmax ? qseq0[i] : 255u;
-                    if (c != 255u && c >= (uint32_t)L) { c = 0; status |= PB_ST_BADCODE; }
+                    uint32_t c = 255u;               /* past the query */
+                    if (i < rmax) {
+                        c = qseq0[i];
+                        if (c >= (uint32_t)L) { c = 0; status |= PB_ST_BADCODE; }
+                    }
                     for (int a = 0; a < L; ++a)
                         wslice[a * LETTER + lane] = c == 255u ? (int8_t)bias : s_mat[a * L + c];
                 } else {
@@ -306,8 +309,11 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
 #pragma unroll
                     for (int b = 0; b < 4; ++b) {
                         const int i = r0 + 4 * w + b;
-                        uint32_t c = i < rows ? qseq[i] : 255u;
-                        if (c != 255u && c >= (uint32_t)L) { c = 0; status |= PB_ST_BADCODE; }
+                        uint32_t c = 255u;           /* past the query */
+                        if (i < rows) {
+                            c = qseq[i];
+                            if (c >= (uint32_t)L) { c = 0; status |= PB_ST_BADCODE; }
+                        }
                         word |= c << (8 * b);
                     }
                     qc[w] = word;
@@ -718,8 +724,11 @@ k_p16_trace(pb_job job, P16Params p, const int *__restrict__ tlist, int ntl, con
 #pragma unroll
                         for (int b = 0; b < 4; ++b) {
                             const int x = r0 + 4 * w + b;
-                            uint32_t c = x < rows ? qseq[x] : 255u;
-                            if (c != 255u && c >= (uint32_t)L) c = 0;
+                            uint32_t c = 255u;
+                            if (x < rows) {
+                                c = qseq[x];
+                                if (c >= (uint32_t)L) c = 0;
+                            }
                             word |= c << (8 * b);
                         }
                         qc[w] = word;

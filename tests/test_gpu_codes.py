@@ -42,3 +42,15 @@ def test_exact_kernels(name, rows):
     q, t = rng.randint(rows[0], rows[1], 70), rng.randint(1, 200, 70)
     a, b = (records(name, m, q, t, 9000, 700, outside) for outside in (False, True))
     assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("name", ["sw_striped_32", "sw_stats_striped_32", "sw_stats_scan_32", "nw_stats_striped_32",
+                                  "sg_qx_stats_scan_32", "nw_scan_16"])
+@pytest.mark.parametrize("alphabet", ["ACGT", "ARNDCQEGHILKMFPSTWYV"])
+def test_pair_kernels(name, alphabet):
+    """Scores inside 16 bits: the pair kernels and their traceback."""
+    rng = np.random.RandomState(len(alphabet))
+    m = pb.matrix_create(alphabet, 2, -3)
+    q, t = rng.randint(1, 300, 300), rng.randint(1, 300, 300)
+    a, b = (records(name, m, q, t, 5, 2, outside) for outside in (False, True))
+    assert np.array_equal(a, b)
