@@ -62,6 +62,7 @@
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 #include <cub/device/device_select.cuh>
+#include <cuda/std/functional>
 #include <dlfcn.h>
 #include <mutex>
 #include <string>
@@ -69,6 +70,7 @@
 #include "pb_cuda.h"
 #include "pb_kernels.cuh"
 #include "pb_resolve.h"
+#include "pb_slices.h"
 
 namespace pb {
 
@@ -1669,7 +1671,7 @@ __global__ void k_p16_map_into(const uint8_t *__restrict__ raw, uint8_t *__restr
         codes[i] = smap[raw[i]];
 }
 
-/* What the CIGARs of a batch are built from and into. */
+/* What the CIGARs of a slice of a batch are built from and into. */
 struct CigarParams {
     int n, sg;
     const uint8_t *ops;             /* steps, at the end of each pair's rows + columns bytes */
@@ -1679,7 +1681,8 @@ struct CigarParams {
     const int64_t *qoff, *toff;
     const int *qlen, *tlen;
     const uint8_t *upper;           /* toupper of every character */
-    uint32_t *cig;                  /* elements, at ooff[k] */
+    uint32_t *cig;                  /* elements, at ooff[k] - cig0 */
+    int64_t cig0;
     int *len, *cnt, *beg;           /* elements (-1: no CIGAR), elements to copy, first positions */
 };
 
@@ -1705,7 +1708,7 @@ __global__ void k_p16_cigar(CigarParams p)
     const int end_q = p.ends[3 * k + 1], end_r = p.ends[3 * k + 2];
     const uint8_t *ops = p.ops + p.ooff[k] + lena + lenb - steps;
     const uint8_t *a = p.q + p.qoff[k], *b = p.t + p.toff[k];
-    uint32_t *out = p.cig + p.ooff[k];
+    uint32_t *out = p.cig + (p.ooff[k] - p.cig0);
     int i = p.info[3 * k + 1], j = p.info[3 * k + 2], n = 0;
     uint32_t op = 0, run = 0;
     auto add = [&](uint32_t o, int c) {
@@ -1748,14 +1751,13 @@ __global__ void k_p16_cigar(CigarParams p)
 }
 
 /* the pairs' elements side by side, a warp per pair */
-__global__ void k_p16_cigar_pack(const uint32_t *__restrict__ cig, const int64_t *__restrict__ ooff,
-                                 const int *__restrict__ cnt, const int64_t *__restrict__ coff, int n,
-                                 uint32_t *__restrict__ out)
+__global__ void k_p16_cigar_pack(CigarParams p, const int64_t *__restrict__ coff, uint32_t *__restrict__ out)
 {
     const int k = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    if (k >= n) return;
-    const int c = cnt[k];
-    for (int x = lane; x < c; x += 32) out[coff[k] + x] = cig[ooff[k] + x];
+    if (k >= p.n) return;
+    const uint32_t *cig = p.cig + (p.ooff[k] - p.cig0);
+    const int c = p.cnt[k];
+    for (int x = lane; x < c; x += 32) out[coff[k] + x] = cig[x];
 }
 
 __global__ void k_p16_ends(const pb_pair_out *__restrict__ o, int n, int *__restrict__ se)
@@ -1775,6 +1777,75 @@ struct TraceCigars {
     int *len, *beg;
     uint32_t **elems;
 };
+
+/* The CIGARs of all pairs, slice by slice: built on the device, packed there,
+ * and copied behind those of the slices before. cp holds the batch's device
+ * arrays. */
+static int trace_cigars(CigarParams cp, int n, const int *h_qlen, const int *h_tlen, const int64_t *h_ooff,
+                        const TraceCigars &cig, cudaStream_t st)
+{
+    pb::P16Frees frees(st);
+    size_t most = 0, have = 0;             /* elements: of a slice, on the host so far */
+    int widest = 0;                        /* pairs of a slice */
+    for (int k0 = 0, k1; k0 < n; k0 = k1) {
+        k1 = cigar_slice_end(h_ooff, h_qlen, h_tlen, n, k0, CIGAR_SLICE);
+        most = std::max(most, (size_t)(h_ooff[k1 - 1] + h_qlen[k1 - 1] + h_tlen[k1 - 1] - h_ooff[k0]));
+        widest = std::max(widest, k1 - k0);
+    }
+    uint32_t *d_cig = nullptr;
+    int *d_len = nullptr;
+    int64_t *d_coff = nullptr;
+    void *d_tmp = nullptr;
+    size_t tmp_bytes = 0;
+    /* the sums run in 64 bits, whatever the type of the counts */
+    auto scan = [&](int items) {
+        return cub::DeviceScan::ExclusiveScan(d_tmp, tmp_bytes, d_len, d_coff, cuda::std::plus<int64_t>{}, (int64_t)0, items, st);
+    };
+    if (scan(widest + 1) != cudaSuccess) return -1;
+    if (cudaMallocAsync((void **)&d_cig, sizeof(uint32_t) * (most + 1), st) == cudaSuccess) frees.add(d_cig);
+    if (cudaMallocAsync((void **)&d_len, sizeof(int) * (4 * (size_t)widest + 1), st) == cudaSuccess) frees.add(d_len);
+    if (cudaMallocAsync((void **)&d_coff, sizeof(int64_t) * ((size_t)widest + 1), st) == cudaSuccess) frees.add(d_coff);
+    if (cudaMallocAsync(&d_tmp, tmp_bytes, st) == cudaSuccess) frees.add(d_tmp);
+    if (frees.v.size() != 4) { cudaGetLastError(); return -1; }
+    const CigarParams all = cp;
+    for (int k0 = 0, k1; k0 < n; k0 = k1) {
+        k1 = cigar_slice_end(h_ooff, h_qlen, h_tlen, n, k0, CIGAR_SLICE);
+        const int m = k1 - k0;
+        /* d_len: [counts, one 0 after them][lengths][first positions] */
+        cp.n = m;
+        cp.info = all.info + 3 * (size_t)k0; cp.ends = all.ends + 3 * (size_t)k0;
+        cp.ooff = all.ooff + k0; cp.qoff = all.qoff + k0; cp.toff = all.toff + k0;
+        cp.qlen = all.qlen + k0; cp.tlen = all.tlen + k0;
+        cp.cig = d_cig; cp.cig0 = h_ooff[k0];
+        cp.cnt = d_len; cp.len = d_len + m + 1; cp.beg = d_len + 2 * (size_t)m + 1;
+        int64_t total = 0;
+        cudaMemsetAsync(d_len + m, 0, sizeof(int), st);
+        k_p16_cigar<<<(m + 63) / 64, 64, 0, st>>>(cp);
+        if (scan(m + 1) != cudaSuccess) return -1;
+        pb_diag_count_launch(1);
+        if (cudaMemcpyAsync(cig.len + k0, cp.len, sizeof(int) * (size_t)m, cudaMemcpyDeviceToHost, st) ||
+            cudaMemcpyAsync(cig.beg + 2 * (size_t)k0, cp.beg, sizeof(int) * 2 * (size_t)m, cudaMemcpyDeviceToHost, st) ||
+            cudaMemcpyAsync(&total, d_coff + m, sizeof total, cudaMemcpyDeviceToHost, st) ||
+            cudaStreamSynchronize(st) != cudaSuccess)
+            return -1;
+        uint32_t *elems = (uint32_t *)realloc(*cig.elems, sizeof(uint32_t) * (have + (size_t)total + 1));
+        if (!elems) return -1;
+        *cig.elems = elems;
+        uint32_t *d_pack = nullptr;
+        if (cudaMallocAsync((void **)&d_pack, sizeof(uint32_t) * (size_t)(total + 1), st) != cudaSuccess) {
+            cudaGetLastError();
+            return -1;
+        }
+        const int64_t threads = 32 * (int64_t)m;
+        k_p16_cigar_pack<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(cp, d_coff, d_pack);
+        pb_diag_count_launch(1);
+        cudaError_t e = cudaMemcpyAsync(elems + have, d_pack, sizeof(uint32_t) * (size_t)total, cudaMemcpyDeviceToHost, st);
+        cudaFreeAsync(d_pack, st);
+        if (e != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) return -1;
+        have += (size_t)total;
+    }
+    return 0;
+}
 
 /* Traceback paths of n pairs from host memory (pairs mode: tmpl carries the
  * matrix table on the device): characters copied and mapped on the device,
@@ -1859,48 +1930,20 @@ static int trace_host(const pb_job *job, const pb_batch *tmpl, const uint8_t *ma
                 rc = -1;
         }
         if (rc == 0 && cig) {
-            /* CIGARs on the device, packed there, and one copy back */
-            uint32_t *d_cig = nullptr, *d_pack = nullptr;
-            int *d_len = nullptr;
-            int64_t *d_coff = nullptr, total = 0;
-            void *d_tmp = nullptr;
-            size_t tmp_bytes = 0;
-            cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, d_len, d_coff, n + 1, st);
-            if (cudaMallocAsync((void **)&d_cig, sizeof(uint32_t) * (size_t)(ob + 1), st) ||
-                cudaMallocAsync((void **)&d_len, sizeof(int) * (4 * (size_t)n + 1), st) ||
-                cudaMallocAsync((void **)&d_coff, sizeof(int64_t) * ((size_t)n + 1), st) ||
-                cudaMallocAsync(&d_tmp, tmp_bytes, st))
-                rc = -1;
-            frees.add(d_cig); frees.add(d_len); frees.add(d_coff); frees.add(d_tmp);
-            if (rc == 0) {
-                /* d_len: [counts, one 0 after them][lengths][first positions] */
-                CigarParams cp;
-                cp.n = n; cp.sg = job->mode.alg == PB_SG;
-                cp.ops = d_ops; cp.ooff = d_ooff; cp.info = d_info; cp.ends = d_se;
-                cp.q = d_qraw; cp.t = d_traw; cp.qoff = d_qoff; cp.toff = d_toff; cp.qlen = d_qlen; cp.tlen = d_tlen;
-                cp.upper = d_map + 256; cp.cig = d_cig;
-                cp.cnt = d_len; cp.len = d_len + n + 1; cp.beg = d_len + 2 * (size_t)n + 1;
-                cudaMemsetAsync(d_len + n, 0, sizeof(int), st);
-                k_p16_cigar<<<(n + 63) / 64, 64, 0, st>>>(cp);
-                cub::DeviceScan::ExclusiveSum(d_tmp, tmp_bytes, d_len, d_coff, n + 1, st);
-                pb_diag_count_launch(1);
-                if (cudaMemcpyAsync(cig->len, cp.len, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost, st) ||
-                    cudaMemcpyAsync(cig->beg, cp.beg, sizeof(int) * 2 * (size_t)n, cudaMemcpyDeviceToHost, st) ||
-                    cudaMemcpyAsync(&total, d_coff + n, sizeof total, cudaMemcpyDeviceToHost, st) ||
-                    cudaStreamSynchronize(st) != cudaSuccess)
-                    rc = -1;
-            }
-            if (rc == 0) {
-                *cig->elems = (uint32_t *)malloc(sizeof(uint32_t) * (size_t)(total + 1));
-                if (!*cig->elems || cudaMallocAsync((void **)&d_pack, sizeof(uint32_t) * (size_t)(total + 1), st)) rc = -1;
-                frees.add(d_pack);
-            }
-            if (rc == 0) {
-                const int64_t threads = 32 * (int64_t)n;
-                k_p16_cigar_pack<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(d_cig, d_ooff, d_len, d_coff, n, d_pack);
-                pb_diag_count_launch(1);
-                if (cudaMemcpyAsync(*cig->elems, d_pack, sizeof(uint32_t) * (size_t)total, cudaMemcpyDeviceToHost, st))
-                    rc = -1;
+            CigarParams cp;
+            cp.sg = job->mode.alg == PB_SG;
+            cp.ops = d_ops; cp.ooff = d_ooff; cp.info = d_info; cp.ends = d_se;
+            cp.q = d_qraw; cp.t = d_traw; cp.qoff = d_qoff; cp.toff = d_toff; cp.qlen = d_qlen; cp.tlen = d_tlen;
+            cp.upper = d_map + 256;
+            /* (with no path among the pairs there is nothing to build) */
+            if (cudaStreamSynchronize(st) != cudaSuccess) rc = -1;
+            int first = 0;
+            while (rc == 0 && first < n && h_info[3 * (size_t)first] < 0) ++first;
+            if (rc == 0 && first < n) {
+                rc = trace_cigars(cp, n, h_qlen, h_tlen, h_ops_off, *cig, st);
+            } else if (rc == 0) {
+                std::fill(cig->len, cig->len + n, -1);
+                std::fill(cig->beg, cig->beg + 2 * (size_t)n, 0);
             }
         }
         if (cudaStreamSynchronize(st) != cudaSuccess) rc = -1;
@@ -1921,8 +1964,9 @@ extern "C" int pb_cuda_trace_pairs_host(const pb_job *job, const pb_batch *tmpl,
 
 /* The same with the CIGARs instead of the paths: h_len[k] elements of pair k
  * (-1: none), its first positions in h_beg[2k..], the elements of all pairs
- * side by side in *h_elems (malloc'd, the caller's). upper256: toupper of
- * every character. */
+ * side by side in *h_elems (malloc'd, the caller's; null when there are none,
+ * as it has to be at the call). upper256: toupper of every character.
+ * h_ops_off: ascending, pair k's rows + columns after it. */
 extern "C" int pb_cuda_trace_cigars_host(const pb_job *job, const pb_batch *tmpl, const uint8_t *mapper256,
                                          const uint8_t *upper256, const char *h_q, const int64_t *h_qoff,
                                          const int *h_qlen, const char *h_t, const int64_t *h_toff, const int *h_tlen,

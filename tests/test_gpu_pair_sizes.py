@@ -5,6 +5,7 @@ score + open out of int8), alphabets of a few and of many letters, and one
 query shared by a task. Every record against the oracle."""
 import random
 
+import numpy as np
 import pytest
 
 import oracle as O
@@ -120,3 +121,34 @@ def test_local_statistics_with_pairs_past_16_bits(name):
         targets.append(rand_seq(rng, rng.randint(0, 200), AA) +
                        (mutate(rng, q, AA, 0.4, 0.03) if rng.random() < 0.7 else rand_seq(rng, rng.randint(1, 700), AA)) or "A")
     _check(name, pb.batch_pairs(name, m, queries, targets, 11, 1), queries, targets, 11, 1, om)
+
+
+def test_batch_cigars_in_several_slices():
+    """A batch of more residues than one slice of CIGARs holds (2^26): 400
+    pairs over and over, some outside the pair kernels' range, against the 400
+    alone."""
+    rng = random.Random(26)
+    m = pb.matrix_create("ACGT", 100, -100)
+    qs, ts = [], []
+    for k in range(400):
+        q = rand_seq(rng, 700 if k % 50 == 7 else rng.randint(20, 180), DNA)
+        qs.append(q)
+        ts.append(rand_seq(rng, 10, DNA) + mutate(rng, q, DNA, 0.1, 0.05) + rand_seq(rng, 20, DNA))
+
+    def run(reps):
+        qb, qo, ql = pb.pack(qs * reps)
+        tb, to, tl = pb.pack(ts * reps)
+        n = len(ql)
+        rec = np.zeros((n, 8), np.int32)
+        out = [np.zeros(int(ql.sum() + tl.sum()), np.uint32)] + [np.zeros(n, np.int32) for _ in range(3)]
+        rc = pb.lib.parasail_b200_batch_pairs_cigar(b"sg_trace_striped_32", m, qb.ctypes.data, qo.ctypes.data, ql.ctypes.data,
+                                                    tb.ctypes.data, to.ctypes.data, tl.ctypes.data, n, 200, 20,
+                                                    rec.ctypes.data, *[x.ctypes.data for x in out])
+        assert rc == 0
+        return [rec.reshape(reps, -1)] + [x.reshape(reps, -1) for x in out]
+
+    one = run(1)
+    assert (one[2] > 0).any() and (one[2] < 0).any()
+    reps = 2 ** 26 // one[1].size + 2
+    for a, b in zip(run(reps), one):
+        assert (a == b).all()
