@@ -272,7 +272,10 @@ void pb_diag_sw16_time(double ms);
 void *pb_cuda_stream(void);   /* the calling thread's stream (a cudaStream_t) */
 /* raise (never lower) a kernel's dynamic shared-memory limit; 0 or -1 */
 int pb_raise_smem(const void *func, int bytes);
-char *pb_single_arena(size_t bytes, size_t host_bytes, char **host);
+#define PB_SINGLE_OUT 256
+char *pb_single_arena(size_t bytes, size_t host_bytes, char **host, char **out);
+/* host memory pinned for the single calls of all threads */
+size_t pb_single_pinned_bytes(void);
 int pb_cuda_exact_single(const pb_batch *tmpl, const uint8_t *h_codes, int tlen, int qlim, int tlim,
                          pb_pair_out *h_out);
 int pb_cuda_sw_single(const pb_device_profile *dp, int open, int gap, const uint8_t *h_codes, int tlen,

@@ -553,19 +553,60 @@ int pb_cuda_align_exact_db(const pb_batch *b)
 }
 
 /* ---- single pairs (the one-pair calls of parasail.h) ----------------------
- * A per-thread device arena holds one pair's descriptors, target codes,
- * scratch and output: one upload, one launch, one download and one
- * synchronisation per call, instead of the batch pipeline's set-up. */
+ * A per-thread device arena holds one pair's descriptors, target codes and
+ * scratch, a pinned block its staging and output: one upload, one launch and
+ * one synchronisation per call, instead of the batch pipeline's set-up. */
 
 namespace {
+
+/* Pinned blocks of one size, a thread's while it lives and then the next
+ * thread's: a thread that ends makes no call to the driver (freeing pinned
+ * memory waits for the device), and a thread pins one block however long the
+ * targets are that it aligns. At most KEEP blocks wait for a thread. */
+struct PinnedBlocks {
+    static constexpr size_t BYTES = 64 << 10, KEEP = 64;
+    std::mutex mu;
+    std::vector<char *> idle;
+    size_t all = 0;              /* blocks, idle or a thread's */
+    char *take()
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        char *p = nullptr;
+        if (!idle.empty()) {
+            p = idle.back();
+            idle.pop_back();
+        } else if (cudaHostAlloc((void **)&p, BYTES, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+            ++all;
+        } else {
+            cudaGetLastError();
+            p = nullptr;
+        }
+        return p;
+    }
+    void give(char *p)
+    {
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            if (idle.size() < KEEP) { idle.push_back(p); return; }
+            --all;
+        }
+        cudaFreeHost(p);
+    }
+};
+
+/* never destroyed: threads may end after the library's static objects */
+PinnedBlocks &pinned_blocks()
+{
+    static PinnedBlocks *blocks = new PinnedBlocks;
+    return *blocks;
+}
 
 struct SingleArena {
     char *d = nullptr;
     size_t cap = 0;
-    char *h = nullptr;       /* pinned host staging of the upload and, read by
-                              * the host after the synchronisation, the output */
-    size_t hcap = 0;
-    ~SingleArena() { if (h) cudaFreeHost(h); }
+    char *pin = nullptr;         /* [output][staging of the upload] */
+    std::vector<char> h;         /* staging of what the block does not hold */
+    ~SingleArena() { if (pin) pinned_blocks().give(pin); }
 };
 thread_local SingleArena g_single;
 
@@ -598,13 +639,15 @@ int pb_raise_smem(const void *func, int bytes)
     return 0;
 }
 
-/* the calling thread's arena of at least `bytes` device bytes, and (host)
- * a zeroed host staging buffer of host_bytes: pinned and mapped, so the
- * upload needs no copy of its own and a kernel writes its output there (one
- * pair: 84.6 -> 78.5 us per call against pageable memory and a download).
- * Every call waits for its stream before it returns, so the buffer is free
- * again. */
-char *pb_single_arena(size_t bytes, size_t host_bytes, char **host)
+/* The calling thread's arena of at least `bytes` device bytes, with (host) a
+ * zeroed staging buffer of host_bytes, and (out) PB_SINGLE_OUT pinned and
+ * mapped bytes that a kernel writes and the host reads after the
+ * synchronisation; null where no memory can be pinned, and the caller copies
+ * its output down. The staging is pinned too where it fits the block (targets
+ * of about 65,000 residues), so that the upload needs no copy of its own: one
+ * pair 84.6 -> 78.5 us per call against pageable memory and a download. Every
+ * call waits for its stream before it returns, so the buffers are free again. */
+char *pb_single_arena(size_t bytes, size_t host_bytes, char **host, char **out)
 {
     if (bytes > g_single.cap) {
         if (g_single.d) cudaFree(g_single.d);
@@ -617,20 +660,22 @@ char *pb_single_arena(size_t bytes, size_t host_bytes, char **host)
         }
         g_single.cap = cap;
     }
-    if (host_bytes > g_single.hcap) {
-        if (g_single.h) cudaFreeHost(g_single.h);
-        const size_t cap = (std::max(host_bytes, (size_t)16 << 10) + 4095) & ~(size_t)4095;
-        if (cudaHostAlloc((void **)&g_single.h, cap, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
-            g_single.h = nullptr;
-            g_single.hcap = 0;
-            cudaGetLastError();
-            return nullptr;
-        }
-        g_single.hcap = cap;
+    if (!g_single.pin) g_single.pin = pinned_blocks().take();
+    *out = g_single.pin;
+    if (g_single.pin && host_bytes <= PinnedBlocks::BYTES - PB_SINGLE_OUT) {
+        *host = g_single.pin + PB_SINGLE_OUT;
+        memset(*host, 0, host_bytes);
+    } else {
+        g_single.h.assign(host_bytes, 0);
+        *host = g_single.h.data();
     }
-    memset(g_single.h, 0, host_bytes);
-    if (host) *host = g_single.h;
     return g_single.d;
+}
+
+size_t pb_single_pinned_bytes(void)
+{
+    std::lock_guard<std::mutex> lock(pinned_blocks().mu);
+    return pinned_blocks().all * PinnedBlocks::BYTES;
 }
 
 /* One pair on the exact kernel from host target codes: on one block, or, where
@@ -651,8 +696,8 @@ int pb_cuda_exact_single(const pb_batch *tmpl, const uint8_t *h_codes, int tlen,
     const size_t o_out = align16(o_ints + 16), o_codes = align16(o_out + sizeof(pb_pair_out));
     const size_t up = align16(o_codes + (size_t)tlen + 16);
     const size_t total = up + sizeof(int) * ((size_t)tl * nv + 16);
-    char *h = nullptr;
-    char *d = pb_single_arena(total, up, &h);
+    char *h = nullptr, *out = nullptr;
+    char *d = pb_single_arena(total, up, &h, &out);
     if (!d) { snprintf(g_err, sizeof g_err, "single-pair arena allocation failed"); return -1; }
     pb::ProfDesc pd;
     pd.prof = dp->d_prof32; pd.prof8 = dp->d_prof8; pd.qcodes = dp->d_qcodes;
@@ -674,7 +719,7 @@ int pb_cuda_exact_single(const pb_batch *tmpl, const uint8_t *h_codes, int tlen,
     p.tlim = tlim > 0 ? reinterpret_cast<const int *>(d + o_ints) + 3 : nullptr;
     p.scratch = reinterpret_cast<int *>(d + up);
     p.soff = reinterpret_cast<const int64_t *>(d + o_soff);
-    p.out = reinterpret_cast<pb_pair_out *>(h + o_out);
+    p.out = reinterpret_cast<pb_pair_out *>(out ? out : d + o_out);
     p.mat = nullptr; p.msize = 0; p.qall = nullptr; p.qoff = nullptr; p.qlen = nullptr;
     p.order = reinterpret_cast<const int *>(d + o_ints);
     p.nt = 0;
@@ -686,8 +731,9 @@ int pb_cuda_exact_single(const pb_batch *tmpl, const uint8_t *h_codes, int tlen,
     }
     pb_diag_count_launch(1);
     CK(cudaGetLastError());
+    if (!out) CK(cudaMemcpyAsync(h_out, d + o_out, sizeof(pb_pair_out), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    memcpy(h_out, h + o_out, sizeof(pb_pair_out));
+    if (out) memcpy(h_out, out, sizeof(pb_pair_out));
     return 0;
 }
 

@@ -254,8 +254,8 @@ int pb_cuda_lane_pair(int bits, const pb_device_profile *dp, const struct pb_mod
     const size_t o_codes = (o_res + sizeof(pb_lane_res) + 15) & ~(size_t)15;
     const size_t up = (o_codes + (size_t)tlen + 16 + 255) & ~(size_t)255;
     const size_t per_warp = pb_cuda_lane_scratch_per_warp(bits, kind, dp->qlen);
-    char *h = nullptr;
-    char *d = pb_single_arena(up + per_warp, up, &h);
+    char *h = nullptr, *out = nullptr;
+    char *d = pb_single_arena(up + per_warp, up, &h, &out);
     if (!d) { pb_cuda_set_error("single-pair arena", "allocation failed"); return -1; }
     const int ints[2] = {tlen, 0};
     memcpy(h + o_ints, ints, sizeof ints);

@@ -1395,9 +1395,10 @@ extern "C" int pb_cuda_align_sw16_multi(const pb_batch *b, pb_pair_out *d_out_al
     return rc;
 }
 
-/* One SW score pair from host target codes: the wavefront kernel on one
- * warp (exact int32, no overflow rerun), its descriptors and the codes in
- * one upload to the thread's arena, the output in one download. */
+/* One SW score pair from host target codes: the wavefront kernel on one warp
+ * (int16x2 where no pair can leave 16 bits, else exact int32: no overflow
+ * rerun), its descriptors and the codes in one upload to the thread's arena,
+ * the output written to the thread's pinned block. */
 extern "C" int pb_cuda_sw_single(const pb_device_profile *dp, int open, int gap, const uint8_t *h_codes, int tlen,
                                  pb_pair_out *h_out)
 {
@@ -1429,8 +1430,8 @@ extern "C" int pb_cuda_sw_single(const pb_device_profile *dp, int open, int gap,
     const size_t o_codes = (o_out + sizeof(pb_pair_out) + 15) & ~(size_t)15;
     const size_t up = (o_codes + (size_t)tlen + 16 + 15) & ~(size_t)15;
     const size_t total = up + sizeof(int2) * (size_t)(tlen + 1) * pb::SW16_WARPS;
-    char *h = nullptr;
-    char *d = pb_single_arena(total, up, &h);
+    char *h = nullptr, *out = nullptr;
+    char *d = pb_single_arena(total, up, &h, &out);
     if (!d) { pb_cuda_set_error("single-pair arena", "allocation failed"); return -1; }
     pb::Sw16Query q;
     q.prof8 = dp->d_prof8; q.prof_off = 0; q.qlen = dp->qlen; q.lp = dp->lp; q.posmax = 32767 - dp->mmax - 1;
@@ -1454,7 +1455,7 @@ extern "C" int pb_cuda_sw_single(const pb_device_profile *dp, int open, int gap,
     p.toff = reinterpret_cast<const int64_t *>(d + o_toff);
     p.tlen = reinterpret_cast<const int *>(d + o_ints) + 1;
     p.scratch = reinterpret_cast<uint32_t *>(d + up);
-    p.out = reinterpret_cast<pb_pair_out *>(h + o_out);
+    p.out = reinterpret_cast<pb_pair_out *>(out ? out : d + o_out);
     int rl = 8;
     double best = -1.0;
     for (int r = 4; r <= 16; r += 4) {
@@ -1472,11 +1473,12 @@ extern "C" int pb_cuda_sw_single(const pb_device_profile *dp, int open, int gap,
             return -1;
         }
     }
-    if (cudaStreamSynchronize(st) != cudaSuccess) {
+    if ((!out && cudaMemcpyAsync(h_out, d + o_out, sizeof *h_out, cudaMemcpyDeviceToHost, st) != cudaSuccess) ||
+        cudaStreamSynchronize(st) != cudaSuccess) {
         pb_cuda_set_error("single-pair SW", cudaGetErrorString(cudaGetLastError()));
         return -1;
     }
-    memcpy(h_out, h + o_out, sizeof *h_out);
+    if (out) memcpy(h_out, out, sizeof *h_out);
     return 0;
 }
 

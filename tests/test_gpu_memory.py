@@ -46,3 +46,63 @@ def test_checkpoints_leave_half_of_the_free_memory():
     run(rec[1])
     assert torch.equal(rec[0], rec[1])
     assert int(rec[0][:, 4].min()) > 0
+
+
+def test_single_calls_pin_one_block_a_thread():
+    """Long targets pin no more memory than short ones, threads that end hand
+    their block on, and results are right at the sizes around the block's."""
+    import ctypes
+    import random
+    import threading
+
+    import oracle as O
+    from conftest import AA, rand_seq
+
+    pinned = pb.lib.pb_single_pinned_bytes
+    pinned.restype = ctypes.c_size_t
+    rng = random.Random(8)
+    m = pb.matrix_lookup("blosum62")
+    om = O.Matrix.from_struct(m)
+    q = rand_seq(rng, 40, AA)
+    sw, nw = (pb.ProfileHandle("parasail_profile_create_" + c, q, m) for c in ("16", "stats_16"))
+    block = 64 << 10
+    text = rand_seq(rng, 2000000, AA)
+
+    def check(n):
+        t = text[-n:]
+        e = O.align(O.SW, 0, 0, q, t, 11, 1, om)
+        got = pb.align_profile("parasail_sw_striped_profile_16", sw, t, 11, 1)
+        assert (got["score"], got["end_query"], got["end_ref"]) == (e["score"], e["end_query"], e["end_ref"]), n
+        alg, sgf = O.alg_of("sg")
+        e = O.align(alg, sgf, 1, q, t, 11, 1, om)
+        got = pb.align_profile("parasail_sg_stats_striped_profile_16", nw, t, 11, 1)
+        assert all(got[k] == e[k] for k in e), n
+
+    check(300)
+    base = pinned()
+    assert base >= block
+    for n in [block - d for d in (1000, 600, 400, 350, 300, 256, 200, 100, 1, 0)] + [block + 1, 2000000, 10]:
+        check(n)
+    assert pinned() == base
+    wrong = []
+
+    def run(n):
+        try:
+            check(n)
+        except BaseException as e:
+            wrong.append(e)
+
+    for _ in range(20):                            # one after the other: one block for all of them
+        th = threading.Thread(target=run, args=(200,))
+        th.start()
+        th.join()
+    assert pinned() <= base + block
+    ths = [threading.Thread(target=run, args=(1000 + k,)) for k in range(6)]
+    for th in ths:
+        th.start()
+    for th in ths:
+        th.join()
+    assert not wrong
+    assert pinned() <= base + 6 * block
+    for p in (sw, nw):
+        p.close()
