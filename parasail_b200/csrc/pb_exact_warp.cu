@@ -614,6 +614,18 @@ bool launch_exact_block(const ExactParams &p, int alg, bool stats, const pb_devi
     const size_t smem = (size_t)prof->size * stride;
     if (smem > 160 * 1024) return false;
     const int R = r32 <= 2 * EB_THREADS ? 2 : 4;
+    /* Score-only calls that the older kernels do faster. Fewer than 32 cells
+     * on one thread: staging the scores takes longer (31 x 1, NW: 18.5 us on a
+     * thread, 25.7 on a block). More than one pass of the warp kernel against a
+     * few columns: the block takes cols + rows / R iterations, the warp kernel
+     * 512 rows in cols + 31 iterations that cost 3.75 to 6 of those (NW, 700 x
+     * 1: 86 us on a warp, 110 on a block; 700 x 10: 121 and 112; 2000 x 1: 172
+     * and 192; 2000 x 8: 229 and 195; 1100 x 1: 131 and 99). */
+    if (!stats) {
+        const long long warp_iters = (r32 + 511) / 512 * (cols + 31LL);
+        if ((long long)rows * cols < 32) return false;
+        if (r32 > 512 && 4LL * (cols + r32 / R) > (R == 4 ? 15 : alg == PB_SG ? 24 : 18) * warp_iters) return false;
+    }
     const int threads = ((r32 + R - 1) / R + 31) & ~31;
     if (R == 2) {
         if (stats) launch_eb<true, 2>(p, alg, threads, (int)smem, stride, st);

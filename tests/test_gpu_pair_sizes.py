@@ -152,3 +152,23 @@ def test_batch_cigars_in_several_slices():
     reps = 2 ** 26 // one[1].size + 2
     for a, b in zip(run(reps), one):
         assert (a == b).all()
+
+
+@pytest.mark.parametrize("qlen,tlens", [(1, (1, 31, 32, 33)), (5, (6, 7)), (31, (1, 2)), (513, (1, 8)), (700, (1, 6, 10)),
+                                        (1024, (1, 10, 30)), (1500, (1, 4)), (2048, (1, 5, 40))])
+def test_single_calls_of_few_cells_or_columns(qlen, tlens):
+    """Score-only calls on either side of the lines between one thread, one
+    warp and one block, against the oracle; the 16-bit forms read the extremes."""
+    rng = random.Random(qlen)
+    b62 = pb.matrix_lookup("blosum62")
+    om = O.Matrix.from_struct(b62)
+    q = rand_seq(rng, qlen, AA)
+    prof, prof16 = (pb.ProfileHandle("parasail_profile_create_" + w, q, b62) for w in ("32", "16"))
+    for name in ("nw_striped", "sg_scan", "sg_qb_de_striped"):
+        alg, sgf = O.alg_of(name.split("_striped")[0].split("_scan")[0])
+        for n in tlens:
+            t = rand_seq(rng, n, AA)
+            e = O.align(alg, sgf, 0, q, t, 11, 1, om)
+            for p, w in ((prof, "32"), (prof16, "16")):
+                got = pb.align_profile("parasail_%s_profile_%s" % (name, w), p, t, 11, 1)
+                assert all(got[k] == e[k] for k in ("score", "end_query", "end_ref")), (name, w, n)
