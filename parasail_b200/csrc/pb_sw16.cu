@@ -87,20 +87,33 @@ __device__ __forceinline__ void fold_best(Sw16Best &best, const Sw16Best &s)
     if (s.j >= 0 && (s.score > best.score || (s.score == best.score && s.j < best.j))) best = s;
 }
 
-/* Does a sequence hold a code outside an alphabet of L letters? (Words as in
- * ResidueWords. A call of its own: inlined it changed the register allocation
- * of k_sw16's column loop, 5% on the large search.) */
+/* Does a sequence hold a code outside an alphabet of L letters? Aligned
+ * 16-byte loads, of those blocks only that hold a byte of the sequence. A call
+ * of its own: inlined it changed the register allocation of k_sw16's column
+ * loop, 5% on the large search. */
 __device__ __noinline__ bool outside_alphabet(const uint8_t *seq, int n, int L)
 {
+    if (n <= 0) return false;
     const uintptr_t p = reinterpret_cast<uintptr_t>(seq);
-    const uint32_t *w = reinterpret_cast<const uint32_t *>(p & ~(uintptr_t)3);
-    const int first = (int)(p & 3), words = n > 0 ? (first + n + 3) >> 2 : 0;
-    const uint32_t head = 0xffffffffu << (8 * first), tail = 0xffffffffu >> (8 * ((4 * words - first - n) & 3));
+    const uint4 *b = reinterpret_cast<const uint4 *>(p & ~(uintptr_t)15);
+    const int first = (int)(p & 15), end = first + n, last = (end - 1) >> 4;
     uint32_t m = 0u;
+    /* word w of the blocks; its bytes before `first` and from `end` on are not
+     * the sequence's */
+    auto edge = [&](uint32_t x, int w) {
+        const int skip = first - 4 * w, keep = end - 4 * w;
+        uint32_t o = codes_outside(x, L);
+        if (skip > 0) o &= skip >= 4 ? 0u : 0xffffffffu << (8 * skip);
+        if (keep < 4) o &= keep <= 0 ? 0u : 0xffffffffu >> (8 * (4 - keep));
+        m |= o;
+    };
+    const uint4 x0 = __ldg(b), x1 = __ldg(b + last);
+    edge(x0.x, 0); edge(x0.y, 1); edge(x0.z, 2); edge(x0.w, 3);
+    edge(x1.x, 4 * last); edge(x1.y, 4 * last + 1); edge(x1.z, 4 * last + 2); edge(x1.w, 4 * last + 3);
 #pragma unroll 8
-    for (int k = 0; k < words; ++k) {
-        const uint32_t x = codes_outside(__ldg(w + k), L);
-        m |= x & (k == 0 ? head : 0xffffffffu) & (k == words - 1 ? tail : 0xffffffffu);
+    for (int k = 1; k < last; ++k) {
+        const uint4 x = __ldg(b + k);
+        m |= codes_outside(x.x, L) | codes_outside(x.y, L) | codes_outside(x.z, L) | codes_outside(x.w, L);
     }
     return m != 0u;
 }
@@ -195,9 +208,10 @@ k_sw16(Sw16Params p, int *task_counter)
         const uint8_t *tseq = p.targets + (valid ? p.toff[pid] : 0);
         /* A code outside the alphabet would index past the slice: such a
          * target counts as empty here and its pair goes to the exact kernel,
-         * which reads the code as letter 0. Looked for once per task (5
-         * queries x 200,000 targets: 54.7 -> 55.0 ms; a check of four codes in
-         * the column loop took 55.9 without a branch, 57.3 with one). */
+         * which reads the code as letter 0. Looked for once per task: 5
+         * queries x 200,000 targets 54.6 -> 54.9 ms, 100 rows x 20,000 targets
+         * 277 -> 285 us (a check of four codes in the column loop: 55.9 ms
+         * without a branch, 57.3 with one). */
         if (outside_alphabet(tseq, len, p.nletters)) len = 0;
         int wmax = len;
 #pragma unroll
