@@ -4,6 +4,7 @@ that run together, the biased and the unbiased form (a penalty that takes
 score + open out of int8), alphabets of a few and of many letters, and one
 query shared by a task. Every record against the oracle."""
 import random
+import re
 
 import numpy as np
 import pytest
@@ -172,3 +173,72 @@ def test_single_calls_of_few_cells_or_columns(qlen, tlens):
             for p, w in ((prof, "32"), (prof16, "16")):
                 got = pb.align_profile("parasail_%s_profile_%s" % (name, w), p, t, 11, 1)
                 assert all(got[k] == e[k] for k in ("score", "end_query", "end_ref")), (name, w, n)
+
+
+def _read_cigar(cigar, q, t, beg_q, beg_t):
+    """[(op, length, start in q, start in t)], the residues under '=' and 'X' compared."""
+    runs, i, j = [], beg_q, beg_t
+    for n, op in re.findall(r"(\d+)([=XID])", cigar):
+        n = int(n)
+        if op in "=X":
+            assert all((q[i + x] == t[j + x]) == (op == "=") for x in range(n)), (cigar, i, j)
+        runs.append((op, n, i, j))
+        i += n * (op != "D")
+        j += n * (op != "I")
+    assert "".join("%d%s" % (n, op) for op, n, _, _ in runs) == cigar
+    assert all(a[0] != b[0] for a, b in zip(runs, runs[1:]))
+    return runs, i, j
+
+
+@pytest.mark.parametrize("alg", ["sw", "nw", "sg", "sg_qx", "sg_de", "sg_qb_db"])
+@pytest.mark.parametrize("alphabet,open_,gap", [(DNA, 5, 2), (AA, 11, 1), (AA, 120, 2)])
+def test_cigars_against_the_oracle(alg, alphabet, open_, gap):
+    """CIGARs read back residue by residue: what they consume, their score and
+    their counts against the score and the statistics that the oracle gives
+    for the path of the same tie rules. Paths over many blocks and passes."""
+    rng = random.Random(open_)
+    m = pb.matrix_create("ACGT", 2, -3) if alphabet is DNA else pb.matrix_lookup("blosum62")
+    om = O.Matrix.from_struct(m)
+    a, sgf = O.alg_of(alg)
+    qs, ts = ["A", "G" * 40], ["A", "A" * 35]
+    for n in EDGES + (200, 333, 512, 600, 1100):
+        for _ in range(2):
+            q = rand_seq(rng, n, alphabet)
+            t = rand_seq(rng, rng.randint(0, 40), alphabet) + mutate(rng, q, alphabet, 0.25, 0.12) + \
+                rand_seq(rng, rng.randint(0, 40), alphabet)
+            qs.append(q)
+            ts.append(t)
+    seen = 0
+    for q, t, g in zip(qs, ts, pb.batch_pairs_cigar(alg + "_trace", m, qs, ts, open_, gap)):
+        e = O.align(a, sgf, 1, q, t, open_, gap, om)
+        assert (g["score"], g["end_query"], g["end_ref"]) == (e["score"], e["end_query"], e["end_ref"])
+        if alg == "sw" and e["score"] == 0:
+            continue
+        runs, i, j = _read_cigar(g["cigar"], q, t, g["beg_query"], g["beg_ref"])
+        # a path begins with a diagonal step: a gap before it is one to the matrix edge
+        lead = runs[0] if runs[0][0] in "ID" else None
+        tail = None
+        if alg == "sw":
+            assert (i, j) == (e["end_query"] + 1, e["end_ref"] + 1)
+        else:
+            assert (i, j) == (len(q), len(t)) and (g["beg_query"], g["beg_ref"]) == (0, 0)
+            if (e["end_query"] + 1, e["end_ref"] + 1) != (len(q), len(t)):
+                tail = runs[-1]
+                assert tail[2:] == (e["end_query"] + 1, e["end_ref"] + 1) and tail[0] in "ID"
+        score = matches = similar = length = 0
+        for run in runs:
+            op, n, x, y = run
+            if op in "ID":
+                free = run is tail or (run is lead and (alg == "sw" or sgf & (O.S1_BEG if op == "I" else O.S2_BEG)))
+                score -= 0 if free else open_ + (n - 1) * gap
+                length += 0 if run is lead or run is tail else n
+                continue
+            length += n
+            for k in range(n):
+                s = O.align(O.NW, 0, 0, q[x + k], t[y + k], 10 ** 6, 10 ** 6, om)["score"]
+                score += s
+                matches += op == "="
+                similar += s > 0
+        assert (score, matches, similar, length) == (e["score"], e["matches"], e["similar"], e["length"]), (alg, len(q), len(t))
+        seen += 1
+    assert seen > 40
