@@ -1175,17 +1175,18 @@ size_t device_memory()
     return seen[dev];
 }
 
-/* Bytes that one chunk's checkpoints may take, where all of them take `want`:
- * a third of the device's memory, so that a chunk of the largest tasks (about
- * 20 MB each at 1500 x 1500) still fills the SMs, but not so much that the pool
- * grows by more than half of what is free, which other allocators and
+/* The chunks that ntasks tasks with `all` bytes of checkpoints run in: chunks
+ * of at most a third of the device's memory, so that one of the largest tasks
+ * (about 20 MB each at 1500 x 1500) still fills the SMs, but not so large that
+ * the pool grows by more than half of what is free, which other allocators and
  * processes may need. The free memory is asked for only where the pool would
- * have to grow: on a shared host that call takes 0.1 to 90 ms, at random (18.9
- * ms passes of 1 M reads became 20-110 ms), and what the pool holds already it
- * keeps. */
-size_t p16_ckpt_budget(size_t want)
+ * have to grow (by more than an eighth of what it holds unused): on a shared
+ * host that call takes 0.1 to 90 ms, at random (18.9 ms passes of 1 M reads
+ * became 20-110 ms). */
+size_t p16_chunks(size_t ntasks, size_t all)
 {
     const size_t cap = device_memory() / 3;
+    auto chunks = [&](size_t bytes) { return std::min(ntasks, all / std::max<size_t>(bytes, 1) + 1); };
     int dev = 0;
     cudaMemPool_t pool;
     uint64_t reserved = 0, used = 0;
@@ -1194,11 +1195,11 @@ size_t p16_ckpt_budget(size_t want)
         cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved);
         cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used);
     }
-    const size_t spare = reserved > used ? (size_t)(reserved - used) : 0;
-    if (std::min(want, cap) <= spare) return cap;
+    const size_t spare = reserved > used ? (size_t)(reserved - used) : 0, n = chunks(cap);
+    if (all / n <= spare + spare / 8) return n;
     size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); return cap; }
-    return std::min(cap, std::max(spare, free_b / 2 + spare / 2));
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); return n; }
+    return chunks(std::min(cap, std::max(spare, free_b / 2 + spare / 2)));
 }
 
 typedef void (*p16_trace_t)(pb_job, P16Params, const int *, int, const pb_pair_out *, int *);
@@ -1392,15 +1393,12 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
         std::stable_sort(torder.begin(), torder.end(), [&](int x, int y) {
             return (long long)hn[x] * (hw[x] + 1) > (long long)hn[y] * (hw[y] + 1);
         });
-        /* chunks of tasks whose checkpoints fit the budget, which is halved when
-         * the allocation fails */
         size_t all_u4 = 0;
         for (int t = 0; t < ntasks; ++t) all_u4 += (size_t)hb[t];
-        size_t budget_u4 = std::max<size_t>(1, ckpt ? p16_ckpt_budget(all_u4 * sizeof(uint4)) / sizeof(uint4) : 1);
         /* Chunks of like make-up: chunk c takes tasks c, c + nch, ... of the
          * order, so that each ends on small tasks (524 k protein pairs in two
          * chunks: 84.2 ms when the first took the largest tasks, 80.7 so). */
-        const int nch = (int)std::min<size_t>((size_t)ntasks, all_u4 / budget_u4 + 1);
+        const int nch = ckpt ? (int)p16_chunks((size_t)ntasks, all_u4 * sizeof(uint4)) : 1;
         std::vector<int> cut(nch + 1, 0);
         if (nch > 1) {
             std::vector<int> dealt;
@@ -1412,7 +1410,8 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
             torder.swap(dealt);
         }
         cut[nch] = ntasks;
-        budget_u4 = all_u4 / nch + (size_t)*std::max_element(hb.begin(), hb.end()) * 2;
+        /* what a chunk may take; halved when its allocation fails */
+        size_t budget_u4 = all_u4 / nch + (size_t)*std::max_element(hb.begin(), hb.end()) * 2;
         /* launch shapes and the pass-boundary buffers, sized for the larger grid */
         int dev = 0, nsm = 0;
         cudaGetDevice(&dev);
