@@ -120,8 +120,9 @@ extern int parasail_b200_batch_db_device(
  * parasail_b200_batch_db_device would give; a search with a pair past the
  * 16-bit range runs once through the full pipeline instead. Plans hold the
  * Smith-Waterman score-only functions (sw_{striped,scan}_profile_{8,16,32,sat})
- * with open > gap and profiles whose scores fit int8; creation returns NULL
- * for anything else. The buffers must outlive the plan. Replaces the
+ * with open > gap and profiles whose scores fit int8 and take at most 200 KB
+ * together (a byte per letter and row, rows padded to a multiple of 64 that
+ * holds 32 more than the query); creation returns NULL for anything else. The buffers must outlive the plan. Replaces the
  * reference aligner's repeated searches of one database
  * (apps/parasail_aligner.cpp:1694-1740) without per-call host work. */
 typedef struct parasail_b200_db_plan parasail_b200_db_plan_t;

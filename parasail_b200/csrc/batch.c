@@ -470,7 +470,7 @@ parasail_b200_db_plan_t *parasail_b200_db_plan_create(const char *funcname, cons
     mapper_bytes(profiles[0]->matrix, pl->mapper);
     if (pb_cuda_db_plan_create(&job, &b, (pb_record *)d_records, &pl->plan) != 0) {
         fprintf(stderr, "%s: '%s' cannot be planned (plans hold Smith-Waterman score-only searches with "
-                "open > gap and int8 profiles)\n", __func__, funcname ? funcname : "(null)");
+                "open > gap and int8 profiles of at most 200 KB together)\n", __func__, funcname ? funcname : "(null)");
         free(profs); free(pl); return NULL;
     }
     free(profs);

@@ -345,12 +345,12 @@ k_exact_warp(ExactParams p, int nitems)
  * cycles per column of 300 rows with statistics). The row above comes from
  * the lane before by shuffle; the last lane of a warp leaves it in shared
  * memory for the next warp, double-buffered, with one barrier per iteration.
- * Bound by the latency of an iteration (shuffles, barrier, R rows), so R is
- * the smallest that keeps the block at 512 threads, matches and similar
+ * Bound by the latency of an iteration (shuffles, barrier, R rows), so R is 2
+ * up to 1,024 rows and 4 up to 2,048, matches and similar
  * share a word (rows + columns below 65,536), the scores are int8 in shared
  * memory, loaded one column ahead, and the extremes are kept per row and
  * sorted into the row regions once, at the end. One sg_qx statistics pair of
- * 300 x 332: 1,174 -> 233 us per call.
+ * 300 x 332: 1,174 -> 221 us per call.
  * Every cell and end rule is k_exact_warp's (without SCANF).
  */
 static constexpr int EB_THREADS = 512;

@@ -134,7 +134,6 @@ struct P16Params {
     const long long *task_ckpt;   /* per task: first uint4 of its checkpoints in `ckpt` */
     uint4 *ckpt;
     const int8_t *mat8;           /* pairs mode: [target letter][query letter] int8, else nullptr */
-    const int32_t *mat32;         /* pairs mode: the same in int32 (the statistics walk) */
     const uint8_t *qall;
     const int64_t *qoff;
     const ProfDesc *profs;        /* db mode */
@@ -215,7 +214,6 @@ int resolve_rounds(const pb_job &job, const pb_lane_args &la, const pb_pair_out 
 pb_lane_args lane_args_of(const pb_batch *b, int q, const pb_pair_out *o1);
 void launch_resolve_plain(const pb_job &job, const pb_pair_out *o1, int qlen_all, const int *tlen, int n,
                           pb_record *rec, int *need, int *counts, cudaStream_t st);
-void launch_sw16(const Sw16Params &p, cudaStream_t st);
 
 }  // namespace pb
 

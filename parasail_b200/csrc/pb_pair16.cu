@@ -303,7 +303,8 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
                         *reinterpret_cast<int4 *>(wslice + a * LETTER + 16 * h) = v;
                     }
                 }
-            } else if (p.mat8) {
+            } else {
+                /* (pairs mode: a task of the database mode shares its query) */
                 uint32_t qc[8];
 #pragma unroll
                 for (int w = 0; w < 8; ++w) {
@@ -337,23 +338,6 @@ k_p16(P16Params p, const int *__restrict__ tlist, int ntl, int *counter)
                         }
                         *reinterpret_cast<uint4 *>(sl + a * LETTER + h * STRIP) =
                             make_uint4(word[0], word[1], word[2], word[3]);
-                    }
-                }
-            } else {
-                /* db mode, lanes of different queries: each copies its own
-                 * (a pass past this lane's profile rows, lp >= qlen + 32, is
-                 * beyond its query: zeros) */
-                const bool in = r0 + P16_PASS <= lp;
-                for (int a = 0; a < L; ++a) {
-                    const int4 *src = reinterpret_cast<const int4 *>(prof8 + (size_t)a * lp + (in ? r0 : 0));
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        int4 v = in ? src[h] : make_int4(0, 0, 0, 0);
-                        if (BIAS) {
-                            v.x = (int)__vadd4((uint32_t)v.x, b4); v.y = (int)__vadd4((uint32_t)v.y, b4);
-                            v.z = (int)__vadd4((uint32_t)v.z, b4); v.w = (int)__vadd4((uint32_t)v.w, b4);
-                        }
-                        *reinterpret_cast<int4 *>(sl + a * LETTER + h * STRIP) = v;
                     }
                 }
             }
@@ -1364,7 +1348,7 @@ int p16_pass(const pb_job &job, const pb_batch *b, int prefix, const pb_pair_out
         memset(&p, 0, sizeof p);
         p.alg = m->alg; p.sgflags = m->sgflags; p.open = m->open; p.gap = m->gap; p.mmax = mmax; p.mmin = mmin;
         p.nletters = L; p.nitems = nslots; p.order = porder; p.rows = rows; p.cols = cols;
-        p.mat8 = d_mat8; p.mat32 = dbmode ? nullptr : b->d_mat;
+        p.mat8 = d_mat8;
         p.qall = b->d_qall; p.qoff = b->d_qoff; p.profs = d_profs; p.nt = dbmode ? b->npairs : 0;
         p.targets = b->d_targets; p.toff = b->d_toff;
         p.out = out;

@@ -460,11 +460,11 @@ k_sw16(Sw16Params p, int *task_counter)
 }
 
 /*
- * Small searches (few warp tasks, e.g. one query against 1,000 targets):
- * the intra-task wavefront. One warp aligns one (query, target) pair in
- * exact int32: a pass covers 256 query rows, 8 per lane, and lane k
+ * Small searches and single pairs whose scores or penalties may pass 16 bits
+ * (the others run on k_sw_wave16): the intra-task wavefront. One warp aligns one (query, target) pair in
+ * exact int32: a pass covers 32 * RL query rows, RL per lane, and lane k
  * computes column t - k at iteration t, so the warp's 32 lanes work on 32
- * columns of one pair at once and the row-to-row dependency chain is 8
+ * columns of one pair at once and the row-to-row dependency chain is RL
  * rows long instead of the inter-task kernel's per-target 16-row strips on
  * a handful of SMs. Row above a lane's first row: the previous lane's last
  * row by __shfl_up_sync, or, for lane 0, the previous pass's bottom row
@@ -476,7 +476,7 @@ k_sw16(Sw16Params p, int *task_counter)
  * dependent operation per row.
  */
 /* RL query rows per lane (4, 8, 12 or 16; a pass covers 32 * RL rows),
- * chosen per launch from the query lengths (wave_rows) */
+ * chosen per launch from the query lengths (sw16_prepare) */
 template <bool GE, int RL>
 __global__ void __launch_bounds__(SW16_WARPS * 32, 2)
 k_sw_wave(Sw16Params p, int *counter)
@@ -909,8 +909,8 @@ __global__ void k_scatter(const pb_pair_out *src, const int *list, int n, pb_pai
 
 }  // namespace
 
-/* the largest profiles k_sw_wave takes into shared memory; also the limit
- * of a plan */
+/* the largest profiles, or staged scores, that the kernels of small searches
+ * take into shared memory; also the documented limit of a plan's profiles */
 static constexpr size_t SW16_WAVE_SMEM = 200 * 1024;
 
 /* Everything the score kernel needs for a batch that depends only on the
