@@ -625,11 +625,13 @@ k_sw_wave(Sw16Params p, int *counter)
  * as it is and cannot raise a maximum after the last. Scores are staged per
  * block as [pass][letter][strip][lane], so that the lanes' loads fall on
  * different banks whatever their letters. One pair (300 x 350) takes 163 ->
- * 85 us per call, 1 query (300) x 1,000 targets 253 -> 128 us per plan run,
+ * 78.5 us per call, 1 query (300) x 1,000 targets 253 -> 107 us per plan run,
  * against the exact 32-bit wavefront (k_sw_wave), which stays for pairs that
- * may pass 16 bits. Up to a task per resident block (9,472 targets) it beats
- * k_sw16's teams: 300 rows x 1,000 / 4,000 / 9,000 targets 128 / 203 / 381 us
- * against 316 / 314 / 475.
+ * may pass 16 bits. It runs up to a task per resident block (9,472 targets),
+ * where it beats k_sw16 at 300 rows and more: 300 rows x 1,000 / 4,000 / 9,000
+ * targets 107 / 172 / 324 us against 316 / 314 / 466 (9,600 targets), 800 rows x
+ * 9,000 749 against 908, 1,500 rows 1,188 against 1,590. At 100 rows the two
+ * are even there (214, 217); at 30 rows k_sw16 would be faster (185, 139).
  */
 template <bool BIAS, int R>
 __global__ void __launch_bounds__(WAVE16_WARPS * 32, 4)
